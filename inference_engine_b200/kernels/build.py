@@ -220,6 +220,8 @@ PART_LIBRARIES = {
     # recurrent mixers with a decaying matrix state (gated-write linear attention, exponential-gate
     # matrix memory, state-space duality): input convolutions, gates, the recurrence, the read-outs
     "recurrent": ["gated_recurrence.cu"],
+    # the same recurrences and the gated delta rule over long portions, in chunks of 64 tokens
+    "chunked": ["chunked_recurrence.cu"],
     # attention with normalised queries and keys and sigmoid weights: the input stage
     "gated_attn": ["gated_attention.cu"],
     # several residual streams mixed and read by every sublayer, and the norm without statistics

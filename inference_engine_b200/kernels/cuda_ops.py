@@ -16,6 +16,7 @@ import ctypes
 import functools
 import os
 from ctypes import c_float, c_int, c_void_p
+from typing import Any
 
 from .build import (ATTENTION_HEAD_DIMS, build_attention, build_core, build_latent_attention, build_part_library,
                     build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
@@ -1001,6 +1002,12 @@ class CudaOps:
             "ie_recurrence_readout": "P I P P I F P I I P I L I I P",
             "ie_lowrank_decay": "P I P P F P I I I P",
         },
+        "chunked": {
+            "ie_chunked_ok": "I I I",
+            "ie_chunked_scratch": "I I I I I",
+            "ie_chunked_recurrence": "P I P I P I P I P I P L P P P I I I I I I F I I P P",
+            "ie_chunked_delta": "P P P P P P L P P P I I I I I I I P P",
+        },
         "gated_attn": {
             "ie_qk_norm_rope_write": "P I P P I I P I I I P P F I P F I F P P P I P I I I I I I I P P",
             "ie_qk_wide_norm_rope_write": "P I P P I I P I P P F F P P P I P I I I I I I I P P",
@@ -1022,6 +1029,8 @@ class CudaOps:
             for fn_name, sig in self._PART_SIGNATURES[name].items():
                 fn = getattr(lib, fn_name)
                 fn.argtypes, fn.restype = [kinds[k] for k in sig.split()], c_int
+            if name == "chunked":
+                lib.ie_chunked_scratch.restype = ctypes.c_longlong
             self._part_libs[name] = lib
         return lib
 
@@ -1135,11 +1144,59 @@ class CudaOps:
             self._stream()), "delta_prep")
         self.launches += 1 if taps > 1 else 0
 
+    # Recurrences over portions in chunks of 64 (`csrc/chunked_recurrence.cu`).
+    takes_chunks = True  # `gated_recurrence` and `delta_rule` know the argument `in_chunks`
+    CHUNK = 64
+    chunks_always = False  # (tests: whatever the sizes, where the kernels take them)
+
+    def chunks_pay(self, longest: int, tokens: int, chunks: int, heads: int, dim: int, vdim: int, delta: bool) -> bool:
+        """Whether chunks beat the token-by-token kernels, from estimates of both in microseconds, set against measurements of 1
+        to 32 requests of 16 to 2,048 tokens at 8 and 16 heads of 64 x 64 to 128 x 128.  Token by token: the longest
+        portion's chain, or all tokens' state traffic when there are many requests.  In chunks: three launches and a block's
+        life, then the work of all chunks; for the delta rule the chain through the longest portion's chunks besides.
+        Examples (16 heads of 128 x 128; token by token / in chunks): 64 tokens 24 / 46 us, 256 tokens 85 / 52, 2,048 tokens 664 /
+        134, 8 requests of 64 tokens 79 / 60, 32 of 32 tokens 153 / 165; delta rule 128 tokens 43 / 64, 256 tokens 82 / 74, 2,048
+        tokens 629 / 264, 32 of 32 tokens 160 / 384."""
+        share, wide = heads * dim * vdim / 262144, dim > 64
+        step = (0.31 if wide else 0.26) if delta else (0.325 if wide else 0.17)
+        one_by_one = max(step * longest, 0.15 * share * tokens)
+        if delta:
+            chain = max(-(-longest // self.CHUNK), heads * -(-vdim // 16) * chunks / self.sm_count) * 4.5
+            return (62 if wide else 36) + chain + 2.0 * share * chunks < one_by_one
+        return (42 if wide else 21) + 2.9 * share * chunks < one_by_one
+
+    def _recurrence_chunks(self, ctx, heads: int, dim: int, vdim: int, delta: bool, rows) -> tuple[int, Any]:
+        """(chunks, scratch) for a step whose portions are worth it, else (0, None).  ``rows``: the 32-bit views that
+        the kernels read in pieces of 16 bytes.  A captured step is judged by its bounds."""
+        bounds, size = getattr(ctx, "bounds", None), self.CHUNK
+        if bounds is not None:
+            longest = tokens = bounds[0]
+            chunks = bounds[0] // size + bounds[1]
+        else:
+            longest, tokens, chunks = ctx.max_q_len, sum(ctx.q_lens), sum(-(-n // size) for n in ctx.q_lens)
+        if not self.chunks_always and not self.chunks_pay(longest, tokens, chunks, heads, dim, vdim, delta):
+            return 0, None
+        lib = self._part_lib("chunked")
+        if not lib.ie_chunked_ok(dim, vdim, int(delta)) or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows):
+            return 0, None
+        floats = lib.ie_chunked_scratch(1, heads, dim, vdim, int(delta))
+        return chunks, ctx.ws.buffer("recurrence.chunks", chunks, floats, self.torch.float32, rows_cap=None)
+
     @_kind("delta.rule")
-    def delta_rule(self, q, k, v, beta, decay, state, slots, ctx, out, heads, kv_heads, dim, vdim) -> None:
-        """The recurrence itself: every request's tokens of this step in order, from and to its slot."""
+    def delta_rule(self, q, k, v, beta, decay, state, slots, ctx, out, heads, kv_heads, dim, vdim,
+                   in_chunks: bool = False) -> None:
+        """The recurrence itself: every request's tokens of this step in order, from and to its slot.  ``in_chunks``: long
+        portions may be taken 64 tokens at a time (the same sums in another order, which depends on the cutting)."""
         if dim > 512:
             raise KernelError(f"the delta rule kernel takes key sizes up to 512, not {dim}")
+        chunks, scratch = self._recurrence_chunks(ctx, heads, dim, vdim, True, (q, k, v, decay, out)) if in_chunks else (0, None)
+        if chunks:
+            self._check(self._part_lib("chunked").ie_chunked_delta(
+                q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
+                state.stride(0), slots.data_ptr(), ctx.cu_q.data_ptr(), out.data_ptr(), ctx.num_seqs, heads, kv_heads, dim,
+                vdim, state.shape[0], chunks, scratch.data_ptr(), self._stream()), "delta_rule_chunks")
+            self.launches += 2
+            return
         self._check(self._part_lib("delta").ie_delta_rule(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
             state.stride(0), slots.data_ptr(), ctx.cu_q.data_ptr(), out.data_ptr(), ctx.num_seqs, heads,
@@ -1356,15 +1413,28 @@ class CudaOps:
 
     @_kind("recurrent.rule")
     def gated_recurrence(self, q, a, w, gates, v, state, slots, ctx, out, heads, dim, vdim, cols, q_scale,
-                         heads_per_unit: int = 1) -> None:
+                         heads_per_unit: int = 1, in_chunks: bool = False) -> None:
         """``S <- diag(a) S + w u^T; o = S^T q`` per head over every request's tokens of the step, from
         and to its slot (``[heads, cols, dim]``).  ``q``, ``a``, ``w``: views ``[N, heads * dim]``;
         ``v``: view ``[N, heads * vdim]``; with ``gates`` (``[N, heads, 3]``) ``a`` is the gates' decay,
         ``u = gate * v``, and column ``vdim`` (if ``cols = vdim + 1``) carries the value 1.  Gates of shape
         ``[1, heads, 3]`` are every token's (a decay that is a constant per head).  So many neighbouring heads as
-        ``heads_per_unit`` share their rows of ``q`` and ``w``, which then hold that many times fewer columns."""
+        ``heads_per_unit`` share their rows of ``q`` and ``w``, which then hold that many times fewer columns.
+        ``in_chunks``: long portions may be taken 64 tokens at a time (the same sums in another order, which
+        depends on the cutting)."""
         if dim > 512:
             raise KernelError(f"the recurrence kernel takes key sizes up to 512, not {dim}")
+        if in_chunks and out.data_ptr() % 16 == 0:
+            chunks, scratch = self._recurrence_chunks(ctx, heads, dim, vdim, False, (q, w, v) if a is None else (q, a, w, v))
+            if chunks:
+                self._check(self._part_lib("chunked").ie_chunked_recurrence(
+                    q.data_ptr(), q.stride(0), self._ptr(a), 0 if a is None else a.stride(0), w.data_ptr(), w.stride(0),
+                    self._ptr(gates), 0 if gates is None or (gates.dim() == 3 and gates.shape[0] == 1) else 3 * heads,
+                    v.data_ptr(), v.stride(0), state.data_ptr(), state.stride(0), slots.data_ptr(), ctx.cu_q.data_ptr(),
+                    out.data_ptr(), ctx.num_seqs, heads, heads_per_unit, dim, vdim, cols, float(q_scale), state.shape[0],
+                    chunks, scratch.data_ptr(), self._stream()), "gated_recurrence_chunks")
+                self.launches += 2
+                return
         self._check(self._part_lib("recurrent").ie_gated_recurrence(
             q.data_ptr(), q.stride(0), self._ptr(a), 0 if a is None else a.stride(0), w.data_ptr(), w.stride(0),
             self._ptr(gates), 0 if gates is None or (gates.dim() == 3 and gates.shape[0] == 1) else 3 * heads,

@@ -23,6 +23,7 @@ with 32-bit sums.
 from __future__ import annotations
 
 from .base import BuildEnv, CacheBinding, Mixer, StateRequest, WeightDecl
+from .recurrent import long_portions
 from .registry import register_part
 
 
@@ -103,7 +104,7 @@ class ChannelDeltaRule(Mixer):
                        q, k, v, beta, decay, self.heads, self.kv_heads, self.dim, self.vdim, self.taps)
         o = ws.buffer("delta.o", n, self.v_size, f32)
         ops.delta_rule(q, k, v, beta, decay, state, group.slots, ctx, o,
-                       self.heads, self.kv_heads, self.dim, self.vdim)
+                       self.heads, self.kv_heads, self.dim, self.vdim, **long_portions(ops, self.dtype))
         out = ws.buffer("delta.out", n, self.v_size, self.dtype)
         ops.gated_rms_heads(o, self.out_norm, self.eps, gate, out, self.heads, self.vdim)
         return ops.linear(out, self.w_o, ws=ws, tag="mixer.delta", out_dtype=f32, allow_split=True)

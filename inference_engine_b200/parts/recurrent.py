@@ -47,6 +47,14 @@ from .base import BuildEnv, Mixer, StateRequest, WeightDecl
 from .registry import build_part, register_part
 
 
+def long_portions(ops, dtype) -> dict:
+    """What lets a recurrence take long portions in chunks, where the operations know how.  Not in a 32-bit model: there the
+    order of every sum is the tokens', however they are cut into steps."""
+    import torch
+
+    return {"in_chunks": True} if dtype != torch.float32 and getattr(ops, "takes_chunks", False) else {}
+
+
 def _part_spec(raw) -> PartSpec:
     return raw if isinstance(raw, PartSpec) else PartSpec(raw["kind"], dict(raw.get("params", {})))
 
@@ -140,7 +148,7 @@ class HGRN2(Mixer):
         o = ws.buffer("hgrn2.o", n, self.v_size, f32)
         ops.gated_recurrence(proj[:, :qk], proj[:, qk: 2 * qk], write, None, proj[:, 2 * qk:],
                              group.state[binding.slot], group.slots, ctx, o, self.heads, self.dim, self.vdim,
-                             self.vdim, 1.0)
+                             self.vdim, 1.0, **long_portions(ops, self.dtype))
         out = ws.buffer("hgrn2.out", n, self.v_size, self.dtype)
         ops.recurrence_readout(o, None, self.out_norm, self.eps, None, out, self.heads, self.vdim, self.vdim)
         return ops.linear(out, self.w_o, ws=ws, tag="hgrn2.delta", out_dtype=f32, allow_split=self.allow_split)
@@ -204,7 +212,8 @@ class MLSTM(Mixer):
         cols = self.vdim + 1
         o = ws.buffer("mlstm.o", n, H * cols, f32)
         ops.gated_recurrence(proj[:, :qk], None, proj[:, qk: 2 * qk], gates, proj[:, 2 * qk: at_g], state,
-                             group.slots, ctx, o, H, self.dim, self.vdim, cols, self.dim ** -0.5)
+                             group.slots, ctx, o, H, self.dim, self.vdim, cols, self.dim ** -0.5,
+                             **long_portions(ops, self.dtype))
         out = ws.buffer("mlstm.out", n, vs, self.dtype)
         ops.recurrence_readout(o, gates, self.out_norm, self.eps, proj[:, at_g: at_i], out, H, self.vdim, cols)
         return ops.linear(out, self.w_o, ws=ws, tag="mlstm.delta", out_dtype=f32, allow_split=self.allow_split)
@@ -270,7 +279,7 @@ class GatedLinearAttention(Mixer):
         o = ws.buffer("gla.o", n, vs, f32)
         ops.gated_recurrence(proj[:, :qk], decay, proj[:, qk: 2 * qk], None, proj[:, 2 * qk: at_g],
                              group.state[binding.slot], group.slots, ctx, o, self.heads, self.dim, self.vdim,
-                             self.vdim, self.dim ** -0.5)
+                             self.vdim, self.dim ** -0.5, **long_portions(ops, self.dtype))
         out = ws.buffer("gla.out", n, vs, self.dtype)
         ops.recurrence_readout(o, None, self.out_norm, self.eps, proj[:, at_g: at_a], out, self.heads, self.vdim,
                                self.vdim, gate_act="silu")
