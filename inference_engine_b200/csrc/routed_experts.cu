@@ -25,63 +25,84 @@ namespace {
 
 constexpr int ROUTE_THREADS = 256;
 
-template <typename T>
+// TOKENS tokens per block: the router's rows are read once for all of them.  A token at a time 2,048 tokens of width 2,048 with 32
+// experts read them 2,048 times (half a GB through the L2, 47 us); few tokens want a block each.
+template <typename T, int TOKENS>
 __global__ void __launch_bounds__(ROUTE_THREADS)
-route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int width,
+route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int num_tokens, int width,
                   int experts, int top, int groups, int keep, int sigmoid_scores,
                   const float* __restrict__ correction, int group_top, float weight_scale,
                   int* __restrict__ ids, float* __restrict__ weights) {
-    extern __shared__ float sm[];  // x[width], score[experts], group_best[groups], choice[experts]
+    extern __shared__ float sm[];  // x[TOKENS][width], then per token score[experts], group_best[groups], choice[experts]
     float* xs = sm;
-    float* score = xs + width;
-    float* gbest = score + experts;
-    float* choice = gbest + groups;
     ie_pdl_trigger();
     ie_pdl_wait();
-    int n = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < width; i += ROUTE_THREADS) xs[i] = ie_load(x + (size_t)n * width + i);
+    const int n0 = blockIdx.x * TOKENS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cnt = min(TOKENS, num_tokens - n0);
+    float* const scores = xs + TOKENS * width;
+    const int per_token = 2 * experts + groups;
+    for (int i = tid; i < TOKENS * width; i += ROUTE_THREADS) xs[i] = i < cnt * width ? ie_load(x + (size_t)n0 * width + i) : 0.f;
     __syncthreads();
     // A warp takes the experts warp, warp + 8, ...; four of them at a time, so that four rows' loads are
     // on their way together.  An expert's sum is the same chain of operations whichever way it is grouped.
     constexpr int WARPS = ROUTE_THREADS / 32, AT_ONCE = 4;
     for (int e0 = warp; e0 < experts; e0 += WARPS * AT_ONCE) {
-        float acc[AT_ONCE];
+        float acc[AT_ONCE][TOKENS];
         if (width % 4 == 0) {  // (four partial sums per lane and expert, added in a fixed order)
-            float a4[AT_ONCE][4];
+            float a4[AT_ONCE][TOKENS][4];
 #pragma unroll
-            for (int u = 0; u < AT_ONCE; ++u) a4[u][0] = a4[u][1] = a4[u][2] = a4[u][3] = 0.f;
+            for (int u = 0; u < AT_ONCE; ++u)
+#pragma unroll
+                for (int t = 0; t < TOKENS; ++t) a4[u][t][0] = a4[u][t][1] = a4[u][t][2] = a4[u][t][3] = 0.f;
             for (int i = lane * 4; i < width; i += 128) {
-                float4 xv = *reinterpret_cast<const float4*>(xs + i);
+                float4 wv[AT_ONCE];
 #pragma unroll
                 for (int u = 0; u < AT_ONCE; ++u) {
                     int e = e0 + u * WARPS;
-                    if (e < experts) {
-                        float4 wv = *reinterpret_cast<const float4*>(w + (size_t)e * width + i);
-                        a4[u][0] = fmaf(xv.x, wv.x, a4[u][0]); a4[u][1] = fmaf(xv.y, wv.y, a4[u][1]);
-                        a4[u][2] = fmaf(xv.z, wv.z, a4[u][2]); a4[u][3] = fmaf(xv.w, wv.w, a4[u][3]);
+                    wv[u] = e < experts ? *reinterpret_cast<const float4*>(w + (size_t)e * width + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int t = 0; t < TOKENS; ++t) {
+                    float4 xv = *reinterpret_cast<const float4*>(xs + t * width + i);
+#pragma unroll
+                    for (int u = 0; u < AT_ONCE; ++u) {
+                        a4[u][t][0] = fmaf(xv.x, wv[u].x, a4[u][t][0]); a4[u][t][1] = fmaf(xv.y, wv[u].y, a4[u][t][1]);
+                        a4[u][t][2] = fmaf(xv.z, wv[u].z, a4[u][t][2]); a4[u][t][3] = fmaf(xv.w, wv[u].w, a4[u][t][3]);
                     }
                 }
             }
 #pragma unroll
-            for (int u = 0; u < AT_ONCE; ++u) acc[u] = (a4[u][0] + a4[u][1]) + (a4[u][2] + a4[u][3]);
+            for (int u = 0; u < AT_ONCE; ++u)
+#pragma unroll
+                for (int t = 0; t < TOKENS; ++t) acc[u][t] = (a4[u][t][0] + a4[u][t][1]) + (a4[u][t][2] + a4[u][t][3]);
         } else {
 #pragma unroll
             for (int u = 0; u < AT_ONCE; ++u) {
                 int e = e0 + u * WARPS;
-                acc[u] = 0.f;
-                if (e < experts)
-                    for (int i = lane; i < width; i += 32) acc[u] = fmaf(xs[i], w[(size_t)e * width + i], acc[u]);
+#pragma unroll
+                for (int t = 0; t < TOKENS; ++t) {
+                    acc[u][t] = 0.f;
+                    if (e < experts)
+                        for (int i = lane; i < width; i += 32) acc[u][t] = fmaf(xs[t * width + i], w[(size_t)e * width + i], acc[u][t]);
+                }
             }
         }
 #pragma unroll
         for (int u = 0; u < AT_ONCE; ++u) {
             int e = e0 + u * WARPS;
-            float total = warp_sum(acc[u]);
-            if (lane == 0 && e < experts) score[e] = bias != nullptr ? total + bias[e] : total;
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) {
+                float total = warp_sum(acc[u][t]);
+                if (lane == 0 && e < experts) scores[t * per_token + e] = bias != nullptr ? total + bias[e] : total;
+            }
         }
     }
     __syncthreads();
-    if (warp != 0) return;
+    if (warp >= cnt) return;  // (a warp per token from here on)
+    const int n = n0 + warp;
+    float* score = scores + warp * per_token;
+    float* gbest = score + experts;
+    float* choice = gbest + groups;
     if (sigmoid_scores) {
         for (int e = lane; e < experts; e += 32) {
             float sg = 1.0f / (1.0f + expf(-score[e]));
@@ -570,16 +591,24 @@ IE_API int ie_route_topk(const void* x, int dtype, const float* w, const float* 
     if (experts < 1 || groups < 1 || experts % groups || top < 1 || top > experts) return (int)cudaErrorInvalidValue;
     if (group_top < 1 || group_top > 2 || (!sigmoid_scores && (correction != nullptr || group_top != 1)))
         return (int)cudaErrorInvalidValue;
-    size_t smem = (size_t)(width + 2 * experts + groups) * sizeof(float);
-    if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
+    // (four tokens a block from as many blocks as the device has SMs on, where their rows fit)
+    constexpr int MANY = 4;
+    size_t one = (size_t)(width + 2 * experts + groups) * sizeof(float);
+    if (one > 48 * 1024) return (int)cudaErrorInvalidValue;
+    const bool many = num_tokens >= MANY * ie_sm_count() && MANY * one <= 48 * 1024;
+    const size_t smem = many ? MANY * one : one;
+    const dim3 grid(many ? (num_tokens + MANY - 1) / MANY : num_tokens);
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == IE_BF16)
-        return ie_launch(route_topk_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(ROUTE_THREADS), smem, s,
-                         (const __nv_bfloat16*)x, w, bias, width, experts, top, groups, keep, sigmoid_scores, correction,
-                         group_top, weight_scale, ids, weights);
-    return ie_launch(route_topk_kernel<float>, dim3(num_tokens), dim3(ROUTE_THREADS), smem, s, (const float*)x, w,
-                     bias, width, experts, top, groups, keep, sigmoid_scores, correction, group_top, weight_scale, ids,
-                     weights);
+#define IE_ROUTE(T, TOKENS)                                                                                              \
+    return ie_launch(route_topk_kernel<T, TOKENS>, grid, dim3(ROUTE_THREADS), smem, s, (const T*)x, w, bias, num_tokens, \
+                     width, experts, top, groups, keep, sigmoid_scores, correction, group_top, weight_scale, ids, weights)
+    if (dtype == IE_BF16) {
+        if (many) IE_ROUTE(__nv_bfloat16, MANY);
+        IE_ROUTE(__nv_bfloat16, 1);
+    }
+    if (many) IE_ROUTE(float, MANY);
+    IE_ROUTE(float, 1);
+#undef IE_ROUTE
 }
 
 IE_API int ie_routed_tile_rows() { return TILE_M; }

@@ -990,6 +990,11 @@ class CudaOps:
             "ie_routed_align": "P I I P P P I P",
             "ie_routed_gate_up": "P P P I P P P I I I I F I F F P",
             "ie_routed_down": "P P P P I P P P I I I I I P",
+            "ie_routed_tc5_ok": "I I",
+            "ie_routed_tc5_max_tiles": "I I",
+            "ie_routed_sort": "P I I P P P I P",
+            "ie_routed_tc5_gate_up": "P P P P P P I I I I I F I F F P P",
+            "ie_routed_tc5_down": "P P P P P P P I I I I I I P P",
         },
         "recurrent": {
             "ie_short_conv_residual": "P I P P L P P P P I I I I I P P",
@@ -1235,6 +1240,20 @@ class CudaOps:
         n, top = ids.shape
         experts, _, ff, hidden = w_gate_up.shape
         pairs = n * top
+        # tcgen05 (`csrc/routed_tc5.cu`) from one token on: 32 experts of 2048 x 1024, 4 a token, at 1 / 8 / 64 / 512 tokens 39 / 78 / 89 /
+        # 109 us, the mma.sync kernels 57 / 115 / 128 / 207.  They keep the widths without whole 16-byte rows.
+        if (x.dtype == torch.bfloat16 and lib.ie_routed_tc5_ok(hidden, ff) and experts <= 3000
+                and not (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16):
+            max_tiles = lib.ie_routed_tc5_max_tiles(pairs, experts)
+            index = ws.buffer(tag + ".order", 1, 4 * max_tiles + 4 + pairs, torch.int32, rows_cap=None)[0]
+            tiles, meta, order = index[: 4 * max_tiles], index[4 * max_tiles: 4 * max_tiles + 4], index[4 * max_tiles + 4:]
+            y = ws.buffer(tag + ".act", pairs, ff, x.dtype)
+            if out is None:
+                out = ws.buffer(tag + ".delta", pairs, hidden, torch.float32).view(top, n, hidden)
+            self._routed_sort(lib, ids, pairs, experts, order, tiles, meta, max_tiles)
+            self._routed_tc5_gate_up(lib, x, w_gate_up, y, order, tiles, meta, max_tiles, top, limit, alpha, up_offset)
+            self._routed_tc5_down(lib, y, w_down, out, weights, order, tiles, meta, max_tiles, n, top)
+            return out
         max_tiles = lib.ie_routed_max_tiles(pairs, experts)
         rows = max_tiles * lib.ie_routed_tile_rows()
         index = ws.buffer(tag + ".index", 1, rows + max_tiles + 4, torch.int32, rows_cap=None)[0]
@@ -1247,6 +1266,26 @@ class CudaOps:
                              limit, alpha, up_offset)
         self._routed_down(lib, y, w_down, out, weights, sorted_pairs, tile_expert, meta, max_tiles, top, n, ff, hidden)
         return out
+
+    @_kind("routed.align")
+    def _routed_sort(self, lib, ids, pairs, experts, order, tiles, meta, max_tiles) -> None:
+        self._check(lib.ie_routed_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
+                                       max_tiles, self._stream()), "routed_sort")
+
+    @_kind("routed.gate_up")
+    def _routed_tc5_gate_up(self, lib, x, w, y, order, tiles, meta, max_tiles, top, limit, alpha, up_offset) -> None:
+        experts, _, ff, hidden = w.shape
+        self._check(lib.ie_routed_tc5_gate_up(
+            x.data_ptr(), w.data_ptr(), y.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(), max_tiles, experts, top,
+            hidden, ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha, up_offset, self._err_ptr,
+            self._stream()), "routed_tc5_gate_up")
+
+    @_kind("routed.down")
+    def _routed_tc5_down(self, lib, y, w, out, weights, order, tiles, meta, max_tiles, n, top) -> None:
+        experts, hidden, ff = w.shape
+        self._check(lib.ie_routed_tc5_down(
+            y.data_ptr(), w.data_ptr(), out.data_ptr(), weights.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
+            max_tiles, experts, top, n, ff, hidden, self._err_ptr, self._stream()), "routed_tc5_down")
 
     @_kind("routed.align")
     def _routed_align(self, lib, ids, pairs, experts, sorted_pairs, tile_expert, meta, max_tiles) -> None:
