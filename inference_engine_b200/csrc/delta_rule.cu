@@ -4,7 +4,7 @@
 // column by column ([heads][vdim][dim]), then the last taps - 1 inputs of the short convolutions
 // ([taps - 1][channels], oldest first).
 //
-//  * delta_prep: per token the short causal convolution (per channel, over the step's earlier
+//  * delta_prep (delta_prep_tile: sixteen tokens at a time): per token the short causal convolution (per channel, over the step's earlier
 //    tokens of the same request and, before them, the slot's kept inputs) and silu of q, k, v;
 //    q and k as unit vectors per head (q also times dim^-1/2); beta = sigmoid(.); the decay
 //    g = exp(-exp(A_log[head]) * softplus(a + dt_bias)).
@@ -111,7 +111,137 @@ delta_prep_kernel(const float* __restrict__ qkvb, int ld, const float* __restric
                         num_slots, err);
 }
 
-// One block per request of the step: the kept inputs become the last taps - 1 of (kept, new).
+// The same for many tokens.  grid: (blocks of PT_TOKENS tokens, units); a thread takes a channel of the unit through its block's
+// tokens, so an input is read once and not once per tap, and sixteen loads are on their way at once (2,048 tokens of 16 heads of
+// 128 x 128: 147 us a token at a time, bound by the units' chains of loads and barriers).  q and k: `dim` at most 128, one
+// channel per thread, whose squares sixteen tokens add up together (every exchange halves the sums a lane still holds).
+constexpr int PT_TOKENS = 16;
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __restrict__ a,
+                       const float* __restrict__ conv_w, const float* __restrict__ A_log,
+                       const float* __restrict__ dt_bias, const float* __restrict__ state, long long state_stride,
+                       const int* __restrict__ slots, const int* __restrict__ seq_of_token,
+                       const int* __restrict__ cu_q, float* __restrict__ q_out, float* __restrict__ k_out,
+                       float* __restrict__ v_out, float* __restrict__ beta, float* __restrict__ decay, int num_tokens,
+                       int heads, int kv_heads, int dim, int vdim, int num_slots, int* err) {
+    __shared__ float red[4][PT_TOKENS];
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    const int n0 = blockIdx.x * PT_TOKENS, cnt = min(PT_TOKENS, num_tokens - n0), unit = blockIdx.y, tid = threadIdx.x;
+    const int qk = kv_heads * dim, channels = 2 * qk + heads * vdim;
+    if (unit == 2 * kv_heads + 2 * heads) {  // the betas
+        for (int i = tid; i < cnt * heads; i += 128) {
+            const size_t n = (size_t)(n0 + i / heads);
+            beta[n * heads + i % heads] = sigmoid_f(qkvb[n * ld + channels + i % heads]);
+        }
+        return;
+    }
+    if (unit >= 2 * kv_heads + heads) {  // a head's decays
+        const int h = unit - 2 * kv_heads - heads;
+        const float rate = expf(A_log[h]);
+        for (int d = tid; d < dim; d += 128) {
+            const float bias = dt_bias[h * dim + d];
+            const size_t at = (size_t)n0 * heads * dim + h * dim + d, step = (size_t)heads * dim;
+            float v[PT_TOKENS];
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS; ++i) v[i] = i < cnt ? a[at + i * step] : 0.f;
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS; ++i)
+                if (i < cnt) decay[at + i * step] = expf(-rate * softplus_f(v[i] + bias));
+        }
+        return;
+    }
+    const bool is_v = unit >= 2 * kv_heads;
+    const int width = is_v ? vdim : dim;
+    const int first_channel = is_v ? 2 * qk + (unit - 2 * kv_heads) * vdim : unit * dim;
+    const size_t tail_at = (size_t)heads * dim * vdim;
+    for (int c0 = 0; c0 < width; c0 += 128) {  // (q and k: once)
+        const int i0 = c0 + tid, c = first_channel + i0;
+        const bool live = i0 < width;
+        float y[PT_TOKENS], w[TAPS];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[j] = live ? conv_w[(size_t)c * TAPS + j] : 0.f;
+        const int seq0 = seq_of_token[n0];
+        if (cnt == PT_TOKENS && n0 + PT_TOKENS <= cu_q[seq0 + 1]) {  // (all of one request)
+            const int t0 = n0 - cu_q[seq0], slot = slots[seq0];
+            if (slot < 0 || slot >= num_slots) {
+                if (tid == 0) ie_report(err, IE_ERR_PAGE, slot, n0);
+                return;
+            }
+            const float* tail = state + (size_t)slot * state_stride + tail_at;
+            float in[PT_TOKENS + TAPS - 1];
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS + TAPS - 1; ++i) {
+                const int back = TAPS - 1 - i;  // (negative: that many tokens into the block)
+                in[i] = !live ? 0.f : t0 - back >= 0 ? qkvb[(size_t)(n0 - back) * ld + c] : tail[(size_t)(TAPS - 1 + t0 - back) * channels + c];
+            }
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS; ++i) {
+                float acc = 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) acc = fmaf(w[j], in[i + j], acc);
+                y[i] = silu_f(acc);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS; ++i) {
+                y[i] = 0.f;
+                if (i < cnt) {
+                    const int n = n0 + i, seq = seq_of_token[n], t = n - cu_q[seq], slot = slots[seq];
+                    if (slot < 0 || slot >= num_slots) {
+                        if (tid == 0) ie_report(err, IE_ERR_PAGE, slot, n);
+                    } else if (live) {
+                        const float* tail = state + (size_t)slot * state_stride + tail_at;
+                        float acc = 0.f;
+#pragma unroll
+                        for (int j = 0; j < TAPS; ++j) {
+                            const int back = TAPS - 1 - j;
+                            acc = fmaf(w[j], t - back >= 0 ? qkvb[(size_t)(n - back) * ld + c] : tail[(size_t)(TAPS - 1 + t - back) * channels + c], acc);
+                        }
+                        y[i] = silu_f(acc);
+                    }
+                }
+            }
+        }
+        if (is_v) {
+            if (live)
+#pragma unroll
+                for (int i = 0; i < PT_TOKENS; ++i)
+                    if (i < cnt) v_out[(size_t)(n0 + i) * heads * vdim + (c - 2 * qk)] = y[i];
+            continue;
+        }
+        float part[PT_TOKENS];
+#pragma unroll
+        for (int i = 0; i < PT_TOKENS; ++i) part[i] = __fmul_rn(y[i], y[i]);
+        const int lane = tid & 31;
+#pragma unroll
+        for (int off = 16, held = PT_TOKENS / 2; off > 1; off >>= 1, held >>= 1) {
+            const bool high = lane & off;
+#pragma unroll
+            for (int k = 0; k < PT_TOKENS / 2; ++k)
+                if (k < held) {
+                    const float send = high ? part[k] : part[k + held], keep = high ? part[k + held] : part[k];
+                    part[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        }
+        part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+        if (!(lane & 1)) red[tid >> 5][lane >> 1] = part[0];
+        __syncthreads();
+        const bool is_q = unit < kv_heads;
+        const float scale = is_q ? 1.0f / sqrtf((float)dim) : 1.0f;
+        float* dst = (is_q ? q_out : k_out) + (size_t)n0 * qk + (is_q ? unit : unit - kv_heads) * dim + i0;
+#pragma unroll
+        for (int i = 0; i < PT_TOKENS; ++i) {
+            float f = 1.0f / sqrtf(((red[0][i] + red[1][i]) + (red[2][i] + red[3][i])) + 1e-6f);
+            if (is_q) f *= scale;
+            if (live && i < cnt) dst[(size_t)i * qk] = y[i] * f;
+        }
+    }
+}
+
+// grid: (requests of the step, blocks of 256 channels): the kept inputs become the last taps - 1 of (kept, new).  A thread owns a
+// channel; with up to four kept rows every value is read before the first is written, so the reads wait for memory together.
 __global__ void delta_conv_tail_kernel(const float* __restrict__ qkvb, int ld, float* __restrict__ state,
                                        long long state_stride, const int* __restrict__ slots,
                                        const int* __restrict__ cu_q, long long matrix_floats, int channels,
@@ -120,18 +250,26 @@ __global__ void delta_conv_tail_kernel(const float* __restrict__ qkvb, int ld, f
     ie_pdl_wait();
     int seq = blockIdx.x;
     int start = cu_q[seq], len = cu_q[seq + 1] - start;
-    int slot = slots[seq];
-    if (len <= 0 || slot < 0 || slot >= num_slots) return;
+    int slot = slots[seq], c = blockIdx.y * blockDim.x + threadIdx.x;
+    if (len <= 0 || slot < 0 || slot >= num_slots || c >= channels) return;
     float* tail = state + (size_t)slot * state_stride + matrix_floats;
-    for (int c = threadIdx.x; c < channels; c += blockDim.x) {
-        // row j takes the input at step-relative time len - (taps - 1) + j; a thread owns a channel and
-        // goes through the rows in rising order, so a kept row is read before it is overwritten
-        for (int j = 0; j < taps - 1; ++j) {
-            int tt = len - (taps - 1) + j;
-            float x = tt >= 0 ? qkvb[(size_t)(start + tt) * ld + c] : tail[(size_t)(taps - 1 + tt) * channels + c];
-            tail[(size_t)j * channels + c] = x;
-        }
+    // row j takes the input at step-relative time len - (taps - 1) + j
+    auto kept = [&](int j) {
+        int tt = len - (taps - 1) + j;
+        return tt >= 0 ? qkvb[(size_t)(start + tt) * ld + c] : tail[(size_t)(taps - 1 + tt) * channels + c];
+    };
+    constexpr int MOST = 4;
+    if (taps - 1 <= MOST) {
+        float v[MOST];
+#pragma unroll
+        for (int j = 0; j < MOST; ++j)
+            if (j < taps - 1) v[j] = kept(j);
+#pragma unroll
+        for (int j = 0; j < MOST; ++j)
+            if (j < taps - 1) tail[(size_t)j * channels + c] = v[j];
+        return;
     }
+    for (int j = 0; j < taps - 1; ++j) tail[(size_t)j * channels + c] = kept(j);  // (rising: read before it is overwritten)
 }
 
 constexpr int DR_THREADS = 128;
@@ -305,14 +443,25 @@ IE_API int ie_delta_prep(const float* qkvb, int ld, const float* a, const float*
     cudaStream_t s = (cudaStream_t)stream;
     size_t smem = (size_t)(dim > vdim ? dim : vdim) * sizeof(float);
     if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-    int units = 2 * kv_heads + 2 * heads + 1;
-    int per_token = num_tokens >= 512 ? (units < 4 ? units : 4) : units;
-    int e = ie_launch(delta_prep_kernel, dim3(num_tokens, per_token), dim3(128), smem, s, qkvb, ld, a, conv_w, A_log, dt_bias,
-                      (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out, k_out, v_out, beta,
-                      decay, heads, kv_heads, dim, vdim, taps, num_slots, err);
+    int units = 2 * kv_heads + 2 * heads + 1, e;
+    const dim3 tiles((num_tokens + PT_TOKENS - 1) / PT_TOKENS, units);
+#define IE_DP_TILE(TAPS)                                                                                               \
+    e = ie_launch(delta_prep_tile_kernel<TAPS>, tiles, dim3(128), 0, s, qkvb, ld, a, conv_w, A_log, dt_bias,           \
+                  (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out, k_out, v_out, beta, decay,      \
+                  num_tokens, heads, kv_heads, dim, vdim, num_slots, err)
+    // (from 64 tokens on the tiles are enough blocks to fill the device; a few tokens get a block per token and unit)
+    const bool tile = num_tokens >= 64 && dim <= 128;
+    if (tile && taps == 4) IE_DP_TILE(4);
+    else if (tile && taps == 3) IE_DP_TILE(3);
+    else if (tile && taps == 2) IE_DP_TILE(2);
+    else
+        e = ie_launch(delta_prep_kernel, dim3(num_tokens, num_tokens >= 512 ? (units < 4 ? units : 4) : units), dim3(128), smem, s,
+                      qkvb, ld, a, conv_w, A_log, dt_bias, (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out,
+                      k_out, v_out, beta, decay, heads, kv_heads, dim, vdim, taps, num_slots, err);
+#undef IE_DP_TILE
     if (e != 0 || taps < 2) return e;
     int channels = 2 * kv_heads * dim + heads * vdim;
-    return ie_launch(delta_conv_tail_kernel, dim3(num_seqs), dim3(256), 0, s, qkvb, ld, state, state_stride, slots,
+    return ie_launch(delta_conv_tail_kernel, dim3(num_seqs, (channels + 255) / 256), dim3(256), 0, s, qkvb, ld, state, state_stride, slots,
                      cu_q, (long long)heads * dim * vdim, channels, taps, num_slots);
 }
 
