@@ -175,6 +175,16 @@ def build_sink_attention(dim: int, vdim: int, bias: str = "none") -> Path:
                          [f"-DSK_D={dim}", f"-DSK_DV={vdim}"] + ([f"-DSK_BIAS={kind}"] if kind else []))
 
 
+PACKED_ATTENTION_SIZES = ((64, 64), (128, 128))  # (key size, value size) that the tcgen05 softmax attention is built for
+
+
+def build_packed_attention(dim: int, vdim: int) -> Path:
+    """The tcgen05 softmax attention of prompt portions for one pair of key and value sizes (compiled on first use)."""
+    if (dim, vdim) not in PACKED_ATTENTION_SIZES:
+        raise BuildError(f"the tcgen05 softmax attention takes sizes {PACKED_ATTENTION_SIZES}, not {dim} and {vdim}")
+    return build_library(f"ie_b200_packed_d{dim}_v{vdim}", ["attention_packed.cu"], [f"-DPA_D={dim}", f"-DPA_DV={vdim}"])
+
+
 def build_retention(dim: int, vdim: int) -> Path:
     """The bfloat16 path's retention kernels for one pair of key and value sizes, each rounded up to a
     multiple of 16 (compiled on first use for the sizes the loaded model has)."""
@@ -245,6 +255,7 @@ def build_all(prune: bool = True) -> list[Path]:
         libs += [build_sigmoid_attention(64, 64), build_sink_attention(64, 64),
                  build_sink_attention(64, 64, "log"), build_sink_attention(64, 64, "table"),
                  build_retention(64, 64), build_state_space(64, 64), build_latent_attention(320, 256)]
+        libs += list(pool.map(lambda sizes: build_packed_attention(*sizes), PACKED_ATTENTION_SIZES))
     if prune:
         keep = {lib.name for lib in libs}
         for old in build_dir().glob("libie_b200_*.so"):

@@ -18,8 +18,8 @@ import os
 from ctypes import c_float, c_int, c_void_p
 from typing import Any
 
-from .build import (ATTENTION_HEAD_DIMS, build_attention, build_core, build_latent_attention, build_part_library,
-                    build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
+from .build import (ATTENTION_HEAD_DIMS, PACKED_ATTENTION_SIZES, build_attention, build_core, build_latent_attention,
+                    build_packed_attention, build_part_library, build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
                     latent_attention_fits)
 
 _ERRORS = {
@@ -146,6 +146,8 @@ class CudaOps:
         self.retention_fused = os.environ.get("IE_B200_RETENTION", "1") != "0"  # the retention kernels of the bfloat16 path
         self._sinkattn_libs: dict[tuple[int, int, str], object] = {}
         self.sink_mma = os.environ.get("IE_B200_SINK_MMA", "1") != "0"  # tensor-core sink attention
+        self.sink_tc5 = os.environ.get("IE_B200_SINK_TC5", "1") != "0"  # ... of prompt portions on tcgen05
+        self._packed_libs: dict[tuple[int, int], object] = {}
         # residual gates' products as partial sums: faster by themselves, slower inside a captured step
         self.gate_split = os.environ.get("IE_B200_GATE_SPLIT", "0") == "1"
         self.sigmoid_mma = os.environ.get("IE_B200_SIGMOID_MMA", "1") != "0"  # tensor-core sigmoid attention
@@ -1803,6 +1805,23 @@ class CudaOps:
             self._sinkattn_libs[(hd, vdim, bias)] = lib
         return lib
 
+    def _packed_lib(self, dim: int, vdim: int):
+        lib = self._packed_libs.get((dim, vdim))
+        if lib is None:
+            path = build_packed_attention(dim, vdim)
+            try:
+                lib = ctypes.CDLL(str(path))
+            except OSError as exc:
+                raise KernelError(f"the kernel library {path} could not be loaded: {exc}") from exc
+            P, I, F = c_void_p, c_int, c_float
+            lib.ie_attention_packed.argtypes = [P, P, P, P, I, P, P, P, I, I, I, I, I, I, F, I, P, P, I, I, F, I, I, P, P]
+            lib.ie_attention_packed.restype = c_int
+            self._packed_libs[(dim, vdim)] = lib
+        return lib
+
+    # from so many rows (tokens x heads of a group) of the longest portion on softmax attention runs on tcgen05
+    PACKED_FROM = 64
+
     # requests that bring at most so many tokens have their window's keys cut among blocks, each of
     # which serves the query heads of one key/value head (tokens x heads of a group: 64 rows at most)
     SINK_SPLIT_ROWS = 8
@@ -1871,6 +1890,17 @@ class CudaOps:
                 splits = -(-tiles // per_split) + kept_splits
                 if splits > 1:
                     scratch = self._scratch(ctx, "attn.sink_partial", ctx.num_tokens * nh * splits * (vdim + 2), q.device)
+            if (scratch is None and self.sink_tc5 and kind == "none" and (hd, vdim) in PACKED_ATTENTION_SIZES
+                    and longest * (nh // nkv) >= self.PACKED_FROM and out.stride(0) % 8 == 0
+                    and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16):
+                self._check(self._packed_lib(hd, vdim).ie_attention_packed(
+                    q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+                    ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, longest, nh, nkv, page_size,
+                    k_cache.shape[0], scale, int(window or 0), self._ptr(sinks), self._ptr(gate),
+                    0 if gate is None else gate.stride(0), by_distance[0], cap, keep, out.stride(0), self._err_ptr,
+                    self._stream()), "sink_attention_mma")
+                self.launch_counts["sink_attention_packed"] = self.launch_counts.get("sink_attention_packed", 0) + 1
+                return
             self._check(lib.ie_sink_attention_mma(
                 q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(),
                 block_tables.shape[1], ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs,
