@@ -3,22 +3,26 @@
 // value size PA_DV: 64 or 128).
 //
 // A block owns 256 rows of one request and one key/value head, a row being a (token, query head of the group) pair, so that a key tile
-// is brought once for the whole group, and walks tiles of 128 keys.  Two row tiles of 128 take turns: while the softmax warps of one work, the
-// tensor core serves the other.  Eleven warps (with a thirteenth a thread would have 128 registers instead of 168, and spill):
+// is brought once for the whole group, and walks tiles of 64 keys.  Two row tiles of 128 take turns, and a row tile's scores are made a key tile
+// ahead of its softmax, so that softmax follows softmax.  Eleven warps (with a thirteenth a thread would have 128 registers instead of
+// 168, and spill):
 //   warps 0-3, 4-7: softmax of row tile 0 and 1, a thread per row (tensor-memory lane);
-//   warp 8: tcgen05.mma.  Per key tile and row tile: O += P V of the tile before (P, in tensor memory, over the scores it was made
-//     from), then S = Q K^T (both from shared memory).  The whole warp runs the loop and one elected lane issues, so that
-//     descriptors stay in uniform registers;
-//   warps 9, 10: gather keys and values from the request's pages by cp.async, swizzled by hand as the tensor core reads them.  (Pages of
-//     16 tokens as TMA boxes are 2 KB each, and the copy engine spends some 300 clocks on any box: 32 of them per key tile would take three
-//     times as long as the tile's products.)
-// Tensor memory: scores of the row tiles in columns 0 and 128, their outputs in 256 and 384.  A row's weights replace its scores 64 keys at a
-// time: 32 columns of weights rounded to bfloat16, two to a column, then 32 columns of what the rounding left (TERMS 2: a weight keeps 16 bits of
+//   warp 8: tcgen05.mma.  Per key tile: S = Q K^T of the next key tile for both row tiles (both operands from shared memory), then
+//     O += P V of this one as each row tile's weights are written (P in tensor memory, over the scores it was made from);
+//   warps 9, 10: gather keys and values by cp.async, swizzled by hand as the tensor core reads them.  (Pages of
+//     16 tokens as TMA boxes are 2 KB each, and the copy engine spends some 300 clocks on any box: they would take longer than a tile's products.)
+// Tensor memory: row tile i's scores of key tile t in columns (2 i + t % 2) 64 .. + 63, its output in 256 + 128 i.  A row's weights replace its
+// scores: 32 columns of weights rounded to bfloat16, two to a column, then 32 columns of what the rounding left (a weight keeps 16 bits of
 // mantissa; both go through the second product).  The maximum that weights are taken against follows a row's running maximum only when that
 // has grown by more than 2^8; only then is the row's output rescaled.  A row's arithmetic depends on its own request alone.
 //
-// What bounds it: the special-function unit (128 x 256 exponentials a key tile: 2,048 clocks) beside the products (head size 128: 1,536 clocks).
-// Sixteen query heads on four of 128, window 1,024, 2,048 tokens: the mma.sync kernel that serves the other sizes takes 148 us.
+// PA_FLAT 1 (latent attention whose keys and values were expanded per head): keys and values are rows of step-wide arrays, a request's
+// context after the one before it; a key is the head's own entries (PA_D - 64) and then up to 64 rotated ones that all heads share.
+//
+// What bounds it: a key tile's products take 1,808 clocks (65 for 128 x 128 x 16, 48 for 128 x 64 x 16, as measured), its exponentials
+// 1,024 of the special-function unit, its softmax instructions about as long as the products.  Scores one tile of 128 keys at a time, made when
+// the softmax before had ended, cost the chain both: 7,000 clocks per 128 keys.
+// Sixteen query heads on four of 128, window 1,024, 2,048 tokens: the mma.sync kernel that serves the other sizes takes 142 us, that form took 40.
 // Every wait is bounded; a block that waits too long records IE_ERR_TIMEOUT, frees its tensor memory and leaves.
 #include "tma.cuh"
 #include <math.h>
@@ -29,24 +33,28 @@
 #ifndef PA_DV
 #define PA_DV 128
 #endif
+#ifndef PA_FLAT
+#define PA_FLAT 0
+#endif
 
 using namespace ie_tma;
 
 namespace {
 constexpr int D = PA_D, DV = PA_DV;
 static_assert((D == 64 || D == 128 || D == 192) && (DV == 64 || DV == 128), "sizes");
+constexpr bool FLAT = PA_FLAT != 0;
 constexpr int TERMS = 2;
-constexpr int BM = 128, ROWS = 2 * BM, KT = 128;
+constexpr int BM = 128, ROWS = 2 * BM, KT = 64;
 constexpr int KH = D / 64, VH = DV / 64;         // runs of 64 entries: 128 bytes, one swizzle atom
-constexpr int HALF = KT * 128;                   // such a run of a tile's 128 rows: 16 KB
-constexpr int K_BYTES = KH * HALF, V_BYTES = VH * HALF, Q_BYTES = 2 * K_BYTES;
-constexpr int KS = D == 64 ? 4 : 2, VS = DV == 64 ? 4 : D == 192 ? 1 : 2;  // tiles of keys and of values in shared memory
+constexpr int Q_RUN = BM * 128, KV_RUN = KT * 128;  // such a run of a row tile, of a key tile
+constexpr int K_BYTES = KH * KV_RUN, V_BYTES = VH * KV_RUN, Q_TILE = KH * Q_RUN, Q_BYTES = 2 * Q_TILE;
+constexpr int KS = D == 192 ? 3 : 4, VS = D == 192 ? 3 : 4;  // tiles of keys and of values in shared memory
 constexpr int SOFTMAX_WARPS = 8, COPY_WARPS = 2, THREADS = (SOFTMAX_WARPS + 1 + COPY_WARPS) * 32;
 constexpr float RESCALE_LAG = 8.0f;              // in powers of two
 constexpr float LOG2E_F = 1.4426950408889634f;
 
 struct __align__(8) Bars {
-    unsigned long long q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_done[2], p_ready[2], o_done[2];
+    unsigned long long q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_done[4], p_ready[4], o_done[2];
     unsigned tmem_base;
     int failed;
 };
@@ -102,6 +110,11 @@ struct Inputs {
     int gate_ld, gate_elements;
     bf16* out;
     int out_ld;
+    // PA_FLAT: q [tokens, heads, D - 64], the rotated entries of (token, head) at q_rot + (token * heads + head) * q_rot_ld; keys and
+    // values at k + row * kv_ld + head * (D - 64) and v + row * kv_ld + head * DV, the shared rotated entries (`rot` of them) at k_rot + row *
+    // k_rot_ld
+    const bf16 *q_rot, *k_rot;
+    int q_rot_ld, k_rot_ld, kv_ld, rot;
 };
 
 // grid: (blocks of 256 rows of the longest portion, key/value heads, requests)
@@ -135,11 +148,8 @@ attention_packed_kernel(const Inputs in, int* err) {
         mbar_init(&bars->q_full, COPY_WARPS);
         for (int s = 0; s < KS; ++s) { mbar_init(&bars->k_full[s], COPY_WARPS); mbar_init(&bars->k_empty[s], 1); }
         for (int s = 0; s < VS; ++s) { mbar_init(&bars->v_full[s], COPY_WARPS); mbar_init(&bars->v_empty[s], 1); }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&bars->s_done[i], 1);
-            mbar_init(&bars->p_ready[i], BM);
-            mbar_init(&bars->o_done[i], 1);
-        }
+        for (int i = 0; i < 4; ++i) { mbar_init(&bars->s_done[i], 1); mbar_init(&bars->p_ready[i], BM); }
+        for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
         bars->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -159,44 +169,48 @@ attention_packed_kernel(const Inputs in, int* err) {
         const unsigned qa = smem_u32(q_s), ka = smem_u32(k_s), va = smem_u32(v_s);
         const bool one = elect_one();
         bool ok = mbar_wait_compact(&bars->q_full, 0);
-        for (int t = 0; t <= tiles && ok; ++t) {
+        // the scores of key tile t for both row tiles.  (What their columns held, the weights of tile t - 2, went into products that
+        // this thread issued before: they are done before these write.)
+        auto scores = [&](int t) {
+            const int slot = t % KS;
+            if (!mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (one) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const unsigned qt = qa + i * Q_TILE, kt = ka + slot * K_BYTES;
+#pragma unroll
+                    for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
+                        umma_ss(tmem + (2 * i + (t & 1)) * KT, umma_desc_sw128(qt + (ks >> 2) * Q_RUN + (ks & 3) * 32),
+                                umma_desc_sw128(kt + (ks >> 2) * KV_RUN + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
+                    umma_commit(&bars->s_done[2 * i + (t & 1)]);
+                }
+                umma_commit(&bars->k_empty[slot]);
+            }
+            __syncwarp();
+            return true;
+        };
+        ok = ok && scores(0);
+        for (int t = 0; t < tiles && ok; ++t) {
+            if (t + 1 < tiles) ok = scores(t + 1);
+            const int slot = t % VS;
+            ok = ok && mbar_wait_compact(&bars->v_full[slot], (t / VS) & 1);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                if (t > 0) {  // the tile before: its weights are written
-                    const int slot = (t - 1) % VS;
-                    ok = ok && (i > 0 || mbar_wait_compact(&bars->v_full[slot], ((t - 1) / VS) & 1)) &&
-                         mbar_wait_compact(&bars->p_ready[i], (t - 1) & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (one) {
-                        const unsigned p = tmem + i * KT, o = tmem + ROWS + i * BM, vt = va + slot * V_BYTES;
+                ok = ok && mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (one) {
+                    const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * V_BYTES;
 #pragma unroll
-                        for (int term = 0; term < TERMS; ++term)
+                    for (int term = 0; term < TERMS; ++term)
 #pragma unroll
-                            for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
-                                umma_ta(o, p + (ks >> 2) * 64 + term * 32 + (ks & 3) * 8, desc_mn(vt + ks * 2048, HALF), idesc_pv,
-                                        t > 1 || term > 0 || ks > 0 ? 1u : 0u);
-                        if (t == tiles) umma_commit(&bars->o_done[i]);
-                        if (i == 1) umma_commit(&bars->v_empty[slot]);
-                    }
-                    __syncwarp();
+                        for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
+                            umma_ta(o, p + term * 32 + ks * 8, desc_mn(vt + ks * 2048, KV_RUN), idesc_pv, t > 0 || term > 0 || ks > 0 ? 1u : 0u);
+                    umma_commit(&bars->o_done[i]);
+                    if (i == 1) umma_commit(&bars->v_empty[slot]);
                 }
-                if (t < tiles) {
-                    const int slot = t % KS;
-                    if (i == 0) ok = mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (one) {
-                        const unsigned qt = qa + i * K_BYTES, kt = ka + slot * K_BYTES;
-#pragma unroll
-                        for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
-                            umma_ss(tmem + i * KT, umma_desc_sw128(qt + (ks >> 2) * HALF + (ks & 3) * 32),
-                                    umma_desc_sw128(kt + (ks >> 2) * HALF + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
-                        umma_commit(&bars->s_done[i]);
-                        if (i == 1) umma_commit(&bars->k_empty[slot]);
-                    }
-                    __syncwarp();
-                }
+                __syncwarp();
             }
         }
         if (!ok) bars->failed = 1;
@@ -230,33 +244,47 @@ attention_packed_kernel(const Inputs in, int* err) {
             return mbar_wait_compact(bar, parity);
         };
         {
-            #pragma unroll 4
+#pragma unroll 4
             for (int p = 0; p < ROWS / AT_ONCE; ++p) {
                 const int r = r0 + AT_ONCE * p;
                 const bool there = r < rows_here;
                 const int rr = row0 + (there ? r : 0), token = rr / group, head = kvh * group + rr - token * group;
-                const bf16* src = in.q + ((size_t)(q0 + token) * in.heads + head) * D + chunk * 8;
-                const unsigned dst = smem_u32(q_s) + (r >> 7) * K_BYTES + (p & (PASSES - 1)) * 1024 + to;
+                const size_t unit = (size_t)(q0 + token) * in.heads + head;
+                const unsigned dst = smem_u32(q_s) + (r >> 7) * Q_TILE + (p & (BM / AT_ONCE - 1)) * 1024 + to;
 #pragma unroll
-                for (int h = 0; h < KH; ++h) cp16(dst + h * HALF, src + h * 64, there ? 16 : 0);
+                for (int h = 0; h < KH; ++h) {
+                    if (FLAT && h == KH - 1) {
+                        const bool rotated = there && chunk * 8 < in.rot;
+                        cp16(dst + h * Q_RUN, rotated ? in.q_rot + unit * in.q_rot_ld + chunk * 8 : in.q, rotated ? 16 : 0);
+                    } else {
+                        cp16(dst + h * Q_RUN, in.q + unit * (FLAT ? D - 64 : D) + chunk * 8 + h * 64, there ? 16 : 0);
+                    }
+                }
             }
             asked(&bars->q_full);
         }
-        const int* table = in.tables + (size_t)seq * in.table_width;
+        const int* table = FLAT ? nullptr : in.tables + (size_t)seq * in.table_width;
+        int before = 0;  // FLAT: rows of the requests before this one
+        if (FLAT)
+            for (int i = 0; i < seq; ++i) before += in.ctx_lens[i];
         bool ok = true;
         for (int t = 0; t < tiles; ++t) {
             const int key0 = key_of(t);
-            int row[PASSES];  // the cache's row of each of the thread's keys; -1: nothing there (reads as zero)
+            int row[PASSES];  // the row of each of the thread's keys; -1: nothing there (reads as zero)
 #pragma unroll
             for (int p = 0; p < PASSES; ++p) {
                 const int pos = key0 + r0 + AT_ONCE * p;
                 row[p] = -1;
                 if ((pos >= lo_min || pos < in.keep_first) && pos <= last_pos) {
-                    const int page = table[pos >> in.page_shift];
-                    if (page < 0 || page >= in.total_pages) {
-                        if (chunk == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
+                    if (FLAT) {
+                        row[p] = before + pos;
                     } else {
-                        row[p] = ((page * in.kv_heads + kvh) << in.page_shift) + (pos & ((1 << in.page_shift) - 1));
+                        const int page = table[pos >> in.page_shift];
+                        if (page < 0 || page >= in.total_pages) {
+                            if (chunk == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
+                        } else {
+                            row[p] = ((page * in.kv_heads + kvh) << in.page_shift) + (pos & ((1 << in.page_shift) - 1));
+                        }
                     }
                 }
             }
@@ -265,18 +293,27 @@ attention_packed_kernel(const Inputs in, int* err) {
             unsigned dst = smem_u32(k_s) + ks * K_BYTES + to;
 #pragma unroll
             for (int p = 0; p < PASSES; ++p) {
-                const bf16* src = in.k + (size_t)max(row[p], 0) * D + chunk * 8;
+                const size_t at = (size_t)max(row[p], 0);
+                const bf16* src = FLAT ? in.k + at * in.kv_ld + kvh * (D - 64) + chunk * 8 : in.k + at * D + chunk * 8;
 #pragma unroll
-                for (int h = 0; h < KH; ++h) cp16(dst + p * 1024 + h * HALF, src + h * 64, row[p] >= 0 ? 16 : 0);
+                for (int h = 0; h < KH; ++h) {
+                    if (FLAT && h == KH - 1) {
+                        const bool rotated = row[p] >= 0 && chunk * 8 < in.rot;
+                        cp16(dst + p * 1024 + h * KV_RUN, rotated ? in.k_rot + at * in.k_rot_ld + chunk * 8 : in.k, rotated ? 16 : 0);
+                    } else {
+                        cp16(dst + p * 1024 + h * KV_RUN, src + h * 64, row[p] >= 0 ? 16 : 0);
+                    }
+                }
             }
             asked(&bars->k_full[ks]);
             if (t >= VS && !slot_free(&bars->v_empty[vs], (t / VS - 1) & 1)) { ok = false; break; }
             dst = smem_u32(v_s) + vs * V_BYTES + to;
 #pragma unroll
             for (int p = 0; p < PASSES; ++p) {
-                const bf16* src = in.v + (size_t)max(row[p], 0) * DV + chunk * 8;
+                const size_t at = (size_t)max(row[p], 0);
+                const bf16* src = FLAT ? in.v + at * in.kv_ld + kvh * DV + chunk * 8 : in.v + at * DV + chunk * 8;
 #pragma unroll
-                for (int h = 0; h < VH; ++h) cp16(dst + p * 1024 + h * HALF, src + h * 64, row[p] >= 0 ? 16 : 0);
+                for (int h = 0; h < VH; ++h) cp16(dst + p * 1024 + h * KV_RUN, src + h * 64, row[p] >= 0 ? 16 : 0);
             }
             asked(&bars->v_full[vs]);
         }
@@ -292,7 +329,7 @@ attention_packed_kernel(const Inputs in, int* err) {
         const int pos_lo = start + min(row0 + i * BM, rows_total - 1) / group;
         const int pos_hi = start + min(row0 + i * BM + BM - 1, rows_total - 1) / group;
         const unsigned lane_addr = (unsigned)((warp & 3) * 32) << 16;
-        const unsigned ts = tmem + i * KT + lane_addr, to = tmem + ROWS + i * BM + lane_addr;
+        const unsigned to = tmem + ROWS + i * BM + lane_addr;
         const float sl2 = in.scale * LOG2E_F;
         const float cap_in = CAP ? in.scale / in.softcap : 0.f, cap_out = CAP ? in.softcap * LOG2E_F : 0.f;
         // m: the maximum that the weights are taken against (in units of log2 e); the sink is a term of the sum without key and value
@@ -300,36 +337,29 @@ attention_packed_kernel(const Inputs in, int* err) {
         bool ok = true;
         for (int t = 0; t < tiles; ++t) {
             const int key0 = key_of(t);
-            if (!mbar_wait_compact(&bars->s_done[i], t & 1)) { ok = false; break; }
+            if (!mbar_wait_compact(&bars->s_done[2 * i + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned ts = tmem + (2 * i + (t & 1)) * KT + lane_addr;
             const bool inner = key0 + KT - 1 <= pos_lo && (in.window <= 0 || key0 >= pos_hi - in.window + 1 || key0 + KT <= in.keep_first);
-            float s[64];
-            auto scores = [&](int half) {
-                tmem_ld64(s, ts + half * 64);
-                if (!inner) {
+            float s[KT];
+            tmem_ld64(s, ts);
+            if (!inner) {
 #pragma unroll
-                    for (int j = 0; j < 64; ++j) {
-                        const int kp = key0 + half * 64 + j;
-                        s[j] = kp <= pos && (kp >= lo || kp < in.keep_first) ? s[j] : -INFINITY;
-                    }
+                for (int j = 0; j < KT; ++j) {
+                    const int kp = key0 + j;
+                    s[j] = kp <= pos && (kp >= lo || kp < in.keep_first) ? s[j] : -INFINITY;
                 }
-            };
-            auto maximum = [&](float before) {
-                float mx[8];
+            }
+            float mx[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) mx[j] = s[j];
+            for (int j = 0; j < 8; ++j) mx[j] = s[j];
 #pragma unroll
-                for (int j = 8; j < 56; j += 16)
+            for (int j = 8; j < 56; j += 16)
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) mx[k] = max3(mx[k], s[j + k], s[j + 8 + k]);
+                for (int k = 0; k < 8; ++k) mx[k] = max3(mx[k], s[j + k], s[j + 8 + k]);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) mx[k] = fmaxf(mx[k], s[56 + k]);
-                return fmaxf(before, fmaxf(max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), mx[6]), mx[7]));
-            };
-            scores(0);
-            float top = maximum(-INFINITY);
-            scores(1);
-            top = maximum(top);
+            for (int k = 0; k < 8; ++k) mx[k] = fmaxf(mx[k], s[56 + k]);
+            const float top = fmaxf(max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), mx[6]), mx[7]);
             // (scores are compared before scale and cap, which keep their order)
             const float m_seen = top == -INFINITY ? m : fmaxf(m, CAP ? cap_out * tanh_fast(top * cap_in) : top * sl2);
             const bool grown = m_seen > m + RESCALE_LAG;  // (from -inf: yes)
@@ -338,7 +368,10 @@ attention_packed_kernel(const Inputs in, int* err) {
                 m = m_seen;
                 l *= alpha;
             }
-            if (t > 0 && __any_sync(0xffffffffu, grown)) {  // (the products before this tile's scores are done)
+            if (t > 0 && __any_sync(0xffffffffu, grown)) {
+                // (the product of the tile before may still be running; the ones before that are done, since this tile's scores are)
+                if (!mbar_wait_compact(&bars->o_done[i], (t - 1) & 1)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
                 for (int d = 0; d < DV; d += 32) {
                     float acc[32];
@@ -349,45 +382,40 @@ attention_packed_kernel(const Inputs in, int* err) {
                 }
             }
             const float m_safe = m == -INFINITY ? 0.f : m;
-            const float2 scale2 = make_float2(sl2, sl2), minus_m = make_float2(-m_safe, -m_safe);
+            const float2 scale2 = make_float2(sl2, sl2), minus_m = make_float2(-m_safe, -m_safe), minus_one = make_float2(-1.f, -1.f);
             float2 sums[2] = {{0.f, 0.f}, {0.f, 0.f}};
-            auto weights = [&](int half) {
 #pragma unroll
-                for (int part = 0; part < 2; ++part) {
-                    unsigned hi[16], rest[16];
+            for (int part = 0; part < 2; ++part) {
+                unsigned hi[16], rest[16];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        const float s0 = s[part * 32 + 2 * k], s1 = s[part * 32 + 2 * k + 1];
-                        float2 x;
-                        if constexpr (CAP) {
-                            x = make_float2(cap_out * tanh_fast(s0 * cap_in) - m_safe, cap_out * tanh_fast(s1 * cap_in) - m_safe);
-                            if (!inner) {
-                                if (s0 == -INFINITY) x.x = -INFINITY;
-                                if (s1 == -INFINITY) x.y = -INFINITY;
-                            }
-                        } else {
-                            x = fma2(make_float2(s0, s1), scale2, minus_m);
+                for (int k = 0; k < 16; ++k) {
+                    const float s0 = s[part * 32 + 2 * k], s1 = s[part * 32 + 2 * k + 1];
+                    float2 x;
+                    if constexpr (CAP) {
+                        x = make_float2(cap_out * tanh_fast(s0 * cap_in) - m_safe, cap_out * tanh_fast(s1 * cap_in) - m_safe);
+                        if (!inner) {
+                            if (s0 == -INFINITY) x.x = -INFINITY;
+                            if (s1 == -INFINITY) x.y = -INFINITY;
                         }
-                        const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                        sums[k & 1] = add2(sums[k & 1], p);
-                        hi[k] = pack2(p.x, p.y);
-                        const float2 r = as_float2(hi[k]);
-                        rest[k] = pack2(p.x - r.x, p.y - r.y);
+                    } else {
+                        x = fma2(make_float2(s0, s1), scale2, minus_m);
                     }
-                    tmem_st16(hi, ts + half * 64 + part * 16);
-                    tmem_st16(rest, ts + half * 64 + 32 + part * 16);
+                    const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                    sums[k & 1] = add2(sums[k & 1], p);
+                    hi[k] = pack2(p.x, p.y);
+                    const float2 r = fma2(as_float2(hi[k]), minus_one, p);  // (exact)
+                    rest[k] = pack2(r.x, r.y);
                 }
-            };
-            weights(1);
-            scores(0);  // (the first half's scores once more: both halves at once would not fit the registers)
-            weights(0);
+                tmem_st16(hi, ts + part * 16);
+                tmem_st16(rest, ts + 32 + part * 16);
+            }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(&bars->p_ready[2 * i + (t & 1)]);
             const float2 both = add2(sums[0], sums[1]);
             l += both.x + both.y;
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(&bars->p_ready[i]);
         }
-        if (ok) ok = mbar_wait_compact(&bars->o_done[i], 0);
+        if (ok) ok = mbar_wait_compact(&bars->o_done[i], (tiles - 1) & 1);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float f = l > 0.f ? 1.0f / l : 0.f;
@@ -418,6 +446,18 @@ attention_packed_kernel(const Inputs in, int* err) {
 }
 }  // namespace
 
+static int launch_packed(const Inputs& in, int num_seqs, int max_q_len, int* err, void* stream) {
+    const long long rows = (long long)max_q_len * (in.heads / in.kv_heads);
+    const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS), in.kv_heads, num_seqs);
+    static IePerDevice allowed, allowed_cap;
+    cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false>, SMEM_BYTES);
+    if (e == cudaSuccess && !FLAT) e = ie_allow_smem(allowed_cap, attention_packed_kernel<!FLAT>, SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    if (!FLAT && in.softcap > 0.f) return ie_launch(attention_packed_kernel<!FLAT>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+    return ie_launch(attention_packed_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+}
+
+#if !PA_FLAT
 // q: [tokens, heads, PA_D]; the caches [pages, kv_heads, page_size, PA_D or PA_DV]; out: rows of bfloat16 `out_ld` entries apart, 16-byte
 // aligned, out_ld a multiple of 8.
 IE_API int ie_attention_packed(const void* q, const void* k_cache, const void* v_cache, const int* tables, int table_width, const int* cu_q,
@@ -433,13 +473,25 @@ IE_API int ie_attention_packed(const void* q, const void* k_cache, const void* v
     int page_shift = 0;
     while ((1 << page_shift) < page_size) ++page_shift;
     const Inputs in{(const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, tables, cu_q, ctx_lens, table_width, heads, kv_heads,
-                    page_shift, total_pages, scale, window, keep_first, softcap, sinks, out_gate, gate_ld, gate_elements, (bf16*)out, out_ld};
-    const long long rows = (long long)max_q_len * (heads / kv_heads);
-    const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS), kv_heads, num_seqs);
-    static IePerDevice allowed, allowed_cap;
-    cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false>, SMEM_BYTES);
-    if (e == cudaSuccess) e = ie_allow_smem(allowed_cap, attention_packed_kernel<true>, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    if (softcap > 0.f) return ie_launch(attention_packed_kernel<true>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
-    return ie_launch(attention_packed_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+                    page_shift, total_pages, scale, window, keep_first, softcap, sinks, out_gate, gate_ld, gate_elements, (bf16*)out, out_ld,
+                    nullptr, nullptr, 0, 0, 0, 0};
+    return launch_packed(in, num_seqs, max_q_len, err, stream);
 }
+#else
+// Every head has keys and values of its own.  q: [tokens, heads, PA_D - 64]; q_rot: the first of a (token, head)'s `rot` rotated entries
+// (a multiple of 8 up to 64), q_rot_ld apart; kv: rows of kv_ld entries, all heads' keys (PA_D - 64 each), then all heads' values
+// (PA_DV each), a row per context position, request after request; k_rot: such a row's shared rotated entries, k_rot_ld apart; out:
+// [tokens, heads * PA_DV].  Everything 16-byte aligned, the distances multiples of 8.
+IE_API int ie_attention_flat(const void* q, const void* q_rot, int q_rot_ld, const void* kv, int kv_ld, const void* k_rot, int k_rot_ld, int rot,
+                             const int* cu_q, const int* ctx_lens, void* out, int num_seqs, int max_q_len, int heads, float scale,
+                             const float* sinks, const float* out_gate, int gate_ld, int* err, void* stream) {
+    if (num_seqs <= 0 || max_q_len <= 0) return 0;
+    if (heads <= 0 || rot < 0 || rot > 64 || rot % 8 || q_rot_ld % 8 || k_rot_ld % 8 || kv_ld % 8 || kv_ld < heads * (D - 64 + DV) ||
+        (((uintptr_t)q | (uintptr_t)q_rot | (uintptr_t)kv | (uintptr_t)k_rot | (uintptr_t)out) & 15))
+        return (int)cudaErrorInvalidValue;
+    const bf16* k = (const bf16*)kv;
+    const Inputs in{(const bf16*)q, k, k + (size_t)heads * (D - 64), nullptr, cu_q, ctx_lens, 0, heads, heads, 0, 0, scale, 0, 0, 0.f, sinks,
+                    out_gate, gate_ld, 0, (bf16*)out, heads * DV, (const bf16*)q_rot, (const bf16*)k_rot, q_rot_ld, k_rot_ld, kv_ld, rot};
+    return launch_packed(in, num_seqs, max_q_len, err, stream);
+}
+#endif

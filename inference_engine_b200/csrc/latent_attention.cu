@@ -382,6 +382,27 @@ int pick_headwise_mma(const void* x, long long x_ld, long long x_hs, const void*
     return split ? launch_headwise_mma<XT, 4, true>(IE_HM_ARGS) : launch_headwise_mma<XT, 4, false>(IE_HM_ARGS);
 #undef IE_HM_ARGS
 }
+
+// A warp per row: the cached rows of the step's requests, whole contexts one after the other, into an array without gaps.
+__global__ void __launch_bounds__(256)
+gather_context_rows_kernel(const uint4* __restrict__ cache, const int* __restrict__ tables, int table_width,
+                           const int* __restrict__ ctx_lens, int num_seqs, int total, int pieces, int page_shift, int total_pages,
+                           uint4* __restrict__ out, int* err) {
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= total) return;
+    int seq = 0, pos = row;
+    while (seq < num_seqs && pos >= ctx_lens[seq]) pos -= ctx_lens[seq++];
+    if (seq >= num_seqs) return;
+    const int page = tables[(size_t)seq * table_width + (pos >> page_shift)];
+    if (page < 0 || page >= total_pages) {
+        if (lane == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, row);
+        return;
+    }
+    const uint4* src = cache + (((size_t)page << page_shift) + (pos & ((1 << page_shift) - 1))) * pieces;
+    for (int i = lane; i < pieces; i += 32) out[(size_t)row * pieces + i] = src[i];
+}
 }  // namespace
 
 IE_API int ie_scale_head_rows(void* out, long long o_ld, long long o_hs, const float* scale, int N, int heads, int o,
@@ -445,4 +466,15 @@ IE_API int ie_headwise_linear(const void* x, long long x_ld, long long x_hs, con
                          x_hs, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_ld, o_hs, scale, N, heads, O, K);
     return ie_launch(headwise_linear_kernel<float>, grid, dim3(256), 0, s, (const float*)x, x_ld, x_hs,
                      (const float*)w, (float*)out, o_ld, o_hs, scale, N, heads, O, K);
+}
+
+// cache: bfloat16 [pages, page_size, row], row a multiple of 8; out: [total, row], the requests' contexts one after the other.
+IE_API int ie_gather_context_rows(const void* cache, const int* tables, int table_width, const int* ctx_lens, int num_seqs, int total,
+                                  int row, int page_size, int total_pages, void* out, int* err, void* stream) {
+    if (total <= 0) return 0;
+    if (row % 8 || page_size < 1 || (page_size & (page_size - 1)) || (((uintptr_t)cache | (uintptr_t)out) & 15)) return (int)cudaErrorInvalidValue;
+    int shift = 0;
+    while ((1 << shift) < page_size) ++shift;
+    return ie_launch(gather_context_rows_kernel, dim3((total + 7) / 8), dim3(256), 0, (cudaStream_t)stream, (const uint4*)cache, tables,
+                     table_width, ctx_lens, num_seqs, total, row / 8, shift, total_pages, (uint4*)out, err);
 }

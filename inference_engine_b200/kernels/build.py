@@ -185,6 +185,19 @@ def build_packed_attention(dim: int, vdim: int) -> Path:
     return build_library(f"ie_b200_packed_d{dim}_v{vdim}", ["attention_packed.cu"], [f"-DPA_D={dim}", f"-DPA_DV={vdim}"])
 
 
+# (unrotated key entries, value size) of latent attention heads whose expanded form it is built for -> its key size
+FLAT_ATTENTION_SIZES = {(64, 64): 128, (128, 128): 192}
+
+
+def build_flat_attention(dim: int, vdim: int) -> Path:
+    """The same for latent attention whose keys (``dim`` entries of a head's own and up to 64 shared ones) and values were
+    expanded per head."""
+    if (dim, vdim) not in FLAT_ATTENTION_SIZES:
+        raise BuildError(f"the expanded latent attention takes sizes {tuple(FLAT_ATTENTION_SIZES)}, not {dim} and {vdim}")
+    return build_library(f"ie_b200_flat_d{dim}_v{vdim}", ["attention_packed.cu"],
+                         [f"-DPA_D={FLAT_ATTENTION_SIZES[dim, vdim]}", f"-DPA_DV={vdim}", "-DPA_FLAT=1"])
+
+
 def build_retention(dim: int, vdim: int) -> Path:
     """The bfloat16 path's retention kernels for one pair of key and value sizes, each rounded up to a
     multiple of 16 (compiled on first use for the sizes the loaded model has)."""
@@ -256,6 +269,7 @@ def build_all(prune: bool = True) -> list[Path]:
                  build_sink_attention(64, 64, "log"), build_sink_attention(64, 64, "table"),
                  build_retention(64, 64), build_state_space(64, 64), build_latent_attention(320, 256)]
         libs += list(pool.map(lambda sizes: build_packed_attention(*sizes), PACKED_ATTENTION_SIZES))
+        libs += list(pool.map(lambda sizes: build_flat_attention(*sizes), FLAT_ATTENTION_SIZES))
     if prune:
         keep = {lib.name for lib in libs}
         for old in build_dir().glob("libie_b200_*.so"):

@@ -18,8 +18,8 @@ import os
 from ctypes import c_float, c_int, c_void_p
 from typing import Any
 
-from .build import (ATTENTION_HEAD_DIMS, PACKED_ATTENTION_SIZES, build_attention, build_core, build_latent_attention,
-                    build_packed_attention, build_part_library, build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
+from .build import (ATTENTION_HEAD_DIMS, FLAT_ATTENTION_SIZES, PACKED_ATTENTION_SIZES, build_attention, build_core,
+                    build_flat_attention, build_latent_attention, build_packed_attention, build_part_library, build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
                     latent_attention_fits)
 
 _ERRORS = {
@@ -148,6 +148,9 @@ class CudaOps:
         self.sink_mma = os.environ.get("IE_B200_SINK_MMA", "1") != "0"  # tensor-core sink attention
         self.sink_tc5 = os.environ.get("IE_B200_SINK_TC5", "1") != "0"  # ... of prompt portions on tcgen05
         self._packed_libs: dict[tuple[int, int], object] = {}
+        self._flat_libs: dict[tuple[int, int], object] = {}
+        # the latent attention of prompts with keys and values expanded per head ("0": always moved to the query side)
+        self.latent_expand = os.environ.get("IE_B200_LATENT_EXPAND", "1") != "0"
         # residual gates' products as partial sums: faster by themselves, slower inside a captured step
         self.gate_split = os.environ.get("IE_B200_GATE_SPLIT", "0") == "1"
         self.sigmoid_mma = os.environ.get("IE_B200_SIGMOID_MMA", "1") != "0"  # tensor-core sigmoid attention
@@ -971,6 +974,79 @@ class CudaOps:
             v_cache.shape[-1], page_size, k_cache.shape[0], scale, window, 0, None, self._ptr(sinks), None, 0, 0.0, 0,
             *self._NO_BIAS, nh * value_dim, self._err_ptr, self._stream()), "paged_attention_latent")
 
+    def latent_expands(self, ctx, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> bool:
+        """Whether a step's latent attention runs on keys and values expanded per head.  Moved to the query side a (query, key) pair
+        costs ``2 * rank + rot_dim`` products a head (the second half twice, for the weights' two terms) on ``mma.sync``;
+        expanded ``dim + rot_dim + vdim`` on tcgen05, after a product over every token of the requests' contexts.  So prompts
+        and long portions do (2,048 tokens of 16 heads: 557 us against 75), decoding requests, whose contexts are long and whose
+        pairs are few, do not.  The estimates: 190 TFLOP/s moved; 900 for the expansion, 350 for its attention and 20 us of
+        launches.  Captured steps of any lengths (``bounds``) know no contexts and do not."""
+        starts = getattr(ctx, "start_positions", None)
+        if (not self.latent_expand or getattr(ctx, "bounds", None) is not None or starts is None or (dim, vdim) not in FLAT_ATTENTION_SIZES
+                or rot_dim % 8 or rot_dim > 64 or rank % 64 or ctx.max_q_len < 64):
+            return False
+        context = pairs = 0
+        for a, n in zip(starts, ctx.q_lens):
+            context += a + n
+            pairs += n * (2 * a + n) // 2
+        if context * heads * (dim + vdim) > 1 << 30:  # (2 GB of expanded keys and values)
+            return False
+        moved = pairs * heads * (3 * rank + rot_dim) * 2 / 190e6
+        return moved > context * rank * heads * (dim + vdim) * 2 / 900e6 + pairs * heads * (dim + rot_dim + 2 * vdim) * 2 / 350e6 + 20
+
+    def _flat_lib(self, dim: int, vdim: int):
+        lib = self._flat_libs.get((dim, vdim))
+        if lib is None:
+            path = build_flat_attention(dim, vdim)
+            try:
+                lib = ctypes.CDLL(str(path))
+            except OSError as exc:
+                raise KernelError(f"the kernel library {path} could not be loaded: {exc}") from exc
+            P, I, F = c_void_p, c_int, c_float
+            lib.ie_attention_flat.argtypes = [P, P, I, P, I, P, I, I, P, P, P, I, I, I, F, P, P, I, P, P]
+            lib.ie_attention_flat.restype = c_int
+            self._flat_libs[(dim, vdim)] = lib
+        return lib
+
+    @_kind("latent.gather")
+    def _gather_context_rows(self, cache, block_tables, ctx, page_size, out) -> None:
+        self._check(self._part_lib("latent").ie_gather_context_rows(
+            cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], ctx.ctx_lens.data_ptr(), ctx.num_seqs, out.shape[0],
+            out.shape[1], page_size, cache.shape[0], out.data_ptr(), self._err_ptr, self._stream()), "gather_context_rows")
+
+    def latent_expanded(self, q, w_kv, cache, block_tables, ctx, positions, table, rot_dims, out, *, heads, dim, rot_dim, vdim, rank,
+                        page_size, interleaved, scale, gate_pre, sinks, ws) -> None:
+        """The latent attention with keys and values expanded per head (``latent_expands`` says when): ``q`` as for
+        :meth:`latent_queries`; ``w_kv`` ``[heads * (dim + vdim), rank]``, all heads' key rows, then all heads' value rows; ``cache``
+        holds the step's own rows too; ``gate_pre`` (a 32-bit view ``[N, heads]`` or None) and ``sinks`` as for the attentions;
+        ``out``: ``[N, heads * vdim]``, gated."""
+        n, row = positions.shape[0], rank + rot_dim
+        plain = ws.buffer("latent.q_plain", n, heads * dim, out.dtype)
+        turned = ws.buffer("latent.q", n, heads * row, out.dtype)  # (its rotated entries alone are written)
+        self.latent_prep(positions, table, rot_dims, heads=heads, dim=dim, rot_dim=rot_dim, rank=rank, page_size=page_size,
+                         interleaved=interleaved, q=q, q_plain=plain, q_abs=turned)
+        total = sum(ctx.start_positions) + sum(ctx.q_lens)
+        rows = ws.buffer("latent.context", total, row, out.dtype, rows_cap=None)
+        self._gather_context_rows(cache, block_tables, ctx, page_size, rows)
+        kv = ws.buffer("latent.expanded", total, heads * (dim + vdim), out.dtype, rows_cap=None)
+        self._expand_latent(rows[:, :rank], w_kv, kv)
+        self._flat_attention(plain, turned[:, rank:], row, kv, rows[:, rank:], row, rot_dim, ctx, out, heads, dim, vdim, scale, sinks,
+                             gate_pre)
+
+    @_kind("latent.headwise")
+    def _expand_latent(self, latent, w_kv, out) -> None:
+        self.torch.mm(latent, w_kv.t(), out=out)
+
+    @_kind("attention.latent")
+    def _flat_attention(self, q, q_rot, q_rot_ld, kv, k_rot, k_rot_ld, rot_dim, ctx, out, heads, dim, vdim, scale, sinks, gate_pre) -> None:
+        if gate_pre is not None and (gate_pre.dtype != self.torch.float32 or gate_pre.dim() != 2 or gate_pre.stride(1) != 1):
+            raise KernelError("latent_expanded: the gate must be a 32-bit view with unit stride")
+        self._check(self._flat_lib(dim, vdim).ie_attention_flat(
+            q.data_ptr(), q_rot.data_ptr(), q_rot_ld, kv.data_ptr(), kv.shape[1], k_rot.data_ptr(), k_rot_ld, rot_dim,
+            ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, ctx.max_q_len, heads, scale,
+            self._ptr(sinks), self._ptr(gate_pre), 0 if gate_pre is None else gate_pre.stride(0), self._err_ptr,
+            self._stream()), "latent_attention_expanded")
+
     # --- kernels of single mixers and feed-forwards (libraries built on first use) -------------
 
     _PART_SIGNATURES = {
@@ -979,6 +1055,7 @@ class CudaOps:
             "ie_headwise_linear": "P L L P P L L P I I I I I P",
             "ie_scale_head_rows": "P L L P I I I P",
             "ie_headwise_mma_ok": "I",
+            "ie_gather_context_rows": "P P I P I I I I I P P P",
             "ie_headwise_mma": "P I L L P P L L P I I I I I L P P I I I I I I P P",
         },
         "delta": {

@@ -20,7 +20,8 @@ token and layer, shared by the heads).  The products with ``W_uk`` and ``W_uv`` 
 query side: ``q_unrotated[n] . (W_uk[n] c) = (W_uk[n]^T q_unrotated[n]) . c``, and
 ``sum_j p_j W_uv[n] c_j = W_uv[n] sum_j p_j c_j``.  So the attention runs with one shared
 key/value head whose key rows are the cached rows and whose value rows are their first
-``kv_rank`` entries, in prompts and in decoding alike, and nothing is expanded per cached token.
+``kv_rank`` entries, and nothing is expanded per cached token.  Prompts and long portions in bfloat16, whose
+pairs of query and key cost more than their tokens, expand keys and values per head instead (``ops.latent_expands``).
 """
 
 from __future__ import annotations
@@ -93,7 +94,9 @@ class LatentAttention(Mixer):
         self.latent_norm = tensors[n["latent_norm"]].float().contiguous()
         uk = tensors[n["uk"]].to(self.dtype).view(self.heads, self.dim, self.kv_rank)
         self.w_uk_t = uk.transpose(1, 2).contiguous()  # [heads, kv_rank, dim]: query side of the key product
-        self.w_uv = tensors[n["uv"]].to(self.dtype).view(self.heads, self.vdim, self.kv_rank).contiguous()
+        # keys' rows, then values' rows: the map that expands a cached latent per head
+        self.w_kv = torch.cat([uk.reshape(-1, self.kv_rank), tensors[n["uv"]].to(self.dtype)]).contiguous()
+        self.w_uv = self.w_kv[self.heads * self.dim:].view(self.heads, self.vdim, self.kv_rank)
         self.w_o = tensors[n["o"]].to(self.dtype).contiguous()
         if "sink" in n:
             self.sinks = tensors[n["sink"]].float().contiguous()
@@ -127,12 +130,19 @@ class LatentAttention(Mixer):
         q = proj[..., : self.q_size]
         if cq is not None:
             q = ops.linear(cq, self.w_uq, ws=ws, tag="latent.uq", out_dtype=torch.float32, allow_split=True)
+        out = ws.buffer("latent.out", n, H * self.vdim, self.dtype)
+        expands = getattr(ops, "latent_expands", None)
+        if (expands is not None and self.dtype == torch.bfloat16 and proj.dim() == 2
+                and expands(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank)):
+            gates = proj[:, at + self.row: at + self.row + H] if gate is not None else None
+            ops.latent_expanded(q, self.w_kv, cache, group.block_tables, ctx, ctx.positions, table, rot_dims, out, vdim=self.vdim,
+                                scale=self.scale, gate_pre=gates, sinks=self.sinks, ws=ws, **sizes)
+            return ops.linear(out, self.w_o, ws=ws, tag="mixer.delta", out_dtype=torch.float32, allow_split=True)
         q_abs = ws.buffer("latent.q", n, H * self.row, self.dtype)
         ops.latent_queries(q, self.w_uk_t, q_abs, ctx.positions, table, rot_dims, **sizes, ws=ws)
         mixed = ws.buffer("latent.mixed", n, H * self.kv_rank, self.dtype)
         ops.paged_attention(q_abs, cache, cache, group.block_tables, ctx, H, 1, self.row,
                             group.page_size, self.scale, 0, mixed, ragged=group.ragged,
                             value_dim=self.kv_rank, sinks=self.sinks)
-        out = ws.buffer("latent.out", n, H * self.vdim, self.dtype)
         ops.headwise_linear(mixed.view(n, H, self.kv_rank), self.w_uv, out.view(n, H, self.vdim), row_scale=gate)
         return ops.linear(out, self.w_o, ws=ws, tag="mixer.delta", out_dtype=torch.float32, allow_split=True)
