@@ -169,50 +169,47 @@ attention_packed_kernel(const Inputs in, int* err) {
         const unsigned qa = smem_u32(q_s), ka = smem_u32(k_s), va = smem_u32(v_s);
         const bool one = elect_one();
         bool ok = mbar_wait_compact(&bars->q_full, 0);
-        // the scores of key tile t for both row tiles.  (What their columns held, the weights of tile t - 2, went into products that
-        // this thread issued before: they are done before these write.)
-        auto scores = [&](int t) {
+        // The scores of row tile i and key tile t.  Their columns held the weights of tile t - 2: the product that read them must be done
+        // (products into different accumulators are not ordered by their issue).
+        auto scores = [&](int i, int t) {
+            if (t >= tiles) return true;
             const int slot = t % KS;
-            if (!mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
+            if ((t >= 2 && !mbar_wait_compact(&bars->o_done[i], t & 1)) || !mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (one) {
+                const unsigned qt = qa + i * Q_TILE, kt = ka + slot * K_BYTES;
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const unsigned qt = qa + i * Q_TILE, kt = ka + slot * K_BYTES;
-#pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
-                        umma_ss(tmem + (2 * i + (t & 1)) * KT, umma_desc_sw128(qt + (ks >> 2) * Q_RUN + (ks & 3) * 32),
-                                umma_desc_sw128(kt + (ks >> 2) * KV_RUN + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
-                    umma_commit(&bars->s_done[2 * i + (t & 1)]);
-                }
-                umma_commit(&bars->k_empty[slot]);
+                for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
+                    umma_ss(tmem + (2 * i + (t & 1)) * KT, umma_desc_sw128(qt + (ks >> 2) * Q_RUN + (ks & 3) * 32),
+                            umma_desc_sw128(kt + (ks >> 2) * KV_RUN + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
+                umma_commit(&bars->s_done[2 * i + (t & 1)]);
+                if (i == 1) umma_commit(&bars->k_empty[slot]);
             }
             __syncwarp();
             return true;
         };
-        ok = ok && scores(0);
-        for (int t = 0; t < tiles && ok; ++t) {
-            if (t + 1 < tiles) ok = scores(t + 1);
+        // O_i += P V of key tile t
+        auto values = [&](int i, int t) {
             const int slot = t % VS;
-            ok = ok && mbar_wait_compact(&bars->v_full[slot], (t / VS) & 1);
+            if ((i == 0 && !mbar_wait_compact(&bars->v_full[slot], (t / VS) & 1)) ||
+                !mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (one) {
+                const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * V_BYTES;
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                ok = ok && mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (one) {
-                    const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * V_BYTES;
+                for (int term = 0; term < TERMS; ++term)
 #pragma unroll
-                    for (int term = 0; term < TERMS; ++term)
-#pragma unroll
-                        for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
-                            umma_ta(o, p + term * 32 + ks * 8, desc_mn(vt + ks * 2048, KV_RUN), idesc_pv, t > 0 || term > 0 || ks > 0 ? 1u : 0u);
-                    umma_commit(&bars->o_done[i]);
-                    if (i == 1) umma_commit(&bars->v_empty[slot]);
-                }
-                __syncwarp();
+                    for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
+                        umma_ta(o, p + term * 32 + ks * 8, desc_mn(vt + ks * 2048, KV_RUN), idesc_pv, t > 0 || term > 0 || ks > 0 ? 1u : 0u);
+                umma_commit(&bars->o_done[i]);
+                if (i == 1) umma_commit(&bars->v_empty[slot]);
             }
-        }
+            __syncwarp();
+            return true;
+        };
+        ok = ok && scores(0, 0) && scores(1, 0) && scores(0, 1);
+        // (a row tile's scores follow the other's second product: the product they wait for is the one before that)
+        for (int t = 0; t < tiles && ok; ++t) ok = (t > 0 || scores(1, 1)) && values(0, t) && (t == 0 || scores(1, t + 1)) && values(1, t) && scores(0, t + 2);
         if (!ok) bars->failed = 1;
     } else if (warp > SOFTMAX_WARPS) {
         // ---- copies: eight threads to a row of 128 bytes, eight rows at a time ----
@@ -220,27 +217,32 @@ attention_packed_kernel(const Inputs in, int* err) {
         const unsigned to = (unsigned)(r0 * 128 + ((chunk ^ (r0 & 7)) << 4));  // (r0 + 8 p: the same place in its group of eight rows)
         constexpr int AT_ONCE = COPY_WARPS * 4, PASSES = KT / AT_ONCE;
         static_assert(AT_ONCE == 8, "rows at a time");
-        // what was asked for last and not announced yet
-        unsigned long long* pending = nullptr;
-        auto announce = [&](unsigned long long* bar) {
+        // Groups of copies in the order in which they are asked for: the queries, then keys and values of every tile in turn.  A group is
+        // announced when DEPTH more have been asked for, or when a slot is not free yet (it may wait for what is on its way): one group
+        // ahead left the memory's latency between any two.
+        constexpr int DEPTH = 4;
+        int asked_for = 0, announced = 0;
+        auto announce = [&]() {
+            const int g = announced++ - 1;  // (0: the queries)
+            unsigned long long* bar = g < 0 ? &bars->q_full : g & 1 ? &bars->v_full[(g >> 1) % VS] : &bars->k_full[(g >> 1) % KS];
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
-        auto settle = [&](bool all) {  // the copies before the last group have landed, or all of them
-            if (all) asm volatile("cp.async.wait_group 0;" ::: "memory");
-            else asm volatile("cp.async.wait_group 1;" ::: "memory");
-            if (pending != nullptr) announce(pending);
-            pending = nullptr;
-        };
-        auto asked = [&](unsigned long long* bar) {
+        auto asked = [&]() {
             asm volatile("cp.async.commit_group;" ::: "memory");
-            settle(false);
-            pending = bar;
+            if (++asked_for - announced > DEPTH) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH) : "memory");
+                announce();
+            }
         };
-        // a slot that is not free yet: whatever is on its way is announced before the wait, since the slot may depend on it
+        auto settle = [&]() {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            while (announced < asked_for) announce();
+        };
         auto slot_free = [&](unsigned long long* bar, int parity) {
-            settle(true);
+            if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+            settle();
             return mbar_wait_compact(bar, parity);
         };
         {
@@ -261,13 +263,24 @@ attention_packed_kernel(const Inputs in, int* err) {
                     }
                 }
             }
-            asked(&bars->q_full);
+            asked();
         }
         const int* table = FLAT ? nullptr : in.tables + (size_t)seq * in.table_width;
         int before = 0;  // FLAT: rows of the requests before this one
         if (FLAT)
             for (int i = 0; i < seq; ++i) before += in.ctx_lens[i];
         bool ok = true;
+        // the pages of the thread's keys, looked up a tile ahead
+        int page_of[PASSES];
+        auto look_up = [&](int t) {
+            const int key0 = key_of(t);
+#pragma unroll
+            for (int p = 0; p < PASSES; ++p) {
+                const int pos = key0 + r0 + AT_ONCE * p;
+                page_of[p] = (pos >= lo_min || pos < in.keep_first) && pos <= last_pos ? table[pos >> in.page_shift] : 0;
+            }
+        };
+        if (!FLAT) look_up(0);
         for (int t = 0; t < tiles; ++t) {
             const int key0 = key_of(t);
             int row[PASSES];  // the row of each of the thread's keys; -1: nothing there (reads as zero)
@@ -279,7 +292,7 @@ attention_packed_kernel(const Inputs in, int* err) {
                     if (FLAT) {
                         row[p] = before + pos;
                     } else {
-                        const int page = table[pos >> in.page_shift];
+                        const int page = page_of[p];
                         if (page < 0 || page >= in.total_pages) {
                             if (chunk == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
                         } else {
@@ -288,6 +301,7 @@ attention_packed_kernel(const Inputs in, int* err) {
                     }
                 }
             }
+            if (!FLAT && t + 1 < tiles) look_up(t + 1);
             const int ks = t % KS, vs = t % VS;
             if (t >= KS && !slot_free(&bars->k_empty[ks], (t / KS - 1) & 1)) { ok = false; break; }
             unsigned dst = smem_u32(k_s) + ks * K_BYTES + to;
@@ -305,7 +319,7 @@ attention_packed_kernel(const Inputs in, int* err) {
                     }
                 }
             }
-            asked(&bars->k_full[ks]);
+            asked();
             if (t >= VS && !slot_free(&bars->v_empty[vs], (t / VS - 1) & 1)) { ok = false; break; }
             dst = smem_u32(v_s) + vs * V_BYTES + to;
 #pragma unroll
@@ -315,9 +329,9 @@ attention_packed_kernel(const Inputs in, int* err) {
 #pragma unroll
                 for (int h = 0; h < VH; ++h) cp16(dst + p * 1024 + h * KV_RUN, src + h * 64, row[p] >= 0 ? 16 : 0);
             }
-            asked(&bars->v_full[vs]);
+            asked();
         }
-        settle(true);
+        settle();
         if (!ok) bars->failed = 1;
     } else {
         // ---- softmax: thread = row = tensor-memory lane ----
