@@ -66,15 +66,21 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
     return p != 0;
 }
-// B with its N entries contiguous (values: 64 entries to 128 bytes, runs of 64 `run` bytes apart, eight keys to 1,024 bytes).
-__device__ __forceinline__ unsigned long long desc_mn(unsigned addr, unsigned run) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((addr >> 4) & 0x3FFF);
-    d |= (unsigned long long)((run >> 4) & 0x3FFF) << 16;
-    d |= (unsigned long long)64 << 32;
-    d |= (unsigned long long)1 << 46;
-    d |= (unsigned long long)2 << 61;
-    return d;
+// Shared-memory descriptors as their two words: the low one (start address and, for values, the distance of the runs, in 16-byte units)
+// moves with the address, the high one (groups of eight rows 1,024 bytes apart, version, 128-byte swizzle) is a constant.  An instruction
+// then costs an addition an operand; descriptors put together anew for each cost the issuing warp 100 clocks an instruction beside
+// the softmax warps, where the tensor core needs 48 and 65.
+constexpr unsigned DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ unsigned desc_low(unsigned addr, unsigned run) { return (addr >> 4) | ((run >> 4) << 16); }
+__device__ __forceinline__ void mma_ss(unsigned d, unsigned a, unsigned b, unsigned idesc, bool accumulate) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
+                 ::"r"(d), "r"(a), "r"(b), "r"(DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_ts(unsigned d, unsigned a, unsigned b, unsigned idesc, bool accumulate) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 y;\n setp.ne.b32 p, %5, 0;\n mov.b64 y, {%2, %3};\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}"
+                 ::"r"(d), "r"(a), "r"(b), "r"(DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
 }
 __device__ __forceinline__ void cp16(unsigned dst, const void* src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -127,7 +133,8 @@ attention_packed_kernel(const Inputs in, int* err) {
     unsigned char* k_s = q_s + Q_BYTES;             // [slot][run][128 keys][128 bytes]
     unsigned char* v_s = k_s + KS * K_BYTES;
     Bars* bars = reinterpret_cast<Bars*>(v_s + VS * V_BYTES);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (one number for the whole warp, as far as the compiler is concerned)
     ie_pdl_trigger();
     // (lengths and block tables are the step's inputs; queries, keys and values are the kernels' before)
     const int seq = blockIdx.z, kvh = blockIdx.y, group = in.heads / in.kv_heads;
@@ -160,13 +167,13 @@ attention_packed_kernel(const Inputs in, int* err) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem = bars->tmem_base;
+    const unsigned tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
     ie_pdl_wait();
 
     if (warp == SOFTMAX_WARPS) {
         // ---- tensor core ----
         const unsigned idesc_qk = umma_idesc_bf16(BM, KT), idesc_pv = umma_idesc_bf16(BM, DV) | (1u << 16);
-        const unsigned qa = smem_u32(q_s), ka = smem_u32(k_s), va = smem_u32(v_s);
+        const unsigned qa = desc_low(smem_u32(q_s), 1024), ka = desc_low(smem_u32(k_s), 1024), va = desc_low(smem_u32(v_s), KV_RUN);
         const bool one = elect_one();
         bool ok = mbar_wait_compact(&bars->q_full, 0);
         // The scores of row tile i and key tile t.  Their columns held the weights of tile t - 2: the product that read them must be done
@@ -177,11 +184,10 @@ attention_packed_kernel(const Inputs in, int* err) {
             if ((t >= 2 && !mbar_wait_compact(&bars->o_done[i], t & 1)) || !mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (one) {
-                const unsigned qt = qa + i * Q_TILE, kt = ka + slot * K_BYTES;
+                const unsigned qt = qa + i * (Q_TILE >> 4), kt = ka + slot * (K_BYTES >> 4), st = tmem + (2 * i + (t & 1)) * KT;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
-                    umma_ss(tmem + (2 * i + (t & 1)) * KT, umma_desc_sw128(qt + (ks >> 2) * Q_RUN + (ks & 3) * 32),
-                            umma_desc_sw128(kt + (ks >> 2) * KV_RUN + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
+                    mma_ss(st, qt + (((ks >> 2) * Q_RUN + (ks & 3) * 32) >> 4), kt + (((ks >> 2) * KV_RUN + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
                 umma_commit(&bars->s_done[2 * i + (t & 1)]);
                 if (i == 1) umma_commit(&bars->k_empty[slot]);
             }
@@ -195,12 +201,12 @@ attention_packed_kernel(const Inputs in, int* err) {
                 !mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (one) {
-                const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * V_BYTES;
+                const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * (V_BYTES >> 4);
 #pragma unroll
                 for (int term = 0; term < TERMS; ++term)
 #pragma unroll
                     for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
-                        umma_ta(o, p + term * 32 + ks * 8, desc_mn(vt + ks * 2048, KV_RUN), idesc_pv, t > 0 || term > 0 || ks > 0 ? 1u : 0u);
+                        mma_ts(o, p + term * 32 + ks * 8, vt + ks * (2048 >> 4), idesc_pv, term > 0 || ks > 0 || t > 0);
                 umma_commit(&bars->o_done[i]);
                 if (i == 1) umma_commit(&bars->v_empty[slot]);
             }
