@@ -165,6 +165,173 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
         }
     }
 }
+
+// The same attention for prompt portions in 32-bit (plain softmax, all positions or a window): a block takes 32 (token, query head of the
+// group) rows of one request and key/value head and brings a tile of 32 keys once for all of them, where the kernel above reads a key
+// row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 72).  Every number is the same chain of operations as there: a
+// score one multiply-add after the other over the row, maxima and sums over a tile's 32 keys by the same exchanges (a warp
+// takes a row, a lane a key), the output's multiply-adds key by key; tiles a row does not see leave it as it is (its maximum stays, a factor
+// of 1, weights of 0).  So results are equal bit for bit, and a portion may be cut anywhere between the two kernels.
+constexpr int T_ROWS = 32, T_KEYS = 32, T_THREADS = 128;
+template <int HD>
+__global__ void __launch_bounds__(T_THREADS)
+paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+                                const int* __restrict__ block_tables, int table_width, const int* __restrict__ cu_q,
+                                const int* __restrict__ ctx_lens, float* __restrict__ out, int nh, int nkv, int page_size, int total_pages,
+                                float scale, int window, int* err) {
+    constexpr int LD = HD + 4, LP = T_KEYS + 4;
+    extern __shared__ __align__(16) float tile_smem[];
+    float* qs = tile_smem;             // [32][LD]
+    float* ks = qs + T_ROWS * LD;      // two of [32][LD]
+    float* vs = ks + 2 * T_KEYS * LD;  // two of [32][HD]
+    float* ps = vs + 2 * T_KEYS * HD;  // [32][LP]: scores, then weights
+    float* alpha_s = ps + T_ROWS * LP; // [32]
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    const int seq = blockIdx.z, kvh = blockIdx.y, group = nh / nkv, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int q0 = cu_q[seq], q_len = cu_q[seq + 1] - q0, row0 = (gridDim.x - 1 - blockIdx.x) * T_ROWS, rows_total = q_len * group;
+    if (row0 >= rows_total) return;
+    const int start = ctx_lens[seq] - q_len, rows_here = min(T_ROWS, rows_total - row0);
+    const int first_pos = start + row0 / group, last_pos = start + (row0 + rows_here - 1) / group;
+    const int lo_min = window > 0 ? max(first_pos - window + 1, 0) : 0;
+    const int* table = block_tables + (size_t)seq * table_width;
+    auto fetch = [&](int t0, int b) {  // four threads a key
+        const int key = tid >> 2, pos = t0 + key;
+        int row = -1;
+        if (pos >= lo_min && pos <= last_pos) {
+            const int page = table[pos / page_size];
+            if (page < 0 || page >= total_pages) {
+                if ((tid & 3) == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
+            } else {
+                row = (page * nkv + kvh) * page_size + pos % page_size;
+            }
+        }
+        const float* kr = k_cache + (size_t)max(row, 0) * HD;
+        const float* vr = v_cache + (size_t)max(row, 0) * HD;
+#pragma unroll
+        for (int c = (tid & 3) * 4; c < HD; c += 16) {
+            const int bytes = row >= 0 ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(ks + (b * T_KEYS + key) * LD + c)), "l"(kr + c), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(vs + (b * T_KEYS + key) * HD + c)), "l"(vr + c), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int t_first = lo_min / T_KEYS * T_KEYS;
+    fetch(t_first, 0);
+    for (int i = tid; i < T_ROWS * HD / 4; i += T_THREADS) {
+        const int r = i / (HD / 4), c = (i % (HD / 4)) * 4, rr = row0 + r, token = rr / group;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows_here) v = *reinterpret_cast<const float4*>(q + ((size_t)(q0 + token) * nh + kvh * group + rr - token * group) * HD + c);
+        *reinterpret_cast<float4*>(qs + r * LD + c) = v;
+    }
+    // scores: 4 rows (8 apart) x 2 keys (16 apart) a thread; softmax: a warp every fourth row; output: 32 * HD / 128 numbers a thread
+    const int sr = tid >> 4, sk = tid & 15;
+    constexpr int DL = HD / 4, RG = T_THREADS / DL, OR = T_ROWS / RG;  // lanes across a row, rows at once, rows of a thread
+    const int od = (tid % DL) * 4, orow = tid / DL;
+    float m[T_ROWS / 4], l[T_ROWS / 4];
+#pragma unroll
+    for (int i = 0; i < T_ROWS / 4; ++i) { m[i] = -INFINITY; l[i] = 0.f; }
+    float acc[OR][4];
+#pragma unroll
+    for (int i = 0; i < OR; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    int b = 0;
+    for (int t0 = t_first; t0 <= last_pos; t0 += T_KEYS, b ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the tile has landed, and everyone is done with the other one and with the weights
+        if (t0 + T_KEYS <= last_pos) fetch(t0 + T_KEYS, b ^ 1);
+        {
+            const float* kt = ks + b * T_KEYS * LD;
+            float s[4][2] = {};
+#pragma unroll 4
+            for (int d = 0; d < HD; d += 4) {
+                float4 x[4], y[2];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(qs + (sr + 8 * i) * LD + d);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) y[j] = *reinterpret_cast<const float4*>(kt + (sk + 16 * j) * LD + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        s[i][j] = fmaf(x[i].x, y[j].x, s[i][j]); s[i][j] = fmaf(x[i].y, y[j].y, s[i][j]);
+                        s[i][j] = fmaf(x[i].z, y[j].z, s[i][j]); s[i][j] = fmaf(x[i].w, y[j].w, s[i][j]);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) ps[(sr + 8 * i) * LP + sk + 16 * j] = s[i][j] * scale;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < T_ROWS / 4; ++i) {
+            const int r = warp + 4 * i;
+            if (r < rows_here) {
+                const int pos = start + (row0 + r) / group, lo = window > 0 ? max(pos - window + 1, 0) : 0, kpos = t0 + lane;
+                const bool valid = kpos >= lo && kpos <= pos;
+                const float s = valid ? ps[r * LP + lane] : -INFINITY;
+                const float m_new = fmaxf(m[i], warp_max(s));
+                const float p = valid ? expf(s - m_new) : 0.f;
+                const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+                l[i] = fmaf(l[i], alpha, warp_sum(p));
+                m[i] = m_new;
+                ps[r * LP + lane] = p;
+                if (lane == 0) alpha_s[r] = alpha;
+            }
+        }
+        __syncthreads();
+        const float* vt = vs + b * T_KEYS * HD + od;
+#pragma unroll
+        for (int i = 0; i < OR; ++i) {
+            const float a = alpha_s[orow + RG * i];
+            acc[i][0] *= a; acc[i][1] *= a; acc[i][2] *= a; acc[i][3] *= a;
+        }
+#pragma unroll 2
+        for (int j = 0; j < T_KEYS; j += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = *reinterpret_cast<const float4*>(vt + (j + k) * HD);
+#pragma unroll
+            for (int i = 0; i < OR; ++i) {
+                const float4 p = *reinterpret_cast<const float4*>(ps + (orow + RG * i) * LP + j);
+                const float pv[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    acc[i][0] = fmaf(pv[k], v[k].x, acc[i][0]); acc[i][1] = fmaf(pv[k], v[k].y, acc[i][1]);
+                    acc[i][2] = fmaf(pv[k], v[k].z, acc[i][2]); acc[i][3] = fmaf(pv[k], v[k].w, acc[i][3]);
+                }
+            }
+        }
+    }
+    __syncthreads();  // (the last tile's factors have been read)
+#pragma unroll
+    for (int i = 0; i < T_ROWS / 4; ++i) {
+        const int r = warp + 4 * i;
+        if (lane == 0 && r < rows_here) alpha_s[r] = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < OR; ++i) {
+        const int r = orow + RG * i, rr = row0 + r, token = rr / group;
+        if (r >= rows_here) continue;
+        const float f = alpha_s[r];
+        *reinterpret_cast<float4*>(out + ((size_t)(q0 + token) * nh + kvh * group + rr - token * group) * HD + od) =
+            make_float4(acc[i][0] * f, acc[i][1] * f, acc[i][2] * f, acc[i][3] * f);
+    }
+}
+
+template <int HD>
+int launch_f32_tile(const float* q, const float* k, const float* v, const int* tables, int width, const int* cu_q, const int* ctx_lens,
+                    float* out, int num_seqs, int max_q_len, int nh, int nkv, int page_size, int total_pages, float scale, int window,
+                    int* err, cudaStream_t s) {
+    constexpr size_t smem = (size_t)(T_ROWS * (HD + 4) + 2 * T_KEYS * (HD + 4) + 2 * T_KEYS * HD + T_ROWS * (T_KEYS + 4) + T_ROWS) * sizeof(float);
+    static IePerDevice allowed;
+    cudaError_t e = ie_allow_smem(allowed, paged_attention_f32_tile_kernel<HD>, smem);
+    if (e != cudaSuccess) return (int)e;
+    const dim3 grid((unsigned)(((long long)max_q_len * (nh / nkv) + T_ROWS - 1) / T_ROWS), nkv, num_seqs);
+    return ie_launch(paged_attention_f32_tile_kernel<HD>, grid, dim3(T_THREADS), smem, s, q, k, v, tables, width, cu_q, ctx_lens, out, nh,
+                     nkv, page_size, total_pages, scale, window, err);
+}
 }  // namespace
 
 IE_API int ie_paged_attention_generic(const void* q, const void* k_cache, const void* v_cache,
@@ -197,4 +364,21 @@ IE_API int ie_paged_attention_generic(const void* q, const void* k_cache, const 
             nh, nkv, hd, hdv, v_stride, page_size, total_pages, scale, window, chunk, head_bias, sinks, out_gate, gate_ld, softcap, keep_first,
             gate_elements, log_r1, log_r2, bias_table, bias_len, out_ld, err);
     return IE_LAUNCH_CHECK();
+}
+
+// 32-bit prompt portions with rows of 32, 64 or 128 entries; everything 16-byte aligned.
+IE_API int ie_paged_attention_f32_tiles(const float* q, const float* k_cache, const float* v_cache, const int* tables, int table_width,
+                                        const int* cu_q, const int* ctx_lens, float* out, int num_seqs, int max_q_len, int nh, int nkv, int hd,
+                                        int page_size, int total_pages, float scale, int window, int* err, void* stream) {
+    if (num_seqs <= 0 || max_q_len <= 0) return 0;
+    if (nkv <= 0 || nh % nkv || page_size < 1 || window < 0 || (long long)total_pages * nkv * page_size > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+#define IE_F32_TILE(HD)                                                                                                              \
+    if (hd == HD)                                                                                                                    \
+    return launch_f32_tile<HD>(q, k_cache, v_cache, tables, table_width, cu_q, ctx_lens, out, num_seqs, max_q_len, nh, nkv, page_size, \
+                               total_pages, scale, window, err, (cudaStream_t)stream)
+    IE_F32_TILE(32);
+    IE_F32_TILE(64);
+    IE_F32_TILE(128);
+#undef IE_F32_TILE
+    return (int)cudaErrorInvalidValue;
 }

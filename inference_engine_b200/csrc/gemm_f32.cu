@@ -9,63 +9,103 @@
 #include "common.cuh"
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+constexpr int BK = 16, TN = 4, BN = 64, THREADS = 128;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                int M, int N, int K) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
+// Two multiply-adds in one instruction, each rounded as one by itself: the kernel is bound by the instructions it issues.
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long twice(float x) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+    return d;
+}
+
+// A block: BM rows x 64 columns, 8 x 16 threads; a thread TM = BM / 8 rows (in pairs) x 4 columns.  The next 16 of k are fetched into registers
+// while these are worked on.  Whatever the tile, an output is the same chain over k.  (377 x 1,024 by 1,536 and 1,024: tiles of 64 x 64 with
+// 4 x 4 a thread, one block per SM and nothing fetched ahead took 56 us each; these, 32 rows a block there, 40.)
+template <int BM>
+__global__ void __launch_bounds__(THREADS)
+gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K) {
+    constexpr int TM = BM / 8, A_LOADS = BM * BK / 4 / THREADS, W_LOADS = BN * BK / 4 / THREADS;
+    __shared__ __align__(16) float As[2][BK][BM + 4];
+    __shared__ __align__(16) float Ws[2][BK][BN + 4];
     ie_pdl_trigger();
     ie_pdl_wait();
-    int tid = threadIdx.x;
-    int tx = tid % 16, ty = tid / 16;          // 16 x 16 threads, each a 4 x 4 patch
-    int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const bool vec = K % 4 == 0 && !(((size_t)A | (size_t)W) & 15);
+    // four consecutive k of one row
+    auto fetch = [&](const float* __restrict__ X, int row, int rows, int k) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row >= rows) return v;
+        const float* p = X + (size_t)row * K + k;
+        if (vec && k + 3 < K) return *reinterpret_cast<const float4*>(p);
+        if (k < K) v.x = p[0];
+        if (k + 1 < K) v.y = p[1];
+        if (k + 2 < K) v.z = p[2];
+        if (k + 3 < K) v.w = p[3];
+        return v;
+    };
+    float4 a[A_LOADS], w[W_LOADS];
+    auto fetch_tile = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < A_LOADS; ++i) a[i] = fetch(A, m0 + (tid + i * THREADS) / 4, M, k0 + (tid % 4) * 4);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
-    // Each thread loads 4 consecutive k of one row of A and of W per tile.
-    int lr = tid / 4, lk = (tid % 4) * 4;
-    bool vec = (K % 4 == 0);
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
-        int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
-        if (gm < M) {
-            const float* p = A + (size_t)gm * K + gk;
-            if (vec && gk + 3 < K) { float4 v = *reinterpret_cast<const float4*>(p); a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w; }
-            else { for (int i = 0; i < 4; ++i) if (gk + i < K) a[i] = p[i]; }
+        for (int i = 0; i < W_LOADS; ++i) w[i] = fetch(W, n0 + (tid + i * THREADS) / 4, N, k0 + (tid % 4) * 4);
+    };
+    auto keep_tile = [&](int b) {
+        const int k = (tid % 4) * 4;
+#pragma unroll
+        for (int i = 0; i < A_LOADS; ++i) {
+            const int r = (tid + i * THREADS) / 4;
+            As[b][k][r] = a[i].x; As[b][k + 1][r] = a[i].y; As[b][k + 2][r] = a[i].z; As[b][k + 3][r] = a[i].w;
         }
-        if (gn < N) {
-            const float* p = W + (size_t)gn * K + gk;
-            if (vec && gk + 3 < K) { float4 v = *reinterpret_cast<const float4*>(p); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
-            else { for (int i = 0; i < 4; ++i) if (gk + i < K) w[i] = p[i]; }
-        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { As[lk + i][lr] = a[i]; Ws[lk + i][lr] = w[i]; }
-        __syncthreads();
+        for (int i = 0; i < W_LOADS; ++i) {
+            const int r = (tid + i * THREADS) / 4;
+            Ws[b][k][r] = w[i].x; Ws[b][k + 1][r] = w[i].y; Ws[b][k + 2][r] = w[i].z; Ws[b][k + 3][r] = w[i].w;
+        }
+    };
+    unsigned long long acc[TM / 2][TN];
+#pragma unroll
+    for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    fetch_tile(0);
+    keep_tile(0);
+    __syncthreads();
+    int b = 0;
+    for (int k0 = 0; k0 < K; k0 += BK, b ^= 1) {
+        const bool more = k0 + BK < K;
+        if (more) fetch_tile(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            float4 av = *reinterpret_cast<const float4*>(&As[k][ty * TM]);
-            float4 wv = *reinterpret_cast<const float4*>(&Ws[k][tx * TN]);
-            float ar[4] = {av.x, av.y, av.z, av.w}, wr[4] = {wv.x, wv.y, wv.z, wv.w};
+            const float4 wv = *reinterpret_cast<const float4*>(&Ws[b][k][tx * TN]);
+            const unsigned long long w2[TN] = {twice(wv.x), twice(wv.y), twice(wv.z), twice(wv.w)};
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < TM / 4; ++i) {
+                const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(&As[b][k][ty * TM + 4 * i]);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) {
+                    acc[2 * i][j] = fma2(av.x, w2[j], acc[2 * i][j]);
+                    acc[2 * i + 1][j] = fma2(av.y, w2[j], acc[2 * i + 1][j]);
+                }
+            }
         }
+        if (more) keep_tile(b ^ 1);  // (everyone is done with that buffer since the last barrier)
         __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        int gm = m0 + ty * TM + i;
+        const int gm = m0 + ty * TM + i;
         if (gm >= M) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            int gn = n0 + tx * TN + j;
-            if (gn < N) C[(size_t)gm * N + gn] = acc[i][j];
+            const int gn = n0 + tx * TN + j;
+            const unsigned long long pair = acc[i / 2][j];
+            if (gn < N) C[(size_t)gm * N + gn] = __uint_as_float(i & 1 ? (unsigned)(pair >> 32) : (unsigned)pair);
         }
     }
 }
@@ -73,7 +113,11 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 
 IE_API int ie_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_f32_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(A, W, C, M, N, K);
+    const int across = (N + BN - 1) / BN;
+    // (64 rows a block once such blocks are two to an SM; below that 32, so that more SMs have one)
+    if ((long long)((M + 63) / 64) * across >= 2ll * ie_sm_count())
+        gemm_f32_kernel<64><<<dim3(across, (M + 63) / 64), THREADS, 0, (cudaStream_t)stream>>>(A, W, C, M, N, K);
+    else
+        gemm_f32_kernel<32><<<dim3(across, (M + 31) / 32), THREADS, 0, (cudaStream_t)stream>>>(A, W, C, M, N, K);
     return IE_LAUNCH_CHECK();
 }

@@ -243,6 +243,7 @@ class CudaOps:
             "ie_gemm_tc5_bf16": [P, P, P, I, I, I, I, I, I, P, P],
             "ie_gemm_tc5_ok": [I, I, I],
             "ie_paged_attention_generic": [P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, F, I, I, P, P, P, I, I, P, P],
+            "ie_paged_attention_f32_tiles": [P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, I, P, P],
             "ie_sample": [P, I, I, P, P, P, P, P, P, I, P, P, P, P, P],
             "ie_bigram_embedding": [P, P, I, P, P, P, P, P, P, L, I, P, I, I, I, I, L, L, P, P],
             "ie_sandwich_norm": [P, P, I, L, P, I, L, P, P, P, F, P, F, P, I, P, I, I, P],
@@ -913,6 +914,17 @@ class CudaOps:
     @_kind("attention.general")
     def paged_attention_general(self, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd,
                                 page_size, scale, window, out) -> None:
+        # 32-bit portions whose rows (tokens x heads of a group) fill half of a block's 32 at least: the tile kernel, which gives
+        # the same bits (377 tokens of 16 heads of 64 on 4: 72 us, by the general kernel 221)
+        bounds = getattr(ctx, "bounds", None)
+        longest = bounds[0] if bounds is not None else getattr(ctx, "max_q_len", 0)
+        if (q.dtype == self.torch.float32 and hd in (32, 64, 128) and longest * (nh // nkv) >= 16
+                and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16):
+            self._check(self._paged_attention_f32_tiles(
+                q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+                ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, longest, nh, nkv, hd, page_size,
+                k_cache.shape[0], scale, window, self._err_ptr, self._stream()), "paged_attention_f32_tiles")
+            return
         self._check(self._paged_attention_generic(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _dtype_code(q),
             block_tables.data_ptr(), block_tables.shape[1], ctx.seq_of_token.data_ptr(),
