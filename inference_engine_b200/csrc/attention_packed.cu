@@ -435,6 +435,9 @@ attention_packed_kernel(const Inputs in, int* err) {
             const float2 both = add2(sums[0], sums[1]);
             l += both.x + both.y;
         }
+        // (the last scores only say that the product three tiles back is done: each of the two still open is waited for, since a wait for the
+        // last alone would take the one before it for its like of two phases ago)
+        if (ok && tiles > 1) ok = mbar_wait_compact(&bars->o_done[i], tiles & 1);
         if (ok) ok = mbar_wait_compact(&bars->o_done[i], (tiles - 1) & 1);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
