@@ -4,13 +4,14 @@
 //
 // A block owns 256 rows of one request and one key/value head, a row being a (token, query head of the group) pair, so that a key tile
 // is brought once for the whole group, and walks tiles of 64 keys.  Two row tiles of 128 take turns, and a row tile's scores are made a key tile
-// ahead of its softmax, so that softmax follows softmax.  Eleven warps (with a thirteenth a thread would have 128 registers instead of
-// 168, and spill):
+// ahead of its softmax, so that softmax follows softmax.  Twelve warps (a thirteenth would leave a thread 128 registers instead of
+// 168, and it would spill):
 //   warps 0-3, 4-7: softmax of row tile 0 and 1, a thread per row (tensor-memory lane);
-//   warp 8: tcgen05.mma.  Per key tile: S = Q K^T of the next key tile for both row tiles (both operands from shared memory), then
-//     O += P V of this one as each row tile's weights are written (P in tensor memory, over the scores it was made from);
-//   warps 9, 10: gather keys and values by cp.async, swizzled by hand as the tensor core reads them.  (Pages of
-//     16 tokens as TMA boxes are 2 KB each, and the copy engine spends some 300 clocks on any box: they would take longer than a tile's products.)
+//   warps 8, 9: tcgen05.mma of row tile 0 and 1.  Per key tile: O += P V as the weights are written (P in tensor memory, over the scores it
+//     was made from), then S = Q K^T of the key tile after the next (both operands from shared memory);
+//   warps 10, 11: gather keys and values by cp.async, every other key tile each, swizzled by hand as the tensor core reads them.  (Pages of
+//     16 tokens as TMA boxes are 2 KB each, and the copy engine spends 120 to 300 clocks on any box: they would take longer than a tile's
+//     products.)
 // Tensor memory: row tile i's scores of key tile t in columns (2 i + t % 2) 64 .. + 63, its output in 256 + 128 i.  A row's weights replace its
 // scores: 32 columns of weights rounded to bfloat16, two to a column, then 32 columns of what the rounding left (a weight keeps 16 bits of
 // mantissa; both go through the second product).  The maximum that weights are taken against follows a row's running maximum only when that
@@ -19,10 +20,12 @@
 // PA_FLAT 1 (latent attention whose keys and values were expanded per head): keys and values are rows of step-wide arrays, a request's
 // context after the one before it; a key is the head's own entries (PA_D - 64) and then up to 64 rotated ones that all heads share.
 //
-// What bounds it: a key tile's products take 1,808 clocks (65 for 128 x 128 x 16, 48 for 128 x 64 x 16, as measured), its exponentials
-// 1,024 of the special-function unit, its softmax instructions about as long as the products.  Scores one tile of 128 keys at a time, made when
-// the softmax before had ended, cost the chain both: 7,000 clocks per 128 keys.
-// Sixteen query heads on four of 128, window 1,024, 2,048 tokens: the mma.sync kernel that serves the other sizes takes 142 us, that form took 40.
+// What bounds it: a key tile's products take 1,840 clocks with two terms and keys of 128 (65 for 128 x 128 x 16, 50 for 128 x 64 x 16, as
+// measured), its exponentials 1,024 of the special-function unit; a tile takes 1,940.  Keys of 64: 1,880, softmax and the way round (weights,
+// product, scores) about as long as each other.  What it was before: scores one tile of 128 keys at a time, made when the softmax before
+// had ended, 7,000 per 128 keys; a tile ahead, with copies fenced by the warps that all shared a tile, 2,700.
+// Sixteen query heads on four of 128: window 1,024, 2,048 tokens 31 us (the mma.sync kernel that serves the other sizes: 142);
+// 8,192 tokens, all positions, 280 us.
 // Every wait is bounded; a block that waits too long records IE_ERR_TIMEOUT, frees its tensor memory and leaves.
 #include "tma.cuh"
 #include <math.h>
@@ -49,7 +52,7 @@ constexpr int KH = D / 64, VH = DV / 64;         // runs of 64 entries: 128 byte
 constexpr int Q_RUN = BM * 128, KV_RUN = KT * 128;  // such a run of a row tile, of a key tile
 constexpr int K_BYTES = KH * KV_RUN, V_BYTES = VH * KV_RUN, Q_TILE = KH * Q_RUN, Q_BYTES = 2 * Q_TILE;
 constexpr int KS = D == 192 ? 3 : 4, VS = D == 192 ? 3 : 4;  // tiles of keys and of values in shared memory
-constexpr int SOFTMAX_WARPS = 8, COPY_WARPS = 2, THREADS = (SOFTMAX_WARPS + 1 + COPY_WARPS) * 32;
+constexpr int SOFTMAX_WARPS = 8, MMA_WARPS = 2, COPY_WARPS = 2, THREADS = (SOFTMAX_WARPS + MMA_WARPS + COPY_WARPS) * 32;
 constexpr float RESCALE_LAG = 8.0f;              // in powers of two
 constexpr float LOG2E_F = 1.4426950408889634f;
 
@@ -123,7 +126,7 @@ struct Inputs {
     int q_rot_ld, k_rot_ld, kv_ld, rot;
 };
 
-// grid: (blocks of 256 rows of the longest portion, key/value heads, requests)
+// grid: (blocks of 256 rows of the longest portion x key/value heads, requests): the rows that see most start first, whatever the head
 template <bool CAP>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_packed_kernel(const Inputs in, int* err) {
@@ -137,9 +140,9 @@ attention_packed_kernel(const Inputs in, int* err) {
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (one number for the whole warp, as far as the compiler is concerned)
     ie_pdl_trigger();
     // (lengths and block tables are the step's inputs; queries, keys and values are the kernels' before)
-    const int seq = blockIdx.z, kvh = blockIdx.y, group = in.heads / in.kv_heads;
+    const int seq = blockIdx.y, kvh = blockIdx.x % in.kv_heads, group = in.heads / in.kv_heads;
     const int q0 = in.cu_q[seq], q_len = in.cu_q[seq + 1] - q0;
-    const int row0 = (gridDim.x - 1 - blockIdx.x) * ROWS, rows_total = q_len * group;  // (the rows that see most start first)
+    const int row0 = ((gridDim.x - 1 - blockIdx.x) / in.kv_heads) * ROWS, rows_total = q_len * group;
     if (row0 >= rows_total) return;
     const int start = in.ctx_lens[seq] - q_len;  // position of the request's first token of this step
     const int rows_here = min(ROWS, rows_total - row0);
@@ -153,8 +156,8 @@ attention_packed_kernel(const Inputs in, int* err) {
 
     if (tid == 0) {
         mbar_init(&bars->q_full, COPY_WARPS);
-        for (int s = 0; s < KS; ++s) { mbar_init(&bars->k_full[s], COPY_WARPS); mbar_init(&bars->k_empty[s], 1); }
-        for (int s = 0; s < VS; ++s) { mbar_init(&bars->v_full[s], COPY_WARPS); mbar_init(&bars->v_empty[s], 1); }
+        for (int s = 0; s < KS; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], MMA_WARPS); }
+        for (int s = 0; s < VS; ++s) { mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], MMA_WARPS); }
         for (int i = 0; i < 4; ++i) { mbar_init(&bars->s_done[i], 1); mbar_init(&bars->p_ready[i], BM); }
         for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
         bars->failed = 0;
@@ -170,174 +173,148 @@ attention_packed_kernel(const Inputs in, int* err) {
     const unsigned tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
     ie_pdl_wait();
 
-    if (warp == SOFTMAX_WARPS) {
-        // ---- tensor core ----
+    if (warp >= SOFTMAX_WARPS && warp < SOFTMAX_WARPS + MMA_WARPS) {
+        // ---- tensor core: a warp per row tile ----
+        const int i = warp - SOFTMAX_WARPS;
         const unsigned idesc_qk = umma_idesc_bf16(BM, KT), idesc_pv = umma_idesc_bf16(BM, DV) | (1u << 16);
-        const unsigned qa = desc_low(smem_u32(q_s), 1024), ka = desc_low(smem_u32(k_s), 1024), va = desc_low(smem_u32(v_s), KV_RUN);
+        const unsigned qa = desc_low(smem_u32(q_s) + i * Q_TILE, 1024), ka = desc_low(smem_u32(k_s), 1024), va = desc_low(smem_u32(v_s), KV_RUN);
+        const unsigned st = tmem + 2 * i * KT, o = tmem + ROWS + i * BM;
         const bool one = elect_one();
         bool ok = mbar_wait_compact(&bars->q_full, 0);
-        // The scores of row tile i and key tile t.  Their columns held the weights of tile t - 2: the product that read them must be done
+        // The scores of key tile t.  Their columns held the weights of tile t - 2: the product that read them must be done
         // (products into different accumulators are not ordered by their issue).
-        auto scores = [&](int i, int t) {
+        auto scores = [&](int t) {
             if (t >= tiles) return true;
             const int slot = t % KS;
             if ((t >= 2 && !mbar_wait_compact(&bars->o_done[i], t & 1)) || !mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (one) {
-                const unsigned qt = qa + i * (Q_TILE >> 4), kt = ka + slot * (K_BYTES >> 4), st = tmem + (2 * i + (t & 1)) * KT;
+                const unsigned kt = ka + slot * (K_BYTES >> 4), s = st + (t & 1) * KT;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a run
-                    mma_ss(st, qt + (((ks >> 2) * Q_RUN + (ks & 3) * 32) >> 4), kt + (((ks >> 2) * KV_RUN + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
+                    mma_ss(s, qa + (((ks >> 2) * Q_RUN + (ks & 3) * 32) >> 4), kt + (((ks >> 2) * KV_RUN + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
                 umma_commit(&bars->s_done[2 * i + (t & 1)]);
-                if (i == 1) umma_commit(&bars->k_empty[slot]);
+                umma_commit(&bars->k_empty[slot]);
             }
             __syncwarp();
             return true;
         };
-        // O_i += P V of key tile t
-        auto values = [&](int i, int t) {
+        // O += P V of key tile t
+        auto values = [&](int t) {
             const int slot = t % VS;
-            if ((i == 0 && !mbar_wait_compact(&bars->v_full[slot], (t / VS) & 1)) ||
-                !mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1)) return false;
+            if (!mbar_wait_compact(&bars->v_full[slot], (t / VS) & 1) || !mbar_wait_compact(&bars->p_ready[2 * i + (t & 1)], (t >> 1) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (one) {
-                const unsigned p = tmem + (2 * i + (t & 1)) * KT, o = tmem + ROWS + i * BM, vt = va + slot * (V_BYTES >> 4);
+                const unsigned p = st + (t & 1) * KT, vt = va + slot * (V_BYTES >> 4);
 #pragma unroll
                 for (int term = 0; term < TERMS; ++term)
 #pragma unroll
                     for (int ks = 0; ks < KT / 16; ++ks)  // 16 keys: 8 columns of weights, 2,048 bytes of values
                         mma_ts(o, p + term * 32 + ks * 8, vt + ks * (2048 >> 4), idesc_pv, term > 0 || ks > 0 || t > 0);
                 umma_commit(&bars->o_done[i]);
-                if (i == 1) umma_commit(&bars->v_empty[slot]);
+                umma_commit(&bars->v_empty[slot]);
             }
             __syncwarp();
             return true;
         };
-        ok = ok && scores(0, 0) && scores(1, 0) && scores(0, 1);
-        // (a row tile's scores follow the other's second product: the product they wait for is the one before that)
-        for (int t = 0; t < tiles && ok; ++t) ok = (t > 0 || scores(1, 1)) && values(0, t) && (t == 0 || scores(1, t + 1)) && values(1, t) && scores(0, t + 2);
+        ok = ok && scores(0) && scores(1);
+        for (int t = 0; t < tiles && ok; ++t) ok = values(t) && scores(t + 2);
         if (!ok) bars->failed = 1;
-    } else if (warp > SOFTMAX_WARPS) {
-        // ---- copies: eight threads to a row of 128 bytes, eight rows at a time ----
-        const int c = tid - (SOFTMAX_WARPS + 1) * 32, chunk = c & 7, r0 = c >> 3;
-        const unsigned to = (unsigned)(r0 * 128 + ((chunk ^ (r0 & 7)) << 4));  // (r0 + 8 p: the same place in its group of eight rows)
-        constexpr int AT_ONCE = COPY_WARPS * 4, PASSES = KT / AT_ONCE;
-        static_assert(AT_ONCE == 8, "rows at a time");
-        // Groups of copies in the order in which they are asked for: the queries, then keys and values of every tile in turn.  A group is
-        // announced when DEPTH more have been asked for, or when a slot is not free yet (it may wait for what is on its way): one group
-        // ahead left the memory's latency between any two.
-        constexpr int DEPTH = 4;
-        int asked_for = 0, announced = 0;
-        auto announce = [&]() {
-            const int g = announced++ - 1;  // (0: the queries)
-            unsigned long long* bar = g < 0 ? &bars->q_full : g & 1 ? &bars->v_full[(g >> 1) % VS] : &bars->k_full[(g >> 1) % KS];
+    } else if (warp >= SOFTMAX_WARPS + MMA_WARPS) {
+        // ---- copies: eight threads to a row of 128 bytes.  A tile's keys and values are one warp's, and the warps take turns: the fence
+        // that hands the copies to the tensor core waits for all that its warp has in flight, so only other warps' copies go on beside it (two
+        // warps that shared a tile and fenced keys and values apart took 2,600 clocks a tile, whatever the key size). ----
+        const int w = warp - SOFTMAX_WARPS - MMA_WARPS, chunk = lane & 7, r0 = lane >> 3;
+        constexpr int PASSES = KT / 4;
+        // row r0 + 4 p: the same place in every other group of four rows
+        const unsigned to0 = (unsigned)(r0 * 128 + ((chunk ^ r0) << 4)), to1 = (unsigned)((r0 + 4) * 128 + ((chunk ^ (r0 + 4)) << 4));
+        auto place = [&](int p) { return (unsigned)(p >> 1) * 1024 + (p & 1 ? to1 : to0); };
+        auto landed = [&]() {
+            asm volatile("cp.async.wait_all;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar);
         };
-        auto asked = [&]() {
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (++asked_for - announced > DEPTH) {
-                asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH) : "memory");
-                announce();
-            }
-        };
-        auto settle = [&]() {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            while (announced < asked_for) announce();
-        };
-        auto slot_free = [&](unsigned long long* bar, int parity) {
-            if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-            settle();
-            return mbar_wait_compact(bar, parity);
-        };
-        {
 #pragma unroll 4
-            for (int p = 0; p < ROWS / AT_ONCE; ++p) {
-                const int r = r0 + AT_ONCE * p;
-                const bool there = r < rows_here;
-                const int rr = row0 + (there ? r : 0), token = rr / group, head = kvh * group + rr - token * group;
-                const size_t unit = (size_t)(q0 + token) * in.heads + head;
-                const unsigned dst = smem_u32(q_s) + (r >> 7) * Q_TILE + (p & (BM / AT_ONCE - 1)) * 1024 + to;
+        for (int p = w; p < ROWS / 4; p += COPY_WARPS) {
+            const int r = r0 + 4 * p;
+            const bool there = r < rows_here;
+            const int rr = row0 + (there ? r : 0), token = rr / group, head = kvh * group + rr - token * group;
+            const size_t unit = (size_t)(q0 + token) * in.heads + head;
+            const unsigned dst = smem_u32(q_s) + (r >> 7) * Q_TILE + place(p & (BM / 4 - 1));
 #pragma unroll
-                for (int h = 0; h < KH; ++h) {
-                    if (FLAT && h == KH - 1) {
-                        const bool rotated = there && chunk * 8 < in.rot;
-                        cp16(dst + h * Q_RUN, rotated ? in.q_rot + unit * in.q_rot_ld + chunk * 8 : in.q, rotated ? 16 : 0);
-                    } else {
-                        cp16(dst + h * Q_RUN, in.q + unit * (FLAT ? D - 64 : D) + chunk * 8 + h * 64, there ? 16 : 0);
-                    }
+            for (int h = 0; h < KH; ++h) {
+                if (FLAT && h == KH - 1) {
+                    const bool rotated = there && chunk * 8 < in.rot;
+                    cp16(dst + h * Q_RUN, rotated ? in.q_rot + unit * in.q_rot_ld + chunk * 8 : in.q, rotated ? 16 : 0);
+                } else {
+                    cp16(dst + h * Q_RUN, in.q + unit * (FLAT ? D - 64 : D) + chunk * 8 + h * 64, there ? 16 : 0);
                 }
             }
-            asked();
         }
+        landed();
+        if (lane == 0) mbar_arrive(&bars->q_full);
         const int* table = FLAT ? nullptr : in.tables + (size_t)seq * in.table_width;
         int before = 0;  // FLAT: rows of the requests before this one
         if (FLAT)
             for (int i = 0; i < seq; ++i) before += in.ctx_lens[i];
         bool ok = true;
-        // the pages of the thread's keys, looked up a tile ahead
-        int page_of[PASSES];
+        // the row of each of the warp's keys, two to a lane, looked up while the copies before are in flight; -1: nothing there (reads as zero)
+        int row_of[2] = {-1, -1};
         auto look_up = [&](int t) {
-            const int key0 = key_of(t);
 #pragma unroll
-            for (int p = 0; p < PASSES; ++p) {
-                const int pos = key0 + r0 + AT_ONCE * p;
-                page_of[p] = (pos >= lo_min || pos < in.keep_first) && pos <= last_pos ? table[pos >> in.page_shift] : 0;
-            }
-        };
-        if (!FLAT) look_up(0);
-        for (int t = 0; t < tiles; ++t) {
-            const int key0 = key_of(t);
-            int row[PASSES];  // the row of each of the thread's keys; -1: nothing there (reads as zero)
-#pragma unroll
-            for (int p = 0; p < PASSES; ++p) {
-                const int pos = key0 + r0 + AT_ONCE * p;
-                row[p] = -1;
+            for (int j = 0; j < 2; ++j) {
+                const int pos = key_of(t) + lane + 32 * j;
+                row_of[j] = -1;
                 if ((pos >= lo_min || pos < in.keep_first) && pos <= last_pos) {
                     if (FLAT) {
-                        row[p] = before + pos;
+                        row_of[j] = before + pos;
                     } else {
-                        const int page = page_of[p];
+                        const int page = table[pos >> in.page_shift];
                         if (page < 0 || page >= in.total_pages) {
-                            if (chunk == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
+                            ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
                         } else {
-                            row[p] = ((page * in.kv_heads + kvh) << in.page_shift) + (pos & ((1 << in.page_shift) - 1));
+                            row_of[j] = ((page * in.kv_heads + kvh) << in.page_shift) + (pos & ((1 << in.page_shift) - 1));
                         }
                     }
                 }
             }
-            if (!FLAT && t + 1 < tiles) look_up(t + 1);
+        };
+        if (w < tiles) look_up(w);
+        for (int t = w; t < tiles; t += COPY_WARPS) {
             const int ks = t % KS, vs = t % VS;
-            if (t >= KS && !slot_free(&bars->k_empty[ks], (t / KS - 1) & 1)) { ok = false; break; }
-            unsigned dst = smem_u32(k_s) + ks * K_BYTES + to;
-#pragma unroll
+            // (with three slots a warp meets a slot every other time it is filled; the time between is over, since the warp has waited for
+            // a later tile's)
+            if ((t >= KS && !mbar_wait_compact(&bars->k_empty[ks], (t / KS - 1) & 1)) ||
+                (t >= VS && !mbar_wait_compact(&bars->v_empty[vs], (t / VS - 1) & 1))) { ok = false; break; }
+            const unsigned kd = smem_u32(k_s) + ks * K_BYTES, vd = smem_u32(v_s) + vs * V_BYTES;
+#pragma unroll 4
             for (int p = 0; p < PASSES; ++p) {
-                const size_t at = (size_t)max(row[p], 0);
-                const bf16* src = FLAT ? in.k + at * in.kv_ld + kvh * (D - 64) + chunk * 8 : in.k + at * D + chunk * 8;
+                const int row = __shfl_sync(0xffffffffu, p < PASSES / 2 ? row_of[0] : row_of[1], (r0 + 4 * p) & 31);
+                const size_t at = (size_t)max(row, 0);
+                const int bytes = row >= 0 ? 16 : 0;
+                const bf16* k = in.k + (FLAT ? at * in.kv_ld + kvh * (D - 64) : at * D) + chunk * 8;
+                const bf16* v = in.v + (FLAT ? at * in.kv_ld + kvh * DV : at * DV) + chunk * 8;
+                const unsigned to = place(p);
 #pragma unroll
                 for (int h = 0; h < KH; ++h) {
                     if (FLAT && h == KH - 1) {
-                        const bool rotated = row[p] >= 0 && chunk * 8 < in.rot;
-                        cp16(dst + p * 1024 + h * KV_RUN, rotated ? in.k_rot + at * in.k_rot_ld + chunk * 8 : in.k, rotated ? 16 : 0);
+                        const bool rotated = row >= 0 && chunk * 8 < in.rot;
+                        cp16(kd + to + h * KV_RUN, rotated ? in.k_rot + at * in.k_rot_ld + chunk * 8 : in.k, rotated ? 16 : 0);
                     } else {
-                        cp16(dst + p * 1024 + h * KV_RUN, src + h * 64, row[p] >= 0 ? 16 : 0);
+                        cp16(kd + to + h * KV_RUN, k + h * 64, bytes);
                     }
                 }
-            }
-            asked();
-            if (t >= VS && !slot_free(&bars->v_empty[vs], (t / VS - 1) & 1)) { ok = false; break; }
-            dst = smem_u32(v_s) + vs * V_BYTES + to;
 #pragma unroll
-            for (int p = 0; p < PASSES; ++p) {
-                const size_t at = (size_t)max(row[p], 0);
-                const bf16* src = FLAT ? in.v + at * in.kv_ld + kvh * DV + chunk * 8 : in.v + at * DV + chunk * 8;
-#pragma unroll
-                for (int h = 0; h < VH; ++h) cp16(dst + p * 1024 + h * KV_RUN, src + h * 64, row[p] >= 0 ? 16 : 0);
+                for (int h = 0; h < VH; ++h) cp16(vd + to + h * KV_RUN, v + h * 64, bytes);
             }
-            asked();
+            if (t + COPY_WARPS < tiles) look_up(t + COPY_WARPS);
+            landed();
+            if (lane == 0) {
+                mbar_arrive(&bars->k_full[ks]);
+                mbar_arrive(&bars->v_full[vs]);
+            }
         }
-        settle();
+        asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok) bars->failed = 1;
     } else {
         // ---- softmax: thread = row = tensor-memory lane ----
@@ -471,7 +448,7 @@ attention_packed_kernel(const Inputs in, int* err) {
 
 static int launch_packed(const Inputs& in, int num_seqs, int max_q_len, int* err, void* stream) {
     const long long rows = (long long)max_q_len * (in.heads / in.kv_heads);
-    const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS), in.kv_heads, num_seqs);
+    const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS * in.kv_heads), num_seqs);
     static IePerDevice allowed, allowed_cap;
     cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false>, SMEM_BYTES);
     if (e == cudaSuccess && !FLAT) e = ie_allow_smem(allowed_cap, attention_packed_kernel<!FLAT>, SMEM_BYTES);
