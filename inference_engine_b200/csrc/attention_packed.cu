@@ -26,6 +26,12 @@
 // had ended, 7,000 per 128 keys; a tile ahead, with copies fenced by the warps that all shared a tile, 2,700.
 // Sixteen query heads on four of 128: window 1,024, 2,048 tokens 31 us (the mma.sync kernel that serves the other sizes: 142);
 // 8,192 tokens, all positions, 280 us.
+//
+// PA_PROMPT: plain attention as Llama-like models have it.  One term of the weights (as the kernel of 128 tokens of a head a block has
+// it), all portions of a step in one grid, and the key tiles of a block's rows cut among a cluster of blocks, whose outputs are added through
+// the cluster's shared memory (through scratch by the block that ended last it took 8 us for 9 parts).  Softmax bounds it: 1,500 clocks a tile
+// with keys of 64, 1,650 with 128 (products 600 and 1,320).  Against the kernel of a head a block, 32 heads on 8, us: 2,048 tokens of 128
+// entries 85 -> 42, 8,192 tokens 849 -> 449, 512 tokens behind 8,192 118 -> 78; of 64 entries 39 -> 35, 424 -> 374, 68 -> 65.
 // Every wait is bounded; a block that waits too long records IE_ERR_TIMEOUT, frees its tensor memory and leaves.
 #include "tma.cuh"
 #include <math.h>
@@ -39,6 +45,9 @@
 #ifndef PA_FLAT
 #define PA_FLAT 0
 #endif
+#ifndef PA_PROMPT
+#define PA_PROMPT 0
+#endif
 
 using namespace ie_tma;
 
@@ -46,7 +55,9 @@ namespace {
 constexpr int D = PA_D, DV = PA_DV;
 static_assert((D == 64 || D == 128 || D == 192) && (DV == 64 || DV == 128), "sizes");
 constexpr bool FLAT = PA_FLAT != 0;
-constexpr int TERMS = 2;
+constexpr bool PROMPT = PA_PROMPT != 0;
+static_assert(!(FLAT && PROMPT), "one form at a time");
+constexpr int TERMS = PROMPT ? 1 : 2;
 constexpr int BM = 128, ROWS = 2 * BM, KT = 64;
 constexpr int KH = D / 64, VH = DV / 64;         // runs of 64 entries: 128 bytes, one swizzle atom
 constexpr int Q_RUN = BM * 128, KV_RUN = KT * 128;  // such a run of a row tile, of a key tile
@@ -61,6 +72,8 @@ struct __align__(8) Bars {
     unsigned tmem_base;
     int failed;
 };
+constexpr int MOST_SHARES = 8;  // blocks of a cluster that every device runs
+static_assert(ROWS * (DV * 4 + 8) <= Q_BYTES + KS * K_BYTES + VS * V_BYTES, "room for the shares");
 constexpr size_t SMEM_BYTES = (size_t)Q_BYTES + KS * K_BYTES + VS * V_BYTES + sizeof(Bars) + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 
@@ -74,7 +87,8 @@ __device__ __forceinline__ bool elect_one() {
 // then costs an addition an operand; descriptors put together anew for each cost the issuing warp 100 clocks an instruction beside
 // the softmax warps, where the tensor core needs 48 and 65.
 constexpr unsigned DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ unsigned desc_low(unsigned addr, unsigned run) { return (addr >> 4) | ((run >> 4) << 16); }
+// (within a cluster an address has the block's number above its 18 bits)
+__device__ __forceinline__ unsigned desc_low(unsigned addr, unsigned run) { return ((addr & 0x3ffff) >> 4) | ((run >> 4) << 16); }
 __device__ __forceinline__ void mma_ss(unsigned d, unsigned a, unsigned b, unsigned idesc, bool accumulate) {
     asm volatile("{\n .reg .pred p;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
@@ -124,10 +138,64 @@ struct Inputs {
     // k_rot_ld
     const bf16 *q_rot, *k_rot;
     int q_rot_ld, k_rot_ld, kv_ld, rot;
+    // PA_PROMPT: the step's requests (those of 16 rows or fewer are another kernel's)
+    int num_seqs;
 };
 
+__device__ __forceinline__ unsigned peer_smem(unsigned addr, int rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A cluster's blocks hold 256 rows' shares of the output (relative to the share's maximum; piece c of 16 bytes of row r in place c ^ (r & 7)), maxima
+// and sums in shared memory, and each adds an even part of the rows, in the order of the shares.  DV / 4 lanes take a row; a lane works one
+// share's factor out.
+__device__ __forceinline__ void add_shares(unsigned o_s, unsigned ml_s, int rank, int shares, bf16* out, int out_ld, int row0, int rows_here,
+                                           int group, int tid) {
+    constexpr int LANES = DV / 4, AT_ONCE = THREADS / LANES;
+    const int c = tid % LANES, end = (rank + 1) * rows_here / shares;
+    for (int r1 = rank * rows_here / shares; r1 < end; r1 += AT_ONCE) {
+        const int r = min(r1 + tid / LANES, end - 1);
+        float m = -INFINITY, l = 0.f;
+        if (c < shares) asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(m), "=f"(l) : "r"(peer_smem(ml_s + r * 8, c)));
+        float4 v[MOST_SHARES];
+#pragma unroll
+        for (int z = 0; z < MOST_SHARES; ++z)
+            if (z < shares)
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[z].x), "=f"(v[z].y), "=f"(v[z].z), "=f"(v[z].w)
+                             : "r"(peer_smem(o_s + r * (DV * 4) + ((c ^ (r & 7)) << 4), z)));
+        float top = m;
+#pragma unroll
+        for (int x = 1; x < MOST_SHARES; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x, LANES));
+        top = __shfl_sync(0xffffffffu, top, 0, LANES);
+        float f = m == -INFINITY ? 0.f : fast_exp2(m - top);
+        float sum = l * f;
+#pragma unroll
+        for (int x = 1; x < MOST_SHARES; x <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x, LANES);
+        sum = __shfl_sync(0xffffffffu, sum, 0, LANES);
+        f *= sum > 0.f ? 1.f / sum : 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int z = 0; z < MOST_SHARES; ++z) {
+            if (z >= shares) break;
+            const float g = __shfl_sync(0xffffffffu, f, z, LANES);
+            acc.x = fmaf(v[z].x, g, acc.x); acc.y = fmaf(v[z].y, g, acc.y); acc.z = fmaf(v[z].z, g, acc.z); acc.w = fmaf(v[z].w, g, acc.w);
+        }
+        if (r1 + tid / LANES < end) {
+            const int rr = row0 + r, token = rr / group;
+            *reinterpret_cast<uint2*>(out + (size_t)token * out_ld + (rr - token * group) * DV + c * 4) = make_uint2(pack2(acc.x, acc.y), pack2(acc.z, acc.w));
+        }
+    }
+}
+
 // grid: (blocks of 256 rows of the longest portion x key/value heads, requests): the rows that see most start first, whatever the head
-template <bool CAP>
+// (PA_PROMPT: (blocks of 256 rows of all portions x key/value heads, shares): SHARED, a cluster of blocks takes a block's key tiles)
+template <bool CAP, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_packed_kernel(const Inputs in, int* err) {
     extern __shared__ unsigned char smem_raw[];
@@ -140,9 +208,18 @@ attention_packed_kernel(const Inputs in, int* err) {
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (one number for the whole warp, as far as the compiler is concerned)
     ie_pdl_trigger();
     // (lengths and block tables are the step's inputs; queries, keys and values are the kernels' before)
-    const int seq = blockIdx.y, kvh = blockIdx.x % in.kv_heads, group = in.heads / in.kv_heads;
+    const int kvh = blockIdx.x % in.kv_heads, group = in.heads / in.kv_heads;
+    int block = (gridDim.x - 1 - blockIdx.x) / in.kv_heads, seq = PROMPT ? -1 : (int)blockIdx.y;
+    if (PROMPT) {  // the grid's blocks are the requests' one after the other
+        for (int i = 0; i < in.num_seqs; ++i) {
+            const int rows = (in.cu_q[i + 1] - in.cu_q[i]) * group, blocks = rows > 16 ? (rows + ROWS - 1) / ROWS : 0;
+            if (block < blocks) { seq = i; break; }
+            block -= blocks;
+        }
+        if (seq < 0) return;
+    }
     const int q0 = in.cu_q[seq], q_len = in.cu_q[seq + 1] - q0;
-    const int row0 = ((gridDim.x - 1 - blockIdx.x) / in.kv_heads) * ROWS, rows_total = q_len * group;
+    const int row0 = block * ROWS, rows_total = q_len * group;
     if (row0 >= rows_total) return;
     const int start = in.ctx_lens[seq] - q_len;  // position of the request's first token of this step
     const int rows_here = min(ROWS, rows_total - row0);
@@ -151,13 +228,16 @@ attention_packed_kernel(const Inputs in, int* err) {
     // the tiles the block walks, by a running number: those that hold kept keys and lie before the window's first, then the window's
     const int win_begin = lo_min / KT, win_end = last_pos / KT;
     const int kept_tiles = in.keep_first > 0 ? min((in.keep_first - 1) / KT + 1, win_begin) : 0;
-    const int tiles = kept_tiles + win_end - win_begin + 1;
-    auto key_of = [&](int t) { return (t < kept_tiles ? t : win_begin + t - kept_tiles) * KT; };
+    const int all_tiles = kept_tiles + win_end - win_begin + 1;
+    const int shares = SHARED ? (int)gridDim.y : 1, share = SHARED ? (int)blockIdx.y : 0;  // (a share may be empty)
+    const int tile0 = share * all_tiles / shares, tiles = (share + 1) * all_tiles / shares - tile0;
+    auto key_of = [&](int t) { t += tile0; return (t < kept_tiles ? t : win_begin + t - kept_tiles) * KT; };
+    const int row_tiles = rows_here > BM ? 2 : 1;  // (a second one without rows is left out)
 
     if (tid == 0) {
-        mbar_init(&bars->q_full, COPY_WARPS);
-        for (int s = 0; s < KS; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], MMA_WARPS); }
-        for (int s = 0; s < VS; ++s) { mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], MMA_WARPS); }
+        mbar_init(&bars->q_full, SOFTMAX_WARPS);
+        for (int s = 0; s < KS; ++s) { mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], row_tiles); }
+        for (int s = 0; s < VS; ++s) { mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], row_tiles); }
         for (int i = 0; i < 4; ++i) { mbar_init(&bars->s_done[i], 1); mbar_init(&bars->p_ready[i], BM); }
         for (int i = 0; i < 2; ++i) mbar_init(&bars->o_done[i], 1);
         bars->failed = 0;
@@ -180,11 +260,11 @@ attention_packed_kernel(const Inputs in, int* err) {
         const unsigned qa = desc_low(smem_u32(q_s) + i * Q_TILE, 1024), ka = desc_low(smem_u32(k_s), 1024), va = desc_low(smem_u32(v_s), KV_RUN);
         const unsigned st = tmem + 2 * i * KT, o = tmem + ROWS + i * BM;
         const bool one = elect_one();
-        bool ok = mbar_wait_compact(&bars->q_full, 0);
+        bool ok = i >= row_tiles || mbar_wait_compact(&bars->q_full, 0);
         // The scores of key tile t.  Their columns held the weights of tile t - 2: the product that read them must be done
         // (products into different accumulators are not ordered by their issue).
         auto scores = [&](int t) {
-            if (t >= tiles) return true;
+            if (t >= tiles || i >= row_tiles) return true;
             const int slot = t % KS;
             if ((t >= 2 && !mbar_wait_compact(&bars->o_done[i], t & 1)) || !mbar_wait_compact(&bars->k_full[slot], (t / KS) & 1)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -217,8 +297,9 @@ attention_packed_kernel(const Inputs in, int* err) {
             __syncwarp();
             return true;
         };
+        const int mine = i < row_tiles ? tiles : 0;
         ok = ok && scores(0) && scores(1);
-        for (int t = 0; t < tiles && ok; ++t) ok = values(t) && scores(t + 2);
+        for (int t = 0; t < mine && ok; ++t) ok = values(t) && scores(t + 2);
         if (!ok) bars->failed = 1;
     } else if (warp >= SOFTMAX_WARPS + MMA_WARPS) {
         // ---- copies: eight threads to a row of 128 bytes.  A tile's keys and values are one warp's, and the warps take turns: the fence
@@ -234,25 +315,6 @@ attention_packed_kernel(const Inputs in, int* err) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
         };
-#pragma unroll 4
-        for (int p = w; p < ROWS / 4; p += COPY_WARPS) {
-            const int r = r0 + 4 * p;
-            const bool there = r < rows_here;
-            const int rr = row0 + (there ? r : 0), token = rr / group, head = kvh * group + rr - token * group;
-            const size_t unit = (size_t)(q0 + token) * in.heads + head;
-            const unsigned dst = smem_u32(q_s) + (r >> 7) * Q_TILE + place(p & (BM / 4 - 1));
-#pragma unroll
-            for (int h = 0; h < KH; ++h) {
-                if (FLAT && h == KH - 1) {
-                    const bool rotated = there && chunk * 8 < in.rot;
-                    cp16(dst + h * Q_RUN, rotated ? in.q_rot + unit * in.q_rot_ld + chunk * 8 : in.q, rotated ? 16 : 0);
-                } else {
-                    cp16(dst + h * Q_RUN, in.q + unit * (FLAT ? D - 64 : D) + chunk * 8 + h * 64, there ? 16 : 0);
-                }
-            }
-        }
-        landed();
-        if (lane == 0) mbar_arrive(&bars->q_full);
         const int* table = FLAT ? nullptr : in.tables + (size_t)seq * in.table_width;
         int before = 0;  // FLAT: rows of the requests before this one
         if (FLAT)
@@ -319,6 +381,30 @@ attention_packed_kernel(const Inputs in, int* err) {
     } else {
         // ---- softmax: thread = row = tensor-memory lane ----
         const int i = warp >> 2, r = i * BM + (tid & (BM - 1));
+        {   // the queries first, eight threads to 128 bytes of a row (while the copying warps fetch the first keys)
+            const int chunk = lane & 7;
+#pragma unroll 4
+            for (int p = warp * 8; p < warp * 8 + 8; ++p) {
+                const int qr = p * 4 + (lane >> 3);
+                const bool there = qr < rows_here;
+                const int rr = row0 + (there ? qr : 0), token = rr / group, head = kvh * group + rr - token * group;
+                const size_t unit = (size_t)(q0 + token) * in.heads + head;
+                const unsigned dst = smem_u32(q_s) + (qr >> 7) * Q_TILE + (qr & (BM - 1)) * 128 + ((chunk ^ (qr & 7)) << 4);
+#pragma unroll
+                for (int h = 0; h < KH; ++h) {
+                    if (FLAT && h == KH - 1) {
+                        const bool rotated = there && chunk * 8 < in.rot;
+                        cp16(dst + h * Q_RUN, rotated ? in.q_rot + unit * in.q_rot_ld + chunk * 8 : in.q, rotated ? 16 : 0);
+                    } else {
+                        cp16(dst + h * Q_RUN, in.q + unit * (FLAT ? D - 64 : D) + chunk * 8 + h * 64, there ? 16 : 0);
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->q_full);
+        }
         const bool exists = r < rows_here;
         const int rr = row0 + (exists ? r : 0), token = rr / group, head = kvh * group + rr - token * group;
         const int pos = exists ? start + token : -1, lo = in.window > 0 ? max(pos - in.window + 1, 0) : 0;
@@ -332,7 +418,8 @@ attention_packed_kernel(const Inputs in, int* err) {
         // m: the maximum that the weights are taken against (in units of log2 e); the sink is a term of the sum without key and value
         float m = in.sinks != nullptr ? in.sinks[head] * LOG2E_F : -INFINITY, l = in.sinks != nullptr ? 1.f : 0.f;
         bool ok = true;
-        for (int t = 0; t < tiles; ++t) {
+        const int mine = i < row_tiles ? tiles : 0;
+        for (int t = 0; t < mine; ++t) {
             const int key0 = key_of(t);
             if (!mbar_wait_compact(&bars->s_done[2 * i + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -400,11 +487,13 @@ attention_packed_kernel(const Inputs in, int* err) {
                     const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                     sums[k & 1] = add2(sums[k & 1], p);
                     hi[k] = pack2(p.x, p.y);
-                    const float2 r = fma2(as_float2(hi[k]), minus_one, p);  // (exact)
-                    rest[k] = pack2(r.x, r.y);
+                    if constexpr (TERMS == 2) {
+                        const float2 r = fma2(as_float2(hi[k]), minus_one, p);  // (exact)
+                        rest[k] = pack2(r.x, r.y);
+                    }
                 }
                 tmem_st16(hi, ts + part * 16);
-                tmem_st16(rest, ts + 32 + part * 16);
+                if constexpr (TERMS == 2) tmem_st16(rest, ts + 32 + part * 16);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -414,9 +503,29 @@ attention_packed_kernel(const Inputs in, int* err) {
         }
         // (the last scores only say that the product three tiles back is done: each of the two still open is waited for, since a wait for the
         // last alone would take the one before it for its like of two phases ago)
-        if (ok && tiles > 1) ok = mbar_wait_compact(&bars->o_done[i], tiles & 1);
-        if (ok) ok = mbar_wait_compact(&bars->o_done[i], (tiles - 1) & 1);
-        if (ok) {
+        if (ok && mine > 1) ok = mbar_wait_compact(&bars->o_done[i], tiles & 1);
+        if (ok && mine > 0) ok = mbar_wait_compact(&bars->o_done[i], (tiles - 1) & 1);
+        if (SHARED) {
+            // (both row tiles' products are done and every copy has landed: queries, keys and values make room for the output)
+            asm volatile("bar.sync 1, %0;" ::"n"(ROWS) : "memory");
+            const bool filled = ok && mine > 0;
+            *reinterpret_cast<float2*>(smem + ROWS * DV * 4 + r * 8) = make_float2(filled ? m : -INFINITY, filled ? l : 0.f);
+            if (filled) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int d = 0; d < DV && i < row_tiles; d += 32) {
+                float acc[32];
+                if (filled) {
+                    tmem_ld32(acc, to + d);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    *reinterpret_cast<float4*>(smem + r * (DV * 4) + (((d / 4 + k) ^ (r & 7)) << 4)) =
+                        make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+            }
+        } else if (ok && i < row_tiles) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float f = l > 0.f ? 1.0f / l : 0.f;
             const float* gate = in.gate == nullptr ? nullptr : in.gate + (size_t)(q0 + token) * in.gate_ld + (in.gate_elements ? head * DV : head);
@@ -441,20 +550,75 @@ attention_packed_kernel(const Inputs in, int* err) {
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (SHARED) {
+        cluster_barrier();
+        add_shares(smem_u32(smem), smem_u32(smem) + ROWS * DV * 4, share, shares, in.out + (size_t)q0 * in.out_ld + kvh * group * DV, in.out_ld,
+                   row0, rows_here, group, tid);
+        cluster_barrier();  // (the others read this block's memory)
+    }
     if (warp == SOFTMAX_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     if (tid == 0 && bars->failed) ie_report(err, IE_ERR_TIMEOUT, blockIdx.x, blockIdx.y);
 }
 }  // namespace
 
+#if PA_PROMPT
+// Plain softmax attention of a step's portions of more than 16 rows (tokens x heads of a group); the output has the queries' form.  `blocks`:
+// at least the blocks of 256 rows that these portions have; the key tiles of each are shared among `shares` blocks (8 at most), a cluster.
+IE_API int ie_attention_prompt(const void* q, const void* k_cache, const void* v_cache, const int* tables, int table_width, const int* cu_q,
+                               const int* ctx_lens, void* out, int num_seqs, int blocks, int heads, int kv_heads, int page_size,
+                               int total_pages, float scale, int window, int shares, int* err, void* stream) {
+    if (num_seqs <= 0 || blocks <= 0) return 0;
+    if (kv_heads <= 0 || heads % kv_heads != 0 || page_size < 1 || (page_size & (page_size - 1)) || window < 0 || shares < 1 ||
+        shares > MOST_SHARES || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) ||
+        (long long)total_pages * kv_heads * page_size > 0x7fffffffll)
+        return (int)cudaErrorInvalidValue;
+    int page_shift = 0;
+    while ((1 << page_shift) < page_size) ++page_shift;
+    const Inputs in{(const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, tables, cu_q, ctx_lens, table_width, heads, kv_heads,
+                    page_shift, total_pages, scale, window, 0, 0.f, nullptr, nullptr, 0, 0, (bf16*)out, heads * DV,
+                    nullptr, nullptr, 0, 0, 0, 0, num_seqs};
+    static IePerDevice allowed, allowed_shared;
+    cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false, false>, SMEM_BYTES);
+    if (e == cudaSuccess) e = ie_allow_smem(allowed_shared, attention_packed_kernel<false, true>, SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    const dim3 grid((unsigned)(blocks * kv_heads), shares);
+    if (shares > 1) return ie_launch_cluster(attention_packed_kernel<false, true>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, dim3(1, shares, 1), in, err);
+    return ie_launch(attention_packed_kernel<false, false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+}
+
+// How many clusters of so many blocks the device runs at one time; 0: unknown.
+IE_API int ie_attention_prompt_clusters(int shares) {
+    if (shares < 1 || shares > MOST_SHARES) return 0;
+    static IePerDevice allowed;
+    if (ie_allow_smem(allowed, attention_packed_kernel<false, true>, SMEM_BYTES) != cudaSuccess) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, shares);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = (unsigned)shares;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, attention_packed_kernel<false, true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return clusters;
+}
+#else
 static int launch_packed(const Inputs& in, int num_seqs, int max_q_len, int* err, void* stream) {
     const long long rows = (long long)max_q_len * (in.heads / in.kv_heads);
     const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS * in.kv_heads), num_seqs);
     static IePerDevice allowed, allowed_cap;
-    cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false>, SMEM_BYTES);
-    if (e == cudaSuccess && !FLAT) e = ie_allow_smem(allowed_cap, attention_packed_kernel<!FLAT>, SMEM_BYTES);
+    cudaError_t e = ie_allow_smem(allowed, attention_packed_kernel<false, false>, SMEM_BYTES);
+    if (e == cudaSuccess && !FLAT) e = ie_allow_smem(allowed_cap, attention_packed_kernel<!FLAT, false>, SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
-    if (!FLAT && in.softcap > 0.f) return ie_launch(attention_packed_kernel<!FLAT>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
-    return ie_launch(attention_packed_kernel<false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+    if (!FLAT && in.softcap > 0.f) return ie_launch(attention_packed_kernel<!FLAT, false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
+    return ie_launch(attention_packed_kernel<false, false>, grid, dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, in, err);
 }
 
 #if !PA_FLAT
@@ -474,7 +638,7 @@ IE_API int ie_attention_packed(const void* q, const void* k_cache, const void* v
     while ((1 << page_shift) < page_size) ++page_shift;
     const Inputs in{(const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, tables, cu_q, ctx_lens, table_width, heads, kv_heads,
                     page_shift, total_pages, scale, window, keep_first, softcap, sinks, out_gate, gate_ld, gate_elements, (bf16*)out, out_ld,
-                    nullptr, nullptr, 0, 0, 0, 0};
+                    nullptr, nullptr, 0, 0, 0, 0, 0};
     return launch_packed(in, num_seqs, max_q_len, err, stream);
 }
 #else
@@ -491,7 +655,8 @@ IE_API int ie_attention_flat(const void* q, const void* q_rot, int q_rot_ld, con
         return (int)cudaErrorInvalidValue;
     const bf16* k = (const bf16*)kv;
     const Inputs in{(const bf16*)q, k, k + (size_t)heads * (D - 64), nullptr, cu_q, ctx_lens, 0, heads, heads, 0, 0, scale, 0, 0, 0.f, sinks,
-                    out_gate, gate_ld, 0, (bf16*)out, heads * DV, (const bf16*)q_rot, (const bf16*)k_rot, q_rot_ld, k_rot_ld, kv_ld, rot};
+                    out_gate, gate_ld, 0, (bf16*)out, heads * DV, (const bf16*)q_rot, (const bf16*)k_rot, q_rot_ld, k_rot_ld, kv_ld, rot, 0};
     return launch_packed(in, num_seqs, max_q_len, err, stream);
 }
+#endif
 #endif

@@ -185,6 +185,18 @@ def build_packed_attention(dim: int, vdim: int) -> Path:
     return build_library(f"ie_b200_packed_d{dim}_v{vdim}", ["attention_packed.cu"], [f"-DPA_D={dim}", f"-DPA_DV={vdim}"])
 
 
+PROMPT_ATTENTION_SIZES = (64, 128)  # head sizes whose plain prompt attention it is built for
+
+
+def build_prompt_attention(head_dim: int) -> Path:
+    """The same for plain softmax attention of one head size: a step's portions in one launch, their keys shared among blocks
+    (compiled on first use)."""
+    if head_dim not in PROMPT_ATTENTION_SIZES:
+        raise BuildError(f"the tcgen05 prompt attention takes head sizes {PROMPT_ATTENTION_SIZES}, not {head_dim}")
+    return build_library(f"ie_b200_prompt_d{head_dim}", ["attention_packed.cu"],
+                         [f"-DPA_D={head_dim}", f"-DPA_DV={head_dim}", "-DPA_PROMPT=1"])
+
+
 # (unrotated key entries, value size) of latent attention heads whose expanded form it is built for -> its key size
 FLAT_ATTENTION_SIZES = {(64, 64): 128, (128, 128): 192}
 
@@ -270,6 +282,7 @@ def build_all(prune: bool = True) -> list[Path]:
                  build_retention(64, 64), build_state_space(64, 64), build_latent_attention(320, 256)]
         libs += list(pool.map(lambda sizes: build_packed_attention(*sizes), PACKED_ATTENTION_SIZES))
         libs += list(pool.map(lambda sizes: build_flat_attention(*sizes), FLAT_ATTENTION_SIZES))
+        libs += list(pool.map(build_prompt_attention, PROMPT_ATTENTION_SIZES))
     if prune:
         keep = {lib.name for lib in libs}
         for old in build_dir().glob("libie_b200_*.so"):

@@ -18,8 +18,8 @@ import os
 from ctypes import c_float, c_int, c_void_p
 from typing import Any
 
-from .build import (ATTENTION_HEAD_DIMS, FLAT_ATTENTION_SIZES, PACKED_ATTENTION_SIZES, build_attention, build_core,
-                    build_flat_attention, build_latent_attention, build_packed_attention, build_part_library, build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
+from .build import (ATTENTION_HEAD_DIMS, FLAT_ATTENTION_SIZES, PACKED_ATTENTION_SIZES, PROMPT_ATTENTION_SIZES, build_attention, build_core,
+                    build_flat_attention, build_latent_attention, build_packed_attention, build_part_library, build_prompt_attention, build_retention, build_sigmoid_attention, build_sink_attention, build_state_space,
                     latent_attention_fits)
 
 _ERRORS = {
@@ -149,6 +149,7 @@ class CudaOps:
         self.sink_tc5 = os.environ.get("IE_B200_SINK_TC5", "1") != "0"  # ... of prompt portions on tcgen05
         self._packed_libs: dict[tuple[int, int], object] = {}
         self._flat_libs: dict[tuple[int, int], object] = {}
+        self._prompt_libs: dict[int, object] = {}
         # the latent attention of prompts with keys and values expanded per head ("0": always moved to the query side)
         self.latent_expand = os.environ.get("IE_B200_LATENT_EXPAND", "1") != "0"
         # residual gates' products as partial sums: faster by themselves, slower inside a captured step
@@ -159,6 +160,7 @@ class CudaOps:
         self._retired_tickets = []
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.attn_tc5 = os.environ.get("IE_B200_ATTN_TC5", "1") != "0"  # tcgen05 prefill attention
+        self.prompt_packed = os.environ.get("IE_B200_PROMPT_PACKED", "1") != "0"  # of these the kernel that packs a group's heads
         self.latent_mma = os.environ.get("IE_B200_LATENT_MMA", "1") != "0"  # tensor-core latent attention
         self.headwise_mma = os.environ.get("IE_B200_HEADWISE_MMA", "1") != "0"  # its per-head products of few rows
         self.prefill_key_splits = os.environ.get("IE_B200_PREFILL_KEY_SPLITS", "1") != "0"
@@ -761,6 +763,86 @@ class CudaOps:
         best = next(ks for ks in range(1, limit + 1) if cost(ks) <= 1.05 * least)  # (the fewest shares among the near-best)
         return best if cost(best) <= 0.75 * cost(1) else 1
 
+    def prompt_shares(self, tiles, nkv: int, fit) -> int:
+        """Into how many parts the packed prompt kernel cuts the key tiles of its blocks of 256 rows (``tiles``: of each block, per
+        key/value head), a cluster of blocks for each: what costs least by this estimate, in key tiles one SM walks.  ``fit(parts)``:
+        how many clusters of so many the device runs at one time.  A block's start and end are worth five, adding the parts three.
+        Blocks that run at one time take as long as the longest, others an even share and half a longest one."""
+        if not tiles:
+            return 1
+
+        def cost(parts: int) -> float:
+            slots = (fit(parts) or self.sm_count // parts) if parts > 1 else self.sm_count
+            longest = -(-max(tiles) // parts) + 5 + (3 if parts > 1 else 0)
+            if len(tiles) * nkv <= slots:
+                return longest
+            return sum(-(-n // parts) + longest - -(-max(tiles) // parts) for n in tiles) * nkv / slots + longest / 2
+
+        best = min(range(1, max(1, min(8, max(tiles))) + 1), key=cost)
+        return best if cost(best) <= 0.9 * cost(1) else 1
+
+    def prompt_packs(self, hd: int, blocks: int, max_ctx: int, longest) -> bool:
+        """Whether prompt portions go to the kernel that packs a group's heads into blocks of 256 rows, rather than the one of 128
+        tokens of one head a block (``blocks``: how many of the latter; ``longest``: the longest portion, if the step says).  A block
+        of the former costs two to three microseconds more to start and end and gets through its keys faster: with
+        128 entries a head, 32 heads on 8, 64 tokens 7.2 us against 4.6, 256 tokens 10.6 against 7.9 (one
+        round of either), 512 tokens 14.5 against 16.6, eight prompts of 256 20.8 against 36.4, 2,048 tokens 41.8 against 85.4; with 64 entries
+        1,024 tokens 19.1 against 18.2, eight prompts of 256 16.8 against 14.8, 2,048 tokens 35.4 against 38.7, 8,192 374 against 424, and,
+        as its clusters share keys at less cost, 17 tokens behind 1,000 7.9 against 13.0, 128 behind 2,048 14.2 against 18.3."""
+        if hd == 128:
+            return max_ctx >= 1024 or 2 * blocks > self.sm_count
+        return max_ctx >= (1024 if longest is not None and 2 * longest <= max_ctx else 2048)
+
+    def _prompt_clusters(self, hd: int, parts: int) -> int:
+        key = (hd, -parts)
+        if key not in self._cluster_fit:
+            self._cluster_fit[key] = int(self._prompt_lib(hd).ie_attention_prompt_clusters(parts))
+        return self._cluster_fit[key]
+
+    def _prompt_lib(self, hd: int):
+        lib = self._prompt_libs.get(hd)
+        if lib is None:
+            path = build_prompt_attention(hd)
+            try:
+                lib = ctypes.CDLL(str(path))
+            except OSError as exc:
+                raise KernelError(f"the kernel library {path} could not be loaded: {exc}") from exc
+            P, I, F = c_void_p, c_int, c_float
+            lib.ie_attention_prompt.argtypes = [P, P, P, P, I, P, P, P, I, I, I, I, I, I, F, I, I, P, P]
+            lib.ie_attention_prompt.restype = c_int
+            lib.ie_attention_prompt_clusters.argtypes = [I]
+            lib.ie_attention_prompt_clusters.restype = c_int
+            self._prompt_libs[hd] = lib
+        return lib
+
+    def _prompt_plan(self, plan, ctx, groups: int, nkv: int, hd: int, window: int):
+        """The packed prompt kernel's blocks of 256 rows per key/value head, and into how many parts their keys are cut."""
+        rows, bounds = 256, getattr(ctx, "bounds", None)
+        if bounds is not None:  # (a captured step: decided from its bounds alone)
+            tokens, seqs, max_ctx = bounds
+            blocks, likely = seqs + tokens * groups // rows, [max_ctx] * (tokens * groups // rows + min(seqs, 2))
+        else:
+            likely = []
+            for n, start, small in zip(ctx.q_lens, ctx.start_positions, plan["small"]):
+                if not small:
+                    likely += [start + -(-min(r + rows, n * groups) // groups) for r in range(0, n * groups, rows)]
+            blocks = len(likely)
+        if not self.prefill_key_splits:
+            return blocks, 1
+        reach = window + rows // groups if window else 0
+        return blocks, self.prompt_shares([-(-(min(last, reach) if window else last) // 64) for last in likely], nkv,
+                                          lambda parts: self._prompt_clusters(hd, parts))
+
+    def _prompt_attention(self, plan, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd, page_size, scale, window, out) -> None:
+        if (nkv, window) not in plan:  # (once for all layers of the step that are alike)
+            plan[nkv, window] = self._prompt_plan(plan, ctx, nh // nkv, nkv, hd, window)
+        blocks, shares = plan[nkv, window]
+        self._check(self._prompt_lib(hd).ie_attention_prompt(
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+            ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, blocks, nh, nkv, page_size, k_cache.shape[0],
+            scale, window, shares, self._err_ptr, self._stream()), "attention_prefill_tc5")
+        self.launch_counts["attention_prefill_packed"] = self.launch_counts.get("attention_prefill_packed", 0) + 1
+
     def paged_attention(self, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd, page_size,
                         scale, window, out, ragged: bool | None = None, value_dim: int | None = None, sinks=None) -> None:
         """Attention of every token of the step over its request's cached keys and values.
@@ -871,6 +953,10 @@ class CudaOps:
         tiles = plan["tiles"]
         fixed = "max_ctx" in plan  # a launch of fixed size: nothing is decided from the step's own lengths
         max_ctx = plan["max_ctx"] if fixed else ctx.max_ctx_len
+        if (self.attn_tc5 and self.prompt_packed and hd in PROMPT_ATTENTION_SIZES and page_size & (page_size - 1) == 0
+                and self.prompt_packs(hd, (plan["likely_tiles"] if fixed else tiles) * nh, max_ctx, None if fixed else max(ctx.q_lens))
+                and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16):
+            return self._prompt_attention(plan, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd, page_size, scale, window, out)
         if self.attn_tc5 and lib.ie_attention_prefill_tc5_ok(page_size, max_ctx):
             # Head sizes 64 and 128, pages of 8 tokens or more: the tcgen05 / TMEM / TMA kernel.
             # While the blocks would fill the GPU less than about twice, a block takes two tiles

@@ -131,3 +131,43 @@ def test_scores_that_grow_along_the_keys():
     ops.sink_attention(q.view(n, -1), k, v, tables, _Ctx([n], [0]), heads, 1, dim, dim, 16, 1.0, None, None, None, out)
     want = _want(q, [(kk, vv)], [n], [0], 1.0, None, 0, None, None, None).view(n, -1)
     assert float((out.double() - want).norm() / want.norm()) < REL
+
+
+@pytest.mark.parametrize("dim,heads,kv_heads", [(64, 6, 2), (64, 2, 2), (128, 8, 1), (128, 4, 2)])
+@pytest.mark.parametrize("lens,starts", [([17], [0]), ([129, 1, 65], [0, 500, 63]), ([40, 300], [1500, 129]), ([700], [0])])
+@pytest.mark.parametrize("window,page", [(0, 16), (100, 8), (1, 1), (0, 64)])
+@pytest.mark.parametrize("shares", [1, 2, 3, 8])
+def test_prompt_portions_and_shared_keys(monkeypatch, dim, heads, kv_heads, lens, starts, window, page, shares):
+    """Plain attention: all portions in one launch, key tiles cut among the blocks of a cluster (some parts empty).  A weight and a
+    result are each rounded by 2^-9 at most, which is 2^-8 in all and, where values cancel in a row, twice that."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops = get_ops()
+    q, k, v, tables, rows = _case(lens, starts, heads, kv_heads, dim, dim, page, window or None, 0, dim + page)
+    ctx, n = _Ctx(lens, starts), q.shape[0]
+    ctx.start_positions, ctx.max_ctx_len = starts, max(a + b for a, b in zip(lens, starts))
+    monkeypatch.setattr(ops, "prompt_packs", lambda *_: True)
+    monkeypatch.setattr(ops, "prompt_shares", lambda *_: shares)
+    out, before = torch.full((n, heads * dim), 7.0, dtype=torch.bfloat16, device="cuda"), ops.launch_counts.get("attention_prefill_packed", 0)
+    ops.paged_attention(q.view(n, -1), k, v, tables, ctx, heads, kv_heads, dim, page, dim ** -0.5, window, out)
+    ops.check_errors()
+    assert ops.launch_counts.get("attention_prefill_packed", 0) == before + 1
+    want, got = _want(q, rows, lens, starts, dim ** -0.5, window or None, 0, None, None, None).view(n, -1), out.double()
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -8
+    assert float(((got - want).norm(dim=1) / want.norm(dim=1)).max()) < 2.0 ** -7
+
+
+def test_a_fixed_launch_serves_shorter_steps():
+    """Bounds for 256 tokens of 4 requests over 2,048 positions, a step of less: blocks without rows leave, parts may be empty."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, lens, starts = get_ops(), [100, 1, 20], [30, 700, 0]
+    for dim in (64, 128):
+        q, k, v, tables, rows = _case(lens, starts, 8, 2, dim, dim, 16, None, 0, dim)
+        ctx, n = _Ctx(lens, starts), q.shape[0]
+        ctx.bounds = (256, 4, 2048)
+        out = torch.full((n, 8 * dim), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(q.view(n, -1), k, v, tables, ctx, 8, 2, dim, 16, dim ** -0.5, 0, out)
+        ops.check_errors()
+        want = _want(q, rows, lens, starts, dim ** -0.5, None, 0, None, None, None).view(n, -1)
+        assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -8
