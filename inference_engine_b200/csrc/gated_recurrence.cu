@@ -196,7 +196,7 @@ lowrank_decay_kernel(const float* __restrict__ y, int y_ld, const float* __restr
                      const float* __restrict__ bias, float inv_tau, float* __restrict__ decay, int num_tokens,
                      int channels, int rank) {
     __shared__ float ws[128 * (LD_RANKS + 1)];
-    __shared__ float ys[LD_TOKENS * LD_RANKS];
+    __shared__ __align__(16) float ys[LD_TOKENS * LD_RANKS];
     ie_pdl_trigger();
     ie_pdl_wait();
     int n0 = blockIdx.x * LD_TOKENS, c0 = blockIdx.y * 128;
@@ -208,6 +208,7 @@ lowrank_decay_kernel(const float* __restrict__ y, int y_ld, const float* __restr
     for (int r0 = 0; r0 < rank; r0 += LD_RANKS) {
         int width = min(LD_RANKS, rank - r0);
         if (r0 > 0) __syncthreads();  // everyone is done with the last piece
+#pragma unroll 8
         for (int row = warp; row < 128; row += 4) {
             int c = c0 + row;
             ws[row * (LD_RANKS + 1) + lane] = (c < channels && lane < width) ? w2[(size_t)c * rank + r0 + lane] : 0.f;
@@ -215,11 +216,20 @@ lowrank_decay_kernel(const float* __restrict__ y, int y_ld, const float* __restr
         for (int t = warp; t < LD_TOKENS; t += 4)
             ys[t * LD_RANKS + lane] = (t < cnt && lane < width) ? y[(size_t)(n0 + t) * y_ld + r0 + lane] : 0.f;
         __syncthreads();
-        const float* wrow = ws + threadIdx.x * (LD_RANKS + 1);
-        for (int r = 0; r < width; ++r) {
-            float wv = wrow[r];
+        // (the channel's weights in registers, four tokens' sums side by side, each in rising order; ranks beyond the last are zeros)
+        float wv[LD_RANKS];
 #pragma unroll
-            for (int t = 0; t < LD_TOKENS; ++t) acc[t] = fmaf(wv, ys[t * LD_RANKS + r], acc[t]);
+        for (int r = 0; r < LD_RANKS; ++r) wv[r] = ws[threadIdx.x * (LD_RANKS + 1) + r];
+#pragma unroll
+        for (int t = 0; t < LD_TOKENS; t += 4) {
+#pragma unroll
+            for (int r = 0; r < LD_RANKS; r += 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 yv = *reinterpret_cast<const float4*>(ys + (t + i) * LD_RANKS + r);
+                    acc[t + i] = fmaf(wv[r + 3], yv.w, fmaf(wv[r + 2], yv.z, fmaf(wv[r + 1], yv.y, fmaf(wv[r], yv.x, acc[t + i]))));
+                }
+            }
         }
     }
     int c = c0 + threadIdx.x;
