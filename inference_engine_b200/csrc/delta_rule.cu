@@ -113,11 +113,12 @@ delta_prep_kernel(const float* __restrict__ qkvb, int ld, const float* __restric
 
 // The same for many tokens.  grid: (blocks of PT_TOKENS tokens, units); a thread takes a channel of the unit through its block's
 // tokens, so an input is read once and not once per tap, and sixteen loads are on their way at once (2,048 tokens of 16 heads of
-// 128 x 128: 147 us a token at a time, bound by the units' chains of loads and barriers).  q and k: `dim` at most 128, one
+// 128 x 128: 147 us a token at a time, bound by the units' chains of loads and barriers; 102 with three blocks an SM, whose 168
+// registers a thread left too few loads in flight; 63 with five).  q and k: `dim` at most 128, one
 // channel per thread, whose squares sixteen tokens add up together (every exchange halves the sums a lane still holds).
 constexpr int PT_TOKENS = 16;
 template <int TAPS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 5)
 delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __restrict__ a,
                        const float* __restrict__ conv_w, const float* __restrict__ A_log,
                        const float* __restrict__ dt_bias, const float* __restrict__ state, long long state_stride,
@@ -229,13 +230,16 @@ delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __re
         if (!(lane & 1)) red[tid >> 5][lane >> 1] = part[0];
         __syncthreads();
         const bool is_q = unit < kv_heads;
-        const float scale = is_q ? 1.0f / sqrtf((float)dim) : 1.0f;
+        if (tid < PT_TOKENS) {  // (a token's factor once, over one of the sums that this thread alone reads)
+            float f = 1.0f / sqrtf(((red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid])) + 1e-6f);
+            if (is_q) f *= 1.0f / sqrtf((float)dim);
+            red[0][tid] = f;
+        }
+        __syncthreads();
         float* dst = (is_q ? q_out : k_out) + (size_t)n0 * qk + (is_q ? unit : unit - kv_heads) * dim + i0;
 #pragma unroll
         for (int i = 0; i < PT_TOKENS; ++i) {
-            float f = 1.0f / sqrtf(((red[0][i] + red[1][i]) + (red[2][i] + red[3][i])) + 1e-6f);
-            if (is_q) f *= scale;
-            if (live && i < cnt) dst[(size_t)i * qk] = y[i] * f;
+            if (live && i < cnt) dst[(size_t)i * qk] = y[i] * red[0][i];
         }
     }
 }
