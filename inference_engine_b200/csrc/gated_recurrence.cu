@@ -617,6 +617,37 @@ recurrence_readout_kernel(const float* __restrict__ o, int cols, const float* __
     const float* src = o + row * cols;
     float den = 1.0f;
     if (gates != nullptr) den = fmaxf(fabsf(src[vdim]), gates[row * 3 + 2]) + 1e-6f;
+    const float* wrow = weight != nullptr && weight_per_head ? weight + (size_t)head * vdim : weight;
+    constexpr int HELD = 4;
+    if (vdim <= 32 * HELD) {
+        // up to 128 values: read once, gates and weights beside them, no division by a 1 (2,000 tokens of 16 heads of 128: 14 us; 29 with every
+        // value read and divided twice and the gates asked for behind the sum)
+        float x[HELD], g[HELD], w[HELD], ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < HELD; ++k) {
+            const int d = lane + 32 * k;
+            const bool in = d < vdim;
+            x[k] = in ? src[d] : 0.f;
+            g[k] = in && gate_pre != nullptr ? gate_pre[n * gate_ld + (size_t)head * vdim + d] : 0.f;
+            w[k] = in && weight != nullptr ? wrow[d] : 1.f;
+        }
+#pragma unroll
+        for (int k = 0; k < HELD; ++k) {
+            if (gates != nullptr) x[k] /= den;
+            ss = fmaf(x[k], x[k], ss);
+        }
+        ss = warp_sum(ss);
+        const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
+#pragma unroll
+        for (int k = 0; k < HELD; ++k) {
+            const int d = lane + 32 * k;
+            float y = x[k] * inv;
+            if (weight != nullptr) y *= w[k];
+            if (gate_pre != nullptr) y *= gate_silu ? silu_f(g[k]) : sigmoid_f(g[k]);
+            if (d < vdim) ie_store(out + row * vdim + d, y);
+        }
+        return;
+    }
     float ss = 0.f;
     for (int d = lane; d < vdim; d += 32) {
         float x = src[d] / den;
@@ -624,7 +655,6 @@ recurrence_readout_kernel(const float* __restrict__ o, int cols, const float* __
     }
     ss = warp_sum(ss);
     float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
-    const float* wrow = weight != nullptr && weight_per_head ? weight + (size_t)head * vdim : weight;
     for (int d = lane; d < vdim; d += 32) {
         float y = (src[d] / den) * inv;
         if (weight != nullptr) y *= wrow[d];
