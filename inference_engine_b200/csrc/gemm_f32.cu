@@ -24,8 +24,9 @@ __device__ __forceinline__ unsigned long long twice(float x) {
 }
 
 // A block: BM rows x 64 columns, 8 x 16 threads; a thread TM = BM / 8 rows (in pairs) x 4 columns.  The next 16 of k are fetched into registers
-// while these are worked on.  Whatever the tile, an output is the same chain over k.  (377 x 1,024 by 1,536 and 1,024: tiles of 64 x 64 with
-// 4 x 4 a thread, one block per SM and nothing fetched ahead took 56 us each; these, 32 rows a block there, 40.)
+// while these are worked on.  Whatever the tile, an output is the same chain over k.  (By 1,024 of k, with the tiles of 64 x 64,
+// 4 x 4 a thread and nothing fetched ahead that were here, and with these, us: 8 rows by 4,096 53 and 33, 377 by 1,536 55 and 51, 2,048 by
+// 2,048 258 and 208.  Reads of shared memory bound them: larger pieces a thread would leave SMs without a block.)
 template <int BM>
 __global__ void __launch_bounds__(THREADS)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K) {
