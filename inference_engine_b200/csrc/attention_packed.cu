@@ -216,11 +216,11 @@ attention_packed_kernel(const Inputs in, int* err) {
             if (block < blocks) { seq = i; break; }
             block -= blocks;
         }
-        if (seq < 0) return;
+        if (seq < 0) { ie_pdl_leave(); return; }
     }
     const int q0 = in.cu_q[seq], q_len = in.cu_q[seq + 1] - q0;
     const int row0 = block * ROWS, rows_total = q_len * group;
-    if (row0 >= rows_total) return;
+    if (row0 >= rows_total) { ie_pdl_leave(); return; }
     const int start = in.ctx_lens[seq] - q_len;  // position of the request's first token of this step
     const int rows_here = min(ROWS, rows_total - row0);
     const int first_pos = start + row0 / group, last_pos = start + (row0 + rows_here - 1) / group;

@@ -215,7 +215,7 @@ attention_prefill_tc5_kernel(const bf16* __restrict__ q, const __grid_constant__
         }
         item -= items;
     }
-    if (seq < 0) return;
+    if (seq < 0) { ie_pdl_leave(); return; }
     int ctx = ctx_lens[seq];
     const int* table = tables + (size_t)seq * table_width;
     int first_qpos = ctx - qlen;

@@ -56,8 +56,14 @@ __device__ __forceinline__ float warp_max(float v) {
 // ie_pdl_wait -- index arithmetic, prefetching weights, which no earlier kernel writes --
 // overlap the predecessor.  ie_pdl_wait returns when the predecessor grid has completed and its
 // writes are visible; every kernel calls it before its first read of activations and before any
-// global write, and every thread calls it, so "my predecessor is done" holds transitively.
+// global write, and every thread calls it, so "my predecessor is done" holds transitively.  Blocks that turn out to have no work
+// call ie_pdl_leave instead and return: a grid is complete only when all of its blocks are, so it is enough that the first one
+// waits, whatever it finds.  (Were all to wait, a thousand empty blocks of 200 KB of shared memory would start, in rounds, only when the
+// predecessor has ended: 12 decoding requests at 3,000 positions and a portion of 20 tokens in a captured step, 46 -> 57 us.)
 __device__ __forceinline__ void ie_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void ie_pdl_leave() {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) ie_pdl_wait();
+}
 __device__ __forceinline__ void ie_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::); }
 
 // 1 (default): launch with the programmatic-serialization attribute; 0: plain launches.

@@ -171,3 +171,48 @@ def test_a_fixed_launch_serves_shorter_steps():
         ops.check_errors()
         want = _want(q, rows, lens, starts, dim ** -0.5, None, 0, None, None, None).view(n, -1)
         assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("dim,packed", [(64, True), (128, True), (64, False), (128, False)])
+def test_a_captured_step_without_long_portions_waits_for_the_decode_attention(monkeypatch, dim, packed):
+    """Portions of two to four tokens (16 rows and fewer) beside decoded tokens of long contexts: a launch of fixed size holds the prompt
+    attention too, none of whose blocks has work.  The product behind it reads what the decode attention writes."""
+    from inference_engine_b200.engine.workspace import Workspace
+    from inference_engine_b200.kernels import get_ops
+
+    ops, heads, kv_heads = get_ops(), 8, 2
+    lens, starts = [2, 1, 4, 3, 1, 1], [5000, 7900, 3001, 6000, 8000, 7000]
+    q, k, v, tables, rows = _case(lens, starts, heads, kv_heads, dim, dim, 16, None, 0, dim + 9)
+    monkeypatch.setattr(ops, "prompt_packs", lambda *_: packed)
+    n, width, out_dim = q.shape[0], heads * dim, 512
+    w = torch.randn(out_dim, width, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda").bfloat16()
+    attended, ws = torch.zeros(n, width, dtype=torch.bfloat16, device="cuda"), Workspace("cuda", min_rows=n)
+
+    def step(bounds):
+        ctx = _Ctx(lens, starts)
+        ctx.start_positions, ctx.max_ctx_len, ctx.ws, ctx.bounds = starts, 8001, ws, bounds
+
+        def run():
+            ops.paged_attention(q.view(n, -1), k, v, tables, ctx, heads, kv_heads, dim, 16, dim ** -0.5, 0, attended)
+            return ops.linear(attended, w, ws=ws, tag="after", out_dtype=torch.float32)
+
+        return ctx, run
+
+    _, eager = step(None)
+    eager()
+    torch.cuda.synchronize()
+    want_rows = attended.double()
+    want = want_rows @ w.double().t()
+    reference = _want(q, rows, lens, starts, dim ** -0.5, None, 0, None, None, None).view(n, -1)
+    assert float((want_rows - reference).norm() / reference.norm()) < 2.0 ** -7
+    ctx, run = step((16, 8, 16384))  # (the context stays: its arrays are the captured launches' inputs)
+    run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    for i in range(50):
+        attended.fill_(math.nan)
+        graph.replay()
+        assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -7, f"replay {i}"
+    ops.check_errors()
