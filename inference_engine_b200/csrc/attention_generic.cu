@@ -64,29 +64,20 @@ __device__ __forceinline__ float dot_row(const float* __restrict__ q, const __nv
     return s;
 }
 
+// One query row by one warp, `qs`: hd floats of the warp's own.
 template <typename T>
-__global__ void __launch_bounds__(WARPS * 32)
-paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
-                               const T* __restrict__ v_cache, const int* __restrict__ block_tables,
-                               int table_width, const int* __restrict__ seq_of_token,
-                               const int* __restrict__ positions, T* __restrict__ out,
-                               int nh, int nkv, int hd, int hdv, int v_stride, int page_size, int total_pages,
-                               float scale, int window, int chunk, const float* __restrict__ head_bias,
-                               const float* __restrict__ sinks, const float* __restrict__ out_gate, int gate_ld,
-                               float softcap, int keep_first, int gate_elements, const float* __restrict__ log_r1,
-                               const float* __restrict__ log_r2, const float* __restrict__ bias_table, int bias_len,
-                               int out_ld, int* err) {
-    extern __shared__ float q_smem[];  // [WARPS][hd]
-    ie_pdl_trigger();
-    ie_pdl_wait();
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int head = blockIdx.x * WARPS + warp;
-    int token = blockIdx.y;
-    if (head >= nh) return;  // whole warp leaves together; no block-wide barrier below
+__device__ __forceinline__ void
+paged_attention_row(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+                    const int* __restrict__ block_tables, int table_width, int token, int head, int seq, int pos, int lane,
+                    float* qs, T* __restrict__ out,
+                    int nh, int nkv, int hd, int hdv, int v_stride, int page_size, int total_pages,
+                    float scale, int window, int chunk, const float* __restrict__ head_bias,
+                    const float* __restrict__ sinks, const float* __restrict__ out_gate, int gate_ld,
+                    float softcap, int keep_first, int gate_elements, const float* __restrict__ log_r1,
+                    const float* __restrict__ log_r2, const float* __restrict__ bias_table, int bias_len,
+                    int out_ld, int* err) {
     int kvh = head / (nh / nkv);
-    int seq = seq_of_token[token], pos = positions[token];
     const int* table = block_tables + (size_t)seq * table_width;
-    float* qs = q_smem + warp * hd;
     const T* qrow = q + ((size_t)token * nh + head) * hd;
     for (int d = lane; d < hd; d += 32) qs[d] = ie_load(qrow + d);
     __syncwarp();
@@ -166,15 +157,60 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
     }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(WARPS * 32)
+paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
+                               const T* __restrict__ v_cache, const int* __restrict__ block_tables,
+                               int table_width, const int* __restrict__ seq_of_token,
+                               const int* __restrict__ positions, T* __restrict__ out,
+                               int nh, int nkv, int hd, int hdv, int v_stride, int page_size, int total_pages,
+                               float scale, int window, int chunk, const float* __restrict__ head_bias,
+                               const float* __restrict__ sinks, const float* __restrict__ out_gate, int gate_ld,
+                               float softcap, int keep_first, int gate_elements, const float* __restrict__ log_r1,
+                               const float* __restrict__ log_r2, const float* __restrict__ bias_table, int bias_len,
+                               int out_ld, int* err) {
+    extern __shared__ float q_smem[];  // [WARPS][hd]
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int head = blockIdx.x * WARPS + warp;
+    int token = blockIdx.y;
+    if (head >= nh) return;  // whole warp leaves together; no block-wide barrier below
+    paged_attention_row(q, k_cache, v_cache, block_tables, table_width, token, head, seq_of_token[token], positions[token], lane,
+                        q_smem + warp * hd, out, nh, nkv, hd, hdv, v_stride, page_size, total_pages, scale, window, chunk, head_bias,
+                        sinks, out_gate, gate_ld, softcap, keep_first, gate_elements, log_r1, log_r2, bias_table, bias_len, out_ld, err);
+}
+
 // The same attention for prompt portions in 32-bit (plain softmax, all positions or a window): a block takes 32 (token, query head of the
 // group) rows of one request and key/value head and brings a tile of 32 keys once for all of them, where the kernel above reads a key
 // row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 72).  Every number is the same chain of operations as there: a
 // score one multiply-add after the other over the row, maxima and sums over a tile's 32 keys by the same exchanges (a warp
 // takes a row, a lane a key), the output's multiply-adds key by key; tiles a row does not see leave it as it is (its maximum stays, a factor
-// of 1, weights of 0).  So results are equal bit for bit, and a portion may be cut anywhere between the two kernels.
+// of 1, weights of 0).  So results are equal bit for bit, and a portion may be cut anywhere between the two kernels; where a value that some
+// row does not see is infinite or not a number, or a page is not there, the block's rows go that kernel's way.  (Masks in the walk
+// over the tiles: 2 to 10 % more time.)
 constexpr int T_ROWS = 32, T_KEYS = 32, T_THREADS = 128;
+
+// A block's rows by that kernel's own code, a warp a row.
 template <int HD>
-__global__ void __launch_bounds__(T_THREADS)
+__device__ __noinline__ void
+rows_one_by_one(const float* q, const float* k_cache, const float* v_cache, const int* block_tables, int table_width, int q0, int row0,
+                int rows_here, int start, int seq, int kvh, float* q_smem, float* out, int nh, int nkv, int page_size, int total_pages,
+                float scale, int window, int* err) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = nh / nkv;
+    for (int rr = row0 + warp; rr < row0 + rows_here; rr += T_THREADS / 32) {
+        const int token = rr / group, head = kvh * group + rr - token * group;
+        paged_attention_row<float>(q, k_cache, v_cache, block_tables, table_width, q0 + token, head, seq, start + token, lane,
+                                   q_smem + warp * HD, out, nh, nkv, HD, HD, HD, page_size, total_pages, scale, window, 0, nullptr, nullptr,
+                                   nullptr, 0, 0.f, 0, 0, nullptr, nullptr, nullptr, 0, nh * HD, err);
+        __syncwarp();
+    }
+}
+
+// (Two blocks an SM at least, which leaves the compiler its registers: with the 86 of its own choice a portion of 16 tokens behind 2,000
+// takes 299 us, with these 266.)
+template <int HD>
+__global__ void __launch_bounds__(T_THREADS, 2)
 paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                                 const int* __restrict__ block_tables, int table_width, const int* __restrict__ cu_q,
                                 const int* __restrict__ ctx_lens, float* __restrict__ out, int nh, int nkv, int page_size, int total_pages,
@@ -186,6 +222,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
     float* vs = ks + 2 * T_KEYS * LD;  // two of [32][HD]
     float* ps = vs + 2 * T_KEYS * HD;  // [32][LP]: scores, then weights
     float* alpha_s = ps + T_ROWS * LP; // [32]
+    int* missing_s = reinterpret_cast<int*>(alpha_s + T_ROWS);  // a key that some row sees has no page
     ie_pdl_trigger();
     ie_pdl_wait();
     const int seq = blockIdx.z, kvh = blockIdx.y, group = nh / nkv, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -195,6 +232,8 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
     const int first_pos = start + row0 / group, last_pos = start + (row0 + rows_here - 1) / group;
     const int lo_min = window > 0 ? max(first_pos - window + 1, 0) : 0;
     const int* table = block_tables + (size_t)seq * table_width;
+    if (tid == 0) *missing_s = 0;
+    __syncthreads();
     auto fetch = [&](int t0, int b) {  // four threads a key
         const int key = tid >> 2, pos = t0 + key;
         int row = -1;
@@ -202,6 +241,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
             const int page = table[pos / page_size];
             if (page < 0 || page >= total_pages) {
                 if ((tid & 3) == 0) ie_report(err, page < 0 ? IE_ERR_TABLE : IE_ERR_PAGE, page, q0 + row0 / group);
+                *missing_s = 1;
             } else {
                 row = (page * nkv + kvh) * page_size + pos % page_size;
             }
@@ -310,21 +350,27 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
         if (lane == 0 && r < rows_here) alpha_s[r] = l[i] > 0.f ? 1.0f / l[i] : 0.f;
     }
     __syncthreads();
+    // A hidden value has a weight of 0 and changes nothing, unless it is infinite or not a number: then an output is not a number.
+    float z = 0.f;
 #pragma unroll
     for (int i = 0; i < OR; ++i) {
         const int r = orow + RG * i, rr = row0 + r, token = rr / group;
         if (r >= rows_here) continue;
         const float f = alpha_s[r];
-        *reinterpret_cast<float4*>(out + ((size_t)(q0 + token) * nh + kvh * group + rr - token * group) * HD + od) =
-            make_float4(acc[i][0] * f, acc[i][1] * f, acc[i][2] * f, acc[i][3] * f);
+        const float4 o = make_float4(acc[i][0] * f, acc[i][1] * f, acc[i][2] * f, acc[i][3] * f);
+        z += (o.x + o.y + o.z + o.w) * 0.f;
+        *reinterpret_cast<float4*>(out + ((size_t)(q0 + token) * nh + kvh * group + rr - token * group) * HD + od) = o;
     }
+    if (__syncthreads_or(z != 0.f || *missing_s))
+        rows_one_by_one<HD>(q, k_cache, v_cache, block_tables, table_width, q0, row0, rows_here, start, seq, kvh, tile_smem, out, nh, nkv,
+                            page_size, total_pages, scale, window, err);
 }
 
 template <int HD>
 int launch_f32_tile(const float* q, const float* k, const float* v, const int* tables, int width, const int* cu_q, const int* ctx_lens,
                     float* out, int num_seqs, int max_q_len, int nh, int nkv, int page_size, int total_pages, float scale, int window,
                     int* err, cudaStream_t s) {
-    constexpr size_t smem = (size_t)(T_ROWS * (HD + 4) + 2 * T_KEYS * (HD + 4) + 2 * T_KEYS * HD + T_ROWS * (T_KEYS + 4) + T_ROWS) * sizeof(float);
+    constexpr size_t smem = (size_t)(T_ROWS * (HD + 4) + 2 * T_KEYS * (HD + 4) + 2 * T_KEYS * HD + T_ROWS * (T_KEYS + 4) + T_ROWS + 1) * sizeof(float);
     static IePerDevice allowed;
     cudaError_t e = ie_allow_smem(allowed, paged_attention_f32_tile_kernel<HD>, smem);
     if (e != cudaSuccess) return (int)e;
