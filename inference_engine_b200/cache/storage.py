@@ -32,25 +32,39 @@ class PagedStorage:
 HEADROOM_BYTES = 512 * 2**20  # left free beside the cache for activations and libraries' workspaces
 
 
-def pages_that_fit(paged_groups, page_size: int, dtype_bytes: int, device, utilization: float) -> int:
-    """How many pages per cache group the device has room for.  The engine may fill the
+SPARE_SHARE = 32  # of the room for the cache, one part in so many at most is kept for scratch that steps could do without
+
+
+def _room(device, utilization: float) -> tuple[float, int, int]:
+    """Bytes that the engine may still take, what is free and what the device has.  The engine may fill the
     fraction ``utilization`` of the device; what is taken already (weights, other processes)
-    counts against that, and ``HEADROOM_BYTES`` stay free.  Every group gets the same number
-    of pages, so a page costs the sum over the groups (the reference sizes its one pool the
-    same way, engine/runtime/engine.py:130-140)."""
+    counts against that, and ``HEADROOM_BYTES`` stay free."""
     import torch
 
+    free_now, capacity = torch.cuda.mem_get_info(device)
+    return utilization * capacity - (capacity - free_now) - HEADROOM_BYTES, free_now, capacity
+
+
+def pages_that_fit(paged_groups, page_size: int, dtype_bytes: int, device, utilization: float, spare: int = 0) -> int:
+    """How many pages per cache group the device has room for, beside ``spare`` bytes of scratch (or so many of them as
+    ``SPARE_SHARE`` allows).  Every group gets the same number of pages, so a page costs the sum over the groups
+    (the reference sizes its one pool the same way, engine/runtime/engine.py:130-140)."""
     if not str(device).startswith("cuda"):
         raise ValueError("pass num_blocks explicitly when not running on CUDA")
-    free_now, capacity = torch.cuda.mem_get_info(device)
-    taken = capacity - free_now
-    room = utilization * capacity - taken - HEADROOM_BYTES
+    room, free_now, capacity = _room(device, utilization)
+    room -= max(0, min(spare, room / SPARE_SHARE))
     page_bytes = sum(g.bytes_per_page(page_size, dtype_bytes) for g in paged_groups)
     pages = int(room // page_bytes) if page_bytes else 1
     if pages < 1:
         raise RuntimeError(f"no GPU memory left for the KV cache ({free_now / 2**30:.1f} GiB free of "
                            f"{capacity / 2**30:.1f}, gpu_memory_utilization {utilization})")
     return pages
+
+
+def spare_that_fits(device, utilization: float) -> int | None:
+    """Bytes of scratch that steps could do without that there is room for once the cache stands (None: not a device whose
+    memory is counted)."""
+    return max(0, int(_room(device, utilization)[0])) if str(device).startswith("cuda") else None
 
 
 class CacheStorage:

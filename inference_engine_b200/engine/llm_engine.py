@@ -23,7 +23,7 @@ from collections import deque
 from typing import Any
 
 from ..cache.manager import CacheManager
-from ..cache.storage import CacheStorage, pages_that_fit
+from ..cache.storage import CacheStorage, pages_that_fit, spare_that_fits
 from ..config.engine_config import EngineConfig
 from ..sampling.params import SamplingParams
 from ..sampling.sampler import Sampler
@@ -65,8 +65,10 @@ class LLMEngine:
         block_size, max_num_seqs = config.block_size, config.max_num_seqs
         num_blocks = config.num_blocks
         if num_blocks is None:
+            longest = min(config.max_model_len or model.spec.max_position_embeddings, model.env.max_positions)
+            spare = model.spare_scratch_bytes(ops, config.max_num_batched_tokens, max_num_seqs, max_num_seqs * longest)
             num_blocks = pages_that_fit(model.paged_groups, block_size, 2 if self.dtype == "bfloat16" else 4,
-                                        self.device, config.gpu_memory_utilization)
+                                        self.device, config.gpu_memory_utilization, spare)
         self.max_model_len = min(config.max_model_len or model.spec.max_position_embeddings,
                                  num_blocks * block_size if model.paged_groups else 2**62,
                                  model.env.max_positions)
@@ -76,6 +78,7 @@ class LLMEngine:
         self.storage = CacheStorage(self.cache, model.env.torch_dtype, self.device)
         self.runner = ModelRunner(model, self.cache, self.storage, ops, self.device,
                                   config.max_num_batched_tokens, max_num_seqs)
+        self.runner.ws.spare_bytes = spare_that_fits(self.device, config.gpu_memory_utilization)
         self.scheduler = Scheduler(self.cache, max_num_seqs, config.max_num_batched_tokens,
                                    config.enable_chunked_prefill)
         self.sampler = Sampler(ops, self.device, model.spec.vocab_size)

@@ -145,6 +145,14 @@ class Model:
         per_request = sum(g.num_layers * math.prod(g.shape) for g in self.state_groups)
         return Footprint(parameters, per_token, per_request)
 
+    def spare_scratch_bytes(self, ops, tokens: int, seqs: int, context: int) -> int:
+        """Scratch that the parts' faster ways take at most and could do without (``Part.spare_scratch``)."""
+        most: dict[str, int] = {}
+        for part in self.all_parts():
+            for what, count in part.spare_scratch(ops, tokens, seqs, context).items():
+                most[what] = max(most.get(what, 0), count)
+        return sum(most.values())
+
     # --- forward ----------------------------------------------------------------------------
 
     def forward(self, ctx, logit_rows):

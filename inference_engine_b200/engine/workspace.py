@@ -4,6 +4,9 @@ Every intermediate of a step is a view of a buffer that was allocated once for t
 tokens a step may hold, so steady-state steps allocate nothing and a captured launch
 sequence keeps reading and writing the same addresses.  ``version`` changes whenever a
 buffer had to be replaced by a larger one; whoever captured addresses must capture again.
+
+Beside these there is scratch that a faster way through a step takes and another way does without
+(``spare``): it grows by doubling and stays within ``spare_bytes`` altogether.
 """
 
 from __future__ import annotations
@@ -15,6 +18,9 @@ class Workspace:
         self._buffers: dict[str, object] = {}
         self._views: dict[tuple, tuple] = {}  # last view handed out per buffer
         self.version = 0
+        self.spare_bytes: int | None = None  # what all spare scratch may take (None: whatever is asked for)
+        self._spare: dict = {}  # its buffers' bytes
+        self._addressed: set = set()  # spare scratch whose addresses a capture may hold
 
     def buffer(self, name: str, rows: int, cols: int, dtype, rows_cap: int | None = 0):
         """A ``[rows, cols]`` view named ``name``.  Capacity is at least ``min_rows`` rows
@@ -36,6 +42,50 @@ class Workspace:
         view = buf[:need].view(rows, cols)
         self._views[key] = (rows, cols, view)
         return view
+
+    def _spare_plan(self, wants):
+        """Elements of each buffer that ``wants`` leads to (doubled where one grows, if that much may be taken), or None."""
+        buffers = self._buffers
+        held = [buffers.get((name, dtype)) for name, _, dtype in wants]
+        if all(buf is not None and buf.numel() >= want[1] for buf, want in zip(held, wants)):
+            return {want[::2]: buf.numel() for buf, want in zip(held, wants)}
+        for grown in (lambda n: 1 << max(int(n) - 1, 0).bit_length(), int):
+            plan = {want[::2]: buf.numel() if buf is not None and buf.numel() >= want[1] else grown(max(want[1], 1))
+                    for buf, want in zip(held, wants)}
+            total = sum({**self._spare, **{key: n * key[1].itemsize for key, n in plan.items()}}.values())
+            if self.spare_bytes is None or total <= self.spare_bytes:
+                return plan
+        return None
+
+    def has_spare(self, wants) -> bool:
+        """Whether :meth:`spare` would hand out ``wants``."""
+        return self._spare_plan(wants) is not None
+
+    def spare(self, wants, captured: bool = True):
+        """Flat views of spare scratch for ``wants`` (name, elements, dtype), or None where that would be more than
+        ``spare_bytes``.  ``captured=False``: scratch of steps that are launched one kernel at a time alone, whose growth
+        leaves captured addresses as they are."""
+        import torch
+
+        plan = self._spare_plan(wants)
+        if plan is None:
+            return None
+        captured = captured or (str(self.device).startswith("cuda") and torch.cuda.is_current_stream_capturing())
+        views = []
+        for name, elements, dtype in wants:
+            key = (name, dtype)
+            buf = self._buffers.get(key)
+            if buf is None or buf.numel() < plan[key]:
+                if buf is not None and key in self._addressed:
+                    self.version += 1
+                buf = self._buffers.pop(key, None)
+                del buf  # (given back first: the larger one may need its place)
+                buf = self._buffers[key] = torch.empty(plan[key], dtype=dtype, device=self.device)
+                self._spare[key] = buf.numel() * buf.element_size()
+            if captured:
+                self._addressed.add(key)
+            views.append(buf[:elements])
+        return views
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

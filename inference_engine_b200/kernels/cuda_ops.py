@@ -1087,10 +1087,26 @@ class CudaOps:
         for a, n in zip(starts, ctx.q_lens):
             context += a + n
             pairs += n * (2 * a + n) // 2
-        if context * heads * (dim + vdim) > 1 << 30:  # (2 GB of expanded keys and values)
+        ws = getattr(ctx, "ws", None)
+        if (context * heads * (dim + vdim) > self.EXPANDED_MOST
+                or ws is not None and not ws.has_spare(self._expanded_wants(context, heads, dim, rot_dim, vdim, rank))):
             return False
         moved = pairs * heads * (3 * rank + rot_dim) * 2 / 190e6
         return moved > context * rank * heads * (dim + vdim) * 2 / 900e6 + pairs * heads * (dim + rot_dim + 2 * vdim) * 2 / 350e6 + 20
+
+    EXPANDED_MOST = 1 << 30  # entries of expanded keys and values (2 GB)
+
+    def _expanded_wants(self, context: int, heads: int, dim: int, rot_dim: int, vdim: int, rank: int):
+        """The scratch of the expanded latent attention for so many tokens of context."""
+        bf16 = self.torch.bfloat16
+        return [("latent.context", context * (rank + rot_dim), bf16), ("latent.expanded", context * heads * (dim + vdim), bf16)]
+
+    def latent_scratch_bytes(self, context: int, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> int:
+        """The most of it that steps over ``context`` tokens of requests can take."""
+        if not self.latent_expand or (dim, vdim) not in FLAT_ATTENTION_SIZES:
+            return 0
+        context = min(context, self.EXPANDED_MOST // (heads * (dim + vdim)))
+        return sum(2 * n for _, n, _ in self._expanded_wants(context, heads, dim, rot_dim, vdim, rank))
 
     def _flat_lib(self, dim: int, vdim: int):
         lib = self._flat_libs.get((dim, vdim))
@@ -1124,9 +1140,12 @@ class CudaOps:
         self.latent_prep(positions, table, rot_dims, heads=heads, dim=dim, rot_dim=rot_dim, rank=rank, page_size=page_size,
                          interleaved=interleaved, q=q, q_plain=plain, q_abs=turned)
         total = sum(ctx.start_positions) + sum(ctx.q_lens)
-        rows = ws.buffer("latent.context", total, row, out.dtype, rows_cap=None)
+        # (captured steps never expand: these may grow without their addresses going stale)
+        scratch = ws.spare(self._expanded_wants(total, heads, dim, rot_dim, vdim, rank), captured=False)
+        if scratch is None:
+            raise KernelError(f"latent_expanded: no scratch for {total} tokens of context (latent_expands says when)")
+        rows, kv = scratch[0].view(total, row), scratch[1].view(total, heads * (dim + vdim))
         self._gather_context_rows(cache, block_tables, ctx, page_size, rows)
-        kv = ws.buffer("latent.expanded", total, heads * (dim + vdim), out.dtype, rows_cap=None)
         self._expand_latent(rows[:, :rank], w_kv, kv)
         self._flat_attention(plain, turned[:, rank:], row, kv, rows[:, rank:], row, rot_dim, ctx, out, heads, dim, vdim, scale, sinks,
                              gate_pre)
@@ -1361,8 +1380,16 @@ class CudaOps:
         lib = self._part_lib("chunked")
         if not lib.ie_chunked_ok(dim, vdim, int(delta)) or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows):
             return 0, None
-        floats = lib.ie_chunked_scratch(1, heads, dim, vdim, int(delta))
-        return chunks, ctx.ws.buffer("recurrence.chunks", chunks, floats, self.torch.float32, rows_cap=None)
+        floats = lib.ie_chunked_scratch(chunks, heads, dim, vdim, int(delta))
+        scratch = ctx.ws.spare([("recurrence.chunks", floats, self.torch.float32)])
+        return (0, None) if scratch is None else (chunks, scratch[0])
+
+    def chunk_scratch_bytes(self, tokens: int, seqs: int, heads: int, dim: int, vdim: int, delta: bool) -> int:
+        """The most scratch that steps of so many tokens and requests take in chunks."""
+        lib = self._part_lib("chunked")
+        if not lib.ie_chunked_ok(dim, vdim, int(delta)):
+            return 0
+        return 4 * lib.ie_chunked_scratch(tokens // self.CHUNK + seqs, heads, dim, vdim, int(delta))
 
     @_kind("delta.rule")
     def delta_rule(self, q, k, v, beta, decay, state, slots, ctx, out, heads, kv_heads, dim, vdim,

@@ -127,6 +127,11 @@ class Part:
         """Nested parts (a block returns its mixer, feed-forward and norms)."""
         return []
 
+    def spare_scratch(self, ops, tokens: int, seqs: int, context: int) -> dict[str, int]:
+        """Bytes of scratch, by what it is for, that the part's faster ways take at most in steps of so many tokens and
+        requests over ``context`` tokens in all, and that it does without where there is no room (parts of one kind share it)."""
+        return {}
+
 
 class PositionEncoding(Part):
     category = "position"

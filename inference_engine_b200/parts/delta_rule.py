@@ -23,7 +23,7 @@ with 32-bit sums.
 from __future__ import annotations
 
 from .base import BuildEnv, CacheBinding, Mixer, StateRequest, WeightDecl
-from .recurrent import long_portions
+from .recurrent import long_portions, portion_scratch
 from .registry import register_part
 
 
@@ -79,6 +79,9 @@ class ChannelDeltaRule(Mixer):
         self.w_a1, self.w_a2, self.w_g1, self.w_g2, self.w_o = mat("a1"), mat("a2"), mat("g1"), mat("g2"), mat("o")
         self.conv = torch.cat([vec("q_conv"), vec("k_conv"), vec("v_conv")]).contiguous()  # [channels, taps]
         self.A_log, self.dt_bias, self.out_norm = vec("A_log"), vec("dt_bias"), vec("out_norm")
+
+    def spare_scratch(self, ops, tokens, seqs, context):
+        return portion_scratch(ops, self.dtype, tokens, seqs, self.heads, self.dim, self.vdim, delta=True)
 
     def cache_request(self) -> StateRequest:
         return StateRequest((self.matrix_floats + (self.taps - 1) * self.channels,))

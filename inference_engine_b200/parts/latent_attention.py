@@ -101,6 +101,13 @@ class LatentAttention(Mixer):
         if "sink" in n:
             self.sinks = tensors[n["sink"]].float().contiguous()
 
+    def spare_scratch(self, ops, tokens, seqs, context):
+        import torch
+
+        if self.dtype != torch.bfloat16 or not hasattr(ops, "latent_scratch_bytes"):
+            return {}
+        return {"latent keys and values": ops.latent_scratch_bytes(context, self.heads, self.dim, self.rot_dim, self.vdim, self.kv_rank)}
+
     def cache_request(self) -> PagedKVRequest:
         return PagedKVRequest(1, self.row, None, value_dim=0)
 

@@ -55,6 +55,13 @@ def long_portions(ops, dtype) -> dict:
     return {"in_chunks": True} if dtype != torch.float32 and getattr(ops, "takes_chunks", False) else {}
 
 
+def portion_scratch(ops, dtype, tokens: int, seqs: int, heads: int, dim: int, vdim: int, delta: bool = False) -> dict[str, int]:
+    """The scratch of that (``Part.spare_scratch``)."""
+    if not long_portions(ops, dtype):
+        return {}
+    return {"recurrence in chunks": ops.chunk_scratch_bytes(tokens, seqs, heads, dim, vdim, delta)}
+
+
 def _part_spec(raw) -> PartSpec:
     return raw if isinstance(raw, PartSpec) else PartSpec(raw["kind"], dict(raw.get("params", {})))
 
@@ -133,6 +140,9 @@ class HGRN2(Mixer):
         self.lower = tensors[n["lower"]].float().contiguous()
         self.out_norm = tensors[n["out_norm"]].float().contiguous()
 
+    def spare_scratch(self, ops, tokens, seqs, context):
+        return portion_scratch(ops, self.dtype, tokens, seqs, self.heads, self.dim, self.vdim)
+
     def cache_request(self) -> StateRequest:
         return StateRequest((self.heads * self.vdim * self.dim,))
 
@@ -193,6 +203,9 @@ class MLSTM(Mixer):
         self.i_bias = tensors[n["i_bias"]].float().contiguous()
         self.f_bias = tensors[n["f_bias"]].float().contiguous()
         self.out_norm = tensors[n["out_norm"]].float().contiguous()
+
+    def spare_scratch(self, ops, tokens, seqs, context):
+        return portion_scratch(ops, self.dtype, tokens, seqs, self.heads, self.dim, self.vdim)
 
     def cache_request(self) -> StateRequest:
         return StateRequest((self.matrix_floats + self.heads,))
@@ -261,6 +274,9 @@ class GatedLinearAttention(Mixer):
         self.w_a2 = tensors[n["a2"]].float().contiguous()  # the decay's second map stays 32-bit
         self.a2_bias = tensors[n["a2_bias"]].float().contiguous()
         self.out_norm = tensors[n["out_norm"]].float().contiguous()
+
+    def spare_scratch(self, ops, tokens, seqs, context):
+        return portion_scratch(ops, self.dtype, tokens, seqs, self.heads, self.dim, self.vdim)
 
     def cache_request(self) -> StateRequest:
         return StateRequest((self.heads * self.vdim * self.dim,))

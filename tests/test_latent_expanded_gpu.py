@@ -66,6 +66,27 @@ def test_expanded(heads, dim, rot, rank, lens, starts, page, gate, sink):
     assert rel < REL, f"{rel:.2e}"
 
 
+def test_portions_of_a_growing_context_share_a_workspace():
+    """Each portion's context is longer than the last one's: the scratch grows, captured addresses (the workspace's version) stay."""
+    from inference_engine_b200.engine.workspace import Workspace
+    from inference_engine_b200.kernels import get_ops
+
+    ops, heads, dim, rot, rank, page, g = get_ops(), 2, 64, 32, 64, 16, torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    total, portion = 2000, 400
+    cache, tables = rand(total // page, 1, page, rank + rot).bfloat16(), torch.arange(total // page, dtype=torch.int32, device="cuda")[None]
+    w_kv, shared, outs = (rand(heads * 2 * dim, rank) * rank ** -0.5).bfloat16(), Workspace("cuda", min_rows=portion), []
+    for start in range(0, total, portion):
+        q, ctx = rand(portion, heads * (dim + rot)), _Steps([portion], [start])
+        for ws in (shared, Workspace("cuda")):
+            out = torch.empty(portion, heads * dim, dtype=torch.bfloat16, device="cuda")
+            ops.latent_expanded(q, w_kv, cache, tables, ctx, ctx.positions, None, 0, out, heads=heads, dim=dim, rot_dim=rot, vdim=dim,
+                                rank=rank, page_size=page, interleaved=True, scale=0.1, gate_pre=None, sinks=None, ws=ws)
+            outs.append(out)
+        assert torch.equal(outs[-1], outs[-2]) and shared.version == 0
+    ops.check_errors()
+
+
 def test_which_steps_expand():
     """Prompts and long portions do; decoding requests, short portions and captured steps of any lengths do not."""
     from inference_engine_b200.kernels import get_ops
