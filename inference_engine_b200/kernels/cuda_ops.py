@@ -781,17 +781,41 @@ class CudaOps:
         best = min(range(1, max(1, min(8, max(tiles))) + 1), key=cost)
         return best if cost(best) <= 0.9 * cost(1) else 1
 
+    LEAST_TABLE = 64  # the fewest block-table entries of a captured step; above it half of them at least are a request's
+
     def prompt_packs(self, hd: int, blocks: int, max_ctx: int, longest) -> bool:
         """Whether prompt portions go to the kernel that packs a group's heads into blocks of 256 rows, rather than the one of 128
-        tokens of one head a block (``blocks``: how many of the latter; ``longest``: the longest portion, if the step says).  A block
+        tokens of one head a block (``blocks``: how many of the latter; ``longest``: the longest portion).  A block
         of the former costs two to three microseconds more to start and end and gets through its keys faster: with
-        128 entries a head, 32 heads on 8, 64 tokens 7.2 us against 4.6, 256 tokens 10.6 against 7.9 (one
-        round of either), 512 tokens 14.5 against 16.6, eight prompts of 256 20.8 against 36.4, 2,048 tokens 41.8 against 85.4; with 64 entries
+        128 entries a head, 32 heads on 8, 64 tokens 7.2 us against 4.6, 256 tokens 11.0 against 8.6 (one
+        round of either), 384 tokens 13.0 against 15.7, eight prompts of 64 8.5 against 11.9, 2,048 tokens 41.8 against 85.4, 256 tokens
+        behind 700 15.7 against 17.8; with 64 entries
         1,024 tokens 19.1 against 18.2, eight prompts of 256 16.8 against 14.8, 2,048 tokens 35.4 against 38.7, 8,192 374 against 424, and,
-        as its clusters share keys at less cost, 17 tokens behind 1,000 7.9 against 13.0, 128 behind 2,048 14.2 against 18.3."""
+        as its clusters share keys at less cost, 17 tokens behind 1,000 7.9 against 13.0, 128 behind 2,048 14.2 against 18.3.
+
+        A captured step (``longest`` None: ``blocks`` are those of its bound of tokens, ``max_ctx`` what its longest context has at
+        least) starts as many blocks as any step of its bounds could need and shares keys by its bounds: 64 tokens 14.7 against 7.6,
+        256 16.2 against 11.8, 384 17.2 against 14.4, 512 16.7 against 18.4, eight of 60 11.6 against 21.5, 1,000 23.7 against 37.7; 16 heads on 16,
+        1,000 tokens 23.8 against 22.9, fifteen of 60 14.3 against 18.1; 64 heads on 8, 250 tokens 13.0 against 17.5, 120 15.1 against 11.9."""
         if hd == 128:
-            return max_ctx >= 1024 or 2 * blocks > self.sm_count
-        return max_ctx >= (1024 if longest is not None and 2 * longest <= max_ctx else 2048)
+            if longest is None:
+                return max_ctx >= 1024 or 5 * blocks > 4 * self.sm_count
+            return max_ctx >= 1024 or (4 if 2 * longest <= max_ctx else 2) * blocks > self.sm_count
+        return max_ctx >= (2048 if longest is not None and 2 * longest > max_ctx else 1024)
+
+    def _packs(self, plan, ctx, nh: int, hd: int, page_size: int) -> bool:
+        """The answer for a step, once for all its layers that are alike."""
+        answer = plan.get(("packs", nh))
+        if answer is None:
+            bounds = getattr(ctx, "bounds", None)
+            if bounds is not None:
+                tokens, _, max_ctx = bounds
+                answer = self.prompt_packs(hd, tokens // 128 * nh, max_ctx // 2 if max_ctx > self.LEAST_TABLE * page_size else 0, None)
+            else:
+                lens = [n for n, small in zip(ctx.q_lens, plan["small"]) if not small]
+                answer = self.prompt_packs(hd, sum(-(-n // 128) for n in lens) * nh, ctx.max_ctx_len, max(lens))
+            plan["packs", nh] = answer
+        return answer
 
     def _prompt_clusters(self, hd: int, parts: int) -> int:
         key = (hd, -parts)
@@ -954,7 +978,7 @@ class CudaOps:
         fixed = "max_ctx" in plan  # a launch of fixed size: nothing is decided from the step's own lengths
         max_ctx = plan["max_ctx"] if fixed else ctx.max_ctx_len
         if (self.attn_tc5 and self.prompt_packed and hd in PROMPT_ATTENTION_SIZES and page_size & (page_size - 1) == 0
-                and self.prompt_packs(hd, (plan["likely_tiles"] if fixed else tiles) * nh, max_ctx, None if fixed else max(ctx.q_lens))
+                and self._packs(plan, ctx, nh, hd, page_size)
                 and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16):
             return self._prompt_attention(plan, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd, page_size, scale, window, out)
         if self.attn_tc5 and lib.ie_attention_prefill_tc5_ok(page_size, max_ctx):

@@ -96,6 +96,41 @@ def test_keys_of_a_query_tile_are_shared_when_tiles_are_few_and_contexts_long():
             assert 1 <= ks <= 16 and ks <= max(1, ctx // 256)
 
 
+def test_which_prompt_portions_are_packed():
+    """`CudaOps._packs`: eager steps by their portions, counted in the blocks of 128 tokens of a head that they would be otherwise, and
+    their contexts; captured ones by their bounds, of whose contexts nothing is known unless the tables are wider than the narrowest."""
+    from inference_engine_b200.engine.graphs import DecodeGraphs
+
+    assert CudaOps.LEAST_TABLE == DecodeGraphs.MIN_WIDTH
+    ops = types.SimpleNamespace(sm_count=148, LEAST_TABLE=CudaOps.LEAST_TABLE)
+    ops.prompt_packs = lambda *args: CudaOps.prompt_packs(ops, *args)
+
+    def eager(hd, lens, starts, nh=32, group=4):
+        ctx = types.SimpleNamespace(bounds=None, q_lens=lens, max_ctx_len=max(a + n for a, n in zip(starts, lens)))
+        plan = {"small": [n * group <= 16 for n in lens]}
+        return CudaOps._packs(ops, plan, ctx, nh, hd, 16)
+
+    def captured(hd, tokens, max_ctx, nh=32, page=16):
+        return CudaOps._packs(ops, {"small": []}, types.SimpleNamespace(bounds=(tokens, 16, max_ctx)), nh, hd, page)
+
+    assert not eager(128, [64], [0]) and not eager(128, [256], [0]) and eager(128, [384], [0]) and eager(128, [64] * 8, [0] * 8)
+    assert eager(128, [64], [1500]) and eager(128, [256], [700]) and not eager(128, [64], [900])
+    assert not eager(128, [512], [0], nh=16) and eager(128, [1000], [0], nh=16)
+    assert not eager(128, [1] * 12 + [200], [300] * 12 + [0])  # (decoding requests are another kernel's)
+    assert not eager(64, [1000], [0]) and eager(64, [2048], [0]) and eager(64, [64], [1500]) and not eager(64, [256] * 8, [0] * 8)
+    for tokens in (8, 64, 128, 256, 384):
+        assert not captured(128, tokens, 1024)  # the narrowest tables: a prompt of as many tokens, most likely
+        assert captured(128, tokens, 2048) and captured(64, tokens, 2048)  # longer contexts than 1,024 positions
+        assert not captured(128, tokens, 64 * 64, page=64) and captured(128, tokens, 128 * 64, page=64)
+    assert captured(128, 512, 1024) and captured(128, 1024, 1024) and not captured(64, 1024, 1024)
+    assert not captured(128, 512, 1024, nh=16) and captured(128, 1024, 1024, nh=16)
+    assert captured(128, 256, 1024, nh=64) and not captured(128, 128, 1024, nh=64)
+    # a plan keeps its answer per number of heads, and a fresh one asks again
+    plan, ctx = {"small": []}, types.SimpleNamespace(bounds=(512, 16, 1024))
+    assert CudaOps._packs(ops, plan, ctx, 32, 128, 16) and not CudaOps._packs(ops, plan, ctx, 16, 128, 16)
+    assert CudaOps._packs(ops, plan, ctx, 32, 128, 16)
+
+
 def test_the_history_masks_of_the_repetition_penalty_grow_with_the_histories():
     """The sampler keeps every request's bit mask from step to step (by the request's key) and adds
     only the ids that are new; the result is the mask built from the whole history."""
