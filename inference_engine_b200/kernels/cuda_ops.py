@@ -1374,23 +1374,28 @@ class CudaOps:
     CHUNK = 64
     chunks_always = False  # (tests: whatever the sizes, where the kernels take them)
 
-    def chunks_pay(self, longest: int, tokens: int, chunks: int, heads: int, dim: int, vdim: int, delta: bool) -> bool:
+    def chunks_pay(self, longest: int, tokens: int, chunks: int, heads: int, dim: int, vdim: int, delta: bool, gated: bool = False) -> bool:
         """Whether chunks beat the token-by-token kernels, from estimates of both in microseconds, set against measurements of 1
         to 32 requests of 16 to 2,048 tokens at 8 and 16 heads of 64 x 64 to 128 x 128.  Token by token: the longest
-        portion's chain, or all tokens' state traffic when there are many requests.  In chunks: three launches and a block's
-        life, then the work of all chunks; for the delta rule the chain through the longest portion's chunks besides.
+        portion's chain, or all tokens' state traffic when there are many requests, and a part of the smaller of the two.  In chunks: three
+        launches and a block's life (with ``gated`` values and their normaliser's column a little more), then the work of all chunks;
+        for the delta rule the chain through the longest portion's chunks besides.
         Examples (16 heads of 128 x 128; token by token / in chunks): 64 tokens 24 / 46 us, 256 tokens 85 / 52, 2,048 tokens 664 /
-        134, 8 requests of 64 tokens 79 / 60, 32 of 32 tokens 153 / 165; delta rule 128 tokens 43 / 64, 256 tokens 82 / 74, 2,048
-        tokens 629 / 264, 32 of 32 tokens 160 / 384."""
+        134, 8 requests of 64 tokens 79 / 60, 32 of 32 tokens 153 / 165; whole layers of gated values, 8 heads of 64 x 64, 128 tokens
+        47 / 55, 30 requests of 64 124 / 140, 16 heads of 64 x 128, 8 requests of 64 76 / 89; delta rule 128 tokens 43 / 64, 256 tokens 82 / 74, 2,048
+        tokens 629 / 264, 32 of 32 tokens 160 / 384, whole layers 30 of 64 tokens 542 / 666."""
         share, wide = heads * dim * vdim / 262144, dim > 64
         step = (0.31 if wide else 0.26) if delta else (0.325 if wide else 0.17)
-        one_by_one = max(step * longest, 0.15 * share * tokens)
+        alone, together = step * longest, 0.15 * share * tokens
         if delta:
-            chain = max(-(-longest // self.CHUNK), heads * -(-vdim // 16) * chunks / self.sm_count) * 4.5
+            one_by_one = max(alone, together)
+            chain = max(-(-longest // self.CHUNK), heads * -(-vdim // 16) * chunks / self.sm_count)
+            chain *= 4.5 if longest > self.CHUNK else 7.5  # (portions of one chunk: a block starts for each)
             return (62 if wide else 36) + chain + 2.0 * share * chunks < one_by_one
-        return (42 if wide else 21) + 2.9 * share * chunks < one_by_one
+        one_by_one = max(alone, together) + 0.3 * min(alone, together)
+        return (54 if wide else 29) + (2 if gated else 0) + 2.9 * share * chunks < one_by_one
 
-    def _recurrence_chunks(self, ctx, heads: int, dim: int, vdim: int, delta: bool, rows) -> tuple[int, Any]:
+    def _recurrence_chunks(self, ctx, heads: int, dim: int, vdim: int, delta: bool, rows, gated: bool = False) -> tuple[int, Any]:
         """(chunks, scratch) for a step whose portions are worth it, else (0, None).  ``rows``: the 32-bit views that
         the kernels read in pieces of 16 bytes.  A captured step is judged by its bounds."""
         bounds, size = getattr(ctx, "bounds", None), self.CHUNK
@@ -1399,7 +1404,7 @@ class CudaOps:
             chunks = bounds[0] // size + bounds[1]
         else:
             longest, tokens, chunks = ctx.max_q_len, sum(ctx.q_lens), sum(-(-n // size) for n in ctx.q_lens)
-        if not self.chunks_always and not self.chunks_pay(longest, tokens, chunks, heads, dim, vdim, delta):
+        if not self.chunks_always and not self.chunks_pay(longest, tokens, chunks, heads, dim, vdim, delta, gated):
             return 0, None
         lib = self._part_lib("chunked")
         if not lib.ie_chunked_ok(dim, vdim, int(delta)) or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows):
@@ -1692,7 +1697,7 @@ class CudaOps:
         if dim > 512:
             raise KernelError(f"the recurrence kernel takes key sizes up to 512, not {dim}")
         if in_chunks and out.data_ptr() % 16 == 0:
-            chunks, scratch = self._recurrence_chunks(ctx, heads, dim, vdim, False, (q, w, v) if a is None else (q, a, w, v))
+            chunks, scratch = self._recurrence_chunks(ctx, heads, dim, vdim, False, (q, w, v) if a is None else (q, a, w, v), gates is not None)
             if chunks:
                 self._check(self._part_lib("chunked").ie_chunked_recurrence(
                     q.data_ptr(), q.stride(0), self._ptr(a), 0 if a is None else a.stride(0), w.data_ptr(), w.stride(0),

@@ -131,6 +131,29 @@ def test_which_prompt_portions_are_packed():
     assert CudaOps._packs(ops, plan, ctx, 32, 128, 16)
 
 
+def test_which_portions_are_taken_in_chunks():
+    """`CudaOps.chunks_pay` against what was measured: never where the token-by-token kernels were faster."""
+    ops = types.SimpleNamespace(sm_count=148, CHUNK=CudaOps.CHUNK)
+
+    def pays(lens, heads, dim, vdim, delta=False, gated=False):
+        return CudaOps.chunks_pay(ops, max(lens), sum(lens), sum(-(-n // 64) for n in lens), heads, dim, vdim, delta, gated)
+
+    for gated in (False, True):  # (in whole layers: token by token against chunks, us)
+        assert not pays([128], 8, 64, 64, gated=gated)       # 50 and 53, gated 47 and 55
+        assert not pays([64] * 30, 8, 64, 64, gated=gated)   # 118 and 125, 124 and 140
+        assert not pays([64] * 16, 8, 64, 64, gated=gated)   # 58 and 66, 68 and 81
+        assert pays([200], 8, 64, 64, gated=gated) and pays([200] * 8, 8, 64, 64, gated=gated)
+        assert pays([128] * 4, 16, 64, 128, gated=gated)     # 87 and 77, 104 and 89
+        assert pays([200] * 2, 16, 64, 128, gated=gated) and pays([300] + [1] * 30, 8, 64, 64, gated=gated)
+        assert pays([500, 500, 100, 64, 64, 64], 16, 64, 128, gated=gated)
+    assert pays([64] * 8, 16, 64, 128) and not pays([64] * 8, 16, 64, 128, gated=True)  # 85 and 80, gated 76 and 89
+    assert not pays([64] * 2, 16, 128, 128) and not pays([100] * 2, 16, 128, 128)        # 47 and 55, 65 and 72
+    assert pays([200], 16, 128, 128) and pays([64] * 8, 16, 128, 128) and pays([64] * 16, 16, 128, 128)
+    assert not pays([900] + [1] * 100, 16, 128, 128) and pays([600] + [1] * 30, 16, 128, 128)  # 391 and 655, 263 and 245
+    assert not pays([64], 16, 128, 128, delta=True) and not pays([64] * 30, 16, 128, 128, delta=True)
+    assert pays([513], 16, 128, 128, delta=True) and pays([2048], 16, 128, 128, delta=True)
+
+
 def test_the_history_masks_of_the_repetition_penalty_grow_with_the_histories():
     """The sampler keeps every request's bit mask from step to step (by the request's key) and adds
     only the ids that are new; the result is the mask built from the whole history."""
