@@ -846,8 +846,10 @@ class CudaOps:
             tokens, seqs, max_ctx = bounds
             blocks, likely = seqs + tokens * groups // rows, [max_ctx] * (tokens * groups // rows + min(seqs, 2))
         else:
-            likely = []
-            for n, start, small in zip(ctx.q_lens, ctx.start_positions, plan["small"]):
+            likely, starts = [], getattr(ctx, "start_positions", None)
+            if starts is None:  # (a step that only says its longest context: every portion at the end of one)
+                starts = [ctx.max_ctx_len - n for n in ctx.q_lens]
+            for n, start, small in zip(ctx.q_lens, starts, plan["small"]):
                 if not small:
                     likely += [start + -(-min(r + rows, n * groups) // groups) for r in range(0, n * groups, rows)]
             blocks = len(likely)

@@ -131,6 +131,16 @@ def test_which_prompt_portions_are_packed():
     assert CudaOps._packs(ops, plan, ctx, 32, 128, 16)
 
 
+def test_a_step_that_only_says_its_longest_context_is_planned():
+    """Contexts without the requests' first positions are planned as if every portion ended the longest one."""
+    ops = types.SimpleNamespace(sm_count=148, prefill_key_splits=True, _prompt_clusters=lambda hd, parts: 148 // parts)
+    ops.prompt_shares = lambda *args: CudaOps.prompt_shares(ops, *args)
+    step = dict(bounds=None, q_lens=[128, 1], max_ctx_len=2048)
+    plan = lambda ctx: CudaOps._prompt_plan(ops, {"small": [False, True]}, ctx, 4, 8, 64, 0)  # noqa: E731
+    bare = plan(types.SimpleNamespace(**step))
+    assert bare == plan(types.SimpleNamespace(**step, start_positions=[1920, 2047])) and bare[0] == 2 and bare[1] > 1
+
+
 def test_which_portions_are_taken_in_chunks():
     """`CudaOps.chunks_pay` against what was measured: never where the token-by-token kernels were faster."""
     ops = types.SimpleNamespace(sm_count=148, CHUNK=CudaOps.CHUNK)
