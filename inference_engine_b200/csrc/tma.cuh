@@ -41,13 +41,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, int parity) {
     }
     return false;
 }
-// Whether the phase has completed, without waiting.
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, int parity) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
 // The same wait as a loop that is not unrolled, for kernels with many waits in long loops (the
 // prefill attention: 42 against 50 us on a 2,048-token prompt).
 __device__ __forceinline__ bool mbar_wait_compact(unsigned long long* bar, int parity) {
