@@ -69,3 +69,4 @@ class StepContext:
     # portions): (tokens, sequences, context length) the launch is sized for.  Launch decisions are
     # then taken from these bounds alone, never from the step's own lengths.
     bounds: tuple | None = None
+    most_portion: int | None = None  # with ``bounds``: the most tokens one request may bring (None: all of them)

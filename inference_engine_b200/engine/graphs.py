@@ -17,7 +17,8 @@ Steps with prompt portions (`MixedGraphs`): an eager step costs the host about 1
 1.9 ms for the sixteen layers of the 1B shape, whatever the step holds; up to a few hundred
 tokens the device needs half of that (a 384-token step 2.06 ms eager, 1.31 captured; 512 tokens 2.25
 and 1.62; 1,024 tokens 2.59 and 2.42: beyond that the device is the bound and steps stay eager).  Such steps are captured too, per (tokens, sequences,
-wanted rows, block-table stride), each rounded up to a bucket: the tokens beyond the step's own
+wanted rows, block-table stride), each rounded up to a bucket, and, for models whose recurrences take long portions in
+chunks, whether the longest portion is up to all, a half, a quarter or an eighth of the tokens: the tokens beyond the step's own
 belong to no sequence (their keys and values go to the cache's scratch page), the sequences
 beyond the step's own hold no tokens, and the attention is launched for the most query tiles any step within the bounds can
 have (`StepContext.bounds`).  The reference captures such steps piecewise, around an eager
@@ -183,8 +184,8 @@ class MixedGraphs:
         self.replays = 0
 
     def _key(self, entries):
-        """(tokens, sequences, wanted rows, block-table stride) of the launch that serves these
-        entries, or None if none does."""
+        """(tokens, sequences, wanted rows, block-table stride, tokens of one sequence at most) of the launch that
+        serves these entries, or None if none does."""
         tokens = sum(len(e.tokens) for e in entries)
         t_b = next((t for t in self.token_buckets if t >= tokens), None)
         if t_b is None:
@@ -208,7 +209,12 @@ class MixedGraphs:
             width = self.decode.table_width
             if width < pages:
                 return None
-        return t_b, s_b, r_b, width
+        # (where parts take long portions another way: portions of up to all, a half, a quarter or an eighth of the tokens)
+        most, longest = t_b, max(len(e.tokens) for e in entries)
+        if self.runner.portions_matter and t_b > 64:  # (below they do not)
+            while most // 2 >= longest and 8 * most > t_b:
+                most //= 2
+        return t_b, s_b, r_b, width, most
 
     def can_run(self, entries) -> bool:
         return bool(entries) and any(len(e.tokens) > 1 for e in entries) and self._key(entries) is not None
@@ -221,12 +227,12 @@ class MixedGraphs:
             self._graphs.clear()
             self._version = runner.ws.version
         key = self._key(entries)
-        t_b, s_b, r_b, width = key
+        t_b, s_b, r_b, width, most = key
         wanted = sum(len(e.want) for e in entries)
 
         def build():
             return runner.build_context(entries, pad_to_seqs=s_b, table_width=width, pad_to_tokens=t_b,
-                                        pad_to_rows=r_b)
+                                        pad_to_rows=r_b, most_portion=most)
 
         ctx, rows = build()
         if self._version != runner.ws.version:  # the staging buffer itself had to grow

@@ -145,6 +145,11 @@ class Model:
         per_request = sum(g.num_layers * math.prod(g.shape) for g in self.state_groups)
         return Footprint(parameters, per_token, per_request)
 
+    @property
+    def cuts_portions(self) -> bool:
+        """Whether some part's launches depend on how long a step's longest portion is (not in a 32-bit model)."""
+        return self.env.dtype != "float32" and any(getattr(part, "cuts_portions", False) for part in self.all_parts())
+
     def spare_scratch_bytes(self, ops, tokens: int, seqs: int, context: int) -> int:
         """Scratch that the parts' faster ways take at most and could do without (``Part.spare_scratch``)."""
         most: dict[str, int] = {}

@@ -40,6 +40,8 @@ class ModelRunner:
         self._staging_host = None
         self._staging_dev = None
         self.last_h2d_bytes = 0
+        # whether some part's launches depend on how long a step's longest portion is
+        self.portions_matter = (getattr(ops, "takes_chunks", False) and getattr(model, "cuts_portions", False))
         self._ensure_staging(self._staging_ints(self.max_tokens, self.max_seqs, self.max_seqs, 8))
 
     def contexts_are_ragged(self, ctx_lens) -> tuple[int, ...]:
@@ -98,13 +100,15 @@ class ModelRunner:
 
     def build_context(self, entries: list[StepEntry], pad_to_seqs: int | None = None,
                       table_width: int | None = None, views: bool = True,
-                      pad_to_tokens: int | None = None, pad_to_rows: int | None = None):
+                      pad_to_tokens: int | None = None, pad_to_rows: int | None = None,
+                      most_portion: int | None = None):
         """Pack the step's index data, copy it to the device and return the context and the
         device vector of wanted rows.  ``pad_to_seqs``/``table_width`` give a launch of fixed
         size: missing sequences become single tokens that read and write the scratch page.
         With ``pad_to_tokens`` (and ``pad_to_rows`` wanted rows) the number of tokens is fixed
         too: the tokens beyond the step's own belong to no sequence (their keys and values go to
-        the scratch page), and the sequences beyond the step's own hold no tokens."""
+        the scratch page), and the sequences beyond the step's own hold no tokens; ``most_portion``: the most
+        tokens that one sequence may bring to it."""
         import numpy as np
 
         torch = self._torch
@@ -122,6 +126,8 @@ class ModelRunner:
         pad_tokens = 0
         if pad_to_tokens is not None:
             pad_tokens = pad_to_tokens - sum(q_lens)
+            if most_portion is not None and max(q_lens) > most_portion:
+                raise ValueError(f"a portion of {max(q_lens)} tokens does not fit a launch for portions of up to {most_portion}")
             pad = 0  # (no single-token sequences: see below)
             n = pad_to_tokens
             rows = max(pad_to_rows or 0, sum(len(e.want) for e in entries), 1)
@@ -298,7 +304,7 @@ class ModelRunner:
             q_starts=q_starts, q_lens=q_lens, start_positions=start_positions,
             max_q_len=max(q_lens), max_ctx_len=max(ctx_lens), padded=pad_to_seqs is not None,
             ragged=ragged, decode_order=dview(v_order),
-            bounds=None if pad_to_tokens is None else (n, b, width * ps),
+            bounds=None if pad_to_tokens is None else (n, b, width * ps), most_portion=most_portion,
         )
         return ctx, dview(v_rows)
 

@@ -114,6 +114,8 @@ class Part:
     # tables from device memory, so that it can be captured once and replayed (a part that loops over
     # requests on the host, or reads device values there, says False).
     captures = True
+    # Whether the part takes long portions another way than short ones, by the longest that a captured step may hold.
+    cuts_portions = False
 
     def weights(self) -> dict[str, WeightDecl]:
         """Full tensor names this part reads, with their shapes."""

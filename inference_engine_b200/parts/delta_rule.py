@@ -29,6 +29,8 @@ from .registry import register_part
 
 @register_part("mixer", "channel_delta")
 class ChannelDeltaRule(Mixer):
+    cuts_portions = True
+
     def __init__(self, *, names: dict, hidden_size: int, heads: int, kv_heads: int, dim: int, vdim: int,
                  taps: int, eps: float, dtype) -> None:
         if heads % kv_heads:

@@ -106,6 +106,7 @@ class ConvInput(Mixer):
 @register_part("mixer", "hgrn2")
 class HGRN2(Mixer):
     allow_split = True  # whether the output projection may come back as partial sums
+    cuts_portions = True
 
     def __init__(self, *, names: dict, hidden_size: int, heads: int, dim: int, vdim: int, eps: float, dtype) -> None:
         self.names, self.hidden_size = dict(names), hidden_size
@@ -167,6 +168,7 @@ class HGRN2(Mixer):
 @register_part("mixer", "mlstm")
 class MLSTM(Mixer):
     allow_split = True
+    cuts_portions = True
 
     def __init__(self, *, names: dict, hidden_size: int, heads: int, dim: int, vdim: int, gate_cap: float,
                  eps: float, dtype) -> None:
@@ -236,6 +238,7 @@ class MLSTM(Mixer):
 class GatedLinearAttention(Mixer):
     allow_split = True
     accepts_input_rows = True
+    cuts_portions = True
 
     def __init__(self, *, names: dict, hidden_size: int, heads: int, dim: int, vdim: int, rank: int, tau: float,
                  eps: float, dtype) -> None:

@@ -130,3 +130,38 @@ def test_a_value_that_is_no_number_reaches_no_earlier_token(ops):
     ops.gated_recurrence(q, decay, w, None, v, state, torch.zeros(1, dtype=torch.int32, device="cuda"), _Ctx([n], "cuda"), out, heads,
                          dim, vdim, vdim, 1.0, in_chunks=True)
     assert torch.isfinite(out[:77]).all() and torch.isnan(out[77:]).all()
+
+
+@pytest.mark.parametrize("rule", ["decays", "delta"])
+@pytest.mark.parametrize("lens", [[7, 200, 129], [65], [1, 1, 64, 300]])
+@pytest.mark.parametrize("bounds,most", [((512, 6, 1024), 512), ((1024, 16, 4096), 512)])
+def test_a_launch_for_bounds_serves_every_step_within_them(ops, rule, lens, bounds, most):
+    """A captured step: tokens beyond the step's own belong to no request, requests beyond them have none; blocks for chunks that
+    the step does not have leave.  The bits are those of a launch for the step itself."""
+    heads, dim, vdim, n = 3, 64, 128, sum(lens)
+    g = torch.Generator().manual_seed(n)
+    tokens, seqs, _ = bounds
+    rand = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    pad = lambda t: torch.cat([t, rand(tokens - n, t.shape[1])]).cuda()  # noqa: E731
+    q, k, v, decay = rand(n, heads * dim) * 0.2, rand(n, heads * dim) * 0.2, rand(n, heads * vdim), torch.rand(n, heads * dim, generator=g)
+    beta = torch.rand(n, heads, generator=g)
+    state = rand(seqs + 1, heads * vdim * dim)
+    results = []
+    for captured in (False, True):
+        args = [pad(t) if captured else t.cuda() for t in (q, k, v, decay, beta)]
+        ctx = _Ctx(lens + [0] * (seqs - len(lens) if captured else 0), "cuda")
+        if captured:
+            ctx.bounds, ctx.most_portion = bounds, most
+        slots = torch.tensor(list(range(len(lens))) + [seqs] * (ctx.num_seqs - len(lens)), dtype=torch.int32, device="cuda")
+        st, out = state.cuda(), torch.full((args[0].shape[0], heads * vdim), 7.0, device="cuda")
+        counts = dict(ops.launch_counts)
+        if rule == "delta":
+            ops.delta_rule(args[0], args[1], args[2], args[4], args[3], st, slots, ctx, out, heads, heads, dim, vdim, in_chunks=True)
+        else:
+            ops.gated_recurrence(args[0], args[3], args[1], None, args[2], st, slots, ctx, out, heads, dim, vdim, vdim, 0.5, in_chunks=True)
+        name = "delta_rule_chunks" if rule == "delta" else "gated_recurrence_chunks"
+        assert ops.launch_counts.get(name, 0) == counts.get(name, 0) + 1
+        assert (out[n:] == 7.0).all()
+        results.append((out[:n], st))
+    ops.check_errors()
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])

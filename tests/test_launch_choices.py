@@ -164,6 +164,38 @@ def test_which_portions_are_taken_in_chunks():
     assert pays([513], 16, 128, 128, delta=True) and pays([2048], 16, 128, 128, delta=True)
 
 
+def test_captured_steps_are_told_apart_by_their_longest_portion():
+    """Where parts take long portions another way, a captured step serves portions of up to all, a half, a quarter or an eighth of its
+    tokens; models without such parts have one launch sequence for all."""
+    from inference_engine_b200.engine.batch import StepEntry
+    from inference_engine_b200.engine.graphs import DecodeGraphs, MixedGraphs
+
+    runner = types.SimpleNamespace(page_size=16, portions_matter=True)
+    graphs = MixedGraphs(DecodeGraphs(runner, 64, 512))
+    entries = lambda lens: [StepEntry(i, [0] * n, 0, [n - 1]) for i, n in enumerate(lens)]  # noqa: E731
+    key = lambda lens: graphs._key(entries(lens))  # noqa: E731
+    assert key([200])[0] == key([64] * 3)[0] == 256
+    assert [key(lens)[4] for lens in ([200], [129], [128, 60], [64] * 3, [32] * 6, [10] * 20, [1] * 40 + [100])] == [256, 256, 128, 64, 32, 32, 128]
+    assert key([128, 60]) == key([65] * 3) != key([140, 52])
+    for lens in ([1, 1, 7], [3, 3, 2], [2, 1], [600, 1], [512, 512], [1000], [48] * 8, [49] * 7):
+        assert max(lens) <= key(lens)[4] <= key(lens)[0] and 8 * key(lens)[4] >= key(lens)[0]
+    runner.portions_matter = False
+    assert key([200])[4] == key([64] * 3)[4] == 256
+    # what a launch is told about its portions is what recurrences are judged by
+    seen = []
+    ops = types.SimpleNamespace(CHUNK=64, chunks_always=False, sm_count=148, chunks_pay=lambda *args: seen.append(args) or False)
+    ctx = types.SimpleNamespace(bounds=(256, 4, 1024), most_portion=128)
+    assert CudaOps._recurrence_chunks(ops, ctx, 16, 128, 128, False, ()) == (0, None)
+    ctx.most_portion = None
+    CudaOps._recurrence_chunks(ops, ctx, 16, 128, 128, False, ())
+    assert [args[:3] for args in seen] == [(128, 256, 8), (256, 256, 8)]
+    # ... the delta rule of many heads by the step's tokens, unless its portions are short
+    for most, heads, longest in ((128, 16, 256), (64, 16, 64), (128, 4, 128)):
+        ctx.most_portion = most
+        CudaOps._recurrence_chunks(ops, ctx, heads, 128, 128, True, ())
+        assert seen[-1][0] == longest
+
+
 def test_the_history_masks_of_the_repetition_penalty_grow_with_the_histories():
     """The sampler keeps every request's bit mask from step to step (by the request's key) and adds
     only the ids that are new; the result is the mask built from the whole history."""
