@@ -866,8 +866,7 @@ class CudaOps:
         self._check(self._prompt_lib(hd).ie_attention_prompt(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
             ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, blocks, nh, nkv, page_size, k_cache.shape[0],
-            scale, window, shares, self._err_ptr, self._stream()), "attention_prefill_tc5")
-        self.launch_counts["attention_prefill_packed"] = self.launch_counts.get("attention_prefill_packed", 0) + 1
+            scale, window, shares, self._err_ptr, self._stream()), "attention_prefill_packed")
 
     def paged_attention(self, q, k_cache, v_cache, block_tables, ctx, nh, nkv, hd, page_size,
                         scale, window, out, ragged: bool | None = None, value_dim: int | None = None, sinks=None) -> None:
@@ -2136,8 +2135,7 @@ class CudaOps:
                     ctx.cu_q.data_ptr(), ctx.ctx_lens.data_ptr(), out.data_ptr(), ctx.num_seqs, longest, nh, nkv, page_size,
                     k_cache.shape[0], scale, int(window or 0), self._ptr(sinks), self._ptr(gate),
                     0 if gate is None else gate.stride(0), by_distance[0], cap, keep, out.stride(0), self._err_ptr,
-                    self._stream()), "sink_attention_mma")
-                self.launch_counts["sink_attention_packed"] = self.launch_counts.get("sink_attention_packed", 0) + 1
+                    self._stream()), "sink_attention_packed")
                 return
             self._check(lib.ie_sink_attention_mma(
                 q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(),

@@ -216,3 +216,28 @@ def test_a_captured_step_without_long_portions_waits_for_the_decode_attention(mo
         graph.replay()
         assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -7, f"replay {i}"
     ops.check_errors()
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("window,keep", [(None, 0), (100, 4)])
+@pytest.mark.parametrize("lens,starts,bounds", [([100, 1, 20], [30, 700, 0], (256, 6, 2048)), ([3, 1, 1], [5, 400, 90], (16, 5, 1024)),
+                                                ([2, 1], [1000, 0], (32, 4, 1024))])
+def test_a_captured_step_with_a_sink(dim, window, keep, lens, starts, bounds):
+    """Bounds for more tokens and requests than the step brings: requests beyond its own have no tokens."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, heads, kv_heads, n = get_ops(), 8, 2, sum(lens)
+    q, k, v, tables, rows = _case(lens, starts, heads, kv_heads, dim, dim, 16, window, keep, dim)
+    extra = bounds[1] - len(lens)
+    ctx = _Ctx(lens + [0] * extra, starts + [0] * extra)
+    ctx.bounds, ctx.num_tokens = bounds, bounds[0]
+    tables = torch.cat([tables, torch.full((extra, tables.shape[1]), -1, dtype=torch.int32, device="cuda")])
+    sinks = torch.linspace(-2, 2, heads, device="cuda")
+    padded = torch.zeros(bounds[0], heads * dim, dtype=torch.bfloat16, device="cuda")
+    padded[:n] = q.view(n, -1)
+    out, before = torch.full((bounds[0], heads * dim), 7.0, dtype=torch.bfloat16, device="cuda"), ops.launch_counts.get("sink_attention_packed", 0)
+    ops.sink_attention(padded, k, v, tables, ctx, heads, kv_heads, dim, dim, 16, dim ** -0.5, window, sinks, None, out, keep_first=keep)
+    ops.check_errors()
+    assert ops.launch_counts.get("sink_attention_packed", 0) == before + 1 and bool((out[n:] == 7.0).all())
+    want = _want(q, rows, lens, starts, dim ** -0.5, window, keep, None, sinks, None).view(n, -1)
+    assert float((out[:n].double() - want).norm() / want.norm()) < REL

@@ -437,7 +437,8 @@ def test_decode_attention_with_many_splits_is_the_same_as_one(ops):
 
 @pytest.mark.parametrize("nh,nkv,hd,ps", [(4, 2, 64, 16), (2, 1, 128, 16)])
 @pytest.mark.parametrize("far", [True, False])
-def test_prefill_attention_over_a_long_context(ops, nh, nkv, hd, ps, far):
+@pytest.mark.parametrize("kernel", ["attention_prefill_tc5", "attention_prefill_packed"])
+def test_prefill_attention_over_a_long_context(ops, monkeypatch, nh, nkv, hd, ps, far, kernel):
     """Prompt portions at the end of contexts of 40,000 and 20,500 tokens (2,500 block-table entries:
     a late query tile needs them all).  One key per request stands out, near the context's start or
     24,000 tokens in: the output must be that key's value, whichever page it lies in."""
@@ -445,9 +446,10 @@ def test_prefill_attention_over_a_long_context(ops, nh, nkv, hd, ps, far):
     spike = [77, 1031] if far else [24000, 20400]
     q, k, v, tables, ctx = _attention_case(nh, nkv, hd, ps, q_lens, ctx_lens, torch.bfloat16, seed=21, spike=spike)
     got = torch.empty_like(q)
-    before = ops.launch_counts.get("attention_prefill_tc5", 0)
+    monkeypatch.setattr(ops, "prompt_packed", kernel == "attention_prefill_packed")
+    before = ops.launch_counts.get(kernel, 0)
     ops.paged_attention(q, k, v, tables, ctx, nh, nkv, hd, ps, hd ** -0.5, 0, got)
-    assert ops.launch_counts.get("attention_prefill_tc5", 0) == before + 1  # (the tcgen05 kernel, not the fallback)
+    assert ops.launch_counts.get(kernel, 0) == before + 1  # (this tcgen05 kernel, not the other and not the fallback)
     want = torch.empty_like(q)
     RefOps().paged_attention(q, k, v, tables, ctx, nh, nkv, hd, ps, hd ** -0.5, 0, want)
     torch.testing.assert_close(got.float(), want.float(), atol=2e-2, rtol=2e-2)
@@ -614,7 +616,8 @@ def test_decode_attention_with_keys_as_the_rows_of_the_products(ops, nh, nkv, hd
 @pytest.mark.parametrize("nh,nkv,hd,ps", [(32, 8, 64, 16), (8, 2, 128, 16), (4, 1, 64, 8)])
 @pytest.mark.parametrize("window", [0, 1000])
 @pytest.mark.parametrize("q_lens,ctx_lens", [([200], [3000]), ([130, 1, 260], [2600, 900, 260]), ([17], [1100])])
-def test_prefill_attention_shares_the_keys_of_few_tiles_among_blocks(ops, nh, nkv, hd, ps, window, q_lens, ctx_lens):
+@pytest.mark.parametrize("kernel", ["attention_prefill_tc5", "attention_prefill_packed"])
+def test_prefill_attention_shares_the_keys_of_few_tiles_among_blocks(ops, monkeypatch, nh, nkv, hd, ps, window, q_lens, ctx_lens, kernel):
     """A short portion at the end of a long prompt: too few query tiles to fill the GPU, so the
     keys of every tile are shared among several blocks and merged (head sizes 64 and 128).  One
     far key per request stands out; the result is the same with and without the sharing."""
@@ -623,14 +626,18 @@ def test_prefill_attention_shares_the_keys_of_few_tiles_among_blocks(ops, nh, nk
     want = torch.empty_like(q)
     RefOps().paged_attention(q, k, v, tables, ctx, nh, nkv, hd, ps, hd ** -0.5, window, want)
     outs = []
+    monkeypatch.setattr(ops, "prompt_packed", kernel == "attention_prefill_packed")
+    monkeypatch.setattr(ops, "prompt_packs", lambda *_: True)
     for share in (True, False):
         ops.prefill_key_splits = share
+        before = ops.launch_counts.get(kernel, 0)
         try:
             got = torch.zeros_like(q)
             ops.paged_attention(q, k, v, tables, ctx, nh, nkv, hd, ps, hd ** -0.5, window, got)
             ctx._attention_plans = None
         finally:
             ops.prefill_key_splits = True
+        assert ops.launch_counts.get(kernel, 0) == before + 1
         torch.testing.assert_close(got.float(), want.float(), atol=2e-2, rtol=2e-2)
         outs.append(got)
     torch.testing.assert_close(outs[0].float(), outs[1].float(), atol=1e-2, rtol=1e-2)

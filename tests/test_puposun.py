@@ -389,16 +389,18 @@ def test_attention_sees_its_window_and_the_kept_first_keys(device, window, keep_
     torch.testing.assert_close(torch.cat(got), want, atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.gpu
 @pytest.mark.parametrize("d,window,keep_first,softcap", [
     (16, 50, 3, None), (64, None, 0, 10.0), (128, 160, 70, None), (48, 64, 64, 4.0), (128, 1, 5, None),
     (80, 65, 130, 25.0), (256, 200, 1, None), (96, None, 0, 12.0), (64, 90, 7, None)])
-def test_attention_on_the_tensor_cores(d, window, keep_first, softcap):
+def test_attention_on_the_tensor_cores(monkeypatch, packed, d, window, keep_first, softcap):
     """The bfloat16 kernel against the plain function: portions that start and end inside windows,
     kept positions and tiles of 64, two requests of unequal length in one step (one of them a single
     token), scattered pages, a key per query that stands out at an edge, a zero sink where the
     scores are capped, gates; steps of few tokens cut the keys among blocks (also without a window)."""
     from inference_engine_b200.kernels import get_ops
+    from inference_engine_b200.kernels.build import PACKED_ATTENTION_SIZES
 
     ops, g = get_ops("cuda"), torch.Generator().manual_seed(d + (window or 0))
     T, H, G, ps = 333, 6, 2, 16
@@ -425,7 +427,9 @@ def test_attention_on_the_tensor_cores(d, window, keep_first, softcap):
     tables = torch.tensor([order, other], dtype=torch.int32, device="cuda")
     kc[pages + 3], vc[pages + 3] = 0.5, 0.25
     sinks = torch.zeros(H, device="cuda") if sink else None
-    before = ops.launch_counts.get("sink_attention_mma", 0), ops.launch_counts.get("sink_attention_merge", 0)
+    names = ("sink_attention_mma", "sink_attention_packed", "sink_attention_merge")
+    before = [ops.launch_counts.get(name, 0) for name in names]
+    monkeypatch.setattr(ops, "sink_tc5", packed)
     got, at = [], 0
     portions = [70, 33, 1, 2, 5, 130, 1, 8, 83]  # (few tokens: the key tiles are cut among blocks)
     for n in portions:
@@ -443,8 +447,9 @@ def test_attention_on_the_tensor_cores(d, window, keep_first, softcap):
         torch.testing.assert_close(out[n].float().cpu(), torch.full((H * d,), float(lone)), atol=2e-3, rtol=2e-2)
         at += n
     ops.check_errors()
-    assert at == T and ops.launch_counts.get("sink_attention_mma", 0) == before[0] + len(portions)
-    assert ops.launch_counts.get("sink_attention_merge", 0) > before[1]  # (the steps of few tokens were cut)
+    ran = [ops.launch_counts.get(name, 0) - n for name, n in zip(names, before)]
+    assert at == T and ran[0] + ran[1] == len(portions) and (ran[1] > 0) == (packed and (d, d) in PACKED_ATTENTION_SIZES)
+    assert ran[2] > 0  # (the steps of few tokens were cut)
     # (weights keep 16 bits of mantissa in the second product; outputs are rounded to bfloat16)
     torch.testing.assert_close(torch.cat(got), want, atol=0.015, rtol=0.01)
 

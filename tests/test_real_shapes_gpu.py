@@ -22,6 +22,8 @@ at 128,256 logits would be a gigabyte per run.
 
 from __future__ import annotations
 
+import types
+
 import pytest
 import torch
 
@@ -147,6 +149,8 @@ def test_real_shape_bfloat16_runs_the_kernels_it_is_meant_to(case, monkeypatch):
     name, cfg, *_ = case
     cuts = _cuttings(case)
     _, launches = _run(case, "bfloat16", *cuts["portions"])
+    packed = launches.get("attention_prefill_packed", 0)  # (portions behind a thousand tokens; at head size 128 long ones too)
+    assert packed > 0, launches
     for kernel in ["attention_prefill_tc5", "attention_decode", "gemm_tma"]:
         assert launches.get(kernel, 0) > 0, f"{kernel} never ran: {launches}"
     assert launches.get("gemm_tc5", 0) == 0
@@ -263,12 +267,14 @@ def test_a_long_prompt_in_captured_portions_shares_its_tiles_keys():
         engine = LLMEngine(model, None, (), num_blocks=400, block_size=PAGE, max_num_seqs=4,
                            max_num_batched_tokens=256, max_model_len=2400, enable_cuda_graphs=True,
                            enable_mixed_graphs=mixed, debug_checks=True)
-        before = engine.ops.launch_counts.get("attention_prefill_tc5", 0)
+        before = dict(engine.ops.launch_counts)
         outs.append(engine.generate({"long": prompt}, SamplingParams(temperature=0, max_tokens=4))["long"])
-        assert engine.ops.launch_counts.get("attention_prefill_tc5", 0) > before
+        for kernel in ("attention_prefill_tc5", "attention_prefill_packed"):  # (the first portions, those behind a thousand tokens)
+            assert engine.ops.launch_counts.get(kernel, 0) > before.get(kernel, 0)
         if mixed:
             assert engine.mixed_graphs.replays >= 8
-            assert engine.ops.prefill_key_split(4 * cfg["num_attention_heads"], cfg["head_dim"], 4096) > 1
+            ctx, kv = types.SimpleNamespace(bounds=(256, 4, 4096)), cfg["num_key_value_heads"]
+            assert engine.ops._prompt_plan({}, ctx, cfg["num_attention_heads"] // kv, kv, cfg["head_dim"], 0)[1] > 1
         engine.ops.check_errors()
         del engine, model
         torch.cuda.empty_cache()

@@ -337,14 +337,16 @@ def test_sink_attention_sees_exactly_its_window(device, window):
         assert abs(seen[t] - far_in) < 1e-3 * far_in + 1e-4 and not torch.allclose(want[t], want[t + 1])
 
 
+@pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.gpu
 @pytest.mark.parametrize("d,dv,window", [(16, 32, 50), (64, 64, None), (128, 128, 160), (48, 16, 64), (128, 64, 1),
                                          (80, 112, 65), (256, 256, 200)])
-def test_sink_attention_on_the_tensor_cores(d, dv, window):
+def test_sink_attention_on_the_tensor_cores(monkeypatch, packed, d, dv, window):
     """The bfloat16 kernel against the plain function: portions that start and end inside windows
     and tiles of 64, two requests of unequal length in one step (one of them a single token), scattered
     pages, a key per query that stands out just inside or just outside the window, sinks, gates."""
     from inference_engine_b200.kernels import get_ops
+    from inference_engine_b200.kernels.build import PACKED_ATTENTION_SIZES
 
     ops, g = get_ops("cuda"), torch.Generator().manual_seed(d + dv)
     T, H, G, ps = 333, 6, 2, 16
@@ -371,7 +373,9 @@ def test_sink_attention_on_the_tensor_cores(d, dv, window):
     other = [pages + 3] * pages  # the second request: one token on the scratch page
     tables = torch.tensor([order, other], dtype=torch.int32, device="cuda")
     kc[pages + 3], vc[pages + 3] = 0.5, 0.25
-    before = ops.launch_counts.get("sink_attention_mma", 0)
+    names = ("sink_attention_mma", "sink_attention_packed")
+    before = [ops.launch_counts.get(name, 0) for name in names]
+    monkeypatch.setattr(ops, "sink_tc5", packed)
     got, at = [], 0
     portions = [70, 33, 1, 2, 5, 130, 1, 8, 83]  # (few tokens: the window's key tiles are cut among blocks)
     for n in portions:
@@ -387,7 +391,8 @@ def test_sink_attention_on_the_tensor_cores(d, dv, window):
         torch.testing.assert_close(out[n].float().cpu().view(H, dv), lone.expand(H, dv), atol=2e-3, rtol=2e-2)
         at += n
     ops.check_errors()
-    assert at == T and ops.launch_counts.get("sink_attention_mma", 0) == before + len(portions)  # (the kernel under test did run)
+    ran = [ops.launch_counts.get(name, 0) - n for name, n in zip(names, before)]
+    assert at == T and ran[0] + ran[1] == len(portions) and (ran[1] > 0) == (packed and (d, dv) in PACKED_ATTENTION_SIZES)
     # (weights keep 16 bits of mantissa in the second product; outputs are rounded to bfloat16)
     torch.testing.assert_close(torch.cat(got), want, atol=0.015, rtol=0.01)
 
