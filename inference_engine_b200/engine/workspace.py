@@ -19,7 +19,7 @@ class Workspace:
         self._views: dict[tuple, tuple] = {}  # last view handed out per buffer
         self.version = 0
         self.spare_bytes: int | None = None  # what all spare scratch may take (None: whatever is asked for)
-        self._spare: dict = {}  # its buffers' bytes
+        self._spare: dict = {}  # its buffers' elements
         self._addressed: set = set()  # spare scratch whose addresses a capture may hold
 
     def buffer(self, name: str, rows: int, cols: int, dtype, rows_cap: int | None = 0):
@@ -45,15 +45,15 @@ class Workspace:
 
     def _spare_plan(self, wants):
         """Elements of each buffer that ``wants`` leads to (doubled where one grows, if that much may be taken), or None."""
-        buffers = self._buffers
-        held = [buffers.get((name, dtype)) for name, _, dtype in wants]
-        if all(buf is not None and buf.numel() >= want[1] for buf, want in zip(held, wants)):
-            return {want[::2]: buf.numel() for buf, want in zip(held, wants)}
-        for grown in (lambda n: 1 << max(int(n) - 1, 0).bit_length(), int):
-            plan = {want[::2]: buf.numel() if buf is not None and buf.numel() >= want[1] else grown(max(want[1], 1))
-                    for buf, want in zip(held, wants)}
-            total = sum({**self._spare, **{key: n * key[1].itemsize for key, n in plan.items()}}.values())
-            if self.spare_bytes is None or total <= self.spare_bytes:
+        held = self._spare
+        if all(held.get((name, dtype), -1) >= rows * cols for name, rows, cols, dtype in wants):
+            return held
+        for grown in (lambda n: 1 << max(n - 1, 0).bit_length(), int):
+            plan = dict(held)
+            for name, rows, cols, dtype in wants:
+                if plan.get((name, dtype), -1) < rows * cols:
+                    plan[name, dtype] = grown(max(rows * cols, 1))
+            if self.spare_bytes is None or sum(n * dtype.itemsize for (_, dtype), n in plan.items()) <= self.spare_bytes:
                 return plan
         return None
 
@@ -62,29 +62,38 @@ class Workspace:
         return self._spare_plan(wants) is not None
 
     def spare(self, wants, captured: bool = True):
-        """Flat views of spare scratch for ``wants`` (name, elements, dtype), or None where that would be more than
+        """``[rows, cols]`` views of spare scratch for ``wants`` (name, rows, cols, dtype), or None where that would be more than
         ``spare_bytes``.  ``captured=False``: scratch of steps that are launched one kernel at a time alone, whose growth
         leaves captured addresses as they are."""
         import torch
 
-        plan = self._spare_plan(wants)
-        if plan is None:
-            return None
         captured = captured or (str(self.device).startswith("cuda") and torch.cuda.is_current_stream_capturing())
-        views = []
-        for name, elements, dtype in wants:
+        plan, views = None, []
+        for name, rows, cols, dtype in wants:
             key = (name, dtype)
+            if captured:
+                self._addressed.add(key)
+            hit = self._views.get(key)
+            if hit is not None and hit[0] == rows and hit[1] == cols:
+                views.append(hit[2])
+                continue
+            if plan is None:
+                plan = self._spare_plan(wants)
+                if plan is None:
+                    return None
+            need = rows * cols
             buf = self._buffers.get(key)
-            if buf is None or buf.numel() < plan[key]:
+            if buf is None or buf.numel() < need:
                 if buf is not None and key in self._addressed:
                     self.version += 1
+                self._views.pop(key, None)
                 buf = self._buffers.pop(key, None)
                 del buf  # (given back first: the larger one may need its place)
                 buf = self._buffers[key] = torch.empty(plan[key], dtype=dtype, device=self.device)
-                self._spare[key] = buf.numel() * buf.element_size()
-            if captured:
-                self._addressed.add(key)
-            views.append(buf[:elements])
+                self._spare[key] = plan[key]
+            view = buf[:need].view(rows, cols)
+            self._views[key] = (rows, cols, view)
+            views.append(view)
         return views
 
     def bytes(self) -> int:

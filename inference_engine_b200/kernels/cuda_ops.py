@@ -1124,14 +1124,14 @@ class CudaOps:
     def _expanded_wants(self, context: int, heads: int, dim: int, rot_dim: int, vdim: int, rank: int):
         """The scratch of the expanded latent attention for so many tokens of context."""
         bf16 = self.torch.bfloat16
-        return [("latent.context", context * (rank + rot_dim), bf16), ("latent.expanded", context * heads * (dim + vdim), bf16)]
+        return (("latent.context", context, rank + rot_dim, bf16), ("latent.expanded", context, heads * (dim + vdim), bf16))
 
     def latent_scratch_bytes(self, context: int, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> int:
         """The most of it that steps over ``context`` tokens of requests can take."""
         if not self.latent_expand or (dim, vdim) not in FLAT_ATTENTION_SIZES:
             return 0
         context = min(context, self.EXPANDED_MOST // (heads * (dim + vdim)))
-        return sum(2 * n for _, n, _ in self._expanded_wants(context, heads, dim, rot_dim, vdim, rank))
+        return sum(2 * rows * cols for _, rows, cols, _ in self._expanded_wants(context, heads, dim, rot_dim, vdim, rank))
 
     def _flat_lib(self, dim: int, vdim: int):
         lib = self._flat_libs.get((dim, vdim))
@@ -1169,7 +1169,7 @@ class CudaOps:
         scratch = ws.spare(self._expanded_wants(total, heads, dim, rot_dim, vdim, rank), captured=False)
         if scratch is None:
             raise KernelError(f"latent_expanded: no scratch for {total} tokens of context (latent_expands says when)")
-        rows, kv = scratch[0].view(total, row), scratch[1].view(total, heads * (dim + vdim))
+        rows, kv = scratch
         self._gather_context_rows(cache, block_tables, ctx, page_size, rows)
         self._expand_latent(rows[:, :rank], w_kv, kv)
         self._flat_attention(plain, turned[:, rank:], row, kv, rows[:, rank:], row, rot_dim, ctx, out, heads, dim, vdim, scale, sinks,
@@ -1416,7 +1416,7 @@ class CudaOps:
         if not lib.ie_chunked_ok(dim, vdim, int(delta)) or any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows):
             return 0, None
         floats = lib.ie_chunked_scratch(chunks, heads, dim, vdim, int(delta))
-        scratch = ctx.ws.spare([("recurrence.chunks", floats, self.torch.float32)])
+        scratch = ctx.ws.spare((("recurrence.chunks", 1, floats, self.torch.float32),))
         return (0, None) if scratch is None else (chunks, scratch[0])
 
     def chunk_scratch_bytes(self, tokens: int, seqs: int, heads: int, dim: int, vdim: int, delta: bool) -> int:

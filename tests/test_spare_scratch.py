@@ -37,7 +37,7 @@ def test_a_long_prompt_in_portions_leaves_captured_steps_alone():
         ctx = _ctx(ws, [2048], [start])
         assert ops.latent_expands(ctx, **LATENT)
         views = ws.spare(ops._expanded_wants(start + 2048, **LATENT), captured=False)
-        assert [v.numel() for v in views] == [(start + 2048) * 288, (start + 2048) * 1024]
+        assert [tuple(v.shape) for v in views] == [(start + 2048, 288), (start + 2048, 1024)]
         places.add(views[1].data_ptr())
         assert ws.version == 0
     assert len(places) <= 4  # (doubled, not replaced for every portion)
@@ -57,7 +57,7 @@ def test_the_chunks_scratch_grows_by_doubling():
 def test_what_there_is_no_room_for_is_done_without():
     ops, ws = _ops(), Workspace("cpu")
     ctx = _ctx(ws, [2048], [0])
-    need = sum(2 * n for _, n, _ in ops._expanded_wants(2048, **LATENT))
+    need = sum(2 * rows * cols for _, rows, cols, _ in ops._expanded_wants(2048, **LATENT))
     ws.spare_bytes = need - 1
     assert not ops.latent_expands(ctx, **LATENT) and ws.spare(ops._expanded_wants(2048, **LATENT)) is None and ws.bytes() == 0
     ws.spare_bytes = need  # (no room to double: exactly what is needed)
