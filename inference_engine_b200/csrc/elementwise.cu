@@ -95,8 +95,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 // thread keeps its part of the row in registers, so the row is read once and all loads are in
 // flight together (a decode step's few rows are bound by latency, not bandwidth).  The order
 // in which a row's squares are added depends only on the row's width.
-// PCH: how many parts of `delta` are loaded at a time (1 when it is a single array: a prefill
-// step's thousands of rows want the registers for occupancy instead).
+// PCH: how many parts of `delta` are loaded at a time (1 when it is a single array, 4 when there are no more: a prefill
+// step's thousands of rows want the registers for occupancy instead; 2,048 rows of 2,048 with four parts 26 us by eights, 20 by fours).
 template <typename OutT, int THREADS, int VPT, int PCH>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ delta, int num_partials,
@@ -186,10 +186,12 @@ static int launch_rmsnorm(float* h, const float* delta, int num_partials, size_t
 #define IE_NORM_ARGS s, h, delta, num_partials, partial_stride, dscale, weight, eps, out, rows, hidden
     bool multi = delta != nullptr && num_partials > 1;
     if (hidden % 4 == 0 && hidden <= 128 * 4 * 2)
-        return multi ? ie_launch(rmsnorm_vec_kernel<OutT, 128, 2, 8>, dim3(num_rows), dim3(128), 0, IE_NORM_ARGS)
+        return multi && num_partials > 4 ? ie_launch(rmsnorm_vec_kernel<OutT, 128, 2, 8>, dim3(num_rows), dim3(128), 0, IE_NORM_ARGS)
+               : multi ? ie_launch(rmsnorm_vec_kernel<OutT, 128, 2, 4>, dim3(num_rows), dim3(128), 0, IE_NORM_ARGS)
                      : ie_launch(rmsnorm_vec_kernel<OutT, 128, 2, 1>, dim3(num_rows), dim3(128), 0, IE_NORM_ARGS);
     if (hidden % 4 == 0 && hidden <= 256 * 4 * 2)
-        return multi ? ie_launch(rmsnorm_vec_kernel<OutT, 256, 2, 8>, dim3(num_rows), dim3(256), 0, IE_NORM_ARGS)
+        return multi && num_partials > 4 ? ie_launch(rmsnorm_vec_kernel<OutT, 256, 2, 8>, dim3(num_rows), dim3(256), 0, IE_NORM_ARGS)
+               : multi ? ie_launch(rmsnorm_vec_kernel<OutT, 256, 2, 4>, dim3(num_rows), dim3(256), 0, IE_NORM_ARGS)
                      : ie_launch(rmsnorm_vec_kernel<OutT, 256, 2, 1>, dim3(num_rows), dim3(256), 0, IE_NORM_ARGS);
     if (hidden % 4 == 0 && hidden <= 512 * 4 * 4)
         return multi ? ie_launch(rmsnorm_vec_kernel<OutT, 512, 4, 4>, dim3(num_rows), dim3(512), 0, IE_NORM_ARGS)
