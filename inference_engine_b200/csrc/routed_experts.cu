@@ -19,55 +19,209 @@
 // bfloat16 products run on mma.sync.m16n8k16 with 32-bit sums, 32-bit products on fused
 // multiply-adds; a row's sums run over k in a fixed order, whatever else is in the tile.
 #include "common.cuh"
+#include <limits.h>
 #include <math.h>
 
 namespace {
 
-constexpr int ROUTE_THREADS = 256;
+// The lane's best of `count` scores (larger first, then the lower index), over the warp: every lane gets the index, -1 if no score
+// is above `floor` (one that is no number is above nothing).
+__device__ __forceinline__ int warp_best(const float* score, int count, float floor, int lane) {
+    float bv = floor;
+    int best = INT_MAX;
+    for (int e = lane; e < count; e += 32)
+        if (score[e] > bv) { bv = score[e]; best = e; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best, o);
+        if (ov > bv || (ov == bv && oi < best)) { bv = ov; best = oi; }
+    }
+    return best == INT_MAX ? -1 : best;
+}
+
+// A warp chooses token n's experts from their logits (score[experts]; gbest[groups] and choice[experts] are its scratch).
+__device__ __forceinline__ void choose_experts(int n, float* score, float* gbest, float* choice, int lane, int experts, int top, int groups,
+                                               int keep, int sigmoid_scores, const float* __restrict__ correction, int group_top,
+                                               float weight_scale, int* __restrict__ ids, float* __restrict__ weights) {
+    const int per = experts / groups;
+    float total = 0.f;
+    if (sigmoid_scores) {
+        for (int e = lane; e < experts; e += 32) {
+            float sg = 1.0f / (1.0f + expf(-score[e]));
+            score[e] = sg;
+            choice[e] = correction != nullptr ? sg + correction[e] : sg;
+        }
+        __syncwarp();
+        if (keep < groups) {
+            for (int g = lane; g < groups; g += 32) {  // the group's best corrected scores, one or two of them
+                float b1 = -INFINITY, b2 = -INFINITY;
+                for (int e = g * per; e < (g + 1) * per; ++e) {
+                    float c = choice[e];
+                    if (c > b1) { b2 = b1; b1 = c; }
+                    else if (c > b2) b2 = c;
+                }
+                gbest[g] = (group_top >= 2 && per >= 2) ? b1 + b2 : b1;
+            }
+            __syncwarp();
+            // The kept groups are marked by +inf.  (A group without any score to compare counts as the lowest, not as none: when nothing
+            // better is left it is kept, the one with the lowest index first.)
+            for (int round = 0; round < keep; ++round) {
+                int best = -1;
+                if (lane == 0) {
+                    float bv = -INFINITY;
+                    for (int g = 0; g < groups; ++g)
+                        if (gbest[g] != INFINITY && (best < 0 || gbest[g] > bv)) { bv = gbest[g]; best = g; }
+                    if (best >= 0) gbest[best] = INFINITY;
+                }
+                if (__shfl_sync(0xffffffffu, best, 0) < 0) break;
+            }
+            __syncwarp();
+            for (int e = lane; e < experts; e += 32)
+                if (gbest[e / per] != INFINITY) choice[e] = -INFINITY;
+            __syncwarp();
+        }
+        for (int j = 0; j < top; ++j) {
+            const int best = warp_best(choice, experts, -INFINITY, lane);
+            const float wj = best < 0 ? 0.f : score[best];
+            if (lane == 0) {
+                ids[(size_t)n * top + j] = best < 0 ? 0 : best;
+                weights[(size_t)n * top + j] = wj;
+                if (best >= 0) choice[best] = -INFINITY;  // taken
+            }
+            total += wj;
+            __syncwarp();
+        }
+    } else {
+        // softmax over all experts (lanes share the work, every lane ends with the same numbers)
+        float m = -INFINITY;
+        for (int e = lane; e < experts; e += 32) m = fmaxf(m, score[e]);
+        m = warp_max(m);
+        float sum = 0.f;
+        for (int e = lane; e < experts; e += 32) {
+            float p = expf(score[e] - m);
+            score[e] = p;
+            sum += p;
+        }
+        sum = warp_sum(sum);
+        float inv = 1.0f / sum;
+        for (int e = lane; e < experts; e += 32) score[e] *= inv;
+        __syncwarp();
+        // keep the best groups: a group that is not kept gets its experts' scores hidden (negated - 1)
+        if (keep < groups) {
+            for (int g = lane; g < groups; g += 32) {
+                float b = -1.f;
+                for (int e = g * per; e < (g + 1) * per; ++e) b = fmaxf(b, score[e]);
+                gbest[g] = b;
+            }
+            __syncwarp();
+            for (int round = 0; round < keep; ++round) {
+                const int best = warp_best(gbest, groups, -1.f, lane);
+                if (best < 0) break;
+                if (lane == 0) gbest[best] = -2.f - gbest[best];  // marked as kept
+                __syncwarp();
+            }
+            for (int e = lane; e < experts; e += 32)
+                if (gbest[e / per] >= 0.f) score[e] = -1.f - score[e];
+            __syncwarp();
+        }
+        for (int j = 0; j < top; ++j) {
+            const int best = max(warp_best(score, experts, -1e-30f, lane), 0);
+            const float s = score[best], bv = s >= 0.f ? s : 0.f;  // (no score to choose: expert 0 without weight)
+            __syncwarp();
+            if (lane == 0) {
+                ids[(size_t)n * top + j] = best;
+                weights[(size_t)n * top + j] = bv;
+                score[best] = -1.f - s;  // taken
+            }
+            total += bv;
+            __syncwarp();
+        }
+    }
+    const float f = weight_scale / (total + 1e-20f);
+    if (lane == 0)
+        for (int j = 0; j < top; ++j) weights[(size_t)n * top + j] *= f;
+}
 
 // TOKENS tokens per block: the router's rows are read once for all of them.  A token at a time 2,048 tokens of width 2,048 with 32
-// experts read them 2,048 times (half a GB through the L2, 47 us); few tokens want a block each.
+// experts read them 2,048 times (half a GB through the L2, 47 us); few tokens want a block each.  What bounds it is the way to the
+// L2 and back, so a lane has eight pieces of the router's rows on their way, the first of them before the tokens' own rows have arrived,
+// and the choice is the whole warp's (8 tokens, 32 experts: 20 -> 11 us).
 template <typename T, int TOKENS>
-__global__ void __launch_bounds__(ROUTE_THREADS)
+__global__ void __launch_bounds__(TOKENS > 1 ? 256 : 1024, TOKENS > 1 ? 2 : 1)
 route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int num_tokens, int width,
                   int experts, int top, int groups, int keep, int sigmoid_scores,
-                  const float* __restrict__ correction, int group_top, float weight_scale,
+                  const float* __restrict__ correction, int group_top, float weight_scale, int whole_pieces,
                   int* __restrict__ ids, float* __restrict__ weights) {
-    extern __shared__ float sm[];  // x[TOKENS][width], then per token score[experts], group_best[groups], choice[experts]
+    extern __shared__ __align__(16) float sm[];  // x[TOKENS][width], then per token score[experts], group_best[groups], choice[experts]
     float* xs = sm;
-    ie_pdl_trigger();
-    ie_pdl_wait();
     const int n0 = blockIdx.x * TOKENS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cnt = min(TOKENS, num_tokens - n0);
     float* const scores = xs + TOKENS * width;
     const int per_token = 2 * experts + groups;
-    for (int i = tid; i < TOKENS * width; i += ROUTE_THREADS) xs[i] = i < cnt * width ? ie_load(x + (size_t)n0 * width + i) : 0.f;
+    // A warp takes every so many'th expert, some of them at a time.  An expert's sum is the same chain of operations whichever
+    // way it is grouped: four partial sums per lane, added in a fixed order.
+    constexpr int ROUTE_THREADS = TOKENS > 1 ? 256 : 1024, WARPS = ROUTE_THREADS / 32, AT_ONCE = TOKENS > 1 ? 4 : 1, AHEAD = TOKENS > 1 ? 2 : 8;
+    float4 wv[AHEAD][AT_ONCE];
+    auto ask = [&](int slot, int e0, int i) {
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const int e = e0 + u * WARPS;
+            wv[slot][u] = e < experts && i < width ? *reinterpret_cast<const float4*>(w + (size_t)e * width + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    auto ask_first = [&](int e0) {
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) ask(a, e0, lane * 4 + a * 128);
+    };
+    ie_pdl_trigger();
+    if (width % 4 == 0) ask_first(warp);  // (weights: nothing that the kernel before writes)
+    ie_pdl_wait();
+    if (whole_pieces) {  // rows of whole 16-byte pieces, aligned
+        constexpr int PIECE = 16 / sizeof(T);
+        for (int i = tid * PIECE; i < TOKENS * width; i += ROUTE_THREADS * PIECE) {
+            float4 v[PIECE / 4];
+            if (i < cnt * width) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(x + (size_t)n0 * width + i);
+                const T* t = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+                for (int k = 0; k < PIECE / 4; ++k)
+                    v[k] = make_float4(ie_load(t + 4 * k), ie_load(t + 4 * k + 1), ie_load(t + 4 * k + 2), ie_load(t + 4 * k + 3));
+            } else {
+#pragma unroll
+                for (int k = 0; k < PIECE / 4; ++k) v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < PIECE / 4; ++k) *reinterpret_cast<float4*>(xs + i + 4 * k) = v[k];
+        }
+    } else {
+        for (int i = tid; i < TOKENS * width; i += ROUTE_THREADS) xs[i] = i < cnt * width ? ie_load(x + (size_t)n0 * width + i) : 0.f;
+    }
     __syncthreads();
-    // A warp takes the experts warp, warp + 8, ...; four of them at a time, so that four rows' loads are
-    // on their way together.  An expert's sum is the same chain of operations whichever way it is grouped.
-    constexpr int WARPS = ROUTE_THREADS / 32, AT_ONCE = 4;
     for (int e0 = warp; e0 < experts; e0 += WARPS * AT_ONCE) {
         float acc[AT_ONCE][TOKENS];
-        if (width % 4 == 0) {  // (four partial sums per lane and expert, added in a fixed order)
+        if (width % 4 == 0) {
             float a4[AT_ONCE][TOKENS][4];
 #pragma unroll
             for (int u = 0; u < AT_ONCE; ++u)
 #pragma unroll
                 for (int t = 0; t < TOKENS; ++t) a4[u][t][0] = a4[u][t][1] = a4[u][t][2] = a4[u][t][3] = 0.f;
-            for (int i = lane * 4; i < width; i += 128) {
-                float4 wv[AT_ONCE];
+            if (e0 != warp) ask_first(e0);
+            for (int i0 = lane * 4; i0 < width; i0 += 128 * AHEAD) {
 #pragma unroll
-                for (int u = 0; u < AT_ONCE; ++u) {
-                    int e = e0 + u * WARPS;
-                    wv[u] = e < experts ? *reinterpret_cast<const float4*>(w + (size_t)e * width + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+                for (int a = 0; a < AHEAD; ++a) {
+                    const int i = i0 + a * 128;
+                    if (i < width) {
 #pragma unroll
-                for (int t = 0; t < TOKENS; ++t) {
-                    float4 xv = *reinterpret_cast<const float4*>(xs + t * width + i);
+                        for (int t = 0; t < TOKENS; ++t) {
+                            float4 xv = *reinterpret_cast<const float4*>(xs + t * width + i);
 #pragma unroll
-                    for (int u = 0; u < AT_ONCE; ++u) {
-                        a4[u][t][0] = fmaf(xv.x, wv[u].x, a4[u][t][0]); a4[u][t][1] = fmaf(xv.y, wv[u].y, a4[u][t][1]);
-                        a4[u][t][2] = fmaf(xv.z, wv[u].z, a4[u][t][2]); a4[u][t][3] = fmaf(xv.w, wv[u].w, a4[u][t][3]);
+                            for (int u = 0; u < AT_ONCE; ++u) {
+                                a4[u][t][0] = fmaf(xv.x, wv[a][u].x, a4[u][t][0]); a4[u][t][1] = fmaf(xv.y, wv[a][u].y, a4[u][t][1]);
+                                a4[u][t][2] = fmaf(xv.z, wv[a][u].z, a4[u][t][2]); a4[u][t][3] = fmaf(xv.w, wv[a][u].w, a4[u][t][3]);
+                            }
+                        }
+                        ask(a, e0, i + 128 * AHEAD);
                     }
                 }
             }
@@ -99,110 +253,108 @@ route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const fl
     }
     __syncthreads();
     if (warp >= cnt) return;  // (a warp per token from here on)
-    const int n = n0 + warp;
     float* score = scores + warp * per_token;
-    float* gbest = score + experts;
-    float* choice = gbest + groups;
-    if (sigmoid_scores) {
-        for (int e = lane; e < experts; e += 32) {
-            float sg = 1.0f / (1.0f + expf(-score[e]));
-            score[e] = sg;
-            choice[e] = correction != nullptr ? sg + correction[e] : sg;
+    choose_experts(n0 + warp, score, score + experts, score + experts + groups, lane, experts, top, groups, keep, sigmoid_scores, correction,
+                   group_top, weight_scale, ids, weights);
+}
+
+// The same for many bfloat16 tokens: 16 a block, whose products with the router's rows run on the tensor cores.  A 32-bit number is a sum of
+// three bfloat16 ones, so a product with a bfloat16 number is the sum of three that the tensor cores take whole; 32 of k go through them, whose
+// sums cut off what does not fit, and are added in 32 bits.  A warp takes every sixteenth 32 of k, and the warps' sums meet in a fixed order.
+// (2,048 tokens of width 2,048, 32 experts: 41 us by multiply-adds, four tokens a block, bound by the router's rows' way from the L2; 21 us
+// with eight warps, 14 with sixteen.)
+constexpr int RM_TOKENS = 16, RM_WARPS = 16, RM_EXPERTS = 32;
+
+__device__ __forceinline__ void three(float x, float y, unsigned (&t)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        t[i] = *reinterpret_cast<const unsigned*>(&v);
+        if (i < 2) {
+            x -= __uint_as_float(t[i] << 16);
+            y -= __uint_as_float(t[i] & 0xFFFF0000u);
         }
-        __syncwarp();
-        int per = experts / groups;
-        if (keep < groups) {
-            for (int g = lane; g < groups; g += 32) {  // the group's best corrected scores, one or two of them
-                float b1 = -INFINITY, b2 = -INFINITY;
-                for (int e = g * per; e < (g + 1) * per; ++e) {
-                    float c = choice[e];
-                    if (c > b1) { b2 = b1; b1 = c; }
-                    else if (c > b2) b2 = c;
+    }
+}
+
+__global__ void __launch_bounds__(RM_WARPS * 32)
+route_many_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int num_tokens, int width,
+                  int experts, int top, int groups, int keep, int sigmoid_scores, const float* __restrict__ correction, int group_top,
+                  float weight_scale, int* __restrict__ ids, float* __restrict__ weights) {
+    extern __shared__ __align__(16) float sm[];  // [16 warps][16 tokens][33], then per token score[experts], group_best[groups], choice[experts]
+    constexpr int LD = RM_EXPERTS + 1;
+    float* const scores = sm + RM_WARPS * RM_TOKENS * LD;
+    const int per_token = 2 * experts + groups;
+    const int n0 = blockIdx.x * RM_TOKENS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    // the lane's eight k of 32: two instructions' worth, in an order of its own that both factors share
+    const uint4* x0 = reinterpret_cast<const uint4*>(x + (size_t)min(n0 + g, num_tokens - 1) * width) + t;
+    const uint4* x1 = reinterpret_cast<const uint4*>(x + (size_t)min(n0 + 8 + g, num_tokens - 1) * width) + t;
+    for (int e0 = 0; e0 < experts; e0 += RM_EXPERTS) {
+        float acc[4][4] = {};
+        uint4 a0, a1;
+        float4 wv[4][2];
+        auto ask = [&](int k) {
+            if (k >= width) return;
+            a0 = x0[k / 8];
+            a1 = x1[k / 8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int e = e0 + 8 * j + g;
+                const float4* p = reinterpret_cast<const float4*>(w + (size_t)e * width + k + 8 * t);
+                wv[j][0] = e < experts ? p[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                wv[j][1] = e < experts ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        ask(warp * 32);
+        for (int k = warp * 32; k < width; k += RM_WARPS * 32) {
+            const unsigned av[2][4] = {{a0.x, a1.x, a0.y, a1.y}, {a0.z, a1.z, a0.w, a1.w}};
+            unsigned b[4][2][2][3];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    three(wv[j][h].x, wv[j][h].y, b[j][h][0]);
+                    three(wv[j][h].z, wv[j][h].w, b[j][h][1]);
                 }
-                gbest[g] = (group_top >= 2 && per >= 2) ? b1 + b2 : b1;
+            ask(k + RM_WARPS * 32);  // (the next ones are on their way during the products)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 2; i >= 0; --i)
+                        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                            : "r"(av[h][0]), "r"(av[h][1]), "r"(av[h][2]), "r"(av[h][3]), "r"(b[j][h][0][i]), "r"(b[j][h][1][i]));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[j][i] += c[i];
             }
         }
-        __syncwarp();
-        if (lane != 0) return;
-        if (keep < groups) {
-            for (int round = 0; round < keep; ++round) {  // (a kept group is marked by +inf; ties: the lower index)
-                int best = -1;
-                float bv = -INFINITY;
-                for (int g = 0; g < groups; ++g)
-                    if (gbest[g] != INFINITY && (best < 0 || gbest[g] > bv)) { bv = gbest[g]; best = g; }
-                if (best < 0) break;
-                gbest[best] = INFINITY;
+        float* mine = sm + warp * RM_TOKENS * LD;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mine[(g + 8 * (i >> 1)) * LD + 8 * j + 2 * t + (i & 1)] = acc[j][i];
+        __syncthreads();
+        for (int i = tid; i < RM_TOKENS * RM_EXPERTS; i += RM_WARPS * 32) {
+            const int row = i / RM_EXPERTS, e = e0 + i % RM_EXPERTS;
+            if (e < experts) {
+                float s = 0.f;
+#pragma unroll
+                for (int v = 0; v < RM_WARPS; ++v) s += sm[(v * RM_TOKENS + row) * LD + i % RM_EXPERTS];
+                scores[row * per_token + e] = bias != nullptr ? s + bias[e] : s;
             }
-            for (int g = 0; g < groups; ++g)
-                if (gbest[g] != INFINITY)
-                    for (int e = g * per; e < (g + 1) * per; ++e) choice[e] = -INFINITY;
         }
-        float total = 0.f;
-        for (int j = 0; j < top; ++j) {
-            int best = -1;
-            float bv = -INFINITY;
-            for (int e = 0; e < experts; ++e)
-                if (choice[e] > bv) { bv = choice[e]; best = e; }
-            float wj = best < 0 ? 0.f : score[best];
-            ids[(size_t)n * top + j] = best < 0 ? 0 : best;
-            weights[(size_t)n * top + j] = wj;
-            total += wj;
-            if (best >= 0) choice[best] = -INFINITY;  // taken
-        }
-        float f = weight_scale / (total + 1e-20f);
-        for (int j = 0; j < top; ++j) weights[(size_t)n * top + j] *= f;
-        return;
+        __syncthreads();
     }
-    // softmax over all experts (lanes share the work, every lane ends with the same numbers)
-    float m = -INFINITY;
-    for (int e = lane; e < experts; e += 32) m = fmaxf(m, score[e]);
-    m = warp_max(m);
-    float sum = 0.f;
-    for (int e = lane; e < experts; e += 32) {
-        float p = expf(score[e] - m);
-        score[e] = p;
-        sum += p;
+    for (int row = warp; row < min(RM_TOKENS, num_tokens - n0); row += RM_WARPS) {
+        float* score = scores + row * per_token;
+        choose_experts(n0 + row, score, score + experts, score + experts + groups, lane, experts, top, groups, keep, sigmoid_scores, correction,
+                       group_top, weight_scale, ids, weights);
     }
-    sum = warp_sum(sum);
-    __syncwarp();
-    float inv = 1.0f / sum;
-    for (int e = lane; e < experts; e += 32) score[e] *= inv;
-    __syncwarp();
-    int per = experts / groups;
-    for (int g = lane; g < groups; g += 32) {
-        float b = -1.f;
-        for (int e = g * per; e < (g + 1) * per; ++e) b = fmaxf(b, score[e]);
-        gbest[g] = b;
-    }
-    __syncwarp();
-    if (lane != 0) return;
-    // keep the best groups: a group that is not kept gets its experts' scores hidden (negated - 1)
-    if (keep < groups) {
-        for (int round = 0; round < keep; ++round) {
-            int best = -1;
-            float bv = -1.f;
-            for (int g = 0; g < groups; ++g)
-                if (gbest[g] >= 0.f && gbest[g] > bv) { bv = gbest[g]; best = g; }
-            if (best < 0) break;
-            gbest[best] = -2.f - gbest[best];  // marked as kept
-        }
-        for (int g = 0; g < groups; ++g)
-            if (gbest[g] >= 0.f)
-                for (int e = g * per; e < (g + 1) * per; ++e) score[e] = -1.f - score[e];
-    }
-    float total = 0.f;
-    for (int j = 0; j < top; ++j) {
-        int best = 0;
-        float bv = -1.f;
-        for (int e = 0; e < experts; ++e)
-            if (score[e] >= 0.f && score[e] > bv) { bv = score[e]; best = e; }
-        ids[(size_t)n * top + j] = best;
-        weights[(size_t)n * top + j] = bv < 0.f ? 0.f : bv;
-        total += bv < 0.f ? 0.f : bv;
-        score[best] = -1.f - score[best];  // taken
-    }
-    float f = weight_scale / (total + 1e-20f);
-    for (int j = 0; j < top; ++j) weights[(size_t)n * top + j] *= f;
 }
 
 constexpr int TILE_M = 64, TILE_N = 64, TILE_K = 32;
@@ -598,11 +750,18 @@ IE_API int ie_route_topk(const void* x, int dtype, const float* w, const float* 
     const bool many = num_tokens >= MANY * ie_sm_count() && MANY * one <= 48 * 1024;
     const size_t smem = many ? MANY * one : one;
     const dim3 grid(many ? (num_tokens + MANY - 1) / MANY : num_tokens);
+    const int whole_pieces = width % (dtype == IE_BF16 ? 8 : 4) == 0 && ((uintptr_t)x & 15) == 0;
     cudaStream_t s = (cudaStream_t)stream;
 #define IE_ROUTE(T, TOKENS)                                                                                              \
-    return ie_launch(route_topk_kernel<T, TOKENS>, grid, dim3(ROUTE_THREADS), smem, s, (const T*)x, w, bias, num_tokens, \
-                     width, experts, top, groups, keep, sigmoid_scores, correction, group_top, weight_scale, ids, weights)
+    return ie_launch(route_topk_kernel<T, TOKENS>, grid, dim3(TOKENS > 1 ? 256 : 1024), smem, s, (const T*)x, w, bias, num_tokens, \
+                     width, experts, top, groups, keep, sigmoid_scores, correction, group_top, weight_scale, whole_pieces, ids, weights)
     if (dtype == IE_BF16) {
+        // (16 tokens a block from as many tokens on as four a block fill the device with, and rows of whole 32s)
+        const size_t scratch = (size_t)RM_WARPS * RM_TOKENS * (RM_EXPERTS + 1) + (size_t)RM_TOKENS * (2 * experts + groups);
+        if (num_tokens >= MANY * ie_sm_count() && width % 32 == 0 && whole_pieces && !((uintptr_t)w & 15) && scratch * sizeof(float) <= 48 * 1024)
+            return ie_launch(route_many_kernel, dim3((num_tokens + RM_TOKENS - 1) / RM_TOKENS), dim3(RM_WARPS * 32), scratch * sizeof(float), s,
+                             (const __nv_bfloat16*)x, w, bias, num_tokens, width, experts, top, groups, keep, sigmoid_scores, correction,
+                             group_top, weight_scale, ids, weights);
         if (many) IE_ROUTE(__nv_bfloat16, MANY);
         IE_ROUTE(__nv_bfloat16, 1);
     }
