@@ -1,7 +1,8 @@
 // The routed feed-forward's two grouped products on the fifth-generation tensor cores, bfloat16 in, 32-bit sums in tensor memory.
 //
-//  * routed_sort: the step's (token, choice) pairs in the order of their experts, without gaps, and a list of tiles: up to 256
-//    neighbouring pairs of one expert, an expert's pairs in equal tiles.
+//  * routed_sort: the step's (token, choice) pairs in the order of their experts, and a list of tiles: up to so many neighbouring
+//    pairs of one expert (256 for the kernels here), an expert's pairs in equal tiles.  With `align` 8 an expert's run and its tiles start at
+//    multiples of 8 (for the kernels of routed_tiled.cu); the places between hold -1.
 //  * routed_tc5<true>: per tile and 128 hidden features: gate and up products, then the activation, to y[place in the order].
 //  * routed_tc5<false>: per tile and 256 output features: y times the expert's down matrix, times the pair's routing weight, to
 //    out[choice][token][:].
@@ -220,17 +221,18 @@ routed_tc5_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     if (threadIdx.x == 0 && sh->failed) ie_report(err, IE_ERR_TIMEOUT, blockIdx.x, blockIdx.y);
 }
 
-// One block.  order[pairs]: the pairs by expert (an id outside the experts leaves its pair out); tiles and meta as above.  A pair's rank among its
+// One block.  order[pairs, or more with the gaps]: the pairs by expert (an id outside the experts leaves its pair out); tiles as above; meta: how
+// many tiles, how many places.  A pair's rank among its
 // expert's comes from the counter it raises; up to KEPT pairs of a thread keep it in registers, the rest take theirs in a second pass.
 constexpr int SORT_THREADS = 1024, KEPT = 8;
 __global__ void __launch_bounds__(SORT_THREADS)
 routed_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ order, int4* __restrict__ tiles,
-                   int* __restrict__ meta, int max_tiles) {
+                   int* __restrict__ meta, int max_tiles, int most, int align, int places) {
     extern __shared__ int ism[];  // count[experts], first[experts], tile[experts]
     int* count = ism;
     int* first = count + experts;
     int* tile0 = first + experts;
-    __shared__ int total_tiles;
+    __shared__ int total_tiles, total_places;
     ie_pdl_trigger();
     ie_pdl_wait();
     const int tid = threadIdx.x;
@@ -241,6 +243,8 @@ routed_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int* __r
         mine[k] = i < pairs ? ids[i] : -1;
     }
     for (int e = tid; e < experts; e += SORT_THREADS) count[e] = 0;
+    if (align > 1)
+        for (int i = tid; i < places; i += SORT_THREADS) order[i] = -1;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < KEPT; ++k)
@@ -254,9 +258,10 @@ routed_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int* __r
     }
     __syncthreads();
     if (tid < 32) {  // running sums of pairs and tiles over the experts, 32 at a time
-        int at = 0, t = 0;
+        int at = 0, t = 0;  // (places and tiles so far)
         for (int e0 = 0; e0 < experts; e0 += 32) {
-            const int e = e0 + tid, c = e < experts ? count[e] : 0, k = (c + MOST_PAIRS - 1) / MOST_PAIRS;
+            const int e = e0 + tid, pairs_of = e < experts ? count[e] : 0, k = (pairs_of + most - 1) / most;
+            const int c = (pairs_of + align - 1) / align * align;
             int sc = c, sk = k;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -270,15 +275,15 @@ routed_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int* __r
             at += __shfl_sync(0xffffffffu, sc, 31);
             t += __shfl_sync(0xffffffffu, sk, 31);
         }
-        if (tid == 0) total_tiles = t;
+        if (tid == 0) { total_tiles = t; total_places = at; }
     }
     __syncthreads();
-    if (tid == 0) meta[0] = min(total_tiles, max_tiles);
+    if (tid == 0) { meta[0] = min(total_tiles, max_tiles); meta[1] = total_places; }
     for (int e = tid; e < experts; e += SORT_THREADS) {
-        const int c = count[e], k = (c + MOST_PAIRS - 1) / MOST_PAIRS;
-        for (int j = 0; j < k; ++j) {  // (equal tiles, the earlier ones a pair longer)
-            const int each = c / k, more = c - each * k, at = j * each + min(j, more);
-            if (tile0[e] + j < max_tiles) tiles[tile0[e] + j] = make_int4(e, first[e] + at, each + (j < more ? 1 : 0), 0);
+        const int c = count[e], k = (c + most - 1) / most, units = (c + align - 1) / align;
+        for (int j = 0; j < k; ++j) {  // (equal tiles, the earlier ones a pair, or `align` of them, longer)
+            const int each = units / k, more = units - each * k, at = (j * each + min(j, more)) * align;
+            if (tile0[e] + j < max_tiles) tiles[tile0[e] + j] = make_int4(e, first[e] + at, min((each + (j < more ? 1 : 0)) * align, c - at), 0);
         }
     }
 #pragma unroll
@@ -313,14 +318,19 @@ bool make_expert_map(CUtensorMap* map, const void* base, int matrices, int rows,
 IE_API int ie_routed_tc5_ok(int hidden, int ff) { return encode_fn() != nullptr && hidden % 8 == 0 && ff % 8 == 0 && hidden > 0 && ff > 0; }
 
 // The most tiles `pairs` pairs over `experts` experts can need.
-IE_API int ie_routed_tc5_max_tiles(int pairs, int experts) { return pairs / MOST_PAIRS + (pairs < experts ? pairs : experts); }
+IE_API int ie_routed_tc5_max_tiles(int pairs, int experts, int most) { return pairs / most + (pairs < experts ? pairs : experts); }
 
-IE_API int ie_routed_sort(const int* ids, int pairs, int experts, int* order, int* tiles, int* meta, int max_tiles, void* stream) {
+IE_API int ie_routed_tc5_most() { return MOST_PAIRS; }
+
+// places: the length of `order` (with `align` > 1: room for the gaps).
+IE_API int ie_routed_sort(const int* ids, int pairs, int experts, int* order, int* tiles, int* meta, int max_tiles, int most, int align,
+                          int places, void* stream) {
     if (pairs <= 0) return 0;
+    if (most < align || align < 1 || (long long)places < pairs + (align - 1ll) * (pairs < experts ? pairs : experts)) return (int)cudaErrorInvalidValue;
     const size_t smem = (size_t)3 * experts * sizeof(int);
     if (smem > 40 * 1024 || ((uintptr_t)tiles & 15)) return (int)cudaErrorInvalidValue;
     return ie_launch(routed_sort_kernel, dim3(1), dim3(SORT_THREADS), smem, (cudaStream_t)stream, ids, pairs, experts, order,
-                     (int4*)tiles, meta, max_tiles);
+                     (int4*)tiles, meta, max_tiles, most, align, places);
 }
 
 // x: [N, K], w: [experts, 2, F, K], y: [pairs, F] in the order of the pairs.

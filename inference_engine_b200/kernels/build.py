@@ -251,7 +251,7 @@ PART_LIBRARIES = {
     # the latent attention's input stage and per-head products
     "latent": ["latent_attention.cu"],
     "delta": ["delta_rule.cu"],  # the gated delta rule: convolutions, the recurrence, the read-out norm
-    "routed": ["routed_experts.cu", "routed_tc5.cu"],  # routing and the grouped products of the routed feed-forward
+    "routed": ["routed_experts.cu", "routed_tc5.cu", "routed_tiled.cu"],  # routing and the grouped products of the routed feed-forward
     # recurrent mixers with a decaying matrix state (gated-write linear attention, exponential-gate
     # matrix memory, state-space duality): input convolutions, gates, the recurrence, the read-outs
     "recurrent": ["gated_recurrence.cu"],

@@ -1212,10 +1212,18 @@ class CudaOps:
             "ie_routed_gate_up": "P P P I P P P I I I I F I F F P",
             "ie_routed_down": "P P P P I P P P I I I I I P",
             "ie_routed_tc5_ok": "I I",
-            "ie_routed_tc5_max_tiles": "I I",
-            "ie_routed_sort": "P I I P P P I P",
+            "ie_routed_tc5_max_tiles": "I I I",
+            "ie_routed_tc5_most": "",
+            "ie_routed_sort": "P I I P P P I I I I P",
             "ie_routed_tc5_gate_up": "P P P P P P I I I I I F I F F P P",
             "ie_routed_tc5_down": "P P P P P P P I I I I I I P P",
+            "ie_routed_tiled_few": "",
+            "ie_routed_tiled_most": "",
+            "ie_routed_tiled_align": "",
+            "ie_routed_tiled_places": "I I",
+            "ie_routed_tiled_gather": "P P P P I I I P",
+            "ie_routed_tiled_gate_up": "P P P P P P I I I I I I I F I F F P P",
+            "ie_routed_tiled_down": "P P P P P P P I I I I I I I P P",
         },
         "recurrent": {
             "ie_short_conv_residual": "P I P P L P P P P I I I I I P P",
@@ -1483,13 +1491,14 @@ class CudaOps:
         # 109 us, the mma.sync kernels 57 / 115 / 128 / 207.  They keep the widths without whole 16-byte rows.
         if (x.dtype == torch.bfloat16 and lib.ie_routed_tc5_ok(hidden, ff) and experts <= 3000
                 and not (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16):
-            max_tiles = lib.ie_routed_tc5_max_tiles(pairs, experts)
+            most = lib.ie_routed_tc5_most()
+            max_tiles = lib.ie_routed_tc5_max_tiles(pairs, experts, most)
             index = ws.buffer(tag + ".order", 1, 4 * max_tiles + 4 + pairs, torch.int32, rows_cap=None)[0]
             tiles, meta, order = index[: 4 * max_tiles], index[4 * max_tiles: 4 * max_tiles + 4], index[4 * max_tiles + 4:]
             y = ws.buffer(tag + ".act", pairs, ff, x.dtype)
             if out is None:
                 out = ws.buffer(tag + ".delta", pairs, hidden, torch.float32).view(top, n, hidden)
-            self._routed_sort(lib, ids, pairs, experts, order, tiles, meta, max_tiles)
+            self._routed_sort(lib, ids, pairs, experts, order, tiles, meta, max_tiles, most, 1, pairs)
             self._routed_tc5_gate_up(lib, x, w_gate_up, y, order, tiles, meta, max_tiles, top, limit, alpha, up_offset)
             self._routed_tc5_down(lib, y, w_down, out, weights, order, tiles, meta, max_tiles, n, top)
             return out
@@ -1506,10 +1515,55 @@ class CudaOps:
         self._routed_down(lib, y, w_down, out, weights, sorted_pairs, tile_expert, meta, max_tiles, top, n, ff, hidden)
         return out
 
+    def routed_experts_tiled(self, x, ids, weights, experts, *, limit, alpha, up_offset, ws, tag="moe", out=None):
+        """`routed_experts` on weights laid out in tiles (`ExpertTiles`; `csrc/routed_tiled.cu`)."""
+        lib = self._part_lib("routed")
+        n, top = ids.shape
+        count, ff, hidden = experts.experts, experts.ff, experts.hidden
+        pairs = n * top
+        if not x.is_contiguous() or x.data_ptr() % 16:
+            x = ws.buffer(tag + ".x", n, hidden, x.dtype).copy_(x)
+        # Few tokens are a stream of weights, many a matter of products.  The line is where tiles of 64 pairs hold every expert's.
+        few = n <= lib.ie_routed_tiled_few()
+        most, align, places = lib.ie_routed_tiled_most(), lib.ie_routed_tiled_align(), lib.ie_routed_tiled_places(pairs, count)
+        max_tiles = lib.ie_routed_tc5_max_tiles(pairs, count, most)
+        index = ws.buffer(tag + ".order", 1, 4 * max_tiles + 4 + places, self.torch.int32, rows_cap=None)[0]
+        tiles, meta, order = index[: 4 * max_tiles], index[4 * max_tiles: 4 * max_tiles + 4], index[4 * max_tiles + 4:]
+        y = ws.buffer(tag + ".act", places, -(-ff // 64) * 64, x.dtype)
+        if out is None:
+            out = ws.buffer(tag + ".delta", pairs, hidden, self.torch.float32).view(top, n, hidden)
+        self._routed_sort(lib, ids, pairs, count, order, tiles, meta, max_tiles, most, align, places)
+        if not few:
+            xs = ws.buffer(tag + ".sorted", places, -(-hidden // 64) * 64, x.dtype)
+            self._routed_gather(lib, x, xs, order, meta, places, top)
+            x = xs
+        self._routed_tiled_gate_up(lib, x, experts, y, order, tiles, meta, max_tiles, few, top, n, places, limit, alpha, up_offset)
+        self._routed_tiled_down(lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, top, n, places)
+        return out
+
     @_kind("routed.align")
-    def _routed_sort(self, lib, ids, pairs, experts, order, tiles, meta, max_tiles) -> None:
+    def _routed_gather(self, lib, x, xs, order, meta, places, top) -> None:
+        self._check(lib.ie_routed_tiled_gather(x.data_ptr(), xs.data_ptr(), order.data_ptr(), meta.data_ptr(), places, top, x.shape[1],
+                                               self._stream()), "routed_gather")
+
+    @_kind("routed.gate_up")
+    def _routed_tiled_gate_up(self, lib, x, experts, y, order, tiles, meta, max_tiles, few, top, n, places, limit, alpha, up_offset) -> None:
+        self._check(lib.ie_routed_tiled_gate_up(
+            x.data_ptr(), experts.gate_up.data_ptr(), y.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(), max_tiles,
+            int(few), top, n, places, experts.hidden, experts.ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha,
+            up_offset, self._err_ptr, self._stream()), "routed_few_gate_up" if few else "routed_pair_gate_up")
+
+    @_kind("routed.down")
+    def _routed_tiled_down(self, lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, top, n, places) -> None:
+        self._check(lib.ie_routed_tiled_down(
+            y.data_ptr(), experts.down.data_ptr(), out.data_ptr(), weights.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
+            max_tiles, int(few), top, n, places, experts.ff, experts.hidden, self._err_ptr, self._stream()),
+            "routed_few_down" if few else "routed_pair_down")
+
+    @_kind("routed.align")
+    def _routed_sort(self, lib, ids, pairs, experts, order, tiles, meta, max_tiles, most, align, places) -> None:
         self._check(lib.ie_routed_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
-                                       max_tiles, self._stream()), "routed_sort")
+                                       max_tiles, most, align, places, self._stream()), "routed_sort")
 
     @_kind("routed.gate_up")
     def _routed_tc5_gate_up(self, lib, x, w, y, order, tiles, meta, max_tiles, top, limit, alpha, up_offset) -> None:

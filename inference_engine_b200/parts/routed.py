@@ -20,7 +20,7 @@ more slice, or the parts of a split product, behind the chosen experts' slices. 
 output from one last product that can be told where to go (``forward(x, ctx, slices_before)``).
 
 The experts' matrices are stacked (``[experts, 2, ff, hidden]`` gates then ups, and
-``[experts, hidden, ff]``), a step's (token, expert) pairs are sorted by expert on the device, and
+``[experts, hidden, ff]``; in bfloat16 on the GPU, with widths that are multiples of 8, in tiles: `ExpertTiles`), a step's (token, expert) pairs are sorted by expert on the device, and
 two grouped products run over the sorted list; nothing about the routing is read by the host.  The
 result is ``[top, N, hidden]``: slice ``j`` holds the weighted output of every token's ``j``-th
 choice, and the next norm adds the slices in order, like the parts of a split matrix product.
@@ -28,9 +28,44 @@ choice, and the next norm adds the slices in order, like the parts of a split ma
 
 from __future__ import annotations
 
+from dataclasses import dataclass
+from typing import Any
+
 from ..config.spec import PartSpec
 from .base import BuildEnv, FeedForward, WeightDecl
 from .registry import build_part, register_part
+
+
+@dataclass
+class ExpertTiles:
+    """The experts' bfloat16 matrices as the tensor cores read them: tiles of 128 rows by 64 columns, 16 KB each, a row's pieces
+    of eight columns turned by its number (piece p of row r lies at place ``p ^ (r % 8)``).  ``gate_up``: ``[experts, ff / 64, hidden / 64,
+    128, 64]``, 64 features' gate and up rows in turn, eight of each; ``down``: ``[experts, hidden / 128, ff / 64, 128, 64]``.  What
+    fills the last tiles up is zero."""
+
+    experts: int
+    ff: int
+    hidden: int
+    gate_up: Any
+    down: Any
+
+    @staticmethod
+    def fit(experts: int, ff: int, hidden: int) -> bool:
+        return experts <= 3000 and hidden % 8 == 0 and ff % 8 == 0
+
+    @classmethod
+    def of(cls, gate_up, down):
+        """From ``[experts, 2, ff, hidden]`` and ``[experts, hidden, ff]``."""
+        import torch
+
+        count, _, ff, hidden = gate_up.shape
+        f, h, rows = -(-ff // 64), -(-hidden // 64), -(-hidden // 128)
+        row, piece = torch.arange(128, device=down.device)[:, None], torch.arange(8, device=down.device)[None, :]
+        pad = torch.nn.functional.pad
+        gu = pad(gate_up, (0, h * 64 - hidden, 0, f * 64 - ff)).view(count, 2, f, 8, 8, h, 8, 8).permute(0, 2, 5, 3, 1, 4, 6, 7)
+        dn = pad(down, (0, f * 64 - ff, 0, rows * 128 - hidden)).view(count, rows, 128, f, 8, 8).permute(0, 1, 3, 2, 4, 5)
+        turned = lambda t, a, b: t.reshape(count, a, b, 128, 8, 8)[:, :, :, row, piece ^ (row % 8)].view(count, a, b, 128, 64)  # noqa: E731
+        return cls(count, ff, hidden, turned(gu, f, h), turned(dn, rows, f))
 
 
 @register_part("feed_forward", "routed_experts")
@@ -61,7 +96,7 @@ class RoutedExperts(FeedForward):
         self.hidden_size, self.intermediate_size = hidden_size, intermediate_size
         self.limit = None if limit is None else float(limit)
         self.alpha, self.up_offset, self.dtype = float(alpha), float(up_offset), dtype
-        self.w_router = self.w_gate_up = self.w_down = None
+        self.w_router = self.w_gate_up = self.w_down = self.tiles = None
 
     @classmethod
     def from_spec(cls, params: dict, env: BuildEnv, **_):
@@ -113,6 +148,16 @@ class RoutedExperts(FeedForward):
             for e in range(self.experts)]).contiguous()
         self.w_down = torch.stack([tensors[self._name(e, "down")].to(self.dtype)
                                    for e in range(self.experts)]).contiguous()
+        if (self.dtype == torch.bfloat16 and self.w_down.is_cuda
+                and ExpertTiles.fit(self.experts, self.intermediate_size, self.hidden_size)):
+            self.tiles = ExpertTiles.of(self.w_gate_up, self.w_down)
+            self.w_gate_up = self.w_down = None
+
+    def _experts(self, x, ids, weights, ctx, out=None):
+        rest = {"limit": self.limit, "alpha": self.alpha, "up_offset": self.up_offset, "ws": ctx.ws, "tag": "moe", "out": out}
+        if self.tiles is not None:
+            return ctx.ops.routed_experts_tiled(x, ids, weights, self.tiles, **rest)
+        return ctx.ops.routed_experts(x, ids, weights, self.w_gate_up, self.w_down, **rest)
 
     def forward(self, x, ctx):
         import torch
@@ -129,10 +174,7 @@ class RoutedExperts(FeedForward):
         else:
             ctx.ops.route_topk(x, self.w_router, self.groups, self.keep_groups, ids, weights, bias=self.router_bias)
         if self.shared is None:
-            return ctx.ops.routed_experts(x, ids, weights, self.w_gate_up, self.w_down,
-                                          limit=self.limit, alpha=self.alpha, up_offset=self.up_offset,
-                                          ws=ctx.ws, tag="moe")
+            return self._experts(x, ids, weights, ctx)
         both = self.shared.forward(x, ctx, slices_before=self.top)  # [top + parts, N, hidden]
-        ctx.ops.routed_experts(x, ids, weights, self.w_gate_up, self.w_down, limit=self.limit, alpha=self.alpha,
-                               up_offset=self.up_offset, ws=ctx.ws, tag="moe", out=both[: self.top])
+        self._experts(x, ids, weights, ctx, out=both[: self.top])
         return both

@@ -1,0 +1,91 @@
+"""The routed feed-forward on weights laid out in tiles against plain sums in 64 bits: edges of the tiles of pairs, ragged widths, few
+tokens and many; and the router's products on the tensor cores."""
+
+import pytest
+import torch
+
+from tests.test_routed_tc5_gpu import _want
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(x, ids, weights, gate_up, down, limit, alpha, offset):
+    from inference_engine_b200.engine.workspace import Workspace
+    from inference_engine_b200.kernels import get_ops
+    from inference_engine_b200.parts.routed import ExpertTiles
+
+    ops = get_ops()
+    before = dict(ops.launch_counts)
+    out = ops.routed_experts_tiled(x, ids, weights, ExpertTiles.of(gate_up, down), limit=limit, alpha=alpha, up_offset=offset, ws=Workspace("cuda"))
+    ops.check_errors()
+    return out, {name for name, n in ops.launch_counts.items() if n > before.get(name, 0)}
+
+
+# pairs per expert: around the rounding to 32, an accumulator's 256, a tile's 384, several tiles; experts nobody chose; up to 64 tokens
+@pytest.mark.parametrize("counts", [[0, 1, 31, 32, 33, 63], [255, 256, 257, 0, 320, 64], [383, 384, 385, 0, 770, 8], [0, 0, 2300, 0], [1, 0, 15, 16, 17],
+                                    [0, 64, 0], [1]])
+@pytest.mark.parametrize("hidden,ff,limit", [(128, 64, None), (320, 136, 1.5), (72, 264, None), (520, 128, 0.7)])
+def test_pairs_per_expert(counts, hidden, ff, limit):
+    g = torch.Generator(device="cuda").manual_seed(hidden + len(counts))
+    experts, n, top = len(counts), sum(counts), 1
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(n)].view(n, top).int().cuda()
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, gate_up, down = rand(n, hidden).bfloat16(), (rand(experts, 2, ff, hidden) * hidden ** -0.5).bfloat16(), (rand(experts, hidden, ff) * ff ** -0.5).bfloat16()
+    args = (x, ids, torch.rand(n, top, generator=g, device="cuda"), gate_up, down, limit, 1.3, 0.5)
+    got, ran = _run(*args)
+    assert ("routed_few_down" if n <= 64 else "routed_pair_down") in ran
+    # y is rounded to 8 bits in both, from sums that differ in the last of 24: a few roundings fall the other way
+    want = _want(*args)
+    torch.testing.assert_close(got.double(), want, atol=2e-2, rtol=1e-2)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-3
+
+
+@pytest.mark.parametrize("tokens,top,experts", [(2600, 4, 8), (33, 2, 4), (64, 3, 40), (65, 3, 40), (301, 3, 40)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_several_choices_per_token(tokens, top, experts, aligned):
+    """More pairs than the sorting block keeps in registers (8,192); rows that start anywhere; an id that is no expert."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    hidden, ff = 64, 72
+    ids = torch.rand(tokens, experts, generator=g, device="cuda").topk(top, dim=-1).indices.int()
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x = rand(tokens * hidden + 8).bfloat16()[0 if aligned else 1:][: tokens * hidden].view(tokens, hidden)
+    gate_up, down = (rand(experts, 2, ff, hidden) * 0.1).bfloat16(), (rand(experts, hidden, ff) * 0.1).bfloat16()
+    args = (x, ids, torch.rand(tokens, top, generator=g, device="cuda"), gate_up, down, None, 1.0, 0.0)
+    got, want = _run(*args)[0], _want(*args)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-3
+    ids[5, 0] = experts
+    got, want = _run(*args)[0], _want(*args)
+    got[0, 5] = want[0, 5] = 0.0  # (a pair without an expert is nobody's)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-3
+
+
+@pytest.mark.parametrize("tokens,width,experts,top,groups,keep", [(600, 64, 7, 2, 1, 1), (1000, 2048, 32, 4, 4, 2), (593, 288, 40, 3, 8, 3), (2048, 96, 64, 4, 1, 1)])
+@pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])
+def test_router_of_many_tokens(tokens, width, experts, top, groups, keep, scoring):
+    from inference_engine_b200.kernels import get_ops
+
+    ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(width)
+    x = torch.randn(tokens, width, generator=g, device="cuda").bfloat16()
+    w = torch.randn(experts, width, generator=g, device="cuda") * width ** -0.5
+    bias = torch.randn(experts, generator=g, device="cuda") * 0.1
+    correction = torch.randn(experts, generator=g, device="cuda") * 0.01 if scoring == "sigmoid" else None
+    ids, weights = torch.empty(tokens, top, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+    ops.route_topk(x, w, groups, keep, ids, weights, bias=bias, scoring=scoring, correction=correction)
+    logits = x.double() @ w.double().T + bias.double()
+    scores = logits.softmax(-1) if scoring == "softmax" else logits.sigmoid()
+    choice = scores + (correction.double() if correction is not None else 0)
+    best = choice.view(tokens, groups, -1).amax(-1)
+    kept = torch.zeros(tokens, groups, dtype=torch.bool, device="cuda").scatter_(1, best.topk(keep, dim=-1).indices, True)
+    allowed = choice.masked_fill(~kept.repeat_interleave(experts // groups, dim=1), -1.0)
+    ranked = allowed.sort(dim=-1, descending=True)
+    # sums of 32 bits: where two scores (or two groups) are further apart than 1e-5 the choice is the same
+    gap = (ranked.values[:, :top] - ranked.values[:, 1: top + 1]).amin(-1) if top < experts else torch.ones(tokens, device="cuda")
+    if keep < groups:
+        by_group = best.sort(dim=-1, descending=True).values
+        gap = torch.minimum(gap, by_group[:, keep - 1] - by_group[:, keep])
+    sure = gap > 1e-5
+    assert sure.float().mean() > 0.97
+    assert torch.equal(ids[sure].long(), ranked.indices[sure, :top])
+    want = scores.gather(1, ids.long())
+    want = want / want.sum(-1, keepdim=True)
+    torch.testing.assert_close(weights[sure].double(), want[sure], atol=2e-6, rtol=2e-5)
