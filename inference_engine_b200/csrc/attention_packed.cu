@@ -77,11 +77,6 @@ static_assert(ROWS * (DV * 4 + 8) <= Q_BYTES + KS * K_BYTES + VS * V_BYTES, "roo
 constexpr size_t SMEM_BYTES = (size_t)Q_BYTES + KS * K_BYTES + VS * V_BYTES + sizeof(Bars) + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 
-__device__ __forceinline__ bool elect_one() {
-    unsigned p;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-    return p != 0;
-}
 // Shared-memory descriptors as their two words: the low one (start address and, for values, the distance of the runs, in 16-byte units)
 // moves with the address, the high one (groups of eight rows 1,024 bytes apart, version, 128-byte swizzle) is a constant.  An instruction
 // then costs an addition an operand; descriptors put together anew for each cost the issuing warp 100 clocks an instruction beside

@@ -16,8 +16,10 @@
 // copy is used.
 //
 // The weights do not depend on the kernel that runs before this one, so under programmatic
-// dependent launch the producer fills the ring before it waits for that kernel; only the copy
-// of X (the kernel's activations, one TMA box per 64 k) comes after the wait.
+// dependent launch the producer fills the ring before it waits for that kernel; only the copies
+// of X (the kernel's activations) come after the wait, up to eight blocks of 64 k each.  The producer's warp stays converged and
+// elects a thread, so that the copies' operands are the warp's (`elect_one`): with a copy of X for every 64 k, issued behind a branch on the
+// lane's number, a decode step of the 1B shape at 8 rows took 730 us, 380 of them these products; 703 and 355 so.
 //
 // Matrices with few output features are also cut along k (grid.y = splits) so that every SM
 // has a block; the partial sums go to out[split][M][N] and the consumer of the product adds
@@ -37,12 +39,13 @@ constexpr int STAGE_BYTES = BN * BK * 2;  // 16 KB: one k block of 128 features
 constexpr int MAX_KBLOCKS = 32;           // k-slice of a block: at most 2048
 constexpr int MAX_OPS = 12;               // copies in flight (ring slots)
 constexpr int MAX_KPO = 4;                // k blocks per copy
+constexpr int X_KBLOCKS = 8;              // k blocks of X per copy
 // Shared memory for tiles: what the 227 KB of an SM leave beside X (8 NT rows x 2048 k)
 __host__ __device__ constexpr int ring_bytes(int nt) { return nt == 1 ? 192 * 1024 : 160 * 1024; }
 
 #ifdef IE_TEST_STARVE
 // Self-test build only (kernels/build.py: build_selftest).  While this flag is set, every block
-// leaves out the last box of X although the barrier was told to expect all of them: the
+// leaves out the last copy of X although its barrier was told to expect it: the
 // consumers' wait for X must run out, the block must record IE_ERR_TIMEOUT and return.  The
 // copies of W that were asked for meanwhile are few and complete long before the wait gives up.
 static __device__ int g_starve_last_x;
@@ -56,16 +59,16 @@ static __device__ int g_starve_last_x;
 // writes out[m][i] = silu(gate_i) * up_i, silu(g) = g / (1 + exp(-g)) (engine/model/layers.py:277-281),
 // N / 2 values per token, instead of the product itself; the inner dimension is not cut (one split).
 template <int NT, typename OutT, bool GATED = false>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1)
 gemm_tma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
-                OutT* __restrict__ out, int M, int N, int K, int kblocks_per_split, int ops, int kpo, int w3d,
+                OutT* __restrict__ out, int M, int N, int K, int kblocks_per_split, int ops, int kpo, int w3d, int xkb,
                 int* err) {
     constexpr int XR = 8 * NT;                 // rows of X staged (missing rows read as zero)
     constexpr int XBOX_BYTES = XR * BK * 2;
     extern __shared__ unsigned char smem_raw[];
     // swizzled TMA tiles want 1024-byte alignment; the launch reserves the slack
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int n0 = blockIdx.x * BN;
     int split = blockIdx.y;
     int total_kblocks = (K + BK - 1) / BK;
@@ -94,36 +97,38 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     ie_pdl_trigger();
 
     if (warp == CWARPS) {
-        // ---- producer: one thread ----
-        if (lane == 0) {
-            auto copy_w = [&](int o) {  // copy o of this block into slot o % ops
-                int s = o % ops;
-                mbar_expect_tx(&full[s], op_bytes);
-                if (w3d)
-                    tma_load_3d(ring + (size_t)s * op_bytes, &w_map, 0, n0, kb0 + o * kpo, &full[s]);
-                else
-                    tma_load_2d(ring + (size_t)s * op_bytes, &w_map, (kb0 + o) * BK, n0, &full[s]);
-            };
-            int issued = 0;
-            // the weights need nobody's results: fill the ring right away
-            for (; issued < nops && issued < ops; ++issued) copy_w(issued);
-            ie_pdl_wait();  // X is the previous kernel's output
-            if (nkb > 0) {
-                mbar_expect_tx(x_full, nkb * XBOX_BYTES);
-                for (int kb = 0; kb < nkb; ++kb) {
+        // ---- producer: one thread of a converged warp ----
+        const bool one = elect_one();
+        auto copy_w = [&](int o, int slot) {  // copy o of this block
+            if (!one) return;
+            mbar_expect_tx(&full[slot], op_bytes);
+            if (w3d)
+                tma_load_3d(ring + (size_t)slot * op_bytes, &w_map, 0, n0, kb0 + o * kpo, &full[slot]);
+            else
+                tma_load_2d(ring + (size_t)slot * op_bytes, &w_map, (kb0 + o) * BK, n0, &full[slot]);
+        };
+        int issued = 0;
+        // the weights need nobody's results: fill the ring right away
+        for (; issued < nops && issued < ops; ++issued) copy_w(issued, issued);
+        __syncwarp();
+        ie_pdl_wait();  // X is the previous kernel's output
+        if (one && nkb > 0) mbar_expect_tx(x_full, (nkb + xkb - 1) / xkb * xkb * XBOX_BYTES);
+        for (int kb = 0; kb < nkb; kb += xkb) {
+            if (one) {
 #ifdef IE_TEST_STARVE
-                    if (g_starve_last_x && kb == nkb - 1) break;
+                if (g_starve_last_x && kb + xkb >= nkb) break;
 #endif
-                    tma_load_2d(xs + (size_t)kb * XBOX_BYTES, &x_map, (kb0 + kb) * BK, 0, x_full);
-                }
+                if (w3d) tma_load_3d(xs + (size_t)kb * XBOX_BYTES, &x_map, 0, 0, kb0 + kb, x_full);
+                else tma_load_2d(xs + (size_t)kb * XBOX_BYTES, &x_map, (kb0 + kb) * BK, 0, x_full);
             }
-            for (; issued < nops; ++issued) {
-                int round = issued / ops;  // this slot's round-th reuse: wait for its release
-                if (!mbar_wait(&empty[issued % ops], (round - 1) & 1)) { failed = 1; break; }
-                copy_w(issued);
-            }
-        } else {
-            ie_pdl_wait();
+        }
+        __syncwarp();
+        int slot = 0, phase = 0;
+        for (; issued < nops; ++issued) {  // wait for the slot's release
+            if (!__all_sync(0xffffffffu, mbar_wait(&empty[slot], phase))) { failed = 1; break; }
+            copy_w(issued, slot);
+            __syncwarp();
+            if (++slot == ops) { slot = 0; phase ^= 1; }
         }
     } else {
         // ---- consumers: warp w owns features n0 + 32 w .. + 31 (two 16-row tiles) ----
@@ -226,7 +231,8 @@ int launch(const void* X, const void* W, OutT* out, int M, int N, int K, int kbl
     } else if (!make_map_bf16(&wm, W, N, K, BN)) {
         return (int)cudaErrorNotSupported;
     }
-    if (!make_map_bf16(&xm, X, M, K, 8 * NT)) return (int)cudaErrorNotSupported;
+    const int xkb = w3d ? (kblocks_per_split < X_KBLOCKS ? kblocks_per_split : X_KBLOCKS) : 1;
+    if (w3d ? !make_map_bf16_3d(&xm, X, M, K, 8 * NT, xkb) : !make_map_bf16(&xm, X, M, K, 8 * NT)) return (int)cudaErrorNotSupported;
     int ops = ring_bytes(NT) / (kpo * STAGE_BYTES);
     if (ops > MAX_OPS) ops = MAX_OPS;
     size_t smem = (size_t)ring_bytes(NT) + (size_t)MAX_KBLOCKS * 8 * NT * BK * 2 + (2 * MAX_OPS + 1) * 8 + 1024;
@@ -235,7 +241,7 @@ int launch(const void* X, const void* W, OutT* out, int M, int N, int K, int kbl
     if (e != cudaSuccess) return (int)e;
     dim3 grid((N + BN - 1) / BN, splits);
     return ie_launch(gemm_tma_kernel<NT, OutT, GATED>, grid, dim3(THREADS), smem, s, wm, xm, out, M, N, K,
-                     kblocks_per_split, ops, kpo, w3d, err);
+                     kblocks_per_split, ops, kpo, w3d, xkb, err);
 }
 }  // namespace
 

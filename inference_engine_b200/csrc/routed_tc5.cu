@@ -225,7 +225,7 @@ routed_tc5_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 // many tiles, how many places.  A pair's rank among its
 // expert's comes from the counter it raises; up to KEPT pairs of a thread keep it in registers, the rest take theirs in a second pass.
 constexpr int SORT_THREADS = 1024, KEPT = 8;
-__global__ void __launch_bounds__(SORT_THREADS)
+__global__ void __launch_bounds__(SORT_THREADS, 1)
 routed_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ order, int4* __restrict__ tiles,
                    int* __restrict__ meta, int max_tiles, int most, int align, int places) {
     extern __shared__ int ism[];  // count[experts], first[experts], tile[experts]

@@ -119,14 +119,6 @@ __device__ __forceinline__ void put_gated(const Args& in, const float (&a)[16], 
         if (i + (high ? 1 : 0) < n) *reinterpret_cast<bf16*>(y + i * 128 + (piece ^ ((i & 6) << 4))) = __float2bfloat16_rn(v);
     }
 }
-// The thread of a converged warp that issues its copies and products.  Those take their operands from registers that a warp shares: with a branch on the
-// lane's number, and values that the compiler cannot tell are the warp's, every one of them cost its thread some 150 clocks (64 of k
-// 950 clocks, whatever the pairs).
-__device__ __forceinline__ bool elect_one() {
-    unsigned p;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ int warps_own(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 // Shared-memory descriptors as their two words: the low one moves with the address, the high one (groups of eight rows 1,024 bytes apart, version,
 // 128-byte swizzle) is a constant.  (Within a cluster an address has the block's number above its 18 bits.)

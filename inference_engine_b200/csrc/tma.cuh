@@ -54,6 +54,13 @@ __device__ __forceinline__ bool mbar_wait_compact(unsigned long long* bar, int p
     }
     return false;
 }
+// The thread of a converged warp that issues its copies and products.  Those take their operands from registers that a warp shares: behind a
+// branch on the lane's number, with values that the compiler cannot tell are the warp's, each costs its thread some 150 clocks.
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
 // One box of a 2-D tensor map into shared memory; x is the inner (contiguous) coordinate and
 // x * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
