@@ -43,9 +43,9 @@ constexpr int HALVES = HD / 64;           // 64-wide column halves of a K or V r
 constexpr int BM = 128;             // query rows per block
 constexpr int KT = 64;              // keys per tile
 constexpr int SOFTMAX_THREADS = 128;
-// Head size 128: a thread gets a tcgen05.mma out about every 117 clocks whatever its size, and a
-// tile's sixteen products would keep one thread busy longer than the softmax takes, so each of the
-// two products has an issuing warp of its own.
+// Head size 128: a tile's sixteen products and their waits would keep one warp busy longer than the softmax takes, so each of the
+// two products has an issuing warp of its own.  (The issuing and copying warps stay converged and elect a thread, see tma.cuh: 300 prompt
+// tokens of 32 heads of 64 9.3 -> 8.9 us a layer.)
 constexpr bool SPLIT_ISSUE = HD == 128;
 constexpr int THREADS = SPLIT_ISSUE ? 224 : 192;  // + the copy warp and the tensor-core warp(s)
 constexpr int KV_STAGES = HD == 64 ? 3 : 4;   // head size 128: 132 KB of shared memory, one block per SM as its tensor memory asks
@@ -63,6 +63,12 @@ constexpr float RESCALE_LAG = 8.0f;         // in powers of two
 // Instruction descriptor: bfloat16 x bfloat16 -> float, M = 128, N = 64; b_mn: B is MN-major.
 __device__ __forceinline__ unsigned instr_desc(bool b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+}
+// D or += A B; A in tensor memory, B's descriptor by its low word.
+__device__ __forceinline__ void mma_ta(unsigned d, unsigned a, unsigned b_low, unsigned idesc, bool accumulate) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 y;\n setp.ne.b32 p, %5, 0;\n mov.b64 y, {%2, %3};\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}"
+                 ::"r"(d), "r"(a), "r"(b_low), "r"(UMMA_DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
 }
 #ifdef IE_TC5_TIMING
 __device__ long long g_tc5_clocks[16];
@@ -192,7 +198,7 @@ attention_prefill_tc5_kernel(const bf16* __restrict__ q, const __grid_constant__
     unsigned char* v_s = k_s + KV_STAGES * KV_BYTES;
     int* table_s = reinterpret_cast<int*>(v_s + KV_STAGES * KV_BYTES);  // MAX_TABLE ints
     Barriers* bars = reinterpret_cast<Barriers*>(table_s + MAX_TABLE);
-    int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     int head = blockIdx.y, G = nh / nkv, kvh = head / G;
     ie_pdl_trigger();
     // (lengths and block tables are the step's inputs; queries, keys and values are the previous
@@ -272,142 +278,147 @@ attention_prefill_tc5_kernel(const bf16* __restrict__ q, const __grid_constant__
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    unsigned tmem = bars->tmem_base;
+    unsigned tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
     unsigned tmem_o = tmem + 2 * KT, tmem_q = tmem + 2 * KT + HD;
     // In all three roles g counts the key tiles over both parts: ring stage g % 3, S buffer
     // g & 1 and the barriers' phases go on from the first part into the second.
 
     if (warp == 4) {
-        // ---- copies: one thread ----
+        // ---- copies: one thread of a converged warp (`elect_one`) ----
         ie_pdl_wait();
-        if (lane == 0) {
-            int g = 0;
-            bool ok = true;
-            for (int pi = 0; pi < nparts && ok; ++pi) {
-                const Part& pt = parts[pi];
-                for (int t = 0; t < pt.n_tiles; ++t, ++g) {
-                    int stage = g % KV_STAGES;
-                    if (g >= KV_STAGES && !mbar_wait_compact(&bars->kv_empty[stage], (g / KV_STAGES - 1) & 1)) { ok = false; break; }
-                    mbar_expect_tx(&bars->kv_full[stage], 2 * KV_BYTES);
-                    int entry = ((pt.key_begin + t * KT) >> page_shift) - first_entry;
-                    for (int p = 0; p < pages_per_tile; ++p) {
-                        int page = table_s[min(entry + p, MAX_TABLE - 1)];
-                        int row = (page * nkv + kvh) << page_shift;
+        const bool one = elect_one();
+        int g = 0;
+        bool ok = true;
+        for (int pi = 0; pi < nparts && ok; ++pi) {
+            const int n_tiles = warps_own(parts[pi].n_tiles), first = warps_own(parts[pi].key_begin);
+            for (int t = 0; t < n_tiles; ++t, ++g) {
+                int stage = g % KV_STAGES;
+                if (g >= KV_STAGES && !warp_wait(&bars->kv_empty[stage], (g / KV_STAGES - 1) & 1)) { ok = false; break; }
+                if (one) mbar_expect_tx(&bars->kv_full[stage], 2 * KV_BYTES);
+                int entry = ((first + t * KT) >> page_shift) - first_entry;
+                const int pages = table_s[min(entry + min(lane, pages_per_tile - 1), MAX_TABLE - 1)];  // a lane's page
+                for (int p = 0; p < pages_per_tile; ++p) {
+                    const int row = (__shfl_sync(0xffffffffu, pages, p) * nkv + kvh) << page_shift;
+                    if (one)
 #pragma unroll
                         for (int h = 0; h < HALVES; ++h) {  // 64 dims to a box
                             int at = stage * KV_BYTES + h * HALF_BYTES + p * page_size * 128;
                             tma_load_2d(k_s + at, &k_map, h * 64, row, &bars->kv_full[stage]);
                             tma_load_2d(v_s + at, &v_map, h * 64, row, &bars->kv_full[stage]);
                         }
-                    }
                 }
+                __syncwarp();
             }
-            if (!ok) bars->failed = 1;
         }
+        if (!ok) bars->failed = 1;
     } else if (!SPLIT_ISSUE && warp == 5) {
         // ---- tensor core: one thread issues both products (head size 64: the exponentials bound
         // the kernel, a second issuing warp only takes issue slots from the softmax warps) ----
-        if (lane == 0) {
-            unsigned idesc_qk = instr_desc(false), idesc_pv = instr_desc(true);
-            bool ok = true;
-            auto issue_s = [&](int g) {  // S = Q K^T of key tile g into S buffer g & 1
-                int stage = g % KV_STAGES;
-                if (!mbar_wait_compact(&bars->kv_full[stage], (g / KV_STAGES) & 1)) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unsigned ka = smem_u32(k_s + stage * KV_BYTES);
+        const bool one = elect_one();
+        const unsigned idesc_qk = instr_desc(false), idesc_pv = instr_desc(true), k_low = umma_desc_low(smem_u32(k_s)), v_low = umma_desc_low(smem_u32(v_s));
+        bool ok = true;
+        auto issue_s = [&](int g) {  // S = Q K^T of key tile g into S buffer g & 1
+            int stage = g % KV_STAGES;
+            if (!warp_wait(&bars->kv_full[stage], (g / KV_STAGES) & 1)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (one) {
+                const unsigned ka = k_low + stage * (KV_BYTES >> 4);
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a half
-                    umma_ta(tmem + (g & 1) * KT, tmem_q + ks * 8, umma_desc_sw128(ka + (ks >> 2) * HALF_BYTES + (ks & 3) * 32),
-                            idesc_qk, ks > 0);
+                    mma_ta(tmem + (g & 1) * KT, tmem_q + ks * 8, ka + (((ks >> 2) * HALF_BYTES + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
                 umma_commit(&bars->s_done[g & 1]);
-                return true;
-            };
-            int g = 0;
-            for (int pi = 0; pi < nparts && ok; ++pi) {
-                int n_tiles = parts[pi].n_tiles;
-                // the part's Q is in tensor memory (and the softmax warps are done with the
-                // accumulator of the part before)
-                ok = mbar_wait_compact(&bars->q_full, pi & 1) && (n_tiles == 0 || issue_s(g));
-                for (int t = 0; t < n_tiles && ok; ++t, ++g) {
-                    if (t + 1 < n_tiles) {
-                        // its S buffer held the weights of tile g - 1: that product must have read them
-                        if (g > 0 && !mbar_wait_compact(&bars->o_done, (g - 1) & 1)) { ok = false; break; }
-                        ok = issue_s(g + 1);
-                    }
-                    if (!ok || !mbar_wait_compact(&bars->p_ready[g & 1], (g >> 1) & 1)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    int stage = g % KV_STAGES;
-                    unsigned va = smem_u32(v_s + stage * KV_BYTES);
+            }
+            __syncwarp();
+            return true;
+        };
+        int g = 0;
+        for (int pi = 0; pi < nparts && ok; ++pi) {
+            const int n_tiles = warps_own(parts[pi].n_tiles);
+            // the part's Q is in tensor memory (and the softmax warps are done with the
+            // accumulator of the part before)
+            ok = warp_wait(&bars->q_full, pi & 1) && (n_tiles == 0 || issue_s(g));
+            for (int t = 0; t < n_tiles && ok; ++t, ++g) {
+                if (t + 1 < n_tiles) {
+                    // its S buffer held the weights of tile g - 1: that product must have read them
+                    if (g > 0 && !warp_wait(&bars->o_done, (g - 1) & 1)) { ok = false; break; }
+                    ok = issue_s(g + 1);
+                }
+                if (!ok || !warp_wait(&bars->p_ready[g & 1], (g >> 1) & 1)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                int stage = g % KV_STAGES;
+                if (one) {
+                    const unsigned va = v_low + stage * (KV_BYTES >> 4);
 #pragma unroll
                     for (int h = 0; h < HALVES; ++h)  // 64 output dims per product
 #pragma unroll
                         for (int ks = 0; ks < KT / 16; ++ks)  // P: 8 columns of two keys each; V: 16 keys = 2048 bytes
-                            umma_ta(tmem_o + h * 64, tmem + (g & 1) * KT + ks * 8,
-                                    umma_desc_sw128(va + h * HALF_BYTES + ks * 2048), idesc_pv, (t > 0 || ks > 0) ? 1u : 0u);
+                            mma_ta(tmem_o + h * 64, tmem + (g & 1) * KT + ks * 8, va + ((h * HALF_BYTES + ks * 2048) >> 4), idesc_pv, t > 0 || ks > 0);
                     umma_commit(&bars->o_done);
                     umma_commit(&bars->kv_empty[stage]);
                 }
+                __syncwarp();
             }
-            if (!ok) bars->failed = 1;
         }
+        if (!ok) bars->failed = 1;
     } else if (SPLIT_ISSUE && warp == 5) {
         // ---- tensor core, first product: one thread issues S = Q K^T of every key tile ----
-        // (a thread gets a tcgen05.mma out about every 117 clocks whatever its size, so the two
-        // products of a tile are issued by a thread each)
-        if (lane == 0) {
-            unsigned idesc_qk = instr_desc(false);
-            bool ok = true;
-            int g = 0;
-            for (int pi = 0; pi < nparts && ok; ++pi) {
-                // the part's Q is in tensor memory
-                ok = mbar_wait_compact(&bars->q_full, pi & 1);
-                for (int t = 0; t < parts[pi].n_tiles && ok; ++t, ++g) {
-                    // S buffer g & 1 held the weights of tile g - 2: that product must have read
-                    // them.  (Waited for right after S(g - 1) went out, so the barrier cannot be
-                    // more than one phase ahead.  For a part's first two tiles the wait for Q
-                    // covers it: the softmax warps had waited for all products of the part before,
-                    // and by now this barrier may be any number of phases ahead.)
-                    if (t >= 2 && !mbar_wait_compact(&bars->o_done, (g - 2) & 1)) { ok = false; break; }
-                    int stage = g % KV_STAGES;
-                    if (!mbar_wait_compact(&bars->kv_full[stage], (g / KV_STAGES) & 1)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    unsigned ka = smem_u32(k_s + stage * KV_BYTES);
+        const bool one = elect_one();
+        const unsigned idesc_qk = instr_desc(false), k_low = umma_desc_low(smem_u32(k_s));
+        bool ok = true;
+        int g = 0;
+        for (int pi = 0; pi < nparts && ok; ++pi) {
+            const int n_tiles = warps_own(parts[pi].n_tiles);
+            // the part's Q is in tensor memory
+            ok = warp_wait(&bars->q_full, pi & 1);
+            for (int t = 0; t < n_tiles && ok; ++t, ++g) {
+                // S buffer g & 1 held the weights of tile g - 2: that product must have read
+                // them.  (Waited for right after S(g - 1) went out, so the barrier cannot be
+                // more than one phase ahead.  For a part's first two tiles the wait for Q
+                // covers it: the softmax warps had waited for all products of the part before,
+                // and by now this barrier may be any number of phases ahead.)
+                if (t >= 2 && !warp_wait(&bars->o_done, (g - 2) & 1)) { ok = false; break; }
+                int stage = g % KV_STAGES;
+                if (!warp_wait(&bars->kv_full[stage], (g / KV_STAGES) & 1)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (one) {
+                    const unsigned ka = k_low + stage * (KV_BYTES >> 4);
 #pragma unroll
                     for (int ks = 0; ks < HD / 16; ++ks)  // 32 bytes further along k per step, 4 steps to a half
-                        umma_ta(tmem + (g & 1) * KT, tmem_q + ks * 8,
-                                umma_desc_sw128(ka + (ks >> 2) * HALF_BYTES + (ks & 3) * 32), idesc_qk, ks > 0);
+                        mma_ta(tmem + (g & 1) * KT, tmem_q + ks * 8, ka + (((ks >> 2) * HALF_BYTES + (ks & 3) * 32) >> 4), idesc_qk, ks > 0);
                     umma_commit(&bars->s_done[g & 1]);
                 }
+                __syncwarp();
             }
-            if (!ok) bars->failed = 1;
         }
+        if (!ok) bars->failed = 1;
     } else if (SPLIT_ISSUE && warp == 6) {
         // ---- tensor core, second product: one thread issues O += P V of every key tile ----
-        if (lane == 0) {
-            unsigned idesc_pv = instr_desc(true);
-            bool ok = true;
-            int g = 0;
-            for (int pi = 0; pi < nparts && ok; ++pi) {
-                for (int t = 0; t < parts[pi].n_tiles; ++t, ++g) {
-                    int stage = g % KV_STAGES;
-                    // (the softmax warps are done with the accumulator of the part before: they
-                    // read it before they wrote this part's Q and its first weights)
-                    if (!mbar_wait_compact(&bars->kv_full[stage], (g / KV_STAGES) & 1) ||
-                        !mbar_wait_compact(&bars->p_ready[g & 1], (g >> 1) & 1)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    unsigned va = smem_u32(v_s + stage * KV_BYTES);
+        const bool one = elect_one();
+        const unsigned idesc_pv = instr_desc(true), v_low = umma_desc_low(smem_u32(v_s));
+        bool ok = true;
+        int g = 0;
+        for (int pi = 0; pi < nparts && ok; ++pi) {
+            const int n_tiles = warps_own(parts[pi].n_tiles);
+            for (int t = 0; t < n_tiles; ++t, ++g) {
+                int stage = g % KV_STAGES;
+                // (the softmax warps are done with the accumulator of the part before: they
+                // read it before they wrote this part's Q and its first weights)
+                if (!warp_wait(&bars->kv_full[stage], (g / KV_STAGES) & 1) || !warp_wait(&bars->p_ready[g & 1], (g >> 1) & 1)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (one) {
+                    const unsigned va = v_low + stage * (KV_BYTES >> 4);
 #pragma unroll
                     for (int h = 0; h < HALVES; ++h)  // 64 output dims per product
 #pragma unroll
                         for (int ks = 0; ks < KT / 16; ++ks)  // P: 8 columns of two keys each; V: 16 keys = 2048 bytes
-                            umma_ta(tmem_o + h * 64, tmem + (g & 1) * KT + ks * 8,
-                                    umma_desc_sw128(va + h * HALF_BYTES + ks * 2048), idesc_pv, (t > 0 || ks > 0) ? 1u : 0u);
+                            mma_ta(tmem_o + h * 64, tmem + (g & 1) * KT + ks * 8, va + ((h * HALF_BYTES + ks * 2048) >> 4), idesc_pv, t > 0 || ks > 0);
                     umma_commit(&bars->o_done);
                     umma_commit(&bars->kv_empty[stage]);
                 }
+                __syncwarp();
             }
-            if (!ok) bars->failed = 1;
         }
+        if (!ok) bars->failed = 1;
     } else {
         // ---- softmax: thread = query row = TMEM lane ----
         int row = tid;

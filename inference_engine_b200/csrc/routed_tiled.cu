@@ -119,25 +119,18 @@ __device__ __forceinline__ void put_gated(const Args& in, const float (&a)[16], 
         if (i + (high ? 1 : 0) < n) *reinterpret_cast<bf16*>(y + i * 128 + (piece ^ ((i & 6) << 4))) = __float2bfloat16_rn(v);
     }
 }
-__device__ __forceinline__ int warps_own(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-// Shared-memory descriptors as their two words: the low one moves with the address, the high one (groups of eight rows 1,024 bytes apart, version,
-// 128-byte swizzle) is a constant.  (Within a cluster an address has the block's number above its 18 bits.)
-constexpr unsigned DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ unsigned desc_low(unsigned addr) { return ((addr & 0x3ffff) >> 4) | (64u << 16); }
 // D = or += A B^T.  PAIR: D in both blocks' tensor memory, A and B half in each block's shared memory, issued in the first block.
 template <bool PAIR>
 __device__ __forceinline__ void mma(unsigned d, unsigned a, unsigned b, unsigned idesc, bool accumulate) {
     if (PAIR)
         asm volatile("{\n .reg .pred p;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
                      " tcgen05.mma.cta_group::2.kind::f16 [%0], x, y, %4, p;\n}"
-                     ::"r"(d), "r"(a), "r"(b), "r"(DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+                     ::"r"(d), "r"(a), "r"(b), "r"(UMMA_DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
     else
         asm volatile("{\n .reg .pred p;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
                      " tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
-                     ::"r"(d), "r"(a), "r"(b), "r"(DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+                     ::"r"(d), "r"(a), "r"(b), "r"(UMMA_DESC_HIGH), "r"(idesc), "r"((unsigned)accumulate) : "memory");
 }
-// A wait of the whole warp.
-__device__ __forceinline__ bool warp_wait(unsigned long long* bar, int parity) { return __all_sync(0xffffffffu, mbar_wait_compact(bar, parity)); }
 // An arrival at the barrier of both blocks when all that this thread issued so far is done.
 __device__ __forceinline__ void pair_commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -222,7 +215,7 @@ gemm_pair_kernel(const __grid_constant__ Args in) {
         const bool one = elect_one();
         int s = 0, phase = 0, turn = 0;
         bool ok = true;
-        const unsigned w_low = desc_low(smem_u32(ring));
+        const unsigned w_low = umma_desc_low(smem_u32(ring));
         for (int t = cluster; t < total && ok; t += clusters) {
             const int n = warps_own(tile_at(t).z), cols = columns(n);
             const unsigned idesc = umma_idesc_bf16(256, cols), second = (unsigned)(cols / 2 * BK * 2) >> 4;
@@ -417,7 +410,7 @@ gemm_few_kernel(const __grid_constant__ Args in) {
         __syncwarp();
     } else if (warp == 1) {
         const bool one = elect_one();
-        const unsigned idesc = umma_idesc_bf16(ROWS, n_pad), w_low = desc_low(smem_u32(ring));
+        const unsigned idesc = umma_idesc_bf16(ROWS, n_pad), w_low = umma_desc_low(smem_u32(ring));
         bool ok = true;
         int s = 0, phase = 0;
         for (int kb = 0; kb < nkb; ++kb) {

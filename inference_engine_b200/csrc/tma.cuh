@@ -61,6 +61,9 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
     return p != 0;
 }
+// A number that all lanes hold, as the warp's; a wait of the whole warp.
+__device__ __forceinline__ int warps_own(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, int parity) { return __all_sync(0xffffffffu, mbar_wait_compact(bar, parity)); }
 // One box of a 2-D tensor map into shared memory; x is the inner (contiguous) coordinate and
 // x * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
@@ -85,6 +88,10 @@ __device__ __forceinline__ unsigned long long umma_desc_sw128(unsigned addr) {
     d |= (unsigned long long)2 << 61;                  // layout: 128-byte swizzle
     return d;
 }
+// The same as its two words: the low one moves with the address, the high one is a constant.  (Within a cluster an address has the block's
+// number above its 18 bits.)
+constexpr unsigned UMMA_DESC_HIGH = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ unsigned umma_desc_low(unsigned addr) { return ((addr & 0x3ffff) >> 4) | (64u << 16); }
 // Instruction descriptor: bfloat16 x bfloat16 -> float, both operands K-major, D is m x n.
 __device__ __forceinline__ unsigned umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
@@ -111,12 +118,6 @@ __device__ __forceinline__ void tmem_ld16(float (&v)[16], unsigned taddr) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// D (TMEM) = or += A B; A in tensor memory: lane = row, a 32-bit column = two consecutive k.
-__device__ __forceinline__ void umma_ta(unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
 // One row (this thread's TMEM lane) of 64 columns starting at `taddr`.
 __device__ __forceinline__ void tmem_ld64(float (&v)[64], unsigned taddr) {
     unsigned* r = reinterpret_cast<unsigned*>(v);
