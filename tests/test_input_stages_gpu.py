@@ -1,0 +1,50 @@
+"""Input stages that take rows in pieces of four against the kernels that take them entry by entry: the same sums in another order."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(positions, rot_dims):
+    angle = torch.arange(positions, device="cuda").float()[:, None] * (10000.0 ** (-torch.arange(0, rot_dims, 2, device="cuda") / rot_dims))
+    return torch.stack([angle.cos(), angle.sin()], dim=1).contiguous()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,rot_dims,interleaved,from_keys", [
+    (16, 4, 128, 128, 0, False, False), (5, 1, 64, 64, 64, True, True), (8, 2, 128, 64, 64, False, False), (3, 3, 36, 12, 16, False, False),
+    (4, 2, 8, 128, 4, True, False)])
+@pytest.mark.parametrize("norm", ["weights", "unit", "values", "none"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_heads_in_pieces_of_four(heads, kv_heads, dim, vdim, rot_dims, interleaved, from_keys, norm, dtype):
+    from inference_engine_b200.kernels import get_ops
+
+    ops, n, page = get_ops(), 37, 8
+    g = torch.Generator(device="cuda").manual_seed(dim + heads)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    need = (heads + kv_heads) * dim + (0 if from_keys else kv_heads * vdim)
+    aligned = rand(n, need + 4)[:, :need] if (need + 4) % 4 == 0 else None
+    assert aligned is not None
+    ragged = torch.empty(n, need + 5, device="cuda")[:, :need].copy_(aligned)  # rows that no piece of 16 bytes fits: entry by entry
+    positions = torch.randint(0, 50, (n,), generator=g, device="cuda", dtype=torch.int32)
+    slots = torch.randperm(8 * page, generator=g, device="cuda")[:n].int()
+    slots[3] = -1 if norm == "none" else slots[3]  # a slot that is not there
+    results = []
+    for proj in (aligned, ragged):
+        q = torch.zeros(n, heads * dim, dtype=dtype, device="cuda")
+        k, v = (torch.zeros(8, kv_heads, page, size, dtype=dtype, device="cuda") for size in (dim, vdim))
+        extra = {"bias": (torch.arange(need, device="cuda") % 7 - 3).float() * 0.1, "unit_norm": norm == "unit", "value_norm": norm == "values"}
+        if norm == "unit":
+            extra.update(q_head_scale=torch.arange(1, heads + 1, device="cuda").float(), warm_coef=0.1, warm_every=8, value_scale=0.5)
+        weights = [torch.linspace(0.5, 1.5, dim, device="cuda") for _ in range(2)] if norm == "weights" else [None, None]
+        ops.qk_norm_rope_write(proj, positions, _table(50, rot_dims) if rot_dims else None, rot_dims, *weights, 1e-5, q, k, v, slots, heads,
+                               kv_heads, dim, vdim, page, values_from_keys=from_keys, interleaved=interleaved, **extra)
+        if norm == "none":
+            with pytest.raises(Exception, match="page"):
+                ops.check_errors()
+        else:
+            ops.check_errors()
+        results.append((q, k, v))
+    for a, b in zip(*results):
+        # sums of at most 128 squares in another order: 2^-24 sqrt(128) of a value; in bfloat16 some then round the other way, by 2^-8
+        torch.testing.assert_close(a.float(), b.float(), rtol=1e-5 if dtype == torch.float32 else 2 ** -7, atol=1e-6)
