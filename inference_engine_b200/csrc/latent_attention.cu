@@ -57,6 +57,28 @@ __device__ __forceinline__ float turned(const Src& src, int d, const float* cs, 
     return fmaf(v, c, -src[interleaved ? d + 1 : d + half] * s);
 }
 
+// Entries d .. d + 3 of the same, of a row in one part (rot_dims, and half of it where entries half apart form pairs, multiples of 4).
+__device__ __forceinline__ float4 turned4(const float* src, int d, const float* cs, int rot_dims, int interleaved) {
+    const float4 v = *reinterpret_cast<const float4*>(src + d);
+    if (cs == nullptr || d >= rot_dims) return v;
+    const int half = rot_dims / 2;
+    if (interleaved) {
+        const float2 c = *reinterpret_cast<const float2*>(cs + d / 2), s = *reinterpret_cast<const float2*>(cs + half + d / 2);
+        return make_float4(fmaf(v.x, c.x, -v.y * s.x), fmaf(v.y, c.x, v.x * s.x), fmaf(v.z, c.y, -v.w * s.y), fmaf(v.w, c.y, v.z * s.y));
+    }
+    const int j = d >= half ? d - half : d;
+    const float sign = d >= half ? 1.f : -1.f;
+    const float4 o = *reinterpret_cast<const float4*>(src + (d >= half ? j : d + half)), c = *reinterpret_cast<const float4*>(cs + j);
+    const float4 s = *reinterpret_cast<const float4*>(cs + half + j);
+    return make_float4(fmaf(v.x, c.x, sign * o.x * s.x), fmaf(v.y, c.y, sign * o.y * s.y), fmaf(v.z, c.z, sign * o.z * s.z), fmaf(v.w, c.w, sign * o.w * s.w));
+}
+
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
+    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+    *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(o);
+}
+
 // What a call asks for is what has a pointer: queries (q), gates (gate_pre), the cached row (dkv and
 // slot_mapping), the queries' latent (cq).  Each input is a row `*_ld` numbers long per token, in `parts` parts
 // `part_stride` apart.
@@ -69,7 +91,8 @@ struct LatentIn {
     const float* norm_w;
     const float* cq_norm_w;
     float eps;
-    bool fours;  // sizes and addresses of cq and dkv allow pieces of four
+    bool fours;    // sizes and addresses of cq and dkv allow pieces of four
+    bool all_fours;  // those of everything that is asked for, and the rotation
     __device__ Row row(const float* p, int ld, int n) const { return Row{p + (size_t)n * ld, parts, part_stride}; }
 };
 
@@ -154,6 +177,85 @@ latent_prep_kernel(LatentIn in, const int* __restrict__ positions,
         if (i < n_cq) ie_store(cq_out + (size_t)n * n_cq + i, rows[i] * inv_q * in.cq_norm_w[i]);
         else if (i - n_cq < rank) ie_store(dst + i - n_cq, rows[i] * inv_c * in.norm_w[i - n_cq]);
         else ie_store(dst + i - n_cq, turned(part, i - n_cq - rank, cs, rot_dims, interleaved));
+    }
+}
+
+// The same for many tokens, of products in one part whose sizes and addresses allow pieces of four: a warp per token, no barriers, four of
+// a lane's pieces on their way at a time.  (2,048 tokens of 16 heads of 128 + 64 and a latent of 512, the cached rows and the queries in a
+// launch each: 28 us with a block per token; 17 so.  Most of that was code fetched to be executed once, the sums over parts unrolled in
+// every place: little code counts as much as few trips to memory here.)
+constexpr int LW_WARPS = 4, LW_PIECES = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(LW_WARPS * 32)
+latent_prep_warp_kernel(LatentIn in, const int* __restrict__ positions, const float* __restrict__ table, int rot_dims, int table_rows,
+                        int interleaved, T* __restrict__ q_plain, T* __restrict__ q_abs, float* __restrict__ gate, T* __restrict__ cq_out,
+                        T* __restrict__ cache, const int* __restrict__ slot_mapping, int num_tokens, int heads, int dim, int rot_dim,
+                        int rank, int total_slots, int* err) {
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    const int n = blockIdx.x * LW_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (n >= num_tokens) return;
+    const int hq = dim + rot_dim, krow = rank + rot_dim, pos = positions[n];
+    const int slot = in.dkv != nullptr && slot_mapping != nullptr ? slot_mapping[n] : -1;
+    bool turn = table != nullptr && rot_dims > 0, cached = in.dkv != nullptr && slot_mapping != nullptr;
+    if (turn && (pos < 0 || pos >= table_rows)) {
+        if (lane == 0) ie_report(err, IE_ERR_POSITION, pos, n);
+        turn = false;
+    }
+    if (cached && (slot < 0 || slot >= total_slots)) {
+        if (lane == 0) ie_report(err, IE_ERR_PAGE, slot, n);
+        cached = false;
+    }
+    const float* cs = turn ? table + (size_t)pos * rot_dims : nullptr;
+    if (in.gate_pre != nullptr)
+        for (int h = lane; h < heads; h += 32) gate[(size_t)n * heads + h] = 1.0f / (1.0f + expf(-in.gate_pre[(size_t)n * in.gate_ld + h]));
+    if (in.q != nullptr) {
+        const float* row = in.q + (size_t)n * in.q_ld;
+        for (int i0 = lane * 4; i0 < heads * hq; i0 += 128 * LW_PIECES) {
+            float4 v[LW_PIECES];  // (all loads before the first store)
+            T* to[LW_PIECES];
+#pragma unroll
+            for (int k = 0; k < LW_PIECES; ++k) {
+                const int i = i0 + 128 * k, h = i / hq, d = i - h * hq;
+                const bool plain = d < dim;
+                to[k] = plain ? q_plain + ((size_t)n * heads + h) * dim + d : q_abs + ((size_t)n * heads + h) * krow + rank + d - dim;
+                if (i < heads * hq) v[k] = turned4(row + i - d + dim, d - dim, plain ? nullptr : cs, rot_dims, interleaved);
+            }
+#pragma unroll
+            for (int k = 0; k < LW_PIECES; ++k)
+                if (i0 + 128 * k < heads * hq) store4(to[k], v[k]);
+        }
+    }
+    // the cached row's latent, then the queries' own: the first pass over a row takes its sum of squares, the second finds it in the cache
+    for (int part = 0; part < 2; ++part) {
+        const float* row = part == 0 ? (cached ? in.dkv + (size_t)n * in.dkv_ld : nullptr) : in.cq != nullptr ? in.cq + (size_t)n * in.cq_ld : nullptr;
+        if (row == nullptr) continue;
+        const int count = part == 0 ? rank : in.q_rank;
+        const float* w = part == 0 ? in.norm_w : in.cq_norm_w;
+        T* dst = part == 0 ? cache + (size_t)slot * krow : cq_out + (size_t)n * in.q_rank;
+        float ss = 0.f;
+#pragma unroll 4
+        for (int i = lane * 4; i < count; i += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(row + i);
+            ss += fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+        }
+        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)count + in.eps);
+        for (int i0 = lane * 4; i0 < count; i0 += 128 * LW_PIECES) {
+            float4 v[LW_PIECES], f[LW_PIECES];
+#pragma unroll
+            for (int k = 0; k < LW_PIECES; ++k)
+                if (i0 + 128 * k < count) {
+                    v[k] = *reinterpret_cast<const float4*>(row + i0 + 128 * k);
+                    f[k] = *reinterpret_cast<const float4*>(w + i0 + 128 * k);
+                }
+#pragma unroll
+            for (int k = 0; k < LW_PIECES; ++k)
+                if (i0 + 128 * k < count)
+                    store4(dst + i0 + 128 * k, make_float4(v[k].x * inv * f[k].x, v[k].y * inv * f[k].y, v[k].z * inv * f[k].z, v[k].w * inv * f[k].w));
+        }
+        if (part == 0)
+            for (int d = lane * 4; d < rot_dim; d += 128) store4(dst + rank + d, turned4(row + rank, d, cs, rot_dims, interleaved));
     }
 }
 
@@ -422,11 +524,26 @@ IE_API int ie_latent_prep(const float* q, int q_ld, const float* gate_pre, int g
     if (rot_dims < 0 || rot_dims % 2 || rot_dims > rot_dim) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
     if (parts < 1) return (int)cudaErrorInvalidValue;
-    LatentIn in{q, q_ld, gate_pre, gate_ld, dkv, dkv_ld, cq, cq_ld, q_rank, parts, (size_t)part_stride, norm_w, cq_norm_w, eps, false};
+    LatentIn in{q, q_ld, gate_pre, gate_ld, dkv, dkv_ld, cq, cq_ld, q_rank, parts, (size_t)part_stride, norm_w, cq_norm_w, eps, false, false};
     in.fours = q_rank % 4 == 0 && rank % 4 == 0 && rot_dim % 4 == 0 && cq_ld % 4 == 0 && dkv_ld % 4 == 0 && part_stride % 4 == 0 &&
                ((reinterpret_cast<uintptr_t>(cq) | reinterpret_cast<uintptr_t>(dkv)) % 16 == 0);
+    in.all_fours = parts == 1 && in.fours && dim % 4 == 0 && rot_dims % (interleaved ? 4 : 8) == 0 && q_ld % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(q_plain) | reinterpret_cast<uintptr_t>(q_abs) |
+                     reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(cq_norm_w) |
+                     reinterpret_cast<uintptr_t>(cq_out) | reinterpret_cast<uintptr_t>(cache)) % 16 == 0);
     size_t smem = ((cq ? q_rank : 0) + (dkv ? rank + rot_dim : 0)) * sizeof(float);
     if (smem > 40 * 1024) return (int)cudaErrorInvalidValue;
+    // (from four tokens an SM on: fewer are done sooner with a block each)
+    if (in.all_fours && num_tokens >= 4 * ie_sm_count()) {
+        const dim3 grid((num_tokens + LW_WARPS - 1) / LW_WARPS), block(LW_WARPS * 32);
+        if (dtype == IE_BF16)
+            return ie_launch(latent_prep_warp_kernel<__nv_bfloat16>, grid, block, 0, s, in, positions, table, rot_dims, table_rows, interleaved,
+                             (__nv_bfloat16*)q_plain, (__nv_bfloat16*)q_abs, gate, (__nv_bfloat16*)cq_out, (__nv_bfloat16*)cache,
+                             slot_mapping, num_tokens, heads, dim, rot_dim, rank, total_slots, err);
+        return ie_launch(latent_prep_warp_kernel<float>, grid, block, 0, s, in, positions, table, rot_dims, table_rows, interleaved,
+                         (float*)q_plain, (float*)q_abs, gate, (float*)cq_out, (float*)cache, slot_mapping, num_tokens, heads, dim, rot_dim,
+                         rank, total_slots, err);
+    }
     if (dtype == IE_BF16)
         return ie_launch(latent_prep_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(LP_THREADS), smem, s, in, positions, table,
                          rot_dims, table_rows, interleaved, (__nv_bfloat16*)q_plain, (__nv_bfloat16*)q_abs, gate,

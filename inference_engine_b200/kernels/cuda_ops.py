@@ -1153,17 +1153,24 @@ class CudaOps:
             cache.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], ctx.ctx_lens.data_ptr(), ctx.num_seqs, out.shape[0],
             out.shape[1], page_size, cache.shape[0], out.data_ptr(), self._err_ptr, self._stream()), "gather_context_rows")
 
+    @staticmethod
+    def latent_query_buffers(n: int, heads: int, dim: int, row: int, dtype, ws):
+        """Where the queries' unrotated and rotated entries go for :meth:`latent_expanded` (of the second the rotated entries alone are
+        written)."""
+        return ws.buffer("latent.q_plain", n, heads * dim, dtype), ws.buffer("latent.q", n, heads * row, dtype)
+
     def latent_expanded(self, q, w_kv, cache, block_tables, ctx, positions, table, rot_dims, out, *, heads, dim, rot_dim, vdim, rank,
-                        page_size, interleaved, scale, gate_pre, sinks, ws) -> None:
+                        page_size, interleaved, scale, gate_pre, sinks, ws, queries=None) -> None:
         """The latent attention with keys and values expanded per head (``latent_expands`` says when): ``q`` as for
         :meth:`latent_queries`; ``w_kv`` ``[heads * (dim + vdim), rank]``, all heads' key rows, then all heads' value rows; ``cache``
         holds the step's own rows too; ``gate_pre`` (a 32-bit view ``[N, heads]`` or None) and ``sinks`` as for the attentions;
-        ``out``: ``[N, heads * vdim]``, gated."""
+        ``out``: ``[N, heads * vdim]``, gated.  ``queries``: the buffers of :meth:`latent_query_buffers`, if :meth:`latent_prep` has
+        filled them already (``q`` is not read then)."""
         n, row = positions.shape[0], rank + rot_dim
-        plain = ws.buffer("latent.q_plain", n, heads * dim, out.dtype)
-        turned = ws.buffer("latent.q", n, heads * row, out.dtype)  # (its rotated entries alone are written)
-        self.latent_prep(positions, table, rot_dims, heads=heads, dim=dim, rot_dim=rot_dim, rank=rank, page_size=page_size,
-                         interleaved=interleaved, q=q, q_plain=plain, q_abs=turned)
+        plain, turned = queries or self.latent_query_buffers(n, heads, dim, row, out.dtype, ws)
+        if queries is None:
+            self.latent_prep(positions, table, rot_dims, heads=heads, dim=dim, rot_dim=rot_dim, rank=rank, page_size=page_size,
+                             interleaved=interleaved, q=q, q_plain=plain, q_abs=turned)
         total = sum(ctx.start_positions) + sum(ctx.q_lens)
         # (captured steps never expand: these may grow without their addresses going stale)
         scratch = ws.spare(self._expanded_wants(total, heads, dim, rot_dim, vdim, rank), captured=False)

@@ -123,9 +123,15 @@ class LatentAttention(Mixer):
                      interleaved=self.interleaved)
         proj = ops.linear(x, self.w_in, ws=ws, tag="latent.in", out_dtype=torch.float32, allow_split=True)
         at = self.q_size if self.q_rank is None else self.q_rank  # where the latent's columns start
-        gate = cq = None
+        gate = cq = queries = None
         extra = {}
-        if "gate" in self.names:
+        expands = getattr(ops, "latent_expands", None)
+        expands = (expands is not None and self.dtype == torch.bfloat16 and proj.dim() == 2
+                   and expands(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank))
+        if expands and self.q_rank is None:  # the queries are columns of this product too: one launch for all
+            queries = ops.latent_query_buffers(n, H, self.dim, self.row, self.dtype, ws)
+            extra.update(q=proj[..., : self.q_size], q_plain=queries[0], q_abs=queries[1])
+        elif "gate" in self.names and not expands:
             gate = ws.buffer("latent.gate", n, H, torch.float32)
             extra.update(gate_pre=proj[..., at + self.row: at + self.row + H], gate=gate)
         if self.q_rank is not None:
@@ -138,12 +144,10 @@ class LatentAttention(Mixer):
         if cq is not None:
             q = ops.linear(cq, self.w_uq, ws=ws, tag="latent.uq", out_dtype=torch.float32, allow_split=True)
         out = ws.buffer("latent.out", n, H * self.vdim, self.dtype)
-        expands = getattr(ops, "latent_expands", None)
-        if (expands is not None and self.dtype == torch.bfloat16 and proj.dim() == 2
-                and expands(ctx, H, self.dim, self.rot_dim, self.vdim, self.kv_rank)):
-            gates = proj[:, at + self.row: at + self.row + H] if gate is not None else None
+        if expands:
+            gates = proj[:, at + self.row: at + self.row + H] if "gate" in self.names else None
             ops.latent_expanded(q, self.w_kv, cache, group.block_tables, ctx, ctx.positions, table, rot_dims, out, vdim=self.vdim,
-                                scale=self.scale, gate_pre=gates, sinks=self.sinks, ws=ws, **sizes)
+                                scale=self.scale, gate_pre=gates, sinks=self.sinks, ws=ws, queries=queries, **sizes)
             return ops.linear(out, self.w_o, ws=ws, tag="mixer.delta", out_dtype=torch.float32, allow_split=True)
         q_abs = ws.buffer("latent.q", n, H * self.row, self.dtype)
         ops.latent_queries(q, self.w_uk_t, q_abs, ctx.positions, table, rot_dims, **sizes, ws=ws)
