@@ -1396,18 +1396,19 @@ class CudaOps:
         portion's chain, or all tokens' state traffic when there are many requests, and a part of the smaller of the two.  In chunks: three
         launches and a block's life (with ``gated`` values and their normaliser's column a little more), then the work of all chunks;
         for the delta rule the chain through the longest portion's chunks besides.
-        Examples (16 heads of 128 x 128; token by token / in chunks): 64 tokens 24 / 46 us, 256 tokens 85 / 52, 2,048 tokens 664 /
-        134, 8 requests of 64 tokens 79 / 60, 32 of 32 tokens 153 / 165; whole layers of gated values, 8 heads of 64 x 64, 128 tokens
-        47 / 55, 30 requests of 64 124 / 140, 16 heads of 64 x 128, 8 requests of 64 76 / 89; delta rule 128 tokens 43 / 64, 256 tokens 82 / 74, 2,048
-        tokens 629 / 264, 32 of 32 tokens 160 / 384, whole layers 30 of 64 tokens 542 / 666."""
+        Examples (us, token by token / in chunks; 16 heads of 128 x 128): 64 tokens 21 / 40, 256 tokens 64 / 42, 2,048 tokens 461 /
+        124, 8 requests of 64 tokens 84 / 54, 32 of 32 tokens 160 / 146; whole layers of gated values, 8 heads of 64 x 64, 128 tokens
+        47 / 55, 30 requests of 64 124 / 140, 16 heads of 64 x 128, 8 requests of 64 76 / 89; delta rule 128 tokens 47 / 56, 256 tokens
+        86 / 63, 2,048 tokens 629 / 216, 8 requests of 128 tokens 137 / 122, 32 of 32 tokens 166 / 261, of 64 283 / 273; 8 heads, 8
+        requests of 250 tokens 164 / 120."""
         share, wide = heads * dim * vdim / 262144, dim > 64
         step = (0.31 if wide else 0.26) if delta else (0.325 if wide else 0.17)
         alone, together = step * longest, 0.15 * share * tokens
         if delta:
             one_by_one = max(alone, together)
             chain = max(-(-longest // self.CHUNK), heads * -(-vdim // 16) * chunks / self.sm_count)
-            chain *= 4.5 if longest > self.CHUNK else 7.5  # (portions of one chunk: a block starts for each)
-            return (62 if wide else 36) + chain + 2.0 * share * chunks < one_by_one
+            chain *= 3.7 if longest > self.CHUNK else 7.5  # (portions of one chunk: a block starts for each)
+            return (48 if wide else 33) + chain + 2.0 * share * chunks < one_by_one
         one_by_one = max(alone, together) + 0.3 * min(alone, together)
         return (54 if wide else 29) + (2 if gated else 0) + 2.9 * share * chunks < one_by_one
 

@@ -165,3 +165,28 @@ def test_a_launch_for_bounds_serves_every_step_within_them(ops, rule, lens, boun
         results.append((out[:n], st))
     ops.check_errors()
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", ["v", "k"])
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 36)])
+def test_delta_rule_with_a_value_that_is_no_number(ops, value, what, dim, vdim):
+    """It reaches no earlier token, also of its own sixteen, and those come out as without it."""
+    n, heads, at = 150, 2, 77
+    g = torch.Generator().manual_seed(3)
+    rand = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)  # noqa: E731
+    q, k = (unit(rand(n, heads, dim)).view(n, -1) for _ in range(2))
+    v, beta, decay = rand(n, heads * vdim), torch.sigmoid(rand(n, heads)), torch.sigmoid(rand(n, heads * dim) + 4)
+    outs = []
+    for spoilt in (False, True):
+        if spoilt:
+            (v if what == "v" else k)[at, :3] = value
+        out, state = torch.zeros(n, heads * vdim, device="cuda"), torch.zeros(1, heads * vdim * dim, device="cuda")
+        ops.delta_rule(q, k, v, beta, decay, state, torch.zeros(1, dtype=torch.int32, device="cuda"), _Ctx([n], "cuda"), out, heads, heads, dim,
+                       vdim, in_chunks=True)
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all() and torch.isfinite(outs[1][:at]).all()
+    assert not torch.isfinite(outs[1][at:, :3]).all(dim=1).any()
+    # (the spoilt chunk goes token by token: the same sums in another order)
+    assert float((outs[0][:at] - outs[1][:at]).norm() / outs[0][:at].norm()) < REL
