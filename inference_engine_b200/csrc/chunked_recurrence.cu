@@ -28,7 +28,7 @@
 // 128 x 128, us with FMAs / so: outputs 79 / 66 (delta rule 81 / 70), solve 75 / 54, chain 111 / 84; all together 142 / 122 and 270 /
 // 214.  Errors against 64 bits, over keys of 64 and 128, as parts of the results: outputs 1.4e-7 / 1.3e-7, of the delta rule 2.6e-7 /
 // 2.1e-7, its states 1.9e-7 / 1.8e-7.
-#include "common.cuh"
+#include "split32.cuh"
 #include <float.h>
 
 namespace {
@@ -70,58 +70,6 @@ __device__ __forceinline__ void fetch_rows(float* dst, const float* src, size_t 
     }
 }
 
-// ---- 32-bit products on the tensor cores ----
-// A number is a sum of two that the tensor cores take (11 bits each; the second, of at most 12, loses its last one), and a product three of
-// theirs: what is left out is about 2^-23 of it.  Sums of 16 products go through the tensor cores, which cut off what does not fit
-// where the 32-bit adders round, and are added in those; the products with second parts go first, so that little is cut off.  Against 64 bits
-// a chain of 64 or 128 such multiply-adds is no further off than one of the FMA pipe's, unless its terms grow towards its end.
-// (Three parts of 8 bits and six products are exact and take the tensor cores as long, but more instructions: the same error, the delta
-// rule's chain 104 us with them and 83 so.  The conversion instruction for these formats runs at an eighth of the adders' rate: 142 us.)
-struct Two {
-    unsigned hi, lo;
-};
-__device__ __forceinline__ unsigned long long packed(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ unsigned nearest(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
-// (the tensor cores ignore the last 13 bits; what is no number stays in the second part)
-__device__ __forceinline__ void two(float x, float y, Two& a, Two& b) {
-    a.hi = nearest(x);
-    b.hi = nearest(y);
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(packed(x, y)), "l"(packed(__uint_as_float(a.hi), __uint_as_float(b.hi))));
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(a.lo), "=r"(b.lo) : "l"(d));
-}
-__device__ __forceinline__ void add_to(float (&acc)[4], const float (&c)[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i += 2) {
-        unsigned long long d;
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(packed(acc[i], acc[i + 1])), "l"(packed(c[i], c[i + 1])));
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[i]), "=f"(acc[i + 1]) : "l"(d));
-    }
-}
-// c = a b (first) or c += a b.  a: (row g, k t'), (g + 8, t'), (g, t''), (g + 8, t'') with g = lane / 4; b: (k t', column g), (t'', g): t' and t'' are
-// the lane's two k of eight, the same for both.
-__device__ __forceinline__ void mma8(float (&c)[4], bool first, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    if (first)
-        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-            : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-    else
-        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// c = a b over 16 of k, eights of it in a[0], b[0] and a[1], b[1]
-__device__ __forceinline__ void mma6(float (&c)[4], const Two (&a)[2][4], const Two (&b)[2][2]) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        mma8(c, h == 0, a[h][0].lo, a[h][1].lo, a[h][2].lo, a[h][3].lo, b[h][0].hi, b[h][1].hi);
-        mma8(c, false, a[h][0].hi, a[h][1].hi, a[h][2].hi, a[h][3].hi, b[h][0].lo, b[h][1].lo);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) mma8(c, false, a[h][0].hi, a[h][1].hi, a[h][2].hi, a[h][3].hi, b[h][0].hi, b[h][1].hi);
-}
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 // Rows that the tensor cores read along k lie DIM + 8 apart, rows that they read across it so many columns + 4: no two lanes that are
@@ -139,8 +87,10 @@ __device__ __forceinline__ void tile_product(float (&acc)[N][4], const float* a,
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const float2 x = of_a(ld2(a0 + k + 8 * h), 0, k + 8 * h + t2), y = of_a(ld2(a1 + k + 8 * h), 1, k + 8 * h + t2);
-            two(x.x, x.y, av[h][0], av[h][2]);
-            two(y.x, y.y, av[h][1], av[h][3]);
+            av[h][0] = apart(x.x);
+            av[h][1] = apart(y.x);
+            av[h][2] = apart(x.y);
+            av[h][3] = apart(y.y);
         }
 #pragma unroll
         for (int n = 0; n < N; ++n) {
