@@ -183,7 +183,8 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 
 // The same attention for prompt portions in 32-bit (plain softmax, all positions or a window): a block takes 32 (token, query head of the
 // group) rows of one request and key/value head and brings a tile of 32 keys once for all of them, where the kernel above reads a key
-// row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 72).  Every number is the same chain of operations as there: a
+// row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 62 with a row's exchanges after the other's, 40 with all of a
+// warp's rows side by side).  Every number is the same chain of operations as there: a
 // score one multiply-add after the other over the row, maxima and sums over a tile's 32 keys by the same exchanges (a warp
 // takes a row, a lane a key), the output's multiply-adds key by key; tiles a row does not see leave it as it is (its maximum stays, a factor
 // of 1, weights of 0).  So results are equal bit for bit, and a portion may be cut anywhere between the two kernels; where a value that some
@@ -269,8 +270,9 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
     constexpr int DL = HD / 4, RG = T_THREADS / DL, OR = T_ROWS / RG;  // lanes across a row, rows at once, rows of a thread
     const int od = (tid % DL) * 4, orow = tid / DL;
     float m[T_ROWS / 4], l[T_ROWS / 4];
+    int pos[T_ROWS / 4];
 #pragma unroll
-    for (int i = 0; i < T_ROWS / 4; ++i) { m[i] = -INFINITY; l[i] = 0.f; }
+    for (int i = 0; i < T_ROWS / 4; ++i) { m[i] = -INFINITY; l[i] = 0.f; pos[i] = start + (row0 + warp + 4 * i) / group; }
     float acc[OR][4];
 #pragma unroll
     for (int i = 0; i < OR; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -303,20 +305,38 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
                 for (int j = 0; j < 2; ++j) ps[(sr + 8 * i) * LP + sk + 16 * j] = s[i][j] * scale;
         }
         __syncthreads();
+        {
+            // (all rows' exchanges side by side; what rows beyond the block's give is not used)
+            const int kpos = t0 + lane;
+            float p[T_ROWS / 4], m_new[T_ROWS / 4], sum[T_ROWS / 4];
+            bool valid[T_ROWS / 4];
 #pragma unroll
-        for (int i = 0; i < T_ROWS / 4; ++i) {
-            const int r = warp + 4 * i;
-            if (r < rows_here) {
-                const int pos = start + (row0 + r) / group, lo = window > 0 ? max(pos - window + 1, 0) : 0, kpos = t0 + lane;
-                const bool valid = kpos >= lo && kpos <= pos;
-                const float s = valid ? ps[r * LP + lane] : -INFINITY;
-                const float m_new = fmaxf(m[i], warp_max(s));
-                const float p = valid ? expf(s - m_new) : 0.f;
-                const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
-                l[i] = fmaf(l[i], alpha, warp_sum(p));
-                m[i] = m_new;
-                ps[r * LP + lane] = p;
-                if (lane == 0) alpha_s[r] = alpha;
+            for (int i = 0; i < T_ROWS / 4; ++i) {
+                valid[i] = kpos <= pos[i] && kpos >= (window > 0 ? max(pos[i] - window + 1, 0) : 0);
+                p[i] = valid[i] ? ps[(warp + 4 * i) * LP + lane] : -INFINITY;
+                m_new[i] = p[i];
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < T_ROWS / 4; ++i) m_new[i] = fmaxf(m_new[i], __shfl_xor_sync(0xffffffffu, m_new[i], off));
+#pragma unroll
+            for (int i = 0; i < T_ROWS / 4; ++i) {
+                m_new[i] = fmaxf(m[i], m_new[i]);
+                p[i] = valid[i] ? expf(p[i] - m_new[i]) : 0.f;
+                sum[i] = p[i];
+                ps[(warp + 4 * i) * LP + lane] = p[i];
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < T_ROWS / 4; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], off);
+#pragma unroll
+            for (int i = 0; i < T_ROWS / 4; ++i) {
+                const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
+                l[i] = fmaf(l[i], alpha, sum[i]);
+                m[i] = m_new[i];
+                if (lane == 0) alpha_s[warp + 4 * i] = alpha;
             }
         }
         __syncthreads();
