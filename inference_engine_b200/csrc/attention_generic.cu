@@ -183,8 +183,8 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 
 // The same attention for prompt portions in 32-bit (plain softmax, all positions or a window): a block takes 32 (token, query head of the
 // group) rows of one request and key/value head and brings a tile of 32 keys once for all of them, where the kernel above reads a key
-// row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 62 with a row's exchanges after the other's, 40 with all of a
-// warp's rows side by side).  Every number is the same chain of operations as there: a
+// row per warp and lane (377 tokens of 16 heads of 64 on 4: 221 us, here 45 by itself; 38 since no exponential
+// is behind a branch and the products' loops are unrolled; a portion of 16 tokens behind 2,000 172 and 126).  Every number is the same chain of operations as there: a
 // score one multiply-add after the other over the row, maxima and sums over a tile's 32 keys by the same exchanges (a warp
 // takes a row, a lane a key), the output's multiply-adds key by key; tiles a row does not see leave it as it is (its maximum stays, a factor
 // of 1, weights of 0).  So results are equal bit for bit, and a portion may be cut anywhere between the two kernels; where a value that some
@@ -208,8 +208,8 @@ rows_one_by_one(const float* q, const float* k_cache, const float* v_cache, cons
     }
 }
 
-// (Two blocks an SM at least, which leaves the compiler its registers: with the 86 of its own choice a portion of 16 tokens behind 2,000
-// takes 299 us, with these 266.)
+// (Two blocks an SM at least, which leaves the compiler its registers: with the 86 of its own choice the loops are not interleaved.  256 threads
+// a block took as long for few blocks and longer for many: what a tile costs is the chain through it.)
 template <int HD>
 __global__ void __launch_bounds__(T_THREADS, 2)
 paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
@@ -284,7 +284,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
         {
             const float* kt = ks + b * T_KEYS * LD;
             float s[4][2] = {};
-#pragma unroll 4
+#pragma unroll 16
             for (int d = 0; d < HD; d += 4) {
                 float4 x[4], y[2];
 #pragma unroll
@@ -323,7 +323,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
 #pragma unroll
             for (int i = 0; i < T_ROWS / 4; ++i) {
                 m_new[i] = fmaxf(m[i], m_new[i]);
-                p[i] = valid[i] ? expf(p[i] - m_new[i]) : 0.f;
+                p[i] = expf(valid[i] ? p[i] - m_new[i] : -INFINITY);  // (exactly 0, without a branch)
                 sum[i] = p[i];
                 ps[(warp + 4 * i) * LP + lane] = p[i];
             }
@@ -333,7 +333,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
                 for (int i = 0; i < T_ROWS / 4; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], off);
 #pragma unroll
             for (int i = 0; i < T_ROWS / 4; ++i) {
-                const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
+                const float alpha = expf(m[i] == -INFINITY ? m[i] : m[i] - m_new[i]);
                 l[i] = fmaf(l[i], alpha, sum[i]);
                 m[i] = m_new[i];
                 if (lane == 0) alpha_s[warp + 4 * i] = alpha;
@@ -346,7 +346,7 @@ paged_attention_f32_tile_kernel(const float* __restrict__ q, const float* __rest
             const float a = alpha_s[orow + RG * i];
             acc[i][0] *= a; acc[i][1] *= a; acc[i][2] *= a; acc[i][3] *= a;
         }
-#pragma unroll 2
+#pragma unroll
         for (int j = 0; j < T_KEYS; j += 4) {
             float4 v[4];
 #pragma unroll
