@@ -328,8 +328,8 @@ chunk_state_kernel(const float* __restrict__ a, int a_ld, const float* __restric
     float* us = ws + CHUNK * DIM;   // [64][CB]
     float* rest = us + CHUNK * CB;  // [THREADS]
     float* bs = rest + THREADS;     // [64]
-    ie_pdl_trigger();
     ie_pdl_wait();
+    ie_pdl_trigger();  // (chunk_out reads what was there before this kernel without waiting for it: see there)
     int seq, chunk;
     const int head = blockIdx.y, c0 = blockIdx.z * CB, tid = threadIdx.x;
     if (!find_chunk(cu_q, num_seqs, blockIdx.x, seq, chunk)) return;
@@ -345,19 +345,18 @@ chunk_state_kernel(const float* __restrict__ a, int a_ld, const float* __restric
     const float* wp = w + (size_t)n0 * w_ld + (head / heads_per_unit) * dim + d;
     const float* ap = a + (size_t)n0 * a_ld + head * dim + d;  // (not read with gates)
     float run = 1.f;
-#pragma unroll 1
-    for (int j1 = (part + 1) * EACH; j1 > part * EACH; j1 -= 16) {
-        float wv[16], av[16];
+    {
+        float wv[EACH], av[EACH];  // (all on their way at once: 513 tokens of 8 heads of 128 x 128 18 us by sixteens, 12.5 so)
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            int j = j1 - 1 - i;
+        for (int i = 0; i < EACH; ++i) {
+            int j = (part + 1) * EACH - 1 - i;
             bool there = j < cnt && d < dim;
             wv[i] = there ? wp[(size_t)j * w_ld] : 0.f;
             av[i] = there ? (g != nullptr ? g[j * gate_stride] : ap[(size_t)j * a_ld]) : 1.f;
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            ws[(j1 - 1 - i) * DIM + d] = wv[i] * run;
+        for (int i = 0; i < EACH; ++i) {
+            ws[((part + 1) * EACH - 1 - i) * DIM + d] = wv[i] * run;
             run *= av[i];
         }
     }
@@ -500,12 +499,17 @@ chunk_out_kernel(const float* __restrict__ q, int q_ld, const float* __restrict_
     float* ws = ahead + 4 * DIM;            // [64][DIM + 8], then the pieces: two of [32][CB + 4]
     float* quad = ws + CHUNK * LD;          // [16][DIM]
     ie_pdl_trigger();
-    ie_pdl_wait();
+    // The scores need nothing of the two kernels before, chunk_state and chunk_scan or the delta rule's two, and so do not wait for them: the first
+    // of those lets the second start, and that one this, only once all that ran before is done.  (Scores formed meanwhile: 513 tokens of 8 heads 22 us after them, 18 so; 2,048 of the delta rule's 16, whose chain leaves 20 SMs idle, 70 and 61.)
     int seq, chunk;
     const int head = blockIdx.y, c0 = blockIdx.z * CB, tid = threadIdx.x, unit = head / heads_per_unit;
-    if (!find_chunk(cu_q, num_seqs, blockIdx.x, seq, chunk)) return;
-    const int n0 = cu_q[seq] + chunk * CHUNK, cnt = min(CHUNK, cu_q[seq + 1] - n0), slot = slots[seq];
-    if (slot < 0 || slot >= num_slots) return;
+    const bool there = find_chunk(cu_q, num_seqs, blockIdx.x, seq, chunk);
+    const int slot = there ? slots[seq] : -1;
+    if (slot < 0 || slot >= num_slots) {
+        ie_pdl_wait();  // (what runs next waits for this kernel alone: it is not done before those are)
+        return;
+    }
+    const int n0 = cu_q[seq] + chunk * CHUNK, cnt = min(CHUNK, cu_q[seq + 1] - n0);
     const size_t place = (size_t)blockIdx.x * heads + head;
     const float* g = gates != nullptr ? gates + (size_t)n0 * gate_stride + head * 3 : nullptr;
     const float *qp = q + (size_t)n0 * q_ld + unit * dim, *wp = w + (size_t)n0 * w_ld + unit * dim, *ap = a + (size_t)n0 * a_ld + head * dim;
@@ -531,6 +535,7 @@ chunk_out_kernel(const float* __restrict__ q, int q_ld, const float* __restrict_
         }
         cp_commit();
     };
+    ie_pdl_wait();
     fetch(0);
     fetch(1);
     if (g != nullptr) {  // u = gate * v, on the scores' side
@@ -687,8 +692,8 @@ delta_solve_kernel(const float* __restrict__ k, const float* __restrict__ v, con
     float* inv = bs + CHUNK;                  // [4][16][24]: the groups' inverses, [j][i]
     float* ws = inv + 4 * GROUP * LI;         // [64][DIM + 8], then U [64][136]
     float* quad = ws + CHUNK * LD;            // [16][DIM]
-    ie_pdl_trigger();
     ie_pdl_wait();
+    ie_pdl_trigger();  // (as in chunk_state)
     int seq, chunk;
     const int head = blockIdx.y, tid = threadIdx.x, kvh = head / (heads / kv_heads);
     if (!find_chunk(cu_q, num_seqs, blockIdx.x, seq, chunk)) return;
