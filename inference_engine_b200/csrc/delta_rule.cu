@@ -114,7 +114,8 @@ delta_prep_kernel(const float* __restrict__ qkvb, int ld, const float* __restric
 // The same for many tokens.  grid: (blocks of PT_TOKENS tokens, units); a thread takes a channel of the unit through its block's
 // tokens, so an input is read once and not once per tap, and sixteen loads are on their way at once (2,048 tokens of 16 heads of
 // 128 x 128: 147 us a token at a time, bound by the units' chains of loads and barriers; 102 with three blocks an SM, whose 168
-// registers a thread left too few loads in flight; 63 with five).  q and k: `dim` at most 128, one
+// registers a thread left too few loads in flight; 63 with five, 57 since the
+// block's rows are asked for before it is known whose they are).  q and k: `dim` at most 128, one
 // channel per thread, whose squares sixteen tokens add up together (every exchange halves the sums a lane still holds).
 constexpr int PT_TOKENS = 16;
 template <int TAPS>
@@ -163,19 +164,29 @@ delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __re
         float y[PT_TOKENS], w[TAPS];
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) w[j] = live ? conv_w[(size_t)c * TAPS + j] : 0.f;
+        // The rows of the block and those before it, on their way before it is known which request's they are.
         const int seq0 = seq_of_token[n0];
-        if (cnt == PT_TOKENS && n0 + PT_TOKENS <= cu_q[seq0 + 1]) {  // (all of one request)
-            const int t0 = n0 - cu_q[seq0], slot = slots[seq0];
+        float in[PT_TOKENS + TAPS - 1];
+        if (cnt == PT_TOKENS) {
+            const float* row = qkvb + (size_t)n0 * ld + c;
+#pragma unroll
+            for (int i = 0; i < PT_TOKENS + TAPS - 1; ++i) {
+                const int at = i - (TAPS - 1);  // (negative: that many rows before the block)
+                in[i] = live && n0 + at >= 0 ? row[(ptrdiff_t)at * ld] : 0.f;
+            }
+        }
+        const int start = cu_q[seq0], end = cu_q[seq0 + 1], slot = slots[seq0];
+        if (cnt == PT_TOKENS && n0 + PT_TOKENS <= end) {  // (all of one request)
+            const int t0 = n0 - start;
             if (slot < 0 || slot >= num_slots) {
                 if (tid == 0) ie_report(err, IE_ERR_PAGE, slot, n0);
                 return;
             }
-            const float* tail = state + (size_t)slot * state_stride + tail_at;
-            float in[PT_TOKENS + TAPS - 1];
+            if (live && t0 < TAPS - 1) {  // the first are the kept ones
+                const float* tail = state + (size_t)slot * state_stride + tail_at;
 #pragma unroll
-            for (int i = 0; i < PT_TOKENS + TAPS - 1; ++i) {
-                const int back = TAPS - 1 - i;  // (negative: that many tokens into the block)
-                in[i] = !live ? 0.f : t0 - back >= 0 ? qkvb[(size_t)(n0 - back) * ld + c] : tail[(size_t)(TAPS - 1 + t0 - back) * channels + c];
+                for (int i = 0; i < TAPS - 1; ++i)
+                    if (i + t0 < TAPS - 1) in[i] = tail[(size_t)(i + t0) * channels + c];
             }
 #pragma unroll
             for (int i = 0; i < PT_TOKENS; ++i) {
@@ -240,6 +251,139 @@ delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __re
 #pragma unroll
         for (int i = 0; i < PT_TOKENS; ++i) {
             if (live && i < cnt) dst[(size_t)i * qk] = y[i] * red[0][i];
+        }
+    }
+}
+
+// The same where channels come in aligned pieces of four: a warp per unit and 8 tokens, a lane four neighbouring channels.  Rows of the block
+// and those before it go to shared memory, all on their way at once, and every lane reads what it fetched itself: no barriers, no
+// registers that wait for memory, little code.  The exponentials and divisions bound it (27 million instructions here, 41 there), then
+// the warps in flight.  (2,048 tokens of 16 heads of 128 x 128: the kernel above 57 us, this one 45, with 16 tokens a warp and half as many
+// warps an SM 56; 4,000 tokens of 32 heads on 16 150 and 111; the bytes of the first take 20.)
+constexpr int PW_TOKENS = 8, PW_LD = PW_TOKENS + 1;
+template <int TAPS> constexpr int pw_floats() { return (PW_TOKENS + TAPS - 1) * 128 + 32 * PW_LD; }
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __restrict__ a, const float* __restrict__ conv_w,
+                       const float* __restrict__ A_log, const float* __restrict__ dt_bias, const float* __restrict__ state,
+                       long long state_stride, const int* __restrict__ slots, const int* __restrict__ seq_of_token,
+                       const int* __restrict__ cu_q, float* __restrict__ q_out, float* __restrict__ k_out, float* __restrict__ v_out,
+                       float* __restrict__ beta, float* __restrict__ decay, int num_tokens, int heads, int kv_heads, int dim, int vdim,
+                       int num_slots, int* err) {
+    extern __shared__ __align__(16) float pw_smem[];
+    ie_pdl_trigger();
+    ie_pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = blockIdx.y * 4 + warp;
+    const int n0 = blockIdx.x * PW_TOKENS, cnt = min(PW_TOKENS, num_tokens - n0), qk = kv_heads * dim, channels = 2 * qk + heads * vdim;
+    float* rows = pw_smem + warp * pw_floats<TAPS>();            // [PW_TOKENS + TAPS - 1][128]
+    float* sums = rows + (PW_TOKENS + TAPS - 1) * 128;           // [32 lanes][PW_TOKENS + 1]
+    auto bring = [&](int row, const float* src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(rows + row * 128 + lane * 4)), "l"(src) : "memory");
+    };
+    if (unit > 2 * kv_heads + 2 * heads) return;
+    if (unit == 2 * kv_heads + 2 * heads) {  // the betas
+        for (int i = lane; i < cnt * heads; i += 32) {
+            const size_t n = (size_t)(n0 + i / heads);
+            beta[n * heads + i % heads] = sigmoid_f(qkvb[n * ld + channels + i % heads]);
+        }
+        return;
+    }
+    const bool is_decay = unit >= 2 * kv_heads + heads, is_v = unit >= 2 * kv_heads && !is_decay;
+    const int width = is_v ? vdim : dim;
+    // the block's tokens, one a lane: its place in its request, and the slot
+    int t_of = 0, slot_of = 0;
+    if (!is_decay && lane < cnt) {
+        const int seq = seq_of_token[n0 + lane];
+        t_of = n0 + lane - cu_q[seq];
+        slot_of = slots[seq];
+        if (slot_of < 0 || slot_of >= num_slots) {
+            ie_report(err, IE_ERR_PAGE, slot_of, n0 + lane);
+            slot_of = -1;
+        }
+    }
+    for (int c0 = 0; c0 < width; c0 += 128) {  // (q, k and decays: once)
+        const int i0 = c0 + lane * 4;
+        const bool live = i0 < width;
+        if (is_decay) {
+            const int h = unit - 2 * kv_heads - heads;
+            const size_t at = (size_t)n0 * heads * dim + h * dim + i0, step = (size_t)heads * dim;
+            if (live)
+                for (int i = 0; i < cnt; ++i) bring(i, a + at + i * step);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (!live) continue;
+            const float rate = expf(A_log[h]);
+            const float4 b = *reinterpret_cast<const float4*>(dt_bias + h * dim + i0);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll 2
+            for (int i = 0; i < cnt; ++i) {
+                const float4 x = *reinterpret_cast<const float4*>(rows + i * 128 + lane * 4);
+                *reinterpret_cast<float4*>(decay + at + i * step) =
+                    make_float4(expf(-rate * softplus_f(x.x + b.x)), expf(-rate * softplus_f(x.y + b.y)),
+                                expf(-rate * softplus_f(x.z + b.z)), expf(-rate * softplus_f(x.w + b.w)));
+            }
+            continue;
+        }
+        const int c = (is_v ? 2 * qk + (unit - 2 * kv_heads) * vdim : unit * dim) + i0;
+        if (live)
+            for (int i = 0; i < cnt + TAPS - 1; ++i)
+                if (n0 + i >= TAPS - 1) bring(i, qkvb + (size_t)(n0 + i - (TAPS - 1)) * ld + c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        float w[4][TAPS];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) w[e][j] = live ? conv_w[(size_t)(c + e) * TAPS + j] : 0.f;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll 2
+        for (int i = 0; i < cnt; ++i) {
+            const int t = __shfl_sync(0xffffffffu, t_of, i), slot = __shfl_sync(0xffffffffu, slot_of, i);
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && slot >= 0) {
+                float4 x[TAPS];
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) x[j] = *reinterpret_cast<const float4*>(rows + (i + j) * 128 + lane * 4);
+                if (t < TAPS - 1) {  // the first look back to the kept ones
+                    const float* tail = state + (size_t)slot * state_stride + (size_t)heads * dim * vdim + c;
+#pragma unroll
+                    for (int j = 0; j < TAPS - 1; ++j)
+                        if (t + j < TAPS - 1) {
+                            const float* kept = tail + (size_t)(t + j) * channels;
+                            x[j] = make_float4(kept[0], kept[1], kept[2], kept[3]);
+                        }
+                }
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) {
+                    y.x = fmaf(w[0][j], x[j].x, y.x);
+                    y.y = fmaf(w[1][j], x[j].y, y.y);
+                    y.z = fmaf(w[2][j], x[j].z, y.z);
+                    y.w = fmaf(w[3][j], x[j].w, y.w);
+                }
+                y = make_float4(silu_f(y.x), silu_f(y.y), silu_f(y.z), silu_f(y.w));
+            }
+            if (is_v) {
+                if (live) *reinterpret_cast<float4*>(v_out + (size_t)(n0 + i) * heads * vdim + (c - 2 * qk)) = y;
+            } else {
+                *reinterpret_cast<float4*>(rows + i * 128 + lane * 4) = y;  // (a row that no later token looks back to)
+                sums[lane * PW_LD + i] = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)));
+            }
+        }
+        if (is_v) continue;
+        // a token's sum per lane, by halves of the lanes; then its factor
+        __syncwarp();
+        float sum = 0.f;
+#pragma unroll
+        for (int l = 0; l < PW_TOKENS; ++l) sum += sums[(lane / PW_TOKENS * PW_TOKENS + l) * PW_LD + lane % PW_TOKENS];
+#pragma unroll
+        for (int off = PW_TOKENS; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        float f = 1.0f / sqrtf(sum + 1e-6f);
+        if (unit < kv_heads) f *= 1.0f / sqrtf((float)dim);
+        float* dst = (unit < kv_heads ? q_out : k_out) + (size_t)n0 * qk + (unit < kv_heads ? unit : unit - kv_heads) * dim + i0;
+#pragma unroll 4
+        for (int i = 0; i < cnt; ++i) {
+            const float factor = __shfl_sync(0xffffffffu, f, i);
+            if (!live) continue;
+            const float4 y = *reinterpret_cast<const float4*>(rows + i * 128 + lane * 4);
+            *reinterpret_cast<float4*>(dst + (size_t)i * qk) = make_float4(y.x * factor, y.y * factor, y.z * factor, y.w * factor);
         }
     }
 }
@@ -453,9 +597,25 @@ IE_API int ie_delta_prep(const float* qkvb, int ld, const float* a, const float*
     e = ie_launch(delta_prep_tile_kernel<TAPS>, tiles, dim3(128), 0, s, qkvb, ld, a, conv_w, A_log, dt_bias,           \
                   (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out, k_out, v_out, beta, decay,      \
                   num_tokens, heads, kv_heads, dim, vdim, num_slots, err)
+#define IE_DP_WARP(TAPS)                                                                                               \
+    {                                                                                                                  \
+        static IePerDevice allowed;                                                                                    \
+        cudaError_t e2 = ie_allow_smem(allowed, delta_prep_warp_kernel<TAPS>, 4 * pw_floats<TAPS>() * sizeof(float));  \
+        if (e2 != cudaSuccess) return (int)e2;                                                                         \
+        e = ie_launch(delta_prep_warp_kernel<TAPS>, dim3((num_tokens + PW_TOKENS - 1) / PW_TOKENS, (units + 3) / 4), dim3(128), 4 * pw_floats<TAPS>() * sizeof(float), \
+                      s, qkvb, ld, a, conv_w, A_log, dt_bias, (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out, \
+                      k_out, v_out, beta, decay, num_tokens, heads, kv_heads, dim, vdim, num_slots, err);              \
+    }
     // (from 64 tokens on the tiles are enough blocks to fill the device; a few tokens get a block per token and unit)
     const bool tile = num_tokens >= 64 && dim <= 128;
-    if (tile && taps == 4) IE_DP_TILE(4);
+    // (a warp per unit and 8 tokens from 256 tokens on: 128 tokens of 16 heads of 128 x 128 8.6 us in tiles, 9.6 so, 256 of 8 heads of 64 x 64
+    // 9.7 and 8.8)
+    const bool fours = tile && num_tokens >= 256 && dim % 4 == 0 && vdim % 4 == 0 && ld % 4 == 0 &&
+                       !(((size_t)qkvb | (size_t)a | (size_t)dt_bias | (size_t)q_out | (size_t)k_out | (size_t)v_out | (size_t)decay) & 15);
+    if (fours && taps == 4) IE_DP_WARP(4)
+    else if (fours && taps == 3) IE_DP_WARP(3)
+    else if (fours && taps == 2) IE_DP_WARP(2)
+    else if (tile && taps == 4) IE_DP_TILE(4);
     else if (tile && taps == 3) IE_DP_TILE(3);
     else if (tile && taps == 2) IE_DP_TILE(2);
     else
@@ -463,6 +623,7 @@ IE_API int ie_delta_prep(const float* qkvb, int ld, const float* a, const float*
                       qkvb, ld, a, conv_w, A_log, dt_bias, (const float*)state, state_stride, slots, seq_of_token, cu_q, q_out,
                       k_out, v_out, beta, decay, heads, kv_heads, dim, vdim, taps, num_slots, err);
 #undef IE_DP_TILE
+#undef IE_DP_WARP
     if (e != 0 || taps < 2) return e;
     int channels = 2 * kv_heads * dim + heads * vdim;
     return ie_launch(delta_conv_tail_kernel, dim3(num_seqs, (channels + 255) / 256), dim3(256), 0, s, qkvb, ld, state, state_stride, slots,

@@ -86,3 +86,42 @@ def test_latent_rows_of_many_tokens(heads, dim, rot_dim, rank, rot_dims, interle
     for a, b in zip(*results):
         # (sums of at most 512 squares in another order)
         torch.testing.assert_close(a.float(), b.float(), rtol=1e-5 if dtype == torch.float32 else 2 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("lens", [[256], [300, 1, 2, 3, 70], [5] * 60])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps", [(4, 4, 128, 128, 4), (4, 2, 64, 256, 3), (8, 8, 36, 20, 2)])
+@pytest.mark.parametrize("missing", [False, True])
+def test_delta_rule_inputs_of_many_tokens(lens, heads, kv_heads, dim, vdim, taps, missing):
+    from types import SimpleNamespace
+
+    from inference_engine_b200.kernels import get_ops
+    from inference_engine_b200.kernels.cuda_ops import KernelError
+
+    ops, n, channels = get_ops(), sum(lens), 2 * kv_heads * dim + heads * vdim
+    g = torch.Generator(device="cuda").manual_seed(n + dim)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, a, w, rates, bias = rand(n, channels + heads), rand(n, heads * dim), rand(channels, taps), rand(heads), rand(heads * dim)
+    state = rand(len(lens), heads * dim * vdim + (taps - 1) * channels)
+    ctx = SimpleNamespace(num_seqs=len(lens), cu_q=torch.tensor([0, *lens]).cumsum(0).int().cuda(),
+                          seq_of_token=torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().cuda())
+    slots = torch.randperm(len(lens), generator=torch.Generator().manual_seed(1)).int()
+    if missing:
+        slots[-1] = len(lens)
+    good = n - lens[-1] if missing else n  # (tokens of a request without a slot get anything)
+    results = []
+    for offset in (0, 1):  # decays that no piece of 16 bytes fits: a thread per channel
+        decay = torch.zeros(n * heads * dim + 4, device="cuda")[offset:offset + n * heads * dim].view(n, heads * dim)
+        outs = [torch.zeros(n, size, device="cuda") for size in (kv_heads * dim, kv_heads * dim, heads * vdim, heads)] + [decay]
+        kept = state.clone()
+        ops.delta_prep(x, a, w, rates, bias, kept, slots.cuda(), ctx, *outs, heads, kv_heads, dim, vdim, taps)
+        if missing:
+            with pytest.raises(KernelError):
+                ops.check_errors()
+        else:
+            ops.check_errors()
+        results.append(outs[:4] + [decay.contiguous(), kept])
+    for i, (one, other) in enumerate(zip(*results)):
+        if i < 2:  # sums of at most 128 squares in another order
+            torch.testing.assert_close(one[:good], other[:good], rtol=2e-6, atol=0)
+        else:
+            assert torch.equal(one[:good], other[:good])
