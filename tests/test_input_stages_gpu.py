@@ -125,3 +125,23 @@ def test_delta_rule_inputs_of_many_tokens(lens, heads, kv_heads, dim, vdim, taps
             torch.testing.assert_close(one[:good], other[:good], rtol=2e-6, atol=0)
         else:
             assert torch.equal(one[:good], other[:good])
+
+
+@pytest.mark.parametrize("tokens,channels,rank", [(1, 128, 1), (37, 100, 7), (300, 300, 16), (1000, 2048, 32), (9000, 384, 31), (130, 200, 33)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_low_rank_decays(tokens, channels, rank, biased):
+    """Whatever the tokens a block takes, a number is the same one: as of its token by itself."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(tokens)
+    y, w = torch.randn(tokens, rank + 3, generator=g, device="cuda")[:, 2: rank + 2], torch.randn(channels, rank, generator=g, device="cuda")
+    bias = torch.randn(channels, generator=g, device="cuda") if biased else None
+    out, one = torch.zeros(tokens, channels, device="cuda"), torch.zeros(1, channels, device="cuda")
+    ops.lowrank_decay(y, w, bias, 16.0, out)
+    x = y.double() @ w.double().T + (0 if bias is None else bias.double())
+    # the sum's error (rank + 1 roundings of at most the terms' sizes) through a slope of at most 1 / 16, and a few of the result's own
+    size = y.double().abs() @ w.double().abs().T + (0 if bias is None else bias.double().abs())
+    assert ((out.double() - torch.exp(torch.nn.functional.logsigmoid(x) / 16)).abs() <= (rank + 1) * 2 ** -24 / 16 * size + 2 ** -21).all()
+    for row in {0, tokens // 2, tokens - 1}:
+        ops.lowrank_decay(y[row:row + 1], w, bias, 16.0, one)
+        assert torch.equal(one[0], out[row])
