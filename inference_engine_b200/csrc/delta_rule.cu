@@ -16,7 +16,7 @@
 //    Each sum over rows is taken in an order that depends on `dim` alone.
 //  * gated_rms_heads: o / rms(o) per head, times a weight, times sigmoid(gate).
 // Everything here is 32-bit.
-#include "common.cuh"
+#include "gated_rows.cuh"
 #include <math.h>
 
 namespace {
@@ -669,6 +669,9 @@ IE_API int ie_gated_rms_heads(const float* o, const float* weight, float eps, co
     if (rows <= 0) return 0;
     dim3 grid((unsigned)((rows + 3) / 4));
     cudaStream_t s = (cudaStream_t)stream;
+    if (gated_rows_fit(o, weight, gate_pre, vdim, out, rows, vdim))
+        return out_dtype == IE_BF16 ? launch_gated_rows(o, weight, 0, eps, gate_pre, vdim, 0, (__nv_bfloat16*)out, rows, 1, vdim, s)
+                                    : launch_gated_rows(o, weight, 0, eps, gate_pre, vdim, 0, (float*)out, rows, 1, vdim, s);
     if (out_dtype == IE_BF16)
         return ie_launch(gated_rms_heads_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, o, weight, eps, gate_pre,
                          (__nv_bfloat16*)out, rows, vdim);

@@ -35,7 +35,7 @@
 // a time through a ring of four shared-memory buffers, three chunks on their way); recurrence_readout (normaliser,
 // unit root mean square per head, weight, output gate).  Every sum is taken in an order that
 // depends on the sizes alone, never on how a request's tokens were cut into steps or batched.
-#include "common.cuh"
+#include "gated_rows.cuh"
 #include <math.h>
 
 namespace {
@@ -838,6 +838,10 @@ IE_API int ie_recurrence_readout(const float* o, int cols, const float* gates, c
     if (rows <= 0) return 0;
     dim3 grid((unsigned)((rows + 3) / 4));
     cudaStream_t s = (cudaStream_t)stream;
+    if (gates == nullptr && cols == vdim && gated_rows_fit(o, weight, gate_pre, gate_pre != nullptr ? gate_ld : 0, out, rows, vdim))
+        return out_dtype == IE_BF16
+                   ? launch_gated_rows(o, weight, weight_per_head, eps, gate_pre, gate_ld, gate_silu, (__nv_bfloat16*)out, rows, heads, vdim, s)
+                   : launch_gated_rows(o, weight, weight_per_head, eps, gate_pre, gate_ld, gate_silu, (float*)out, rows, heads, vdim, s);
     if (out_dtype == IE_BF16)
         return ie_launch(recurrence_readout_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, o, cols, gates, weight,
                          weight_per_head, eps, gate_pre, gate_ld, gate_silu, (__nv_bfloat16*)out, rows, heads, vdim);

@@ -145,3 +145,25 @@ def test_low_rank_decays(tokens, channels, rank, biased):
     for row in {0, tokens // 2, tokens - 1}:
         ops.lowrank_decay(y[row:row + 1], w, bias, 16.0, one)
         assert torch.equal(one[0], out[row])
+
+
+@pytest.mark.parametrize("heads,vdim", [(16, 128), (7, 36), (5, 4)])
+@pytest.mark.parametrize("silu,weighted", [(False, "heads"), (True, "all"), (True, None), (None, "heads")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_rows_in_pieces_of_four(heads, vdim, silu, weighted, dtype):
+    from inference_engine_b200.kernels import get_ops
+
+    ops, tokens = get_ops(), 2501
+    g = torch.Generator(device="cuda").manual_seed(vdim)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    rows, wide = rand(tokens * heads * vdim), rand(tokens, heads * vdim + 8)
+    weight = None if weighted is None else rand(heads * vdim if weighted == "heads" else vdim)
+    results = []
+    for offset in (0, 1):  # rows that no piece of 16 bytes fits: an entry a lane at a time
+        o = torch.empty(rows.numel() + 4, device="cuda")[offset:offset + rows.numel()].copy_(rows).view(tokens, heads * vdim)
+        out = torch.zeros(tokens, heads * vdim, dtype=dtype, device="cuda")
+        gate = None if silu is None else wide[:, 4: 4 + heads * vdim]
+        ops.recurrence_readout(o, None, weight, 1e-5, gate, out, heads, vdim, vdim, gate_act="silu" if silu else "sigmoid")
+        results.append(out.float())
+    # sums of at most 128 squares in another order; in bfloat16 some then round the other way
+    torch.testing.assert_close(*results, rtol=2e-6 if dtype == torch.float32 else 2 ** -7, atol=0)
