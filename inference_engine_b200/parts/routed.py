@@ -55,17 +55,20 @@ class ExpertTiles:
 
     @classmethod
     def of(cls, gate_up, down):
-        """From ``[experts, 2, ff, hidden]`` and ``[experts, hidden, ff]``."""
+        """From ``[experts, 2, ff, hidden]`` and ``[experts, hidden, ff]``, an expert at a time: what is made on the way is one expert's."""
         import torch
 
         count, _, ff, hidden = gate_up.shape
         f, h, rows = -(-ff // 64), -(-hidden // 64), -(-hidden // 128)
         row, piece = torch.arange(128, device=down.device)[:, None], torch.arange(8, device=down.device)[None, :]
         pad = torch.nn.functional.pad
-        gu = pad(gate_up, (0, h * 64 - hidden, 0, f * 64 - ff)).view(count, 2, f, 8, 8, h, 8, 8).permute(0, 2, 5, 3, 1, 4, 6, 7)
-        dn = pad(down, (0, f * 64 - ff, 0, rows * 128 - hidden)).view(count, rows, 128, f, 8, 8).permute(0, 1, 3, 2, 4, 5)
-        turned = lambda t, a, b: t.reshape(count, a, b, 128, 8, 8)[:, :, :, row, piece ^ (row % 8)].view(count, a, b, 128, 64)  # noqa: E731
-        return cls(count, ff, hidden, turned(gu, f, h), turned(dn, rows, f))
+        turned = lambda t, a, b: t.reshape(a, b, 128, 8, 8)[:, :, row, piece ^ (row % 8)].view(a, b, 128, 64)  # noqa: E731
+        tiles = cls(count, ff, hidden, gate_up.new_empty(count, f, h, 128, 64), down.new_empty(count, rows, f, 128, 64))
+        for e in range(count):
+            gu = pad(gate_up[e], (0, h * 64 - hidden, 0, f * 64 - ff)).view(2, f, 8, 8, h, 8, 8).permute(1, 4, 2, 0, 3, 5, 6)
+            dn = pad(down[e], (0, f * 64 - ff, 0, rows * 128 - hidden)).view(rows, 128, f, 8, 8).permute(0, 2, 1, 3, 4)
+            tiles.gate_up[e], tiles.down[e] = turned(gu, f, h), turned(dn, rows, f)
+        return tiles
 
 
 @register_part("feed_forward", "routed_experts")
