@@ -139,12 +139,13 @@ __device__ __noinline__ float one_chain(const float* __restrict__ a, const float
 // served together meet in no bank, and one load feeds two of the tensor cores' eights.
 // VEC: rows of whole 16-byte pieces, aligned.
 // What bounds it: the products and what takes the operands apart, 10 clocks of a scheduler for a product that takes 8, and, of short steps, the way
-// to the first stage and back.  By 1,024 of k, us, with the kernel above / so: 8 rows by 4,096 29 / 10, 377 by 1,536 44 / 29, 377 by 1,024
-// 43 / 23, 2,048 by 2,048 203 / 164; 160 by 2,048 of 8,192 of k 330 / 144.  (A warp the whole of k of its tile: 31, 25 and 187 for
+// to the first stage and back.  By 1,024 of k, us, with the kernel above / so: 8 rows by 4,096 29 / 10, 377 by 1,536 44 / 27, 377 by 1,024
+// 43 / 23, 2,048 by 2,048 203 / 158; 160 by 2,048 of 8,192 of k 330 / 145.  (Three stages, so that four blocks of 32 x 32 fit an SM; with four
+// stages and three blocks 29, 23, 164 and 143.)  (A warp the whole of k of its tile: 31, 25 and 187 for
 // 377 by 1,536, by 1,024 and 2,048 by 2,048 with tiles of 16 x 16 a warp, 29, 29 and 148 with 32 x 32; 64 x 64 a block of 16 warps 29, 29
 // and 180.)
 template <int BM, int BN, int WM, int STAGES, bool VEC>
-__global__ void __launch_bounds__(BM / WM * BN / 32 * 128, 1)
+__global__ void __launch_bounds__(BM / WM * BN / 32 * 128, BM == 32 ? 4 : 1)
 gemm_f32_mma_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K) {
     constexpr int WN = 32, TILES = BM / WM * BN / WN, T = TILES * 128, ROWS = BM + BN, STEP = 64, SLAB = ROWS * 16, MT = WM / 16, NT = WN / 8;
     constexpr int PASS = T / 16;  // rows that the block's threads fetch at once
@@ -270,7 +271,7 @@ IE_API int ie_gemm_f32(const float* A, const float* W, float* C, int M, int N, i
         const long long blocks = (long long)((M + 31) / 32) * ((N + 31) / 32);
         const bool few = M <= 16 || 2 * blocks <= ie_sm_count();
         cudaError_t e = few ? launch_mma<16, 32, 16, 5>(A, W, C, M, N, K, vec, (cudaStream_t)stream)
-                            : launch_mma<32, 32, 32, 4>(A, W, C, M, N, K, vec, (cudaStream_t)stream);
+                            : launch_mma<32, 32, 32, 3>(A, W, C, M, N, K, vec, (cudaStream_t)stream);
         return e != cudaSuccess ? (int)e : IE_LAUNCH_CHECK();
     }
     const int across = (N + BN - 1) / BN;
