@@ -180,8 +180,34 @@ latent_prep_kernel(LatentIn in, const int* __restrict__ positions,
     }
 }
 
+// The sum of 256 threads' numbers as the kernel above adds them up, thread 32 w + lane's in s[w] of a lane: over every 32, by halves of them,
+// then one 32 after the other.
+__device__ __forceinline__ float block_order_sum(float (&s)[LP_THREADS / 32], int lane) {
+    constexpr int WARPS = LP_THREADS / 32;
+    static_assert(WARPS == 8, "");
+#pragma unroll
+    for (int off = 16, held = WARPS / 2; off > 0; off >>= 1, held >>= 1) {
+        if (held > 0) {  // (every exchange halves the sums a lane still holds)
+            const bool high = lane & off;
+#pragma unroll
+            for (int k = 0; k < WARPS / 2; ++k)
+                if (k < held) {
+                    const float send = high ? s[k] : s[k + held], keep = high ? s[k + held] : s[k];
+                    s[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+        }
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) sum += __shfl_sync(0xffffffffu, s[0], 4 * w);
+    return sum;
+}
+
 // The same for many tokens, of products in one part whose sizes and addresses allow pieces of four: a warp per token, no barriers, four of
-// a lane's pieces on their way at a time.  (2,048 tokens of 16 heads of 128 + 64 and a latent of 512, the cached rows and the queries in a
+// a lane's pieces on their way at a time.  Every number is the same chain of operations as there, also the sums of squares: a token's results do not depend on
+// how many others the step has.  (2,048 tokens of 16 heads of 128 + 64 and a latent of 512, the cached rows and the queries in a
 // launch each: 28 us with a block per token; 17 so.  Most of that was code fetched to be executed once, the sums over parts unrolled in
 // every place: little code counts as much as few trips to memory here.)
 constexpr int LW_WARPS = 4, LW_PIECES = 4;
@@ -227,20 +253,29 @@ latent_prep_warp_kernel(LatentIn in, const int* __restrict__ positions, const fl
                 if (i0 + 128 * k < heads * hq) store4(to[k], v[k]);
         }
     }
-    // the cached row's latent, then the queries' own: the first pass over a row takes its sum of squares, the second finds it in the cache
+    // The sums of squares: a first pass over (the queries' latent, the cached row's), which the second finds in the cache.
+    const int n_cq = in.cq != nullptr ? in.q_rank : 0, both = n_cq + (cached ? rank : 0);
+    const float *cq_row = in.cq + (size_t)n * in.cq_ld, *dkv_row = in.dkv + (size_t)n * in.dkv_ld;
+    float sq[LP_THREADS / 32] = {}, sc[LP_THREADS / 32] = {};
+#pragma unroll 1
+    for (int i0 = lane * 4; i0 < both; i0 += LP_THREADS * 4)
+#pragma unroll
+        for (int w = 0; w < LP_THREADS / 32; ++w) {
+            const int i = i0 + w * 128;
+            if (i >= both) continue;
+            const float4 v = *reinterpret_cast<const float4*>(i < n_cq ? cq_row + i : dkv_row + i - n_cq);
+            const float s = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+            if (i < n_cq) sq[w] += s;
+            else sc[w] += s;
+        }
+    // the cached row's latent, then the queries' own
     for (int part = 0; part < 2; ++part) {
-        const float* row = part == 0 ? (cached ? in.dkv + (size_t)n * in.dkv_ld : nullptr) : in.cq != nullptr ? in.cq + (size_t)n * in.cq_ld : nullptr;
-        if (row == nullptr) continue;
+        if (part == 0 ? !cached : in.cq == nullptr) continue;
+        const float* row = part == 0 ? dkv_row : cq_row;
         const int count = part == 0 ? rank : in.q_rank;
         const float* w = part == 0 ? in.norm_w : in.cq_norm_w;
         T* dst = part == 0 ? cache + (size_t)slot * krow : cq_out + (size_t)n * in.q_rank;
-        float ss = 0.f;
-#pragma unroll 4
-        for (int i = lane * 4; i < count; i += 128) {
-            const float4 v = *reinterpret_cast<const float4*>(row + i);
-            ss += fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
-        }
-        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)count + in.eps);
+        const float inv = 1.0f / sqrtf((part == 0 ? block_order_sum(sc, lane) : block_order_sum(sq, lane)) / (float)count + in.eps);
         for (int i0 = lane * 4; i0 < count; i0 += 128 * LW_PIECES) {
             float4 v[LW_PIECES], f[LW_PIECES];
 #pragma unroll
