@@ -16,16 +16,20 @@
 // after tile (a cluster takes every so many'th), with two accumulators of 256 columns: while the epilogue's warps read one, the tensor
 // cores fill the other, and the copies of the next tile's operands run ahead of both.  More than 256 pairs take both.  (2,048 tokens, 4 of 32 experts of
 // 2,048 x 1,024 each: 119 + 59 us with an SM a tile on plain matrices, 82 + 47 so, where the weights' bytes and the products take 43 + 21.)
-//   warp 0, one thread of each block: copies into a ring of six slots of 36 KB (more and smaller ones for steps of fewer than 257 tokens, whose tiles are smaller);
+//   warp 0, one thread of each block: copies into a ring of six slots of 36 KB (more and smaller ones where tiles are smaller, as in steps of fewer than 257 tokens);
 //   warp 1, one thread: in the first block tcgen05.mma for both (tcgen05.commit hands slots back and accumulators over in both blocks), in the
 //   second it passes on which slots are full;
 //   warps 2-9: read the accumulator of their block.
 //
-// Few tokens (`few`: up to 64, and so tiles of at most 64 pairs): a stream of weights.  128 rows a block and 72 KB of ring, three blocks an SM:
+// Few tokens (`few`: up to 64, tiles of at most 64 pairs): a stream of weights.  128 rows a block and 72 KB of ring, three blocks an SM:
 // all blocks of a step start at once and share the memory evenly, and what one waits for at its start and end the others use.  (256 rows and an SM's
 // whole memory a block: 8 tokens over 32 experts of 2,048 x 1,024 were 160 blocks of 1 MB in two rounds of 148, 49 + 26 us; 30 + 12 so.)
 // The down product's weights are asked for while the gated product still runs (whose blocks let the next kernel start once they have
 // seen the sorted pairs, so those are there).
+//
+// How many pairs a tile may have (`most`) goes into the sort, and both kernels cut their memory for it.  A step's tokens alone do not bound it: a token
+// that names an expert more than once (routing does where its scores are no numbers, or where the kept groups have too few experts) has as many
+// pairs there.
 //
 // Every wait is bounded; a block that waits too long records IE_ERR_TIMEOUT, and it (both of a cluster) leaves.
 #include "tma.cuh"
@@ -62,6 +66,7 @@ struct Args {
     int places;              // rows of a k block of x, and of y
     int w_blocks, kbs;       // tiles of 128 rows per expert, k blocks
     int slots, slot_bytes;   // (many pairs) of the ring
+    int most;                // pairs of a tile that there is room for
     int K, F;                // (few, gate-up) columns of x; features of the result
     bf16* y;
     float* out;
@@ -178,6 +183,7 @@ gemm_pair_kernel(const __grid_constant__ Args in) {
     auto tile_at = [&](int t) {  // (expert, first place, pairs, the tile's number along the features)
         const int r = t / in.feature_blocks;
         int4 v = in.tiles[r];
+        v.z = min(v.z, in.most);
         v.w = t - r * in.feature_blocks;
         return v;
     };
@@ -350,7 +356,7 @@ gemm_few_kernel(const __grid_constant__ Args in) {
         return;
     }
     const int4 tile = __ldcg(in.tiles + blockIdx.y);
-    const int n = warps_own(tile.z), n_pad = (n + 15) & ~15, x_bytes = n_pad * BK * 2, slot_bytes = W_BYTES + x_bytes;
+    const int n = min(warps_own(tile.z), FEW_PAIRS), n_pad = (n + 15) & ~15, x_bytes = n_pad * BK * 2, slot_bytes = W_BYTES + x_bytes;
     const int slots = min(FEW_RING / slot_bytes, FEW_SLOTS);  // at least 3 (a slot is a multiple of 1 KB)
     const int nkb = in.kbs;
 
@@ -558,8 +564,8 @@ int launch(const Args& in, int few, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
     const long long most = (long long)in.max_tiles * in.feature_blocks;
     const int pairs = clusters_at_once<GATED>(), clusters = most < pairs ? (int)most : pairs;
-    Args args = in;  // (a token has an expert once: a tile has no more pairs than the step has tokens)
-    const int rows = in.N <= MOST_COLS ? (in.N + 31) / 32 * 16 : MOST_PAIRS / 2;
+    Args args = in;
+    const int rows = in.most <= MOST_COLS ? (in.most + 31) / 32 * 16 : MOST_PAIRS / 2;
     args.slot_bytes = W_BYTES + rows * BK * 2;
     args.slots = RING_BYTES / args.slot_bytes < MOST_SLOTS ? RING_BYTES / args.slot_bytes : MOST_SLOTS;
     return ie_launch_cluster(gemm_pair_kernel<GATED>, dim3(2 * clusters), dim3(THREADS), SMEM_BYTES, s, dim3(2, 1, 1), args);
@@ -569,12 +575,16 @@ int launch(const Args& in, int few, cudaStream_t s) {
 // Up to so many tokens the kernel for few of them runs.
 IE_API int ie_routed_tiled_few() { return FEW_PAIRS; }
 
-// The most pairs of a tile, and the multiple at which an expert's places start, for `routed_sort`.
-IE_API int ie_routed_tiled_most() { return MOST_PAIRS; }
+// The most pairs of a tile of a step of N tokens, and the multiple at which an expert's places start, for `routed_sort`.  (An expert that no
+// token names twice is one tile up to 320 pairs; a multiple of 32, and so of the places' 8.)
+IE_API int ie_routed_tiled_most(int N) { return N <= FEW_PAIRS ? FEW_PAIRS : N <= MOST_COLS ? (N + 31) / 32 * 32 : MOST_PAIRS; }
 IE_API int ie_routed_tiled_align() { return 8; }
 
 // Places to have room for: every expert's up to 7 more, and what the last tile's copies read beyond its pairs.
 IE_API int ie_routed_tiled_places(int pairs, int experts) { return (pairs + 7 * (pairs < experts ? pairs : experts) + MOST_PAIRS + 7) / 8 * 8; }
+
+// Whether there is room for tiles of up to `most` pairs.
+static bool fits(int few, int most, int N) { return most > 0 && most <= (few ? FEW_PAIRS : MOST_PAIRS) && (!few || N <= FEW_PAIRS); }
 
 IE_API int ie_routed_tiled_gather(const void* x, void* xs, const int* order, const int* meta, int places, int top, int K, void* stream) {
     if (places <= 0) return 0;
@@ -583,12 +593,12 @@ IE_API int ie_routed_tiled_gather(const void* x, void* xs, const int* order, con
                      top, K / 8, (K + BK - 1) / BK, places);
 }
 
-// y: [k blocks of F][places][64].  few: x holds the tokens' rows [N, K]; else what `gather` wrote.  w: [experts][ceil(F / 64)][ceil(K / 64)] tiles.
+// most: the pairs of a tile, as `routed_sort` was told.  y: [k blocks of F][places][64].  few: x holds the tokens' rows [N, K]; else what `gather` wrote.  w: [experts][ceil(F / 64)][ceil(K / 64)] tiles.
 IE_API int ie_routed_tiled_gate_up(const void* x, const void* w, void* y, const int* order, const int* tiles, const int* count, int max_tiles,
-                                   int few, int top, int N, int places, int K, int F, float limit, int clamp, float alpha, float up_offset,
+                                   int few, int most, int top, int N, int places, int K, int F, float limit, int clamp, float alpha, float up_offset,
                                    int* err, void* stream) {
     if (max_tiles <= 0) return 0;
-    if (K <= 0 || F <= 0 || K % 8 || F % 8 || ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y)) & 15) || (few && N > FEW_PAIRS))
+    if (K <= 0 || F <= 0 || K % 8 || F % 8 || ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y)) & 15) || !fits(few, most, N))
         return (int)cudaErrorInvalidValue;
     Args in = {};
     in.w = (const unsigned char*)w;
@@ -606,6 +616,7 @@ IE_API int ie_routed_tiled_gate_up(const void* x, const void* w, void* y, const 
     in.order = order;
     in.top = top;
     in.N = N;
+    in.most = most;
     in.limit = limit;
     in.clamp = clamp;
     in.alpha = alpha;
@@ -616,9 +627,9 @@ IE_API int ie_routed_tiled_gate_up(const void* x, const void* w, void* y, const 
 
 // w: [experts][ceil(H / 128)][ceil(F / 64)] tiles; out: [top, N, H] 32-bit.  few: launched right behind ie_routed_tiled_gate_up.
 IE_API int ie_routed_tiled_down(const void* y, const void* w, float* out, const float* weights, const int* order, const int* tiles,
-                                const int* count, int max_tiles, int few, int top, int N, int places, int F, int H, int* err, void* stream) {
+                                const int* count, int max_tiles, int few, int most, int top, int N, int places, int F, int H, int* err, void* stream) {
     if (max_tiles <= 0) return 0;
-    if (H <= 0 || F <= 0 || H % 8 || F % 8 || ((((uintptr_t)y | (uintptr_t)w)) & 15) || (few && N > FEW_PAIRS)) return (int)cudaErrorInvalidValue;
+    if (H <= 0 || F <= 0 || H % 8 || F % 8 || ((((uintptr_t)y | (uintptr_t)w)) & 15) || !fits(few, most, N)) return (int)cudaErrorInvalidValue;
     Args in = {};
     in.w = (const unsigned char*)w;
     in.x = (const unsigned char*)y;
@@ -636,6 +647,7 @@ IE_API int ie_routed_tiled_down(const void* y, const void* w, float* out, const 
     in.weights = weights;
     in.top = top;
     in.N = N;
+    in.most = most;
     in.err = err;
     return launch<false>(in, few, (cudaStream_t)stream);
 }

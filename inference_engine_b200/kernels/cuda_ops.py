@@ -1225,12 +1225,12 @@ class CudaOps:
             "ie_routed_tc5_gate_up": "P P P P P P I I I I I F I F F P P",
             "ie_routed_tc5_down": "P P P P P P P I I I I I I P P",
             "ie_routed_tiled_few": "",
-            "ie_routed_tiled_most": "",
+            "ie_routed_tiled_most": "I",
             "ie_routed_tiled_align": "",
             "ie_routed_tiled_places": "I I",
             "ie_routed_tiled_gather": "P P P P I I I P",
-            "ie_routed_tiled_gate_up": "P P P P P P I I I I I I I F I F F P P",
-            "ie_routed_tiled_down": "P P P P P P P I I I I I I I P P",
+            "ie_routed_tiled_gate_up": "P P P P P P I I I I I I I I F I F F P P",
+            "ie_routed_tiled_down": "P P P P P P P I I I I I I I I P P",
         },
         "recurrent": {
             "ie_short_conv_residual": "P I P P L P P P P I I I I I P P",
@@ -1533,7 +1533,7 @@ class CudaOps:
             x = ws.buffer(tag + ".x", n, hidden, x.dtype).copy_(x)
         # Few tokens are a stream of weights, many a matter of products.  The line is where tiles of 64 pairs hold every expert's.
         few = n <= lib.ie_routed_tiled_few()
-        most, align, places = lib.ie_routed_tiled_most(), lib.ie_routed_tiled_align(), lib.ie_routed_tiled_places(pairs, count)
+        most, align, places = lib.ie_routed_tiled_most(n), lib.ie_routed_tiled_align(), lib.ie_routed_tiled_places(pairs, count)
         max_tiles = lib.ie_routed_tc5_max_tiles(pairs, count, most)
         index = ws.buffer(tag + ".order", 1, 4 * max_tiles + 4 + places, self.torch.int32, rows_cap=None)[0]
         tiles, meta, order = index[: 4 * max_tiles], index[4 * max_tiles: 4 * max_tiles + 4], index[4 * max_tiles + 4:]
@@ -1545,8 +1545,9 @@ class CudaOps:
             xs = ws.buffer(tag + ".sorted", places, -(-hidden // 64) * 64, x.dtype)
             self._routed_gather(lib, x, xs, order, meta, places, top)
             x = xs
-        self._routed_tiled_gate_up(lib, x, experts, y, order, tiles, meta, max_tiles, few, top, n, places, limit, alpha, up_offset)
-        self._routed_tiled_down(lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, top, n, places)
+        self._routed_tiled_gate_up(lib, x, experts, y, order, tiles, meta, max_tiles, few, most, top, n, places, limit, alpha,
+                                  up_offset)
+        self._routed_tiled_down(lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, most, top, n, places)
         return out
 
     @_kind("routed.align")
@@ -1555,17 +1556,18 @@ class CudaOps:
                                                self._stream()), "routed_gather")
 
     @_kind("routed.gate_up")
-    def _routed_tiled_gate_up(self, lib, x, experts, y, order, tiles, meta, max_tiles, few, top, n, places, limit, alpha, up_offset) -> None:
+    def _routed_tiled_gate_up(self, lib, x, experts, y, order, tiles, meta, max_tiles, few, most, top, n, places, limit, alpha,
+                              up_offset) -> None:
         self._check(lib.ie_routed_tiled_gate_up(
             x.data_ptr(), experts.gate_up.data_ptr(), y.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(), max_tiles,
-            int(few), top, n, places, experts.hidden, experts.ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha,
+            int(few), most, top, n, places, experts.hidden, experts.ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha,
             up_offset, self._err_ptr, self._stream()), "routed_few_gate_up" if few else "routed_pair_gate_up")
 
     @_kind("routed.down")
-    def _routed_tiled_down(self, lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, top, n, places) -> None:
+    def _routed_tiled_down(self, lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, most, top, n, places) -> None:
         self._check(lib.ie_routed_tiled_down(
             y.data_ptr(), experts.down.data_ptr(), out.data_ptr(), weights.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
-            max_tiles, int(few), top, n, places, experts.ff, experts.hidden, self._err_ptr, self._stream()),
+            max_tiles, int(few), most, top, n, places, experts.ff, experts.hidden, self._err_ptr, self._stream()),
             "routed_few_down" if few else "routed_pair_down")
 
     @_kind("routed.align")

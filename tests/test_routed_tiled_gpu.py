@@ -21,8 +21,8 @@ def _run(x, ids, weights, gate_up, down, limit, alpha, offset):
     return out, {name for name, n in ops.launch_counts.items() if n > before.get(name, 0)}
 
 
-# pairs per expert: around the rounding to 32, an accumulator's 256, a tile's 384, several tiles; experts nobody chose; up to 64 tokens
-@pytest.mark.parametrize("counts", [[0, 1, 31, 32, 33, 63], [255, 256, 257, 0, 320, 64], [383, 384, 385, 0, 770, 8], [0, 0, 2300, 0], [1, 0, 15, 16, 17],
+# pairs per expert: around the rounding to 32, an accumulator's 256, a tile's 320, several tiles; experts nobody chose; up to 64 tokens
+@pytest.mark.parametrize("counts", [[0, 1, 31, 32, 33, 63], [255, 256, 257, 0, 320, 64], [319, 321, 640, 641, 0, 8], [383, 384, 385, 0, 770, 8], [0, 0, 2300, 0], [1, 0, 15, 16, 17],
                                     [0, 64, 0], [1]])
 @pytest.mark.parametrize("hidden,ff,limit", [(128, 64, None), (320, 136, 1.5), (72, 264, None), (520, 128, 0.7)])
 def test_pairs_per_expert(counts, hidden, ff, limit):
@@ -89,3 +89,46 @@ def test_router_of_many_tokens(tokens, width, experts, top, groups, keep, scorin
     want = scores.gather(1, ids.long())
     want = want / want.sum(-1, keepdim=True)
     torch.testing.assert_close(weights[sure].double(), want[sure], atol=2e-6, rtol=2e-5)
+
+
+# around the room for 64 pairs of the kernel for few tokens, and for as many pairs as a step has tokens of the other one
+@pytest.mark.parametrize("tokens", [1, 8, 16, 17, 20, 33, 62, 64, 65, 100, 256, 257, 300])
+@pytest.mark.parametrize("repeats", ["one expert", "twice each"])
+def test_tokens_that_name_an_expert_more_than_once(tokens, repeats):
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    experts, top, hidden, ff = 5, 4, 136, 72
+    if repeats == "one expert":
+        ids = torch.zeros(tokens, top, dtype=torch.int32, device="cuda")
+    else:
+        ids = torch.randint(0, experts, (tokens, 2), generator=g, device="cuda", dtype=torch.int32).repeat(1, 2)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, gate_up, down = rand(tokens, hidden).bfloat16(), (rand(experts, 2, ff, hidden) * 0.1).bfloat16(), (rand(experts, hidden, ff) * 0.1).bfloat16()
+    args = (x, ids, torch.rand(tokens, top, generator=g, device="cuda"), gate_up, down, None, 1.0, 0.0)
+    got, ran = _run(*args)
+    assert ("routed_few_down" if tokens <= 64 else "routed_pair_down") in ran
+    want = _want(*args)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-3
+
+
+@pytest.mark.parametrize("tokens", [8, 20, 62, 64, 65, 100, 256, 300, 700])
+@pytest.mark.parametrize("spoilt", ["one", "most", "all"])
+@pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])
+def test_rows_that_are_no_numbers(tokens, spoilt, scoring):
+    """Routing gives them expert 0 for every choice.  The other rows come out as beside good ones, bit for bit."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(tokens)
+    experts, top, hidden, ff = 6, 4, 192, 64
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, router = rand(tokens, hidden).bfloat16(), rand(experts, hidden) * hidden ** -0.5
+    gate_up, down = (rand(experts, 2, ff, hidden) * 0.1).bfloat16(), (rand(experts, hidden, ff) * 0.1).bfloat16()
+    bad = torch.zeros(tokens, dtype=torch.bool, device="cuda")
+    bad[{"one": slice(tokens // 2, tokens // 2 + 1), "most": slice(3, None), "all": slice(None)}[spoilt]] = True
+    outs = []
+    for rows in (x, x.masked_fill(bad[:, None], float("nan"))):
+        ids, weights = torch.empty(tokens, top, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+        ops.route_topk(rows, router, 1, 1, ids, weights, scoring=scoring)
+        outs.append(_run(rows, ids, weights, gate_up, down, None, 1.0, 0.0)[0])
+    assert (ids[bad] == 0).all()
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:, ~bad], outs[1][:, ~bad])
+    assert not torch.isfinite(outs[1][:, bad]).any()
