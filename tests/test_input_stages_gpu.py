@@ -166,5 +166,25 @@ def test_gated_rows_in_pieces_of_four(heads, vdim, silu, weighted, dtype):
         gate = None if silu is None else wide[:, 4: 4 + heads * vdim]
         ops.recurrence_readout(o, None, weight, 1e-5, gate, out, heads, vdim, vdim, gate_act="silu" if silu else "sigmoid")
         results.append(out.float())
-    # sums of at most 128 squares in another order; in bfloat16 some then round the other way
-    torch.testing.assert_close(*results, rtol=2e-6 if dtype == torch.float32 else 2 ** -7, atol=0)
+    assert torch.equal(*results)  # (the same chains of operations)
+    # and so a row's result does not depend on how many there are
+    few = torch.zeros(3, heads * vdim, dtype=dtype, device="cuda")
+    ops.recurrence_readout(rows.view(tokens, -1)[1700:1703], None, weight, 1e-5, None if gate is None else gate[1700:1703], few, heads, vdim, vdim,
+                           gate_act="silu" if silu else "sigmoid")
+    assert torch.equal(few.float(), results[0][1700:1703])
+
+
+@pytest.mark.parametrize("heads,vdim", [(16, 128), (7, 36), (3, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_heads_of_many_and_of_few_tokens(heads, vdim, dtype):
+    """The delta rule's read-out: the same bits for a token among 2,501 and among 3."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, tokens = get_ops(), 2501
+    g = torch.Generator(device="cuda").manual_seed(vdim)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    o, gate, weight = rand(tokens, heads * vdim), rand(tokens, heads * vdim), rand(vdim)
+    out, few = torch.zeros(tokens, heads * vdim, dtype=dtype, device="cuda"), torch.zeros(3, heads * vdim, dtype=dtype, device="cuda")
+    ops.gated_rms_heads(o, weight, 1e-5, gate, out, heads, vdim)
+    ops.gated_rms_heads(o[900:903], weight, 1e-5, gate[900:903], few, heads, vdim)
+    assert torch.equal(out[900:903], few)
