@@ -259,9 +259,10 @@ delta_prep_tile_kernel(const float* __restrict__ qkvb, int ld, const float* __re
 // and those before it go to shared memory, all on their way at once, and every lane reads what it fetched itself: no barriers, no
 // registers that wait for memory, little code.  The exponentials and divisions bound it (27 million instructions here, 41 there), then
 // the warps in flight.  (2,048 tokens of 16 heads of 128 x 128: the kernel above 57 us, this one 45, with 16 tokens a warp and half as many
-// warps an SM 56; 4,000 tokens of 32 heads on 16 150 and 111; the bytes of the first take 20.)
-constexpr int PW_TOKENS = 8, PW_LD = PW_TOKENS + 1;
-template <int TAPS> constexpr int pw_floats() { return (PW_TOKENS + TAPS - 1) * 128 + 32 * PW_LD; }
+// warps an SM 56; 4,000 tokens of 32 heads on 16 150 and 111; the bytes of the first take 20.)  Every number is the same chain of operations as
+// above, also the sums of squares: a token's results do not depend on how many others the step has.
+constexpr int PW_TOKENS = 8, PW_LD = 128 + 4;  // (rows so far apart that eight tokens' pieces of one column meet in no bank)
+template <int TAPS> constexpr int pw_floats() { return (PW_TOKENS + TAPS - 1) * PW_LD; }
 template <int TAPS>
 __global__ void __launch_bounds__(128)
 delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __restrict__ a, const float* __restrict__ conv_w,
@@ -275,10 +276,9 @@ delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __re
     ie_pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = blockIdx.y * 4 + warp;
     const int n0 = blockIdx.x * PW_TOKENS, cnt = min(PW_TOKENS, num_tokens - n0), qk = kv_heads * dim, channels = 2 * qk + heads * vdim;
-    float* rows = pw_smem + warp * pw_floats<TAPS>();            // [PW_TOKENS + TAPS - 1][128]
-    float* sums = rows + (PW_TOKENS + TAPS - 1) * 128;           // [32 lanes][PW_TOKENS + 1]
+    float* rows = pw_smem + warp * pw_floats<TAPS>();  // [PW_TOKENS + TAPS - 1][128 + 4]
     auto bring = [&](int row, const float* src) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(rows + row * 128 + lane * 4)), "l"(src) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(rows + row * PW_LD + lane * 4)), "l"(src) : "memory");
     };
     if (unit > 2 * kv_heads + 2 * heads) return;
     if (unit == 2 * kv_heads + 2 * heads) {  // the betas
@@ -316,7 +316,7 @@ delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __re
             asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
-                const float4 x = *reinterpret_cast<const float4*>(rows + i * 128 + lane * 4);
+                const float4 x = *reinterpret_cast<const float4*>(rows + i * PW_LD + lane * 4);
                 *reinterpret_cast<float4*>(decay + at + i * step) =
                     make_float4(expf(-rate * softplus_f(x.x + b.x)), expf(-rate * softplus_f(x.y + b.y)),
                                 expf(-rate * softplus_f(x.z + b.z)), expf(-rate * softplus_f(x.w + b.w)));
@@ -341,7 +341,7 @@ delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __re
             if (live && slot >= 0) {
                 float4 x[TAPS];
 #pragma unroll
-                for (int j = 0; j < TAPS; ++j) x[j] = *reinterpret_cast<const float4*>(rows + (i + j) * 128 + lane * 4);
+                for (int j = 0; j < TAPS; ++j) x[j] = *reinterpret_cast<const float4*>(rows + (i + j) * PW_LD + lane * 4);
                 if (t < TAPS - 1) {  // the first look back to the kept ones
                     const float* tail = state + (size_t)slot * state_stride + (size_t)heads * dim * vdim + c;
 #pragma unroll
@@ -363,18 +363,29 @@ delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __re
             if (is_v) {
                 if (live) *reinterpret_cast<float4*>(v_out + (size_t)(n0 + i) * heads * vdim + (c - 2 * qk)) = y;
             } else {
-                *reinterpret_cast<float4*>(rows + i * 128 + lane * 4) = y;  // (a row that no later token looks back to)
-                sums[lane * PW_LD + i] = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)));
+                *reinterpret_cast<float4*>(rows + i * PW_LD + lane * 4) = y;  // (a row that no later token looks back to)
             }
         }
         if (is_v) continue;
-        // a token's sum per lane, by halves of the lanes; then its factor
+        // The squares of a token's 32 channels per lane (channel d's with d + 16, then with d + 8 and so on, as a warp of the kernels above adds
+        // them), the four sums of 32, then the token's factor.
         __syncwarp();
-        float sum = 0.f;
+        float part[32];
 #pragma unroll
-        for (int l = 0; l < PW_TOKENS; ++l) sum += sums[(lane / PW_TOKENS * PW_TOKENS + l) * PW_LD + lane % PW_TOKENS];
+        for (int k = 0; k < 32; k += 4) {
+            const float4 y = *reinterpret_cast<const float4*>(rows + lane % PW_TOKENS * PW_LD + lane / PW_TOKENS * 32 + k);
+            part[k] = __fmul_rn(y.x, y.x);
+            part[k + 1] = __fmul_rn(y.y, y.y);
+            part[k + 2] = __fmul_rn(y.z, y.z);
+            part[k + 3] = __fmul_rn(y.w, y.w);
+        }
 #pragma unroll
-        for (int off = PW_TOKENS; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        for (int half = 16; half > 0; half >>= 1)
+#pragma unroll
+            for (int k = 0; k < half; ++k) part[k] += part[k + half];
+        float sum = part[0];
+        sum += __shfl_xor_sync(0xffffffffu, sum, PW_TOKENS);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2 * PW_TOKENS);
         float f = 1.0f / sqrtf(sum + 1e-6f);
         if (unit < kv_heads) f *= 1.0f / sqrtf((float)dim);
         float* dst = (unit < kv_heads ? q_out : k_out) + (size_t)n0 * qk + (unit < kv_heads ? unit : unit - kv_heads) * dim + i0;
@@ -382,7 +393,7 @@ delta_prep_warp_kernel(const float* __restrict__ qkvb, int ld, const float* __re
         for (int i = 0; i < cnt; ++i) {
             const float factor = __shfl_sync(0xffffffffu, f, i);
             if (!live) continue;
-            const float4 y = *reinterpret_cast<const float4*>(rows + i * 128 + lane * 4);
+            const float4 y = *reinterpret_cast<const float4*>(rows + i * PW_LD + lane * 4);
             *reinterpret_cast<float4*>(dst + (size_t)i * qk) = make_float4(y.x * factor, y.y * factor, y.z * factor, y.w * factor);
         }
     }

@@ -121,11 +121,35 @@ def test_delta_rule_inputs_of_many_tokens(lens, heads, kv_heads, dim, vdim, taps
         else:
             ops.check_errors()
         results.append(outs[:4] + [decay.contiguous(), kept])
-    for i, (one, other) in enumerate(zip(*results)):
-        if i < 2:  # sums of at most 128 squares in another order
-            torch.testing.assert_close(one[:good], other[:good], rtol=2e-6, atol=0)
-        else:
-            assert torch.equal(one[:good], other[:good])
+    for one, other in zip(*results):  # (the same chains of operations)
+        assert torch.equal(one[:good], other[:good])
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps", [(4, 4, 128, 128, 4), (4, 2, 64, 128, 3), (8, 8, 36, 20, 2)])
+def test_delta_rule_inputs_whole_and_in_portions(heads, kv_heads, dim, vdim, taps):
+    """700 tokens at once and in portions of 300, 150 and 7: a warp per unit and 8 tokens, tiles of 16, a block per token and unit.  Equal bits."""
+    from types import SimpleNamespace
+
+    from inference_engine_b200.kernels import get_ops
+
+    ops, n, channels = get_ops(), 700, 2 * kv_heads * dim + heads * vdim
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, a, w, rates, bias = rand(n, channels + heads), rand(n, heads * dim), rand(channels, taps), rand(heads), rand(heads * dim)
+    state = rand(1, heads * dim * vdim + (taps - 1) * channels)
+    results = []
+    for step in (700, 300, 150, 7):
+        outs, kept = [torch.zeros(n, size, device="cuda") for size in (kv_heads * dim, kv_heads * dim, heads * vdim, heads, heads * dim)], state.clone()
+        for at in range(0, n, step):
+            cut = slice(at, min(at + step, n))
+            ctx = SimpleNamespace(num_seqs=1, cu_q=torch.tensor([0, cut.stop - at], dtype=torch.int32, device="cuda"),
+                                  seq_of_token=torch.zeros(cut.stop - at, dtype=torch.int32, device="cuda"))
+            ops.delta_prep(x[cut], a[cut], w, rates, bias, kept, torch.zeros(1, dtype=torch.int32, device="cuda"), ctx, *(o[cut] for o in outs),
+                           heads, kv_heads, dim, vdim, taps)
+        ops.check_errors()
+        results.append(outs + [kept])
+    for other in results[1:]:
+        assert all(torch.equal(one, two) for one, two in zip(results[0], other))
 
 
 @pytest.mark.parametrize("tokens,channels,rank", [(1, 128, 1), (37, 100, 7), (300, 300, 16), (1000, 2048, 32), (9000, 384, 31), (130, 200, 33)])
