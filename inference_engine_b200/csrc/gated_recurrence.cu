@@ -772,17 +772,24 @@ IE_API int ie_rotate_heads(float* x, int ld, const int* positions, const float* 
                      table_positions, units, dim, err);
 }
 
+// Tokens a block of ranks of one piece: as many as leave six blocks an SM, 16 at least.  (2,000 tokens of 2,048 channels 21.2 us with 64, 19.0 with 32, 20.5
+// with 16; 8,000 63, 65 and 71.  By itself the kernel is done sooner with 8 where tokens are few, 300 of them 8.0 us against 9.4, but the recurrence behind
+// it starts early with a block or less an SM, and beside twice the blocks several of its own meet on one SM and run as slow as that.  The layer,
+// us, with 8 / 16: 8 heads of 128 x 128, 96 tokens 47 / 43, 128 66 / 51, 160 76 / 57; 4 heads, three requests of 60 42 / 35; others of 16 to 400 tokens and 512
+// to 2,048 channels differ by 2 at most, either way.)
+IE_API int ie_lowrank_decay_tokens(int num_tokens, int channels, int sms) {
+    int each = LD_MOST;
+    while (each > 16 && ((long long)num_tokens + each - 1) / each * ((channels + 127) / 128) < 6ll * sms) each /= 2;
+    return each;
+}
+
 IE_API int ie_lowrank_decay(const float* y, int y_ld, const float* w2, const float* bias, float inv_tau,
                             float* decay, int num_tokens, int channels, int rank, void* stream) {
     if (num_tokens <= 0 || channels <= 0) return 0;
     if (rank < 1) return (int)cudaErrorInvalidValue;
     if (rank <= LD_RANKS) {
-        // (as many tokens a block as leave six blocks an SM: 2,000 tokens of 2,048 channels 21.2 us with 64, 19.0 with 32, 20.5 with 16; 8,000 63, 65
-        // and 71; 300 11.2, 9.7 and 9.4, with 8 8.0)
-        const long long across = (channels + 127) / 128;
-        int each = LD_MOST;
-        while (each > 8 && (num_tokens + each - 1) / each * across < 6ll * ie_sm_count()) each /= 2;
-        return ie_launch(lowrank_decay_long_kernel, dim3((num_tokens + each - 1) / each, (unsigned)across), dim3(128), 0, (cudaStream_t)stream, y, y_ld,
+        const int each = ie_lowrank_decay_tokens(num_tokens, channels, ie_sm_count());
+        return ie_launch(lowrank_decay_long_kernel, dim3((num_tokens + each - 1) / each, (channels + 127) / 128), dim3(128), 0, (cudaStream_t)stream, y, y_ld,
                          w2, bias, inv_tau, decay, num_tokens, channels, rank, each);
     }
     dim3 grid((num_tokens + LD_TOKENS - 1) / LD_TOKENS, (channels + 127) / 128);

@@ -296,3 +296,18 @@ def test_scratch_buffers_are_sized_as_asked():
     assert tuple(again.shape) == (1, 3_000_000) and ctx.ws.version == version and again.data_ptr() == small.data_ptr()
     large = CudaOps._scratch(ops, ctx, "attn.partial", 5_000_000, "cpu")
     assert tuple(large.shape) == (1, 5_000_000) and ctx.ws.version == version + 1 and ctx.ws.bytes() == 4 << 23
+
+
+def test_low_rank_decays_take_no_more_blocks_than_sixteen_tokens_each():
+    """The recurrence behind them starts early: with more and smaller blocks before it, several of its own ran on one SM."""
+    import ctypes
+
+    from inference_engine_b200.kernels.build import build_part_library
+
+    tokens_a_block = ctypes.CDLL(str(build_part_library("recurrent"))).ie_lowrank_decay_tokens
+    for tokens in [1, 2, 15, 16, 17, 60, 96, 128, 160, 200, 256, 300, 513, 2000, 8000, 100000]:
+        for channels in [1, 128, 512, 513, 1024, 2048, 4096]:
+            each = tokens_a_block(tokens, channels, 148)
+            assert 16 <= each <= 64 and each % 4 == 0
+            blocks = -(-tokens // each) * -(-channels // 128)
+            assert each == 16 or blocks >= 6 * 148  # (the blocks of a larger step are larger, and still fill the device)
