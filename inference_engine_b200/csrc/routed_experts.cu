@@ -277,6 +277,14 @@ __device__ __forceinline__ void three(float x, float y, unsigned (&t)[3]) {
     }
 }
 
+// One chain of multiply-adds: for a logit that is no finite number, which three parts, added up or multiplied with an infinite value, do not keep as it is.
+__device__ __noinline__ float route_chain(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, int width) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < width; ++k) s = fmaf(__bfloat162float(x[k]), w[k], s);
+    return s;
+}
+
 __global__ void __launch_bounds__(RM_WARPS * 32)
 route_many_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int num_tokens, int width,
                   int experts, int top, int groups, int keep, int sigmoid_scores, const float* __restrict__ correction, int group_top,
@@ -345,6 +353,7 @@ route_many_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
                 float s = 0.f;
 #pragma unroll
                 for (int v = 0; v < RM_WARPS; ++v) s += sm[(v * RM_TOKENS + row) * LD + i % RM_EXPERTS];
+                if (!isfinite(s) && n0 + row < num_tokens) s = route_chain(x + (size_t)(n0 + row) * width, w + (size_t)e * width, width);
                 scores[row * per_token + e] = bias != nullptr ? s + bias[e] : s;
             }
         }

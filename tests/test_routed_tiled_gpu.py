@@ -132,3 +132,33 @@ def test_rows_that_are_no_numbers(tokens, spoilt, scoring):
     assert (ids[bad] == 0).all()
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:, ~bad], outs[1][:, ~bad])
     assert not torch.isfinite(outs[1][:, bad]).any()
+
+
+@pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])
+def test_router_of_many_tokens_with_infinities(scoring):
+    """An infinite activation gives infinite logits, and a choice, as among few tokens; a weight that rounds beyond bfloat16's range is one like others."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(2)
+    tokens, width, experts, top = 700, 256, 12, 3
+    x = torch.randn(tokens, width, generator=g, device="cuda").bfloat16()
+    w = torch.randn(experts, width, generator=g, device="cuda") * width ** -0.5
+    w[:, 9] = torch.arange(experts, device="cuda") % 2 * 2.0 - 1  # no lower parts
+    w[2, 5], w[7, 6] = 3.4028234e38, float("-inf")
+    x[:, 5], x[300:, 6] = 0.0, 0.0
+    x[:300, 6] = x[:300, 6].abs() + 1
+    x[3, 7], x[17, 100], x[18, 9], x[650, 9] = float("inf"), float("-inf"), float("inf"), float("nan")
+    x[40, 8], x[40, 9] = float("inf"), float("-inf")
+    correction = torch.randn(experts, generator=g, device="cuda") * 0.01 if scoring == "sigmoid" else None
+    results = []
+    for step in (700, 100):
+        ids, weights = torch.full((tokens, top), -1, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+        for at in range(0, tokens, step):
+            ops.route_topk(x[at: at + step], w, 1, 1, ids[at: at + step], weights[at: at + step], scoring=scoring, correction=correction)
+        results.append((ids, weights))
+    (many, many_weights), (few, few_weights) = results
+    assert torch.equal(many, few)
+    # logits of 32-bit sums in another order
+    torch.testing.assert_close(many_weights, few_weights, atol=2e-6, rtol=2e-5, equal_nan=True)
+    if scoring == "sigmoid":
+        assert len(set(few[17].tolist())) == top and len(set(few[18].tolist())) == top  # (a choice, not expert 0 for all)
