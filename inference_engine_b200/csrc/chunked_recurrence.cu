@@ -482,6 +482,8 @@ chunk_scan_kernel(float* __restrict__ add, const float* __restrict__ fade, float
 // normaliser's column.  u: element (n, head, c) at [n * u_ld + head * vdim + c], or with `own` [chunks, heads, 64, vdim].
 // out: [N, heads, cols], times q_scale.  100 KB of shared memory, two blocks per SM: once the scores stand, the state and then u come in
 // pieces of 32 rows, two at a time, where w was.
+// Parts of a product that are subtracted from one another make no number of an infinite one: scores and outputs that come out without a finite value are
+// formed again, one multiply-add after the other.
 template <int DIM, int CB>
 __global__ void __launch_bounds__(THREADS, 2)
 chunk_out_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ a, int a_ld, const float* __restrict__ w,
@@ -626,6 +628,8 @@ chunk_out_kernel(const float* __restrict__ q, int q_ld, const float* __restrict_
         if (p + 2 < PIECES) fetch(p + 2);
     }
     const int c = c0 + nc + NT * t2;  // 2 NT columns from here on
+    auto no_number = [](float x) { return !(fabsf(x) <= FLT_MAX); };
+    bool odd = false;
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -639,10 +643,35 @@ chunk_out_kernel(const float* __restrict__ q, int q_ld, const float* __restrict_
 #pragma unroll
             for (int k = 0; k < 2 * NT; k += 4) {
                 if (c + k >= vdim) break;
+                odd |= no_number(o[k]) || no_number(o[k + 1]) || no_number(o[k + 2]) || no_number(o[k + 3]);
                 if (cols == vdim) st4(to + k, make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]));
                 else { to[k] = o[k]; to[k + 1] = o[k + 1]; to[k + 2] = o[k + 2]; to[k + 3] = o[k + 3]; }  // (rows of an odd length)
             }
         }
+    if (__syncthreads_or(odd)) {
+        for (int i = tid; i < CHUNK * CHUNK; i += THREADS) {
+            const int row = i / CHUNK, j = i % CHUNK;
+            if (j > row || row >= cnt || !no_number(A[Sc::at(row, j)])) continue;
+            float s = 0.f;
+            for (int d = 0; d < dim; ++d) {
+                float x = qp[(size_t)row * q_ld + d];
+                for (int t = j + 1; t <= row; ++t) x *= g != nullptr ? g[t * gate_stride] : ap[(size_t)t * a_ld + d];
+                s = fmaf(x, wp[(size_t)j * w_ld + d], s);
+            }
+            A[Sc::at(row, j)] = g != nullptr ? s * g[j * gate_stride + 1] : s;
+        }
+        __syncthreads();
+        for (int i = tid; i < cnt * CB; i += THREADS) {
+            const int row = i / CB, col = c0 + i % CB;
+            float* to = out + ((size_t)(n0 + row) * heads + head) * cols + col;
+            if (col >= vdim || !no_number(*to)) continue;
+            float s = 0.f;
+            for (int d = 0; d < dim; ++d) s = fmaf(qs[row * LD + d] * ahead[row / GROUP * DIM + d], before[(place * dim + d) * vdim + col], s);
+            for (int j = 0; j <= row; ++j)
+                s = fmaf(A[Sc::at(row, j)], own ? u[(place * CHUNK + j) * vdim + col] : u[(size_t)(n0 + j) * u_ld + head * vdim + col], s);
+            *to = s * q_scale;
+        }
+    }
     if (cols > vdim && c0 == 0) {  // the normaliser's column, whose values are the gates
         for (int i = warp; i < cnt; i += THREADS / 32) {
             float s = 0.f;

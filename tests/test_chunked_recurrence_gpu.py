@@ -190,3 +190,26 @@ def test_delta_rule_with_a_value_that_is_no_number(ops, value, what, dim, vdim):
     assert not torch.isfinite(outs[1][at:, :3]).all(dim=1).any()
     # (the spoilt chunk goes token by token: the same sums in another order)
     assert float((outs[0][:at] - outs[1][:at]).norm() / outs[0][:at].norm()) < REL
+
+
+@pytest.mark.parametrize("where", ["value", "key", "query", "state"])
+@pytest.mark.parametrize("dim,vdim,gated", [(128, 128, False), (64, 36, False), (64, 64, True)])
+def test_infinities_stay_infinities(ops, where, dim, vdim, gated):
+    """Positive numbers, one of them infinite: what is infinite token by token is so in chunks, for all later tokens, and nothing else changes."""
+    n, heads, at, cols = 150, 2, 70, vdim + gated
+    g = torch.Generator().manual_seed(5)
+    rand = lambda *s: (torch.rand(*s, generator=g) + 0.1).cuda()  # noqa: E731
+    q, w, v, decay, gates = rand(n, heads * dim), rand(n, heads * dim), rand(n, heads * vdim), rand(n, heads * dim) * 0.5 + 0.4, rand(n, heads, 3) * 0.5 + 0.4
+    state = rand(1, heads * cols * dim)
+    ({"value": v, "key": w, "query": q, "state": state}[where])[0 if where == "state" else at, 7] = float("inf")
+    results = []
+    for in_chunks in (False, True):
+        out, st = torch.zeros(n, heads * cols, device="cuda"), state.clone()
+        ops.gated_recurrence(q, None if gated else decay, w, gates if gated else None, v, st, torch.zeros(1, dtype=torch.int32, device="cuda"),
+                             _Ctx([n], "cuda"), out, heads, dim, vdim, cols, 0.5, in_chunks=in_chunks)
+        results.append(out)
+    one, chunks = results
+    assert not torch.isnan(one).any() and torch.isinf(one).any()
+    assert torch.equal(torch.isinf(one), torch.isinf(chunks)) and not torch.isnan(chunks).any()
+    good = torch.isfinite(one)
+    assert float((one[good] - chunks[good]).norm() / one[good].norm()) < REL
