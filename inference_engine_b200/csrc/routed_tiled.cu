@@ -106,11 +106,11 @@ __device__ __forceinline__ void load_run(void* dst, const void* src, int bytes, 
 __device__ __forceinline__ const unsigned char* w_tile(const Args& in, int expert, int block, int kb) {
     return in.w + (((size_t)expert * in.w_blocks + block) * in.kbs + kb) * W_BYTES;
 }
-// (The special-function unit's exponential and reciprocal: their error, a few units in the last place of a 32-bit value, vanishes in the
-// rounding to bfloat16.)
+// (The special-function unit's exponential and reciprocal by themselves are off by 12 units in the last place at gates of -8 and by 70 at -50; with them
+// 2,048 tokens, 32 experts of 2,048 x 1,024: layer 181 us, 187 so; 8 tokens 60.4 and 61.1.)
 __device__ __forceinline__ float activated(const Args& in, float g, float u) {
     if (in.clamp) { g = fminf(g, in.limit); u = fminf(fmaxf(u, -in.limit), in.limit); }
-    return __fdividef(g, 1.0f + __expf(-in.alpha * g)) * (u + in.up_offset);
+    return g / (1.0f + expf(-in.alpha * g)) * (u + in.up_offset);
 }
 // Sixteen columns of gates (lanes with bit 3 clear) and their ups (set), of the places from `first` (a multiple of 8) on, n of them there, to feature f
 // of y: a lane takes every second place.  (Features beyond the last: zeros, from zero weights.)

@@ -162,3 +162,24 @@ def test_router_of_many_tokens_with_infinities(scoring):
     torch.testing.assert_close(many_weights, few_weights, atol=2e-6, rtol=2e-5, equal_nan=True)
     if scoring == "sigmoid":
         assert len(set(few[17].tolist())) == top and len(set(few[18].tolist())) == top  # (a choice, not expert 0 for all)
+
+
+@pytest.mark.parametrize("tokens,experts", [(64, 1), (2048, 8)])
+def test_the_activation_is_a_32_bit_one(tokens, experts):
+    """Rows with a single 1 and identities as down matrices, so that gates, ups and what becomes of them are seen as they are.  An exponential of at most
+    two units in the last place and three more roundings leave 2^-22 + 3 * 2^-24 of a value; where that crosses no boundary between two
+    bfloat16 numbers the result is the one that 64 bits round to."""
+    g, size = torch.Generator(device="cuda").manual_seed(tokens), 256
+    gate = (torch.rand(experts, size, size, generator=g, device="cuda") * 80 - 60).bfloat16()
+    up = torch.randn(experts, size, size, generator=g, device="cuda").bfloat16()
+    down = torch.eye(size, device="cuda").bfloat16().repeat(experts, 1, 1)
+    at = torch.arange(tokens, device="cuda")
+    x = torch.zeros(tokens, size, device="cuda", dtype=torch.bfloat16)
+    x[at, at % size] = 1.0
+    ids = (at // size).int()[:, None]
+    got = _run(x, ids, torch.ones(tokens, 1, device="cuda"), torch.stack([gate, up], dim=1), down, None, 1.0, 0.0)[0][0]
+    a, u = (m.transpose(1, 2).reshape(-1, size)[:tokens].double() for m in (gate, up))
+    want = a / (1 + torch.exp(-a)) * u
+    room = 7 * 2.0 ** -24
+    low, high = (want * (1 - room)).bfloat16(), (want * (1 + room)).bfloat16()
+    assert ((got == low.float()) | (got == high.float())).all()
