@@ -17,9 +17,11 @@
 // cores fill the other, and the copies of the next tile's operands run ahead of both.  More than 256 pairs take both.  (2,048 tokens, 4 of 32 experts of
 // 2,048 x 1,024 each: 119 + 59 us with an SM a tile on plain matrices, 82 + 47 so, where the weights' bytes and the products take 43 + 21.)
 //   warp 0, one thread of each block: copies into a ring of six slots of 36 KB (more and smaller ones where tiles are smaller, as in steps of fewer than 257 tokens);
-//   warp 1, one thread: in the first block tcgen05.mma for both (tcgen05.commit hands slots back and accumulators over in both blocks), in the
-//   second it passes on which slots are full;
+//   warp 1 of the first block, one thread: tcgen05.mma for both (tcgen05.commit hands slots back and accumulators over in both blocks);
 //   warps 2-9: read the accumulator of their block.
+// Both blocks' copies are told to the first one's barrier, which is what orders them before the products that read them; copies of rows of 1 and 2 KB
+// of a tensor map can be (cta_group::2), runs of bytes cannot, and they are as fast.  (With a word of the second block's for each of its slots: layer of 2,048 tokens
+// 192 us where nothing orders that word, 294 where it is released to the cluster, a microsecond a word, 193 so; of 65 tokens 90, 211 and 92.)
 //
 // Few tokens (`few`: up to 64, tiles of at most 64 pairs): a stream of weights.  128 rows a block and 72 KB of ring, three blocks an SM:
 // all blocks of a step start at once and share the memory evenly, and what one waits for at its start and end the others use.  (256 rows and an SM's
@@ -57,6 +59,11 @@ __device__ __forceinline__ int parts(int n) { return n > MOST_COLS ? 2 : 1; }
 // The columns of each, rounded up to what the instruction takes.
 __device__ __forceinline__ int columns(int n) { return ((n + parts(n) - 1) / parts(n) + 31) & ~31; }
 
+// (Many pairs) the weights' tiles as rows of 2 KB, boxes of 8; the pairs' rows as rows of 1 KB (8 places), boxes of 16, 8, 4 and 2.
+struct Maps {
+    CUtensorMap w, x[4];
+};
+
 struct Args {
     const unsigned char* w;  // the weights' tiles
     const unsigned char* x;  // the pairs' rows (few, gate-up: the tokens' rows as they are)
@@ -93,10 +100,30 @@ __device__ __forceinline__ unsigned in_first(const void* p) {
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
     return r;
 }
-// (Relaxed, and the waits' scope the block's own: what is handed over was written by copies or read from tensor memory, nothing that a cache
-// would have to be emptied for.  Waits that acquire from the cluster do that each time they look: 147 us instead of 113.)
+// (Of tensor memory alone, which tcgen05's fences order around a relaxed arrival.)
 __device__ __forceinline__ void arrive_at(unsigned cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// A wait for what both blocks do: once it is over, a last look that acquires from the cluster.  (Each look one that acquires: 147 us instead of 113.)
+__device__ __forceinline__ bool warp_wait_cluster(unsigned long long* bar, int parity) {
+    if (!warp_wait(bar, parity)) return false;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n}" ::"r"(smem_u32(bar)), "r"(parity) : "memory");
+    return true;
+}
+// A box of whole rows of a map into this block's shared memory, told to the first block's barrier.
+__device__ __forceinline__ void load_pair(void* dst, const CUtensorMap* map, int row, unsigned first_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(0), "r"(row), "r"(first_bar) : "memory");
+}
+// A run of `kilobytes` (up to 31, even) rows of 1 KB from `row` on, in boxes of 16, 8, 4 and 2 of them.
+__device__ __forceinline__ void load_rows(unsigned char* dst, const CUtensorMap (&maps)[4], int row, int kilobytes, unsigned first_bar) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (kilobytes & (16 >> i)) {
+            load_pair(dst, &maps[i], row, first_bar);
+            dst += (16 >> i) * 1024;
+            row += 16 >> i;
+        }
 }
 // A run of bytes into this block's shared memory.
 __device__ __forceinline__ void load_run(void* dst, const void* src, int bytes, unsigned long long* bar) {
@@ -145,7 +172,7 @@ __device__ __forceinline__ void pair_commit(unsigned long long* bar) {
 // grid: clusters of two blocks.
 template <bool GATED>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ Args in) {
+gemm_pair_kernel(const __grid_constant__ Args in, const __grid_constant__ Maps maps) {
     extern __shared__ unsigned char smem_raw[];
     const unsigned raw = smem_u32(smem_raw) & 0xFFFFFFu;  // (within a cluster the block's number is above)
     unsigned char* ring = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -157,7 +184,7 @@ gemm_pair_kernel(const __grid_constant__ Args in) {
     const int slots = in.slots, slot_bytes = in.slot_bytes;
     if (threadIdx.x == 0) {
         for (int s = 0; s < slots; ++s) {
-            mbar_init(&sh->full[s], rank == 0 ? 2 : 1);  // (the first block's: also the second one's word)
+            mbar_init(&sh->full[s], 1);  // (the first block's, for the copies of both)
             mbar_init(&sh->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -196,61 +223,55 @@ gemm_pair_kernel(const __grid_constant__ Args in) {
             const int4 tile = tile_at(t);
             const int n = warps_own(tile.z), cols = columns(n), rows = cols / 2, bytes = rows * BK * 2;
             const int block = min(2 * warps_own(tile.w) + rank, in.w_blocks - 1);  // (an odd number of them: the last one again, unused)
-            const unsigned char* x = in.x + (size_t)(warps_own(tile.y) + rank * rows) * BK * 2;
-            const unsigned char* w = w_tile(in, warps_own(tile.x), block, 0);
+            int x = (warps_own(tile.y) + rank * rows) >> 3, w = (warps_own(tile.x) * in.w_blocks + block) * nkb * (W_BYTES / 2048);  // (rows of the maps)
             for (int kb = 0; kb < nkb; ++kb, ++use) {
                 if (use >= slots && !warp_wait(&sh->empty[s], phase ^ 1)) { ok = false; break; }
                 if (one) {
                     unsigned char* at = ring + (size_t)s * slot_bytes;
-                    mbar_expect_tx(&sh->full[s], W_BYTES + parts(n) * bytes);
-                    load_run(at, w, W_BYTES, &sh->full[s]);
-                    load_run(at + W_BYTES, x, bytes, &sh->full[s]);
-                    if (n > MOST_COLS) load_run(at + W_BYTES + bytes, x + (size_t)cols * BK * 2, bytes, &sh->full[s]);
+                    const unsigned bar = in_first(&sh->full[s]);
+                    if (rank == 0) mbar_expect_tx(&sh->full[s], 2 * (W_BYTES + parts(n) * bytes));
+                    load_pair(at, &maps.w, w, bar);
+                    load_rows(at + W_BYTES, maps.x, x, rows >> 3, bar);
+                    if (n > MOST_COLS) load_rows(at + W_BYTES + bytes, maps.x, x + (cols >> 3), rows >> 3, bar);
                 }
                 __syncwarp();
-                w += W_BYTES;
-                x += (size_t)in.places * BK * 2;
+                w += W_BYTES / 2048;
+                x += in.places >> 3;
                 if (++s == slots) { s = 0; phase ^= 1; }
             }
         }
         if (!ok) sh->failed = 1;
         else
-            for (int u = max(use - slots, 0); u < use; ++u) mbar_wait_compact(&sh->full[u % slots], (u / slots) & 1);  // (none is in flight at the end)
+            for (int u = max(use - slots, 0); u < use; ++u) mbar_wait_compact(&sh->empty[u % slots], (u / slots) & 1);  // (none is in flight at the end)
         __syncwarp();
     } else if (warp == 1) {
         const bool one = elect_one();
         int s = 0, phase = 0, turn = 0;
         bool ok = true;
         const unsigned w_low = umma_desc_low(smem_u32(ring));
-        for (int t = cluster; t < total && ok; t += clusters) {
+        for (int t = cluster; rank == 0 && t < total && ok; t += clusters) {
             const int n = warps_own(tile_at(t).z), cols = columns(n);
             const unsigned idesc = umma_idesc_bf16(256, cols), second = (unsigned)(cols / 2 * BK * 2) >> 4;
-            if (rank == 0) {
-                for (int part = 0; part < parts(n); ++part) {
-                    const int use_of = turn + part;
-                    if (use_of >= 2 && !warp_wait(&sh->acc_empty[use_of & 1], (use_of / 2 - 1) & 1)) ok = false;
-                }
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int part = 0; part < parts(n); ++part) {
+                const int use_of = turn + part;
+                if (use_of >= 2 && !warp_wait_cluster(&sh->acc_empty[use_of & 1], (use_of / 2 - 1) & 1)) ok = false;
             }
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned acc = tmem + (turn & 1) * MOST_COLS, acc2 = tmem + (~turn & 1) * MOST_COLS;
             for (int kb = 0; kb < nkb; ++kb) {
-                if (!warp_wait(&sh->full[s], phase)) { ok = false; break; }
+                if (!warp_wait_cluster(&sh->full[s], phase)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (one) {
-                    if (rank == 0) {
-                        const unsigned w0 = w_low + s * (slot_bytes >> 4), x0 = w0 + (W_BYTES >> 4);
+                    const unsigned w0 = w_low + s * (slot_bytes >> 4), x0 = w0 + (W_BYTES >> 4);
 #pragma unroll
-                        for (int ks = 0; ks < BK / 16; ++ks) {  // 32 bytes further along k per step
-                            mma<true>(acc, w0 + 2 * ks, x0 + 2 * ks, idesc, kb > 0 || ks > 0);
-                            if (n > MOST_COLS) mma<true>(acc2, w0 + 2 * ks, x0 + second + 2 * ks, idesc, kb > 0 || ks > 0);
-                        }
-                        pair_commit(&sh->empty[s]);
-                        if (kb + 1 == nkb)
-                            for (int part = 0; part < parts(n); ++part) pair_commit(&sh->acc_full[(turn + part) & 1]);
-                    } else {
-                        arrive_at(in_first(&sh->full[s]));
+                    for (int ks = 0; ks < BK / 16; ++ks) {  // 32 bytes further along k per step
+                        mma<true>(acc, w0 + 2 * ks, x0 + 2 * ks, idesc, kb > 0 || ks > 0);
+                        if (n > MOST_COLS) mma<true>(acc2, w0 + 2 * ks, x0 + second + 2 * ks, idesc, kb > 0 || ks > 0);
                     }
+                    pair_commit(&sh->empty[s]);
+                    if (kb + 1 == nkb)
+                        for (int part = 0; part < parts(n); ++part) pair_commit(&sh->acc_full[(turn + part) & 1]);
                 }
                 __syncwarp();
                 if (++s == slots) { s = 0; phase ^= 1; }
@@ -551,8 +572,19 @@ int clusters_at_once() {
     return known[dev];
 }
 
+// Memory as rows of `row_bytes` (a multiple of 16, up to 2 KB), boxes of so many.
+bool make_row_map(CUtensorMap* map, const void* base, long long rows, int row_bytes, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (fn == nullptr) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)row_bytes / 8, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    cuuint32_t box[2] = {(cuuint32_t)row_bytes / 8, (cuuint32_t)box_rows}, elem[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <bool GATED>
-int launch(const Args& in, int few, cudaStream_t s) {
+int launch(const Args& in, int experts, int few, cudaStream_t s) {
     if (few) {
         static IePerDevice allowed;
         cudaError_t e = ie_allow_smem(allowed, gemm_few_kernel<GATED>, FEW_SMEM);
@@ -568,7 +600,11 @@ int launch(const Args& in, int few, cudaStream_t s) {
     const int rows = in.most <= MOST_COLS ? (in.most + 31) / 32 * 16 : MOST_PAIRS / 2;
     args.slot_bytes = W_BYTES + rows * BK * 2;
     args.slots = RING_BYTES / args.slot_bytes < MOST_SLOTS ? RING_BYTES / args.slot_bytes : MOST_SLOTS;
-    return ie_launch_cluster(gemm_pair_kernel<GATED>, dim3(2 * clusters), dim3(THREADS), SMEM_BYTES, s, dim3(2, 1, 1), args);
+    Maps maps;
+    if (!make_row_map(&maps.w, in.w, (long long)experts * in.w_blocks * in.kbs * (W_BYTES / 2048), 2048, W_BYTES / 2048)) return (int)cudaErrorNotSupported;
+    for (int i = 0; i < 4; ++i)
+        if (!make_row_map(&maps.x[i], in.x, (long long)in.kbs * in.places / 8, 1024, 16 >> i)) return (int)cudaErrorNotSupported;
+    return ie_launch_cluster(gemm_pair_kernel<GATED>, dim3(2 * clusters), dim3(THREADS), SMEM_BYTES, s, dim3(2, 1, 1), args, maps);
 }
 }  // namespace
 
@@ -595,10 +631,10 @@ IE_API int ie_routed_tiled_gather(const void* x, void* xs, const int* order, con
 
 // most: the pairs of a tile, as `routed_sort` was told.  y: [k blocks of F][places][64].  few: x holds the tokens' rows [N, K]; else what `gather` wrote.  w: [experts][ceil(F / 64)][ceil(K / 64)] tiles.
 IE_API int ie_routed_tiled_gate_up(const void* x, const void* w, void* y, const int* order, const int* tiles, const int* count, int max_tiles,
-                                   int few, int most, int top, int N, int places, int K, int F, float limit, int clamp, float alpha, float up_offset,
+                                   int experts, int few, int most, int top, int N, int places, int K, int F, float limit, int clamp, float alpha, float up_offset,
                                    int* err, void* stream) {
     if (max_tiles <= 0) return 0;
-    if (K <= 0 || F <= 0 || K % 8 || F % 8 || ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y)) & 15) || !fits(few, most, N))
+    if (K <= 0 || F <= 0 || K % 8 || F % 8 || ((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y)) & 15) || !fits(few, most, N) || experts <= 0 || places % 8)
         return (int)cudaErrorInvalidValue;
     Args in = {};
     in.w = (const unsigned char*)w;
@@ -622,14 +658,14 @@ IE_API int ie_routed_tiled_gate_up(const void* x, const void* w, void* y, const 
     in.alpha = alpha;
     in.up_offset = up_offset;
     in.err = err;
-    return launch<true>(in, few, (cudaStream_t)stream);
+    return launch<true>(in, experts, few, (cudaStream_t)stream);
 }
 
 // w: [experts][ceil(H / 128)][ceil(F / 64)] tiles; out: [top, N, H] 32-bit.  few: launched right behind ie_routed_tiled_gate_up.
 IE_API int ie_routed_tiled_down(const void* y, const void* w, float* out, const float* weights, const int* order, const int* tiles,
-                                const int* count, int max_tiles, int few, int most, int top, int N, int places, int F, int H, int* err, void* stream) {
+                                const int* count, int max_tiles, int experts, int few, int most, int top, int N, int places, int F, int H, int* err, void* stream) {
     if (max_tiles <= 0) return 0;
-    if (H <= 0 || F <= 0 || H % 8 || F % 8 || ((((uintptr_t)y | (uintptr_t)w)) & 15) || !fits(few, most, N)) return (int)cudaErrorInvalidValue;
+    if (H <= 0 || F <= 0 || H % 8 || F % 8 || ((((uintptr_t)y | (uintptr_t)w)) & 15) || !fits(few, most, N) || experts <= 0 || places % 8) return (int)cudaErrorInvalidValue;
     Args in = {};
     in.w = (const unsigned char*)w;
     in.x = (const unsigned char*)y;
@@ -649,5 +685,5 @@ IE_API int ie_routed_tiled_down(const void* y, const void* w, float* out, const 
     in.N = N;
     in.most = most;
     in.err = err;
-    return launch<false>(in, few, (cudaStream_t)stream);
+    return launch<false>(in, experts, few, (cudaStream_t)stream);
 }

@@ -1229,8 +1229,8 @@ class CudaOps:
             "ie_routed_tiled_align": "",
             "ie_routed_tiled_places": "I I",
             "ie_routed_tiled_gather": "P P P P I I I P",
-            "ie_routed_tiled_gate_up": "P P P P P P I I I I I I I I F I F F P P",
-            "ie_routed_tiled_down": "P P P P P P P I I I I I I I I P P",
+            "ie_routed_tiled_gate_up": "P P P P P P I I I I I I I I I F I F F P P",
+            "ie_routed_tiled_down": "P P P P P P P I I I I I I I I I P P",
         },
         "recurrent": {
             "ie_short_conv_residual": "P I P P L P P P P I I I I I P P",
@@ -1560,14 +1560,14 @@ class CudaOps:
                               up_offset) -> None:
         self._check(lib.ie_routed_tiled_gate_up(
             x.data_ptr(), experts.gate_up.data_ptr(), y.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(), max_tiles,
-            int(few), most, top, n, places, experts.hidden, experts.ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha,
+            experts.experts, int(few), most, top, n, places, experts.hidden, experts.ff, 0.0 if limit is None else float(limit), 0 if limit is None else 1, alpha,
             up_offset, self._err_ptr, self._stream()), "routed_few_gate_up" if few else "routed_pair_gate_up")
 
     @_kind("routed.down")
     def _routed_tiled_down(self, lib, y, experts, out, weights, order, tiles, meta, max_tiles, few, most, top, n, places) -> None:
         self._check(lib.ie_routed_tiled_down(
             y.data_ptr(), experts.down.data_ptr(), out.data_ptr(), weights.data_ptr(), order.data_ptr(), tiles.data_ptr(), meta.data_ptr(),
-            max_tiles, int(few), most, top, n, places, experts.ff, experts.hidden, self._err_ptr, self._stream()),
+            max_tiles, experts.experts, int(few), most, top, n, places, experts.ff, experts.hidden, self._err_ptr, self._stream()),
             "routed_few_down" if few else "routed_pair_down")
 
     @_kind("routed.align")

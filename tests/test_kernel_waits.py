@@ -74,3 +74,18 @@ def test_the_look_itself():
     assert "ie_pdl_wait()" in leave and all(f"blockIdx.{axis} == 0" in leave for axis in "xyz")
     seen = [name for source in SOURCES for name, _ in _kernels(source.read_text())]
     assert {"attention_packed_kernel", "attention_prefill_tc5_kernel", "attention_decode_kernel"} <= set(seen)
+
+
+@pytest.mark.parametrize("source", SOURCES, ids=lambda p: p.name)
+def test_words_between_the_blocks_of_a_cluster_order_what_they_hand_over(source):
+    """A relaxed arrival at another block's barrier orders nothing but tensor memory, around which tcgen05's fences stand: directly in front of it one that
+    orders what came before.  Copies are told to the barrier that the reader waits at by the copies themselves."""
+    text = _plain(source.read_text())
+    helpers = re.findall(r"void (\w+)\([^{}]*\{\s*asm volatile\(\"mbarrier\.arrive\.relaxed\.cluster", text)
+    assert len(helpers) == text.count("mbarrier.arrive.relaxed")
+    for helper in helpers:
+        calls = [m.start() for m in re.finditer(rf"\b{helper}\(", text)][1:]
+        assert calls
+        for at in calls:
+            before = re.sub(r"\s+", " ", text[max(at - 200, 0): at])
+            assert re.search(r'tcgen05\.fence::before_thread_sync;" ::: "memory"\); __syncwarp\(\); if \(lane == 0\) $', before), (helper, before[-90:])

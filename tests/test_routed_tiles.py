@@ -48,5 +48,5 @@ def test_more_pairs_than_there_is_room_for_are_refused(lib):
     p, f = ctypes.c_void_p(16), ctypes.c_float
     invalid = 1  # cudaErrorInvalidValue
     for few, most, tokens in ((1, 65, 8), (1, 320, 64), (1, 64, 65), (0, 321, 300), (0, 0, 300)):
-        assert lib.ie_routed_tiled_gate_up(p, p, p, p, p, p, 1, few, most, 4, tokens, 640, 64, 64, f(0), 0, f(1), f(0), None, None) == invalid
-        assert lib.ie_routed_tiled_down(p, p, p, p, p, p, p, 1, few, most, 4, tokens, 640, 64, 64, None, None) == invalid
+        assert lib.ie_routed_tiled_gate_up(p, p, p, p, p, p, 1, 4, few, most, 4, tokens, 640, 64, 64, f(0), 0, f(1), f(0), None, None) == invalid
+        assert lib.ie_routed_tiled_down(p, p, p, p, p, p, p, 1, 4, few, most, 4, tokens, 640, 64, 64, None, None) == invalid
