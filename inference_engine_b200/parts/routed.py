@@ -55,19 +55,38 @@ class ExpertTiles:
 
     @classmethod
     def of(cls, gate_up, down):
-        """From ``[experts, 2, ff, hidden]`` and ``[experts, hidden, ff]``, an expert at a time: what is made on the way is one expert's."""
+        """From ``[experts, 2, ff, hidden]`` and ``[experts, hidden, ff]``."""
+        return cls.laid_out(gate_up.shape[0], lambda e: (gate_up[e, 0], gate_up[e, 1], down[e]))
+
+    @classmethod
+    def laid_out(cls, count, matrices):
+        """From ``matrices(e)``, expert ``e``'s gate and up ``[ff, hidden]`` and down ``[hidden, ff]``, an expert at a time: beside
+        the tiles no more than one expert's matrices are made on the way."""
         import torch
 
-        count, _, ff, hidden = gate_up.shape
+        ff, hidden = matrices(0)[0].shape
         f, h, rows = -(-ff // 64), -(-hidden // 64), -(-hidden // 128)
-        row, piece = torch.arange(128, device=down.device)[:, None], torch.arange(8, device=down.device)[None, :]
-        pad = torch.nn.functional.pad
-        turned = lambda t, a, b: t.reshape(a, b, 128, 8, 8)[:, :, row, piece ^ (row % 8)].view(a, b, 128, 64)  # noqa: E731
-        tiles = cls(count, ff, hidden, gate_up.new_empty(count, f, h, 128, 64), down.new_empty(count, rows, f, 128, 64))
+        new = matrices(0)[0].new_empty
+        tiles = cls(count, ff, hidden, new(count, f, h, 128, 64), new(count, rows, f, 128, 64))
+        steps = lambda n: torch.arange(n, device=tiles.down.device)  # noqa: E731
+
+        def order(blocks, groups, k_blocks):  # pieces [block, k block, group of eight rows, row, place] among a matrix's rows of pieces
+            row = (steps(blocks)[:, None, None] * groups + steps(groups)[:, None]) * 8 + steps(8)  # [block, group, row]
+            piece = steps(k_blocks)[:, None, None] * 8 + (steps(8) ^ steps(8)[:, None])  # [k block, row, place]
+            return (row[:, None, :, :, None] * (k_blocks * 8) + piece[None, :, None]).reshape(-1)
+
+        def pieces(matrix, block, k_blocks):  # zeros up to whole blocks; a piece of 16 bytes is moved as one number
+            more = (0, k_blocks * 64 - matrix.shape[1], 0, -matrix.shape[0] % block)
+            flat = (torch.nn.functional.pad(matrix, more) if any(more) else matrix).reshape(-1)
+            return (flat.clone() if flat.data_ptr() % 16 or flat.storage_offset() % 8 else flat).view(torch.complex128)
+
+        of_gates, of_down = order(f, 8, h), order(rows, 16, f)
+        to_gate_up, to_down = (t.view(count, -1).view(torch.complex128) for t in (tiles.gate_up, tiles.down))
         for e in range(count):
-            gu = pad(gate_up[e], (0, h * 64 - hidden, 0, f * 64 - ff)).view(2, f, 8, 8, h, 8, 8).permute(1, 4, 2, 0, 3, 5, 6)
-            dn = pad(down[e], (0, f * 64 - ff, 0, rows * 128 - hidden)).view(rows, 128, f, 8, 8).permute(0, 2, 1, 3, 4)
-            tiles.gate_up[e], tiles.down[e] = turned(gu, f, h), turned(dn, rows, f)
+            gate, up, down = matrices(e)
+            for which, matrix in enumerate((gate, up)):
+                to_gate_up[e].view(f * h * 8, 2, 64)[:, which] = pieces(matrix, 64, h)[of_gates].view(f * h * 8, 64)
+            torch.index_select(pieces(down, 128, f), 0, of_down, out=to_down[e])
         return tiles
 
 
@@ -146,15 +165,13 @@ class RoutedExperts(FeedForward):
             self.router_bias = tensors[self.router_bias_name].float().contiguous()
         if self.correction_name is not None:
             self.correction = tensors[self.correction_name].float().contiguous()
-        self.w_gate_up = torch.stack([
-            torch.stack([tensors[self._name(e, "gate")].to(self.dtype), tensors[self._name(e, "up")].to(self.dtype)])
-            for e in range(self.experts)]).contiguous()
-        self.w_down = torch.stack([tensors[self._name(e, "down")].to(self.dtype)
-                                   for e in range(self.experts)]).contiguous()
-        if (self.dtype == torch.bfloat16 and self.w_down.is_cuda
+        mine = lambda e, which: tensors[self._name(e, which)].to(self.dtype)  # noqa: E731
+        if (self.dtype == torch.bfloat16 and tensors[self._name(0, "down")].is_cuda
                 and ExpertTiles.fit(self.experts, self.intermediate_size, self.hidden_size)):
-            self.tiles = ExpertTiles.of(self.w_gate_up, self.w_down)
-            self.w_gate_up = self.w_down = None
+            self.tiles = ExpertTiles.laid_out(self.experts, lambda e: (mine(e, "gate"), mine(e, "up"), mine(e, "down")))
+            return
+        self.w_gate_up = torch.stack([torch.stack([mine(e, "gate"), mine(e, "up")]) for e in range(self.experts)]).contiguous()
+        self.w_down = torch.stack([mine(e, "down") for e in range(self.experts)]).contiguous()
 
     def _experts(self, x, ids, weights, ctx, out=None):
         rest = {"limit": self.limit, "alpha": self.alpha, "up_offset": self.up_offset, "ws": ctx.ws, "tag": "moe", "out": out}
