@@ -1,7 +1,8 @@
 // 32-bit products on the tensor cores.
 //
 // A number is a sum of two that the tensor cores take (11 bits each; the second, of at most 12, loses its last one), and a product three of
-// theirs: what is left out is about 2^-23 of it.  Sums of 16 products go through the tensor cores, which cut off what does not fit
+// theirs: what is left out is 2^-21 of it at most (the product of both second parts and the two last bits), 2^-24 in the mean.  So a single product is further off than one
+// multiply-add, which rounds it by 2^-24.  Sums of 16 products go through the tensor cores, which cut off what does not fit
 // where the 32-bit adders round, and are added in those; the products with second parts go first, so that little is cut off.  Against 64 bits
 // a chain of 64 or 128 such multiply-adds is no further off than one of the FMA pipe's, unless its terms grow towards its end.
 // (Three parts of 8 bits and six products are exact and take the tensor cores as long, but more instructions: the same error, the delta
