@@ -183,3 +183,24 @@ def test_the_activation_is_a_32_bit_one(tokens, experts):
     room = 7 * 2.0 ** -24
     low, high = (want * (1 - room)).bfloat16(), (want * (1 + room)).bfloat16()
     assert ((got == low.float()) | (got == high.float())).all()
+
+
+@pytest.mark.parametrize("width,experts", [(2048, 32), (1024, 16)])
+@pytest.mark.parametrize("weights_of", [torch.float32, torch.bfloat16])
+def test_router_of_many_tokens_is_as_exact_as_that_of_few(width, experts, weights_of):
+    """Both kernels' weights against 64 bits, over eight draws; a hundredth more for the draws' own spread."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, tokens, errors = get_ops(), 1000, [0.0, 0.0]
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x = torch.randn(tokens, width, generator=g, device="cuda").bfloat16()
+        w = (torch.randn(experts, width, generator=g, device="cuda") * 0.02).to(weights_of).float()
+        scores = (x.double() @ w.double().T).softmax(-1)
+        for i, step in enumerate((tokens, 500)):
+            ids, weights = torch.empty(tokens, experts, dtype=torch.int32, device="cuda"), torch.empty(tokens, experts, device="cuda")
+            for at in range(0, tokens, step):
+                ops.route_topk(x[at: at + step], w, 1, 1, ids[at: at + step], weights[at: at + step])
+            want = scores.gather(1, ids.long())
+            errors[i] += float((weights.double() - want).norm() / want.norm())
+    assert errors[0] < 1.01 * errors[1]
