@@ -147,8 +147,11 @@ __device__ __forceinline__ void choose_experts(int n, float* score, float* gbest
 // experts read them 2,048 times (half a GB through the L2, 47 us); few tokens want a block each.  What bounds it is the way to the
 // L2 and back, so a lane has eight pieces of the router's rows on their way, the first of them before the tokens' own rows have arrived,
 // and the choice is the whole warp's (8 tokens, 32 experts: 20 -> 11 us).
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(TOKENS > 1 ? 256 : 1024, TOKENS > 1 ? 2 : 1)
+// A step of no more tokens than SMs takes blocks of 1,024 threads, one an SM; one of two, three or four times as many blocks of 256, so many an SM, with
+// fewer registers and so fewer loads ahead each: all blocks run at one time.  (With 1,024 threads every further 148 tokens are another round.  2,048
+// wide, 32 experts, us with them / so: 148 tokens 6.9 / 6.9, 160 12.6 / 7.7, 300 18.7 / 9.0, 500 25.6 / 11.9; 1,024 wide, 16 experts, 500 17.4 / 7.7.)
+template <typename T, int TOKENS, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
 route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int num_tokens, int width,
                   int experts, int top, int groups, int keep, int sigmoid_scores,
                   const float* __restrict__ correction, int group_top, float weight_scale, int whole_pieces,
@@ -161,7 +164,7 @@ route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const fl
     const int per_token = 2 * experts + groups;
     // A warp takes every so many'th expert, some of them at a time.  An expert's sum is the same chain of operations whichever
     // way it is grouped: four partial sums per lane, added in a fixed order.
-    constexpr int ROUTE_THREADS = TOKENS > 1 ? 256 : 1024, WARPS = ROUTE_THREADS / 32, AT_ONCE = TOKENS > 1 ? 4 : 1, AHEAD = TOKENS > 1 ? 2 : 8;
+    constexpr int WARPS = THREADS / 32, AT_ONCE = THREADS > 256 ? 1 : 4, AHEAD = BLOCKS == 1 ? 8 : BLOCKS == 2 ? 2 : 1;
     float4 wv[AHEAD][AT_ONCE];
     auto ask = [&](int slot, int e0, int i) {
 #pragma unroll
@@ -179,7 +182,7 @@ route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const fl
     ie_pdl_wait();
     if (whole_pieces) {  // rows of whole 16-byte pieces, aligned
         constexpr int PIECE = 16 / sizeof(T);
-        for (int i = tid * PIECE; i < TOKENS * width; i += ROUTE_THREADS * PIECE) {
+        for (int i = tid * PIECE; i < TOKENS * width; i += THREADS * PIECE) {
             float4 v[PIECE / 4];
             if (i < cnt * width) {
                 const uint4 raw = *reinterpret_cast<const uint4*>(x + (size_t)n0 * width + i);
@@ -195,7 +198,7 @@ route_topk_kernel(const T* __restrict__ x, const float* __restrict__ w, const fl
             for (int k = 0; k < PIECE / 4; ++k) *reinterpret_cast<float4*>(xs + i + 4 * k) = v[k];
         }
     } else {
-        for (int i = tid; i < TOKENS * width; i += ROUTE_THREADS) xs[i] = i < cnt * width ? ie_load(x + (size_t)n0 * width + i) : 0.f;
+        for (int i = tid; i < TOKENS * width; i += THREADS) xs[i] = i < cnt * width ? ie_load(x + (size_t)n0 * width + i) : 0.f;
     }
     __syncthreads();
     for (int e0 = warp; e0 < experts; e0 += WARPS * AT_ONCE) {
@@ -768,8 +771,9 @@ IE_API int ie_route_topk(const void* x, int dtype, const float* w, const float* 
     const dim3 grid(many ? (num_tokens + MANY - 1) / MANY : num_tokens);
     const int whole_pieces = width % (dtype == IE_BF16 ? 8 : 4) == 0 && ((uintptr_t)x & 15) == 0;
     cudaStream_t s = (cudaStream_t)stream;
-#define IE_ROUTE(T, TOKENS)                                                                                              \
-    return ie_launch(route_topk_kernel<T, TOKENS>, grid, dim3(TOKENS > 1 ? 256 : 1024), smem, s, (const T*)x, w, bias, num_tokens, \
+    const int an_sm = (num_tokens + ie_sm_count() - 1) / ie_sm_count();
+#define IE_ROUTE(T, TOKENS, THREADS, BLOCKS)                                                                             \
+    return ie_launch(route_topk_kernel<T, TOKENS, THREADS, BLOCKS>, grid, dim3(THREADS), smem, s, (const T*)x, w, bias, num_tokens, \
                      width, experts, top, groups, keep, sigmoid_scores, correction, group_top, weight_scale, whole_pieces, ids, weights)
     if (dtype == IE_BF16) {
         // (16 tokens a block from as many tokens on as four a block fill the device with, and rows of whole 32s)
@@ -778,11 +782,17 @@ IE_API int ie_route_topk(const void* x, int dtype, const float* w, const float* 
             return ie_launch(route_many_kernel, dim3((num_tokens + RM_TOKENS - 1) / RM_TOKENS), dim3(RM_WARPS * 32), scratch * sizeof(float), s,
                              (const __nv_bfloat16*)x, w, bias, num_tokens, width, experts, top, groups, keep, sigmoid_scores, correction,
                              group_top, weight_scale, ids, weights);
-        if (many) IE_ROUTE(__nv_bfloat16, MANY);
-        IE_ROUTE(__nv_bfloat16, 1);
+        if (many) IE_ROUTE(__nv_bfloat16, MANY, 256, 2);
+        if (an_sm <= 1) IE_ROUTE(__nv_bfloat16, 1, 1024, 1);
+        if (an_sm <= 2) IE_ROUTE(__nv_bfloat16, 1, 256, 2);
+        if (an_sm == 3) IE_ROUTE(__nv_bfloat16, 1, 256, 3);
+        IE_ROUTE(__nv_bfloat16, 1, 256, 4);
     }
-    if (many) IE_ROUTE(float, MANY);
-    IE_ROUTE(float, 1);
+    if (many) IE_ROUTE(float, MANY, 256, 2);
+    if (an_sm <= 1) IE_ROUTE(float, 1, 1024, 1);
+    if (an_sm <= 2) IE_ROUTE(float, 1, 256, 2);
+    if (an_sm == 3) IE_ROUTE(float, 1, 256, 3);
+    IE_ROUTE(float, 1, 256, 4);
 #undef IE_ROUTE
 }
 

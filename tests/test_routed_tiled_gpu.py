@@ -204,3 +204,28 @@ def test_router_of_many_tokens_is_as_exact_as_that_of_few(width, experts, weight
             want = scores.gather(1, ids.long())
             errors[i] += float((weights.double() - want).norm() / want.norm())
     assert errors[0] < 1.01 * errors[1]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width,experts", [(192, 5), (1028, 40), (50, 3)])
+def test_router_of_one_to_four_tokens_an_sm(dtype, width, experts):
+    """Blocks of 1,024 threads, one an SM, and of 256, up to four: the same bits for a token among any number."""
+    from inference_engine_b200.kernels import get_ops
+
+    ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(width)
+    top, sms = 2, torch.cuda.get_device_properties(0).multi_processor_count
+    x = torch.randn(4 * sms - 1, width, generator=g, device="cuda").to(dtype)
+    w = torch.randn(experts, width, generator=g, device="cuda") * width ** -0.5
+
+    def route(rows):
+        ids, weights = torch.empty(rows.shape[0], top, dtype=torch.int32, device="cuda"), torch.empty(rows.shape[0], top, device="cuda")
+        ops.route_topk(rows, w, 1, 1, ids, weights, scoring="sigmoid")
+        return ids, weights
+
+    ids, weights = route(x)
+    ranked = (x.double() @ w.double().T).sigmoid().sort(dim=-1, descending=True)
+    sure = (ranked.values[:, 0] - ranked.values[:, 1] > 1e-5) & (ranked.values[:, 1] - ranked.values[:, 2] > 1e-5)
+    assert sure.float().mean() > 0.97 and torch.equal(ids[sure].long(), ranked.indices[sure, :top])
+    for tokens in (1, sms, sms + 1, 2 * sms, 2 * sms + 1, 3 * sms, 3 * sms + 1):
+        some = route(x[:tokens])
+        assert torch.equal(some[0], ids[:tokens]) and torch.equal(some[1], weights[:tokens])
