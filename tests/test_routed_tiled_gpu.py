@@ -209,7 +209,7 @@ def test_router_of_many_tokens_is_as_exact_as_that_of_few(width, experts, weight
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width,experts", [(192, 5), (1028, 40), (50, 3)])
 def test_router_of_one_to_four_tokens_an_sm(dtype, width, experts):
-    """Blocks of 1,024 threads, one an SM, and of 256, up to four: the same bits for a token among any number."""
+    """Blocks of 1,024 threads, one an SM, and (bfloat16) of 256, up to four: the same bits for a token among any number."""
     from inference_engine_b200.kernels import get_ops
 
     ops, g = get_ops(), torch.Generator(device="cuda").manual_seed(width)
