@@ -25,8 +25,8 @@
 // What bounds it: the multiply-adds, 40 thousand per token and head of 128 x 128, and what brings their operands from shared memory.  A
 // state in 32 bits must not lose precision, so the products are 32-bit ones, put together from three of the tensor cores' on parts
 // of 11 bits (below); the FMA pipe alone, two operands from shared memory to every few multiply-adds, took longer.  2,048 tokens, 16 heads of
-// 128 x 128, us with FMAs / so: outputs 79 / 66 (delta rule 81 / 70), solve 75 / 54, chain 111 / 84; all together 142 / 122 and 270 /
-// 214.  Errors against 64 bits, over keys of 64 and 128, as parts of the results: outputs 1.4e-7 / 1.3e-7, of the delta rule 2.6e-7 /
+// 128 x 128, us with FMAs / so: outputs 79 / 66 (delta rule 81 / 70), solve 75 / 54, chain 111 / 84; all
+// together 142 / 122 and 270 / 214.  (Outputs 61 since their scores do not wait for the states.)  Errors against 64 bits, over keys of 64 and 128, as parts of the results: outputs 1.4e-7 / 1.3e-7, of the delta rule 2.6e-7 /
 // 2.1e-7, its states 1.9e-7 / 1.8e-7.
 #include "split32.cuh"
 #include <float.h>

@@ -207,8 +207,8 @@ __device__ __forceinline__ float block_order_sum(float (&s)[LP_THREADS / 32], in
 
 // The same for many tokens, of products in one part whose sizes and addresses allow pieces of four: a warp per token, no barriers, four of
 // a lane's pieces on their way at a time.  Every number is the same chain of operations as there, also the sums of squares: a token's results do not depend on
-// how many others the step has.  (2,048 tokens of 16 heads of 128 + 64 and a latent of 512, the cached rows and the queries in a
-// launch each: 28 us with a block per token; 17 so.  Most of that was code fetched to be executed once, the sums over parts unrolled in
+// how many others the step has.  (2,048 tokens of 16 heads of 128 + 64 and a latent of 512: 28 us with a block per token and a launch each
+// for the cached rows and the queries; 22 so with all of it beyond the L2, of which 2 are the order of the sums.  Most of the 28 was code fetched to be executed once, the sums over parts unrolled in
 // every place: little code counts as much as few trips to memory here.)
 constexpr int LW_WARPS = 4, LW_PIECES = 4;
 

@@ -15,7 +15,7 @@
 // rounded up to 32 and an expert of a few more than 256 pairs still is one tile, whose weights are read once.  The blocks stay and take tile
 // after tile (a cluster takes every so many'th), with two accumulators of 256 columns: while the epilogue's warps read one, the tensor
 // cores fill the other, and the copies of the next tile's operands run ahead of both.  More than 256 pairs take both.  (2,048 tokens, 4 of 32 experts of
-// 2,048 x 1,024 each: 119 + 59 us with an SM a tile on plain matrices, 82 + 47 so, where the weights' bytes and the products take 43 + 21.)
+// 2,048 x 1,024 each: 119 + 59 us with an SM a tile on plain matrices, 85 + 47 so, where the weights' bytes and the products take 43 + 21.)
 //   warp 0, one thread of each block: copies into a ring of six slots of 36 KB (more and smaller ones where tiles are smaller, as in steps of fewer than 257 tokens);
 //   warp 1 of the first block, one thread: tcgen05.mma for both (tcgen05.commit hands slots back and accumulators over in both blocks);
 //   warps 2-9: read the accumulator of their block.
@@ -25,7 +25,7 @@
 //
 // Few tokens (`few`: up to 64, tiles of at most 64 pairs): a stream of weights.  128 rows a block and 72 KB of ring, three blocks an SM:
 // all blocks of a step start at once and share the memory evenly, and what one waits for at its start and end the others use.  (256 rows and an SM's
-// whole memory a block: 8 tokens over 32 experts of 2,048 x 1,024 were 160 blocks of 1 MB in two rounds of 148, 49 + 26 us; 30 + 12 so.)
+// whole memory a block: 8 tokens over 32 experts of 2,048 x 1,024 were 160 blocks of 1 MB in two rounds of 148, 49 + 26 us; 28 + 10 so.)
 // The down product's weights are asked for while the gated product still runs (whose blocks let the next kernel start once they have
 // seen the sorted pairs, so those are there).
 //
